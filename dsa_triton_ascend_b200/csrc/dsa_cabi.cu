@@ -15,6 +15,7 @@
 #include "sfa_fwd_sm100.cuh"
 #include "sfa_bwd_simt.cuh"
 #include "sfa_bwd_mma.cuh"
+#include "sfa_bwd_sm100.cuh"
 #include "sli_grad.cuh"
 
 namespace dsa {
@@ -264,8 +265,9 @@ static int sfa_grad_mma_launch(const SfaGradDev& d, int n1, cudaStream_t st) {
 }
 
 template <typename T>
-static int sfa_grad_launch(const DsaSfaGradParams* p, float* acc, cudaStream_t st) {
+static int sfa_grad_launch(const DsaSfaGradParams* p, char* ws, const SfaBwdWs& w, cudaStream_t st) {
   SfaGradDev d;
+  float* acc = reinterpret_cast<float*>(ws + w.acc);
   d.seq.seq_q = p->seq_q; d.seq.seq_k = p->seq_k; d.seq.block_table = nullptr;
   d.seq.layout_q = p->layout_q; d.seq.layout_k = p->layout_kv;
   d.seq.seq_q_cum = p->seq_q_cumulative; d.seq.seq_k_cum = p->seq_k_cumulative;
@@ -286,8 +288,12 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, float* acc, cudaStream_t s
   if (d.rows > 0) {
     const unsigned gy = (unsigned)((p->n1 + kSfaGradHeads - 1) / kSfaGradHeads);
     dim3 grid((unsigned)d.rows, gy, 1);
-    // the contractions run on the tensor cores (mma.sync); on request the CUDA-core kernel
-    if (p->kernel != DSA_KERNEL_PORTABLE) {
+    // D = 512 on tcgen05; other head dims (and tensors off their 16-byte boundaries) on mma.sync; on
+    // request the CUDA-core kernel
+    if (sfa_bwd_sm100_eligible(p)) {
+      const int rc = sfa_bwd_sm100_launch<T>(p, d, ws, w, st);
+      if (rc != DSA_OK) return rc;
+    } else if (p->kernel != DSA_KERNEL_PORTABLE) {
       int rc;
       if (p->d == 512) rc = sfa_grad_mma_launch<T, 512>(d, p->n1, st);
       else if (p->d == 256) rc = sfa_grad_mma_launch<T, 256>(d, p->n1, st);
@@ -301,7 +307,7 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, float* acc, cudaStream_t s
       sfa_bwd_simt_kernel<T><<<grid, kSfaGradThreads, smem, st>>>(d);
     }
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
-    count_launch();
+    if (!sfa_bwd_sm100_eligible(p)) count_launch();
   }
   if (p->key_rows > 0) {
     const int64_t total = p->key_rows * (int64_t)(2 * p->d + p->d_rope);
@@ -605,7 +611,8 @@ int dsa_sfa_grad_workspace_bytes(const DsaSfaGradParams* p, size_t* out_bytes) {
   int st = sfa_grad_validate(p);
   if (st != DSA_OK) return st;
   if (!out_bytes) return DSA_ERR_NULL;
-  *out_bytes = kWorkspaceHeader + (size_t)p->key_rows * (size_t)(2 * p->d + p->d_rope) * sizeof(float);
+  const SfaBwdWs w = sfa_bwd_ws_layout(p, kWorkspaceHeader);
+  *out_bytes = sfa_bwd_sm100_eligible(p) ? w.total : w.zeroed;
   return DSA_OK;
 }
 
@@ -616,10 +623,10 @@ int dsa_sfa_grad(const DsaSfaGradParams* p, void* workspace, size_t workspace_by
   dsa_sfa_grad_workspace_bytes(p, &need);
   if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255u) != 0) return DSA_ERR_WORKSPACE;
   cudaStream_t cs = (cudaStream_t)stream;
-  if (cudaMemsetAsync(workspace, 0, need, cs) != cudaSuccess) return DSA_ERR_CUDA;
-  float* acc = reinterpret_cast<float*>((char*)workspace + kWorkspaceHeader);
-  if (p->dtype == DSA_DTYPE_BF16) return sfa_grad_launch<__nv_bfloat16>(p, acc, cs);
-  return sfa_grad_launch<__half>(p, acc, cs);
+  const SfaBwdWs w = sfa_bwd_ws_layout(p, kWorkspaceHeader);
+  if (cudaMemsetAsync(workspace, 0, w.zeroed, cs) != cudaSuccess) return DSA_ERR_CUDA;
+  if (p->dtype == DSA_DTYPE_BF16) return sfa_grad_launch<__nv_bfloat16>(p, (char*)workspace, w, cs);
+  return sfa_grad_launch<__half>(p, (char*)workspace, w, cs);
 }
 
 static int dense_lse_validate(const DsaDenseLseParams* p) {

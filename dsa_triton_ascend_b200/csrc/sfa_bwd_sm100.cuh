@@ -1,0 +1,715 @@
+// Sparse flash attention backward on tcgen05 tensor cores for D = 512 (+ 64 rope), one KV head, any
+// head count, BSND / TND, token- or block-wise indices.  Same math as sfa_bwd_mma_kernel
+// (sparse_flash_attention_grad_triton.py:100-470, golden sparse_flash_attention_grad_numpy.py:96-135):
+//     S  = q . k^T          dP = dO . k_nope^T
+//     P  = exp(S * scale - max) / sum       dS = P * (dP - delta) * scale
+//     dQ += dS . k          dK += dS^T . q  dV += P^T . dO
+//
+// What bounds it: the scatter-adds.  A selected (row, key) pair adds 1088 fp32 values to d_key /
+// d_value, 4.6 GB for 512 rows x 2048 keys x 64 heads, and the L2 takes whole-line fp32 reductions at
+// 6.2 TB/s (lanes that cover 32-byte sectors only: 3.7 TB/s) whichever instruction brings them (scalar,
+// 16-byte or bulk).  So a block covers 64 heads - every reduction then carries 64 heads - and everything
+// else is arranged to hide behind the stream of reductions:
+//
+//   * A work item is (query row, 64 heads).  Q and dO stay in shared memory for the whole row (136 KB),
+//     keys come 48 at a time (TMA gather4, 54 KB, one buffer).
+//   * Q and dO are stacked: feature block f of both forms one 128-row A operand, so that ONE product
+//     with the key tile yields S (lanes 0..63) and dP (lanes 64..127).  The rope part of S goes to
+//     columns of its own (its lower 64 rows are whatever follows in shared memory; nobody reads them).
+//   * The three gradient products run transposed, FEATURES on the 128 lanes: dV^T and dK^T tiles of
+//     128 features x 48 keys, dQ^T tiles of 128 features x 64 heads.  A warp that drains a dV^T / dK^T
+//     tile holds 32 consecutive features of one key per register: its reduction instruction is one full
+//     128-byte line.  Q, dO and K serve these products as transposed (MN-major) operands straight from
+//     the layout the score product uses.
+//   * P and dS are fp32 values that enter their products as a high and a low io-dtype part
+//     (x = hi + lo up to 2^-16 relative for bf16, 2^-22 for fp16), as in sfa_bwd_mma_kernel.  fp16: P is
+//     scaled by 2^13, dS by a power of two per item that keeps |dS| <= scale * (|dO| |v| + |delta|)
+//     (Cauchy-Schwarz over the item's heads and all keys, taken by the pre-pass) below 2^13.
+//
+// Measured, B1 S1 512 S2 4096 N1 64 k 2048, bf16: 1.29 ms for the operator call (sfa_bwd_mma_kernel: 4.63
+// ms); 4092 rows x 128 heads: 7.6 ms (32.2 ms).  ncu: 3.4 TB/s of reductions, tensor pipe 22 % busy, the
+// load / store unit's data pipe - which a reduction of one line holds for 4.5 cycles - 66 % (77 % while
+// every SM has work).
+//
+// Tensor memory: dQ^T 5 x 64 columns | S, dP 48 | rope part of S 48 | drain ring 2 x 48.
+// Warps (896 threads): 0..7 softmax (lane quarter = warp & 3: quarters 0, 1 hold S of heads 0..63,
+// quarters 2, 3 hold dP; warps 0..3 take keys 0..23, warps 4..7 keys 24..47), 8..19 drain (three groups
+// take the tiles in turn: a group empties its ring slot into registers at once, so that three tiles are
+// being added while two are being computed), 20..24 K gather, 25 issuer of S / dP / dQ, 26 issuer of
+// dV / dK, 27 Q / dO loader.  Waits suspend (try_wait): polling warps take the load / store unit's issue
+// slots from the reductions (1.47 -> 1.36 ms).
+// All waits are bounded; one that gives up sets the status word.
+#pragma once
+
+#include "sfa_bwd_simt.cuh"
+#include "sfa_fwd_sm100.cuh"
+
+namespace dsa {
+
+constexpr int kBwdHeads = 64;        // heads per item
+constexpr int kBwdBK = 48;           // keys per tile
+constexpr int kBwdThreads = 896;
+constexpr int kBwdDrainWarp0 = 8, kBwdDrainGroups = 3, kBwdGatherWarp0 = 20, kBwdGatherWarps = 5;
+constexpr int kBwdIssueA = 25, kBwdIssueB = 26, kBwdLoader = 27;
+constexpr uint32_t kBwdHBlk = kBwdHeads * 128;                    // 64 heads x 64 features
+constexpr uint32_t kBwdQdBlk = 2 * kBwdHBlk;                      // [Q block | dO block]
+constexpr uint32_t kBwdKBlk = kBwdBK * 128;                       // 48 keys x 64 features
+constexpr uint32_t kBwdPMat = kBwdBK * 128;                       // 48 keys x 64 heads, 16 bit
+constexpr uint32_t kBwdOffQd = 0;                                 // 8 x [Q | dO]
+constexpr uint32_t kBwdOffQr = kBwdOffQd + 8 * kBwdQdBlk;
+constexpr uint32_t kBwdOffK = kBwdOffQr + kBwdHBlk;               // 9 blocks
+constexpr uint32_t kBwdOffP = kBwdOffK + 9 * kBwdKBlk;            // P hi, P lo, dS hi, dS lo
+constexpr uint32_t kBwdOffX = kBwdOffP + 4 * kBwdPMat;            // P as fp32 [48 keys][64 heads]
+constexpr uint32_t kBwdOffBar = kBwdOffX + kBwdBK * kBwdHeads * 4;
+constexpr uint32_t kBwdOffRows = kBwdOffBar + 256;               // int32 [3][48]: key rows of the last tiles
+constexpr uint32_t kBwdSmemBytes = kBwdOffRows + 3 * kBwdBK * 4;
+constexpr uint32_t kBwdQBytes = 8 * kBwdQdBlk + kBwdHBlk, kBwdKBytes = 9 * kBwdKBlk;
+static_assert(kBwdOffK % 1024 == 0 && kBwdOffP % 1024 == 0, "operand alignment");
+static_assert(kBwdSmemBytes <= 232448, "shared memory");
+// the drain warps take the registers that the gather, issuer and loader warps give back
+constexpr int kBwdLaunchRegs = 72, kBwdRegsLow = 56, kBwdRegsHigh = 80;
+static_assert((kBwdRegsHigh - kBwdLaunchRegs) * (kBwdGatherWarp0 - kBwdDrainWarp0) <=
+                  (kBwdLaunchRegs - kBwdRegsLow) * (kBwdThreads / 32 - kBwdGatherWarp0),
+              "setmaxnreg: more registers requested than released");
+static_assert(kBwdLaunchRegs * kBwdThreads <= 65536, "register file");
+constexpr uint32_t kBwdTmQ = 0, kBwdTmS = 320, kBwdTmR = 368, kBwdTmD = 416;
+constexpr int kBwdTiles = 9;         // dV^T tiles 0..3, dK^T tiles 4..8 (8: rope)
+
+struct SfaBwdArgs {
+  SfaGradDev p;
+  int32_t* status;
+  const int2* nvalid;        // [rows] .x slots that take part, .y first entry in key_list
+  const int32_t* key_list;   // [rows, slots] their key rows, front-packed
+  const float* delta;        // [rows, n1]
+  const float* bound;        // fp16: [0] largest key norm, [4 + 2 row] largest |dO|, [5 + 2 row] largest |delta|
+  uint32_t idesc_s, idesc_q, idesc_d;
+  int32_t items, hblocks;    // rows * hblocks
+  int32_t key_rows;
+};
+
+__device__ __forceinline__ void red_add_if(bool on, float* addr, float v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p red.global.add.f32 [%0], %1;\n\t}\n" ::"l"(addr),
+               "f"(v), "r"((int)on)
+               : "memory");
+}
+
+// delta = dO . O per (row, head), one warp each; for fp16 also the row's largest |dO| and |delta|.
+template <typename T>
+__global__ void __launch_bounds__(256) sfa_bwd_delta_kernel(const T* __restrict__ d_out, const T* __restrict__ out,
+                                                            float* __restrict__ delta, float* __restrict__ bound,
+                                                            int64_t total, int32_t n1) {
+  const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= total) return;
+  float s = 0.f, n = 0.f;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const uint4 a = reinterpret_cast<const uint4*>(d_out + i * 512)[lane + 32 * u];
+    const uint4 b = reinterpret_cast<const uint4*>(out + i * 512)[lane + 32 * u];
+    const T* av = reinterpret_cast<const T*>(&a);
+    const T* bv = reinterpret_cast<const T*>(&b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float x = to_f32<T>(av[e]);
+      s = fmaf(x, to_f32<T>(bv[e]), s);
+      n = fmaf(x, x, n);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+  }
+  if (lane == 0) {
+    delta[i] = s;
+    if (bound != nullptr) {   // (non-negative floats order like their bit patterns)
+      const int64_t row = i / n1;
+      atomicMax(reinterpret_cast<int*>(bound + 4 + 2 * row), __float_as_int(sqrtf(n)));
+      atomicMax(reinterpret_cast<int*>(bound + 5 + 2 * row), __float_as_int(fabsf(s)));
+    }
+  }
+}
+
+// fp16: largest norm of the value part of a key.
+template <typename T>
+__global__ void __launch_bounds__(256) sfa_bwd_key_norm_kernel(const T* __restrict__ key, float* __restrict__ bound,
+                                                               int64_t key_rows) {
+  const int lane = threadIdx.x & 31;
+  float best = 0.f;
+  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < key_rows; r += (int64_t)gridDim.x * 8) {
+    float n = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint4 a = reinterpret_cast<const uint4*>(key + r * 512)[lane + 32 * u];
+      const T* av = reinterpret_cast<const T*>(&a);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { const float x = to_f32<T>(av[e]); n = fmaf(x, x, n); }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    best = fmaxf(best, n);
+  }
+  if (lane == 0) atomicMax(reinterpret_cast<int*>(bound), __float_as_int(sqrtf(best)));
+}
+
+// fp16: exponent of the power of two that dS of a row is scaled by.
+__device__ __forceinline__ int sfa_bwd_exponent(const SfaBwdArgs& a, int32_t row) {
+  const float b = a.p.scale * (a.bound[4 + 2 * row] * a.bound[0] + a.bound[5 + 2 * row]);
+  if (!(fabsf(b) > 0.f) || !(fabsf(b) < INFINITY)) return 0;
+  return max(-100, min(100, 12 - ilogbf(fabsf(b))));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_constant__ CUtensorMap tmap_kr,
+                     const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_qr,
+                     const __grid_constant__ CUtensorMap tmap_do, const SfaBwdArgs a) {
+  constexpr bool kScaled = !kIsBf16<T>;
+  extern __shared__ __align__(1024) unsigned char bwd_sm[];
+  uint64_t* bars = reinterpret_cast<uint64_t*>(bwd_sm + kBwdOffBar);
+  uint64_t* k_full = bars;          // gather -> issuer A                                 (tx bytes)
+  uint64_t* k_empty = bars + 1;     // dQ of the tile done -> gather                      (commit A)
+  uint64_t* q_full = bars + 2;      // Q, dO landed -> issuer A (issuer B follows it)     (tx bytes)
+  uint64_t* q_empty = bars + 3;     // both issuers through with the item -> loader       (commits A, B)
+  uint64_t* s_full = bars + 4;      // S, dP -> softmax                                   (commit A)
+  uint64_t* s_empty = bars + 5;     // softmax holds them in registers                    (8 warps)
+  uint64_t* p_full = bars + 6;      // P hi / lo stored                                   (4 warps)
+  uint64_t* p_empty = bars + 7;     // dV of the tile done                                (commit B)
+  uint64_t* ds_full = bars + 8;     // dS hi / lo stored                                  (4 warps)
+  uint64_t* ds_empty = bars + 9;    // dK and dQ of the tile done                         (commits A, B)
+  uint64_t* x_full = bars + 10;     // [4] fp32 P handed from an S warp to its dP warp
+  uint64_t* x_empty = bars + 14;    // [4]
+  uint64_t* d_full = bars + 18;     // [3] the drain group's next dV^T / dK^T tile is there (commit B)
+  uint64_t* d_empty = bars + 21;    // [2] ring slot read                                 (4 warps)
+  uint64_t* dq_full = bars + 23;    // dQ^T of the item complete                          (commit A)
+  uint64_t* dq_empty = bars + 24;   // dQ^T read                                          (8 warps)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 26);
+  int32_t* rows_s = reinterpret_cast<int32_t*>(bwd_sm + kBwdOffRows);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int32_t n1 = a.p.n1;
+  const bool misaligned = (ptx::smem_u32(bwd_sm) & 1023u) != 0;
+  if (threadIdx.x == 0) {
+    const int counts[25] = {1, 1, 1, 2, 1, 8, 4, 1, 4, 2, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 4, 4, 1, 8};
+#pragma unroll
+    for (int i = 0; i < 25; ++i) ptx::mbar_init(&bars[i], counts[i]);
+    *abort_flag = misaligned ? 1 : 0;
+    ptx::mbar_fence_init();
+  }
+  // (the operands' padding is read by products whose results nobody uses, and by those of the heads past
+  // n1, which have to be zero: start from zeros)
+  for (uint32_t i = threadIdx.x; i < (kBwdOffBar - kBwdOffK) / 16; i += kBwdThreads)
+    reinterpret_cast<uint4*>(bwd_sm + kBwdOffK)[i] = make_uint4(0, 0, 0, 0);
+  ptx::fence_proxy_async_smem();
+  if (warp == kBwdIssueA) {
+    ptx::tmem_alloc(tmem_slot, 512);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t sm0 = ptx::smem_u32(bwd_sm);
+
+  auto tiles_of = [&](int32_t n) -> int32_t { return (n + kBwdBK - 1) / kBwdBK; };
+  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return ptx::mbar_wait_warp(bar, parity, abort_flag); };
+
+  // Each class of roles sits in its own branch, right under its setmaxnreg: the compiler budgets a
+  // branch by the setmaxnreg that dominates it.
+  if (warp < kBwdDrainWarp0) {
+   if (!*abort_flag) {
+    // -------------------------------------------------------------------- softmax, then dQ^T
+    const int quarter = warp & 3, half = warp >> 2;
+    const bool is_s = quarter < 2;
+    const int hl = (quarter & 1) * 32 + lane;               // head within the item
+    const int pair = (quarter & 1) * 2 + half;
+    const int kk0 = half * 24;                              // this warp's keys of a tile
+    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+    unsigned char* mat_hi = bwd_sm + kBwdOffP + (is_s ? 0u : 2u * kBwdPMat) + (hl & 7) * 2;
+    float* xbuf = reinterpret_cast<float*>(bwd_sm + kBwdOffX) + hl;
+    uint32_t n_tile = 0, n_item = 0;
+    bool ok = true;
+    for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+      const int32_t row = item / a.hblocks, h0 = (item - row * a.hblocks) * kBwdHeads;
+      const int32_t nvalid = a.nvalid[row].x, ntiles = tiles_of(nvalid);
+      const bool head = h0 + hl < n1;
+      const int64_t hi_ = (int64_t)row * n1 + h0 + hl;
+      if (ntiles > 0) {
+        float c0 = 0.f, c1 = 0.f, up = 1.f;                 // S: max, 1 / sum; dP: delta
+        if (head) {
+          if (is_s) {
+            const float l = a.p.softmax_sum[hi_];
+            c0 = l > 0.f ? a.p.softmax_max[hi_] : INFINITY;   // (no sum: P = 0)
+            c1 = l > 0.f ? 1.f / l : 0.f;
+          } else {
+            c0 = a.delta[hi_];
+          }
+        }
+        if constexpr (kScaled) up = is_s ? 8192.f : scalbnf(1.f, sfa_bwd_exponent(a, row));
+        for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
+          const uint32_t ph = n_tile & 1;
+          ok = wait(s_full, ph);
+          if (!ok) break;
+          ptx::tc_fence_after();
+          float v[24];
+          ptx::tmem_ld_x16(lane_addr + kBwdTmS + kk0, reinterpret_cast<uint32_t*>(v));
+          ptx::tmem_ld_x8(lane_addr + kBwdTmS + kk0 + 16, reinterpret_cast<uint32_t*>(v + 16));
+          if (is_s) {
+            float r[24];
+            ptx::tmem_ld_x16(lane_addr + kBwdTmR + kk0, reinterpret_cast<uint32_t*>(r));
+            ptx::tmem_ld_x8(lane_addr + kBwdTmR + kk0 + 16, reinterpret_cast<uint32_t*>(r + 16));
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 24; ++k) v[k] += r[k];
+          } else {
+            ptx::tmem_ld_wait();
+          }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(s_empty);
+          const int32_t cnt = nvalid - t * kBwdBK - kk0;    // valid keys among this warp's 24
+          if (is_s) {
+#pragma unroll
+            for (int k = 0; k < 24; ++k)
+              v[k] = k < cnt ? ex2(fmaf(v[k], a.p.scale, -c0) * 1.4426950408889634f) * c1 : 0.f;
+            ok = wait(&x_empty[pair], ph ^ 1);
+            if (!ok) break;
+#pragma unroll
+            for (int k = 0; k < 24; ++k) xbuf[(kk0 + k) * kBwdHeads] = v[k];
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&x_full[pair]);
+            ok = wait(p_empty, ph ^ 1);
+          } else {
+            ok = wait(&x_full[pair], ph);
+            if (!ok) break;
+#pragma unroll
+            for (int k = 0; k < 24; ++k) v[k] = xbuf[(kk0 + k) * kBwdHeads] * (v[k] - c0) * a.p.scale;
+            if (cnt < 24) {
+#pragma unroll
+              for (int k = 0; k < 24; ++k) v[k] = k < cnt ? v[k] : 0.f;
+            }
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&x_empty[pair]);
+            ok = wait(ds_empty, ph ^ 1);
+          }
+          if (!ok) break;
+#pragma unroll
+          for (int k = 0; k < 24; ++k) {
+            const float x = kScaled ? v[k] * up : v[k];
+            const T hi = from_f32<T>(x);
+            unsigned char* dst = mat_hi + (kk0 + k) * 128 + (((hl >> 3) ^ (k & 7)) << 4);   // (24 is a multiple of 8)
+            *reinterpret_cast<T*>(dst) = hi;
+            *reinterpret_cast<T*>(dst + kBwdPMat) = from_f32<T>(x - to_f32<T>(hi));
+          }
+          ptx::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(is_s ? p_full : ds_full);
+        }
+        if (!ok) break;
+        ok = wait(dq_full, n_item & 1);
+        if (!ok) break;
+        ptx::tc_fence_after();
+      }
+      // dQ^T tile m: this thread's feature is m * 128 + quarter * 32 + lane, a column is a head
+      float down = 1.f;
+      if constexpr (kScaled) { if (ntiles > 0) down = scalbnf(1.f, -sfa_bwd_exponent(a, row)); }
+      const int32_t hn = min(kBwdHeads, n1 - h0);
+#pragma unroll 1
+      for (int m = half; m < 5; m += 2) {
+        const int f = quarter * 32 + lane;
+        if (m == 4 && quarter >= 2) continue;
+        T* dst = m < 4 ? (T*)a.p.d_query + ((int64_t)row * n1 + h0) * 512 + m * 128 + f
+                       : (T*)a.p.d_query_rope + ((int64_t)row * n1 + h0) * 64 + f;
+        const int step = m < 4 ? 512 : 64;
+#pragma unroll 1
+        for (int c = 0; c < kBwdHeads; c += 16) {
+          if (c >= hn) break;
+          float o[16];
+          if (ntiles > 0) {
+            ptx::tmem_ld_x16(lane_addr + kBwdTmQ + m * 64 + c, reinterpret_cast<uint32_t*>(o));
+            ptx::tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = 0.f;
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (c + i < hn) dst[(int64_t)(c + i) * step] = from_f32<T>(o[i] * down);
+        }
+      }
+      if (ntiles > 0) {
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(dq_empty);
+        ++n_item;
+      }
+    }
+   }
+  } else if (warp < kBwdGatherWarp0) {
+   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBwdRegsHigh));
+   if (!*abort_flag) {
+    // -------------------------------------------------------------------- drain: reductions of dV^T / dK^T
+    const int quarter = warp & 3, group = (warp - kBwdDrainWarp0) >> 2;
+    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + kBwdTmD;
+    const int f = quarter * 32 + lane;
+    uint32_t n_drain = 0, n_mine = 0;
+    int turn = 0, rbuf = 0;
+    bool ok = true;
+    for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+      const int32_t row = item / a.hblocks;
+      const int2 nv = a.nvalid[row];
+      const int32_t ntiles = tiles_of(nv.x);
+      float dk_down = 1.f;
+      if constexpr (kScaled) { if (ntiles > 0) dk_down = scalbnf(1.f, -sfa_bwd_exponent(a, row)); }
+      for (int32_t t = 0; t < ntiles && ok; ++t) {
+        const int4* rows4 = reinterpret_cast<const int4*>(rows_s + rbuf * kBwdBK);
+        rbuf = rbuf == 2 ? 0 : rbuf + 1;
+#pragma unroll 1
+        for (int m = 0; m < kBwdTiles; ++m, ++n_drain) {
+          const bool mine = turn == group;
+          turn = turn == kBwdDrainGroups - 1 ? 0 : turn + 1;
+          if (!mine) continue;
+          const uint32_t slot = n_drain & 1;
+          ok = wait(&d_full[group], n_mine++ & 1);
+          if (!ok) break;
+          ptx::tc_fence_after();
+          float v[48];
+          ptx::tmem_ld_x16(lane_addr + slot * kBwdBK, reinterpret_cast<uint32_t*>(v));
+          ptx::tmem_ld_x16(lane_addr + slot * kBwdBK + 16, reinterpret_cast<uint32_t*>(v + 16));
+          ptx::tmem_ld_x16(lane_addr + slot * kBwdBK + 32, reinterpret_cast<uint32_t*>(v + 32));
+          ptx::tmem_ld_wait();
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&d_empty[slot]);
+          if (m == 8 && quarter >= 2) continue;              // the rope tile has 64 features
+          const bool is_v = m < 4;
+          const int32_t width = is_v ? 512 : 576;
+          float* base = is_v ? a.p.dv_acc + m * 128 + f : a.p.dk_acc + (m - 4) * 128 + f;
+          const float down = kScaled ? (is_v ? 1.f / 8192.f : dk_down) : 1.f;
+          // one instruction = 32 features of one key = one full line
+#pragma unroll
+          for (int kb = 0; kb < kBwdBK; kb += 4) {
+            const int4 kr = rows4[kb / 4];
+            const int32_t r[4] = {kr.x, kr.y, kr.z, kr.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              red_add_if(r[i] < a.key_rows, base + (int64_t)r[i] * width, kScaled ? v[kb + i] * down : v[kb + i]);
+          }
+        }
+      }
+    }
+   }
+  } else {
+   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBwdRegsLow));
+   if (*abort_flag) {
+    // nothing started
+   } else if (warp < kBwdIssueA) {
+    // -------------------------------------------------------------------- K gather: 12 groups of 4 keys x 9 blocks
+    const int o = (warp - kBwdGatherWarp0) + kBwdGatherWarps * lane;
+    const bool active = o < 108;
+    const int grp = o / 9, blk = o - grp * 9;
+    unsigned char* dst = bwd_sm + kBwdOffK + blk * kBwdKBlk + grp * 512;
+    if (lane == 0) { ptx::prefetch_tmap(&tmap_kn); ptx::prefetch_tmap(&tmap_kr); }
+    uint32_t n_tile = 0;
+    int rbuf = 0;
+    bool ok = true;
+    for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+      const int2 nv = a.nvalid[item / a.hblocks];
+      const int32_t ntiles = tiles_of(nv.x);
+      const int32_t* list = a.key_list + nv.y;
+      int32_t rn[4], dn0 = 0, dn1 = 0;
+      auto load = [&](int32_t t) {
+        const int32_t left = nv.x - t * kBwdBK;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          rn[i] = active && left > 0 ? list[t * kBwdBK + (grp * 4 + i < left ? grp * 4 + i : 0)] : 0;
+        if (warp == kBwdGatherWarp0) {
+          dn0 = lane < left ? list[t * kBwdBK + lane] : a.key_rows;
+          dn1 = lane < 16 && 32 + lane < left ? list[t * kBwdBK + 32 + lane] : a.key_rows;
+        }
+      };
+      load(0);
+      for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
+        int32_t r[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = rn[i];
+        const int32_t d0 = dn0, d1 = dn1;
+        load(t + 1);
+        ok = wait(k_empty, (n_tile & 1) ^ 1);
+        if (!ok) break;
+        if (warp == kBwdGatherWarp0) {
+          // The drain warps' row numbers (past the keys: no such key).  Three buffers: tile t + 3 is gathered
+          // after dQ of tile t + 2, i.e. after every dK^T tile of t + 1 was issued and so after every drain
+          // group has left tile t behind.
+          rows_s[rbuf * kBwdBK + lane] = d0;
+          if (lane < 16) rows_s[rbuf * kBwdBK + 32 + lane] = d1;
+          rbuf = rbuf == 2 ? 0 : rbuf + 1;
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_expect_tx(k_full, kBwdKBytes);
+        }
+        __syncwarp();
+        if (active) {
+          if (blk == 8) ptx::tma_gather4_2d(dst, &tmap_kr, k_full, 0, r[0], r[1], r[2], r[3]);
+          else ptx::tma_gather4_2d(dst, &tmap_kn, k_full, blk * 64, r[0], r[1], r[2], r[3]);
+        }
+        __syncwarp();
+      }
+    }
+   } else if (warp == kBwdIssueA) {
+    // -------------------------------------------------------------------- issuer A: S / dP, then dQ^T
+    const uint64_t qd_k = ptx::desc_kmajor_sw128(sm0 + kBwdOffQd), qr_k = ptx::desc_kmajor_sw128(sm0 + kBwdOffQr);
+    const uint64_t k_k = ptx::desc_kmajor_sw128(sm0 + kBwdOffK);
+    const uint64_t k_m = ptx::desc_mnmajor_sw128(sm0 + kBwdOffK, kBwdKBlk, 1024);
+    const uint64_t ds_m = ptx::desc_mnmajor_sw128(sm0 + kBwdOffP + 2 * kBwdPMat, 0, 1024);
+    uint32_t n_tile = 0, n_item = 0;
+    bool ok = true;
+    for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+      const int32_t ntiles = tiles_of(a.nvalid[item / a.hblocks].x);
+      if (ntiles == 0) continue;
+      ok = wait(q_full, n_item & 1);
+      for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
+        const uint32_t ph = n_tile & 1;
+        ok = wait(k_full, ph) && wait(s_empty, ph ^ 1);
+        if (!ok) break;
+        ptx::tc_fence_after();
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            ptx::mma_ss(tmem + kBwdTmR, qr_k + i * 2, k_k + ((8 * kBwdKBlk) >> 4) + i * 2, a.idesc_s, i ? 1u : 0u);
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            ptx::mma_ss(tmem + kBwdTmS, qd_k + (((i >> 2) * kBwdQdBlk) >> 4) + (i & 3) * 2,
+                        k_k + (((i >> 2) * kBwdKBlk) >> 4) + (i & 3) * 2, a.idesc_s, i ? 1u : 0u);
+          ptx::mma_commit(s_full);
+        }
+        __syncwarp();
+        ok = wait(ds_full, ph) && (t > 0 || wait(dq_empty, (n_item & 1) ^ 1));
+        if (!ok) break;
+        ptx::tc_fence_after();
+        if (ptx::elect_one()) {
+          ptx::fence_proxy_async_smem();
+#pragma unroll
+          for (int m = 0; m < 5; ++m)
+#pragma unroll
+            for (int ks = 0; ks < 3; ++ks)
+#pragma unroll
+              for (int lo = 0; lo < 2; ++lo)
+                ptx::mma_ss(tmem + kBwdTmQ + m * 64, k_m + ((m * 2 * kBwdKBlk + ks * 2048) >> 4),
+                            ds_m + ((lo * kBwdPMat + ks * 2048) >> 4), a.idesc_q, (t > 0 || ks > 0 || lo > 0) ? 1u : 0u);
+          ptx::mma_commit(k_empty);
+          ptx::mma_commit(ds_empty);
+          if (t == ntiles - 1) {
+            ptx::mma_commit(dq_full);
+            ptx::mma_commit(q_empty);
+          }
+        }
+        __syncwarp();
+      }
+      ++n_item;
+    }
+   } else if (warp == kBwdIssueB) {
+    // -------------------------------------------------------------------- issuer B: dV^T, dK^T
+    const uint64_t q_m = ptx::desc_mnmajor_sw128(sm0 + kBwdOffQd, kBwdQdBlk, 1024);
+    const uint64_t do_m = ptx::desc_mnmajor_sw128(sm0 + kBwdOffQd + kBwdHBlk, kBwdQdBlk, 1024);
+    const uint64_t p_k = ptx::desc_kmajor_sw128(sm0 + kBwdOffP);
+    uint32_t n_tile = 0, n_drain = 0;
+    int turn = 0;
+    bool ok = true;
+    for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+      const int32_t row = item / a.hblocks, h0 = (item - row * a.hblocks) * kBwdHeads;
+      const int32_t ntiles = tiles_of(a.nvalid[row].x);
+      if (ntiles == 0) continue;
+      const int steps = (min(kBwdHeads, n1 - h0) + 15) / 16;       // 16-head steps with real heads
+      for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
+        const uint32_t ph = n_tile & 1;
+#pragma unroll 1
+        for (int m = 0; m < kBwdTiles; ++m, ++n_drain) {
+          if (m == 0) ok = wait(p_full, ph);
+          if (m == 4) ok = wait(ds_full, ph);
+          const uint32_t slot = n_drain & 1;
+          ok = ok && wait(&d_empty[slot], ((n_drain >> 1) & 1) ^ 1);
+          if (!ok) break;
+          ptx::tc_fence_after();
+          if (ptx::elect_one()) {
+            ptx::fence_proxy_async_smem();
+            const uint64_t ad = m < 4 ? do_m + ((m * 2 * kBwdQdBlk) >> 4) : q_m + (((m - 4) * 2 * kBwdQdBlk) >> 4);
+            const uint64_t bd = p_k + (m < 4 ? 0 : (2 * kBwdPMat) >> 4);
+            const uint32_t dst = tmem + kBwdTmD + slot * kBwdBK;
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+              if (s < steps) {
+                ptx::mma_ss(dst, ad + ((s * 2048) >> 4), bd + s * 2, a.idesc_d, s ? 1u : 0u);
+                ptx::mma_ss(dst, ad + ((s * 2048) >> 4), bd + (kBwdPMat >> 4) + s * 2, a.idesc_d, 1u);
+              }
+            }
+            ptx::mma_commit(&d_full[turn]);
+            if (m == 3) ptx::mma_commit(p_empty);
+            if (m == kBwdTiles - 1) {
+              ptx::mma_commit(ds_empty);
+              if (t == ntiles - 1) ptx::mma_commit(q_empty);
+            }
+          }
+          turn = turn == kBwdDrainGroups - 1 ? 0 : turn + 1;
+          __syncwarp();
+        }
+      }
+    }
+   } else if (warp == kBwdLoader) {
+    // -------------------------------------------------------------------- Q / dO loader
+    uint32_t n_item = 0;
+    bool ok = true;
+    if (lane == 0) { ptx::prefetch_tmap(&tmap_q); ptx::prefetch_tmap(&tmap_qr); ptx::prefetch_tmap(&tmap_do); }
+    for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+      const int32_t row = item / a.hblocks, h0 = (item - row * a.hblocks) * kBwdHeads;
+      if (a.nvalid[row].x == 0) continue;
+      if (lane == 0) {
+        ok = ptx::mbar_wait(q_empty, (n_item & 1) ^ 1, abort_flag);
+        if (ok) {
+          ptx::mbar_arrive_expect_tx(q_full, kBwdQBytes);
+#pragma unroll 1
+          for (int b = 0; b < 8; ++b) {
+            ptx::tma_load_3d(bwd_sm + kBwdOffQd + b * kBwdQdBlk, &tmap_q, q_full, b * 64, h0, row);
+            ptx::tma_load_3d(bwd_sm + kBwdOffQd + b * kBwdQdBlk + kBwdHBlk, &tmap_do, q_full, b * 64, h0, row);
+          }
+          ptx::tma_load_3d(bwd_sm + kBwdOffQr, &tmap_qr, q_full, 0, h0, row);
+        }
+      } else {
+        // the other lanes pull the next item's rows into L2
+        const int32_t next = item + gridDim.x;
+        if (next < a.items) {
+          const int32_t nrow = next / a.hblocks, nh0 = (next - nrow * a.hblocks) * kBwdHeads;
+          const int64_t off = ((int64_t)nrow * n1 + nh0) * 1024;
+          for (int32_t i = lane - 1; i < min(kBwdHeads, n1 - nh0) * 8; i += 31) {
+            ptx::prefetch_l2((const unsigned char*)a.p.query + off + (int64_t)i * 128);
+            ptx::prefetch_l2((const unsigned char*)a.p.d_out + off + (int64_t)i * 128);
+          }
+        }
+      }
+      ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+      ++n_item;
+    }
+   }
+  }
+
+  // ---------------------------------------------------------------------- teardown
+  __syncwarp();
+  if (*abort_flag) {
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);  // let copies / MMAs in flight land
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (warp == kBwdIssueA) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, 512);
+  }
+  if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, misaligned ? 2 : 1);
+}
+
+// ---- host side ---------------------------------------------------------------------------------
+inline int64_t sfa_bwd_rows(const DsaSfaGradParams* p) {
+  return p->layout_q == DSA_LAYOUT_TND ? (int64_t)p->s1 : (int64_t)p->batch * p->s1;
+}
+inline bool sfa_bwd_sm100_eligible(const DsaSfaGradParams* p) {
+  if (p->d != 512 || p->d_rope != 64 || p->kernel == DSA_KERNEL_PORTABLE) return false;
+  if (((uintptr_t)p->query | (uintptr_t)p->query_rope | (uintptr_t)p->key | (uintptr_t)p->key_rope |
+       (uintptr_t)p->d_out | (uintptr_t)p->out) & 15u)
+    return false;
+  if (p->key_rows < 1 || p->key_rows >= (1ll << 31) - 1) return false;
+  const int64_t rows = sfa_bwd_rows(p);
+  if (rows < 1 || rows * ((p->n1 + kBwdHeads - 1) / kBwdHeads) >= (1ll << 31)) return false;
+  return rows * p->sparse_count * p->sparse_block_size < (1ll << 31);    // key_list offsets are int32
+}
+// Workspace: header | dk / dv accumulators | bounds (fp16) - zeroed before the call - | nvalid |
+// delta | redo flags and count of the pre-pass (unused) | key_list
+struct SfaBwdWs { size_t acc, bound, zeroed, nvalid, delta, redo, key_list, total; };
+inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
+  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  const size_t rows = (size_t)sfa_bwd_rows(p);
+  SfaBwdWs w;
+  w.acc = header;
+  w.bound = w.acc + up((size_t)p->key_rows * (size_t)(2 * p->d + p->d_rope) * sizeof(float));
+  w.zeroed = w.bound + (p->dtype == DSA_DTYPE_FP16 ? up((rows * 2 + 4) * 4) : 0);
+  w.nvalid = w.zeroed;
+  w.delta = w.nvalid + up(rows * 8);
+  w.redo = w.delta + up(rows * p->n1 * 4);
+  w.key_list = w.redo + up(rows * 4) + 256;
+  w.total = w.key_list + rows * p->sparse_count * p->sparse_block_size * 4;
+  return w;
+}
+
+template <typename T>
+inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, char* ws, const SfaBwdWs& w,
+                                cudaStream_t st) {
+  static std::atomic<int> sm_count[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DSA_ERR_CUDA;
+  int sms = sm_count[dev].load(std::memory_order_acquire);
+  if (sms == 0) {
+    // (idempotent: two threads that get here together do the same thing)
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return DSA_ERR_CUDA;
+    if (cudaFuncSetAttribute(sfa_bwd_sm100_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kBwdSmemBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(sfa_bwd_sm100_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kBwdSmemBytes) != cudaSuccess)
+      return DSA_ERR_CUDA;
+    // (a build with another register count must not run: setmaxnreg.inc could block for good)
+    cudaFuncAttributes fa0, fa1;
+    if (cudaFuncGetAttributes(&fa0, sfa_bwd_sm100_kernel<__nv_bfloat16>) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa1, sfa_bwd_sm100_kernel<__half>) != cudaSuccess || fa0.numRegs != kBwdLaunchRegs ||
+        fa1.numRegs != kBwdLaunchRegs)
+      return DSA_ERR_CUDA;
+    sm_count[dev].store(sms, std::memory_order_release);
+  }
+  const bool bf16 = p->dtype == DSA_DTYPE_BF16;
+  int32_t* status = (int32_t*)ws;
+  int2* nvalid = (int2*)(ws + w.nvalid);
+  int32_t* key_list = (int32_t*)(ws + w.key_list);
+  float* delta = (float*)(ws + w.delta);
+  float* bound = bf16 ? nullptr : (float*)(ws + w.bound);
+  int32_t* redo = (int32_t*)(ws + w.redo);
+  SfaDev f = {};
+  f.seq = d.seq;
+  f.sparse_indices = d.sparse_indices;
+  f.rows = d.rows;
+  f.sparse_count = d.sparse_count; f.sparse_block_size = d.sparse_block_size;
+  const int64_t slots = (int64_t)p->sparse_count * p->sparse_block_size;
+  sfa_compact_kernel<<<(d.rows + 3) / 4, 128, 0, st>>>(f, nvalid, key_list, 1, (int32_t)slots, (int32_t)p->key_rows,
+                                                      redo, redo + d.rows, status);
+  const int64_t pairs = (int64_t)d.rows * p->n1;
+  sfa_bwd_delta_kernel<T><<<(unsigned)((pairs + 7) / 8), 256, 0, st>>>((const T*)p->d_out, (const T*)p->out, delta, bound,
+                                                                      pairs, p->n1);
+  if (!bf16)
+    sfa_bwd_key_norm_kernel<T><<<(unsigned)std::min<int64_t>((p->key_rows + 7) / 8, sms * 4), 256, 0, st>>>(
+        (const T*)p->key, bound, p->key_rows);
+  if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
+  count_launch(bf16 ? 2 : 3);
+  SfaBwdArgs a;
+  a.p = d;
+  a.status = status;
+  a.nvalid = nvalid; a.key_list = key_list; a.delta = delta; a.bound = bound;
+  const uint32_t fmt = bf16 ? 1u : 0u;
+  a.idesc_s = ptx::idesc_f16(fmt, 128, kBwdBK, 0, 0);
+  a.idesc_q = ptx::idesc_f16(fmt, 128, kBwdHeads, 1, 1);
+  a.idesc_d = ptx::idesc_f16(fmt, 128, kBwdBK, 1, 0);
+  a.hblocks = (p->n1 + kBwdHeads - 1) / kBwdHeads;
+  a.items = d.rows * a.hblocks;
+  a.key_rows = (int32_t)p->key_rows;
+  CUtensorMap tkn, tkr, tq, tqr, tdo;
+  if (!make_tmap_gather4_16bit(&tkn, p->key, (uint64_t)p->key_rows, 512, 1024, 64, bf16) ||
+      !make_tmap_gather4_16bit(&tkr, p->key_rope, (uint64_t)p->key_rows, 64, 128, 64, bf16) ||
+      !make_tmap_3d_16bit(&tq, p->query, (uint64_t)d.rows, (uint64_t)p->n1, 512, 1024, (uint64_t)p->n1 * 1024, kBwdHeads,
+                          64, bf16) ||
+      !make_tmap_3d_16bit(&tqr, p->query_rope, (uint64_t)d.rows, (uint64_t)p->n1, 64, 128, (uint64_t)p->n1 * 128,
+                          kBwdHeads, 64, bf16) ||
+      !make_tmap_3d_16bit(&tdo, p->d_out, (uint64_t)d.rows, (uint64_t)p->n1, 512, 1024, (uint64_t)p->n1 * 1024,
+                          kBwdHeads, 64, bf16))
+    return DSA_ERR_CUDA;
+  const int grid = std::min(a.items, sms);
+  sfa_bwd_sm100_kernel<T><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tkn, tkr, tq, tqr, tdo, a);
+  if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
+  count_launch();
+  return DSA_OK;
+}
+
+}  // namespace dsa

@@ -231,3 +231,30 @@ def test_grad_untouched_rows_are_zero_and_repeat_runs_agree():
     assert torch.equal(a[0], b[0]) and torch.equal(a[3], b[3])          # per-row results: no atomics
     for x, y, n in zip(a, b, NAMES):
         sfa_grad_acceptance_rule(host(x), host(y), "fp16", name=n, ulps=1.0)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("S1,S2,N1,K", [
+    (3, 49, 64, 64),       # 47, 48 and 49 keys: one below, at and one past a 48-key tile
+    # 23 and 24 keys, one head.  (Not one or two keys: there dS0 = -dS1, so d_query = dS0 (k0 - k1) cancels
+    # while the checker rounds each dS to the io dtype, 2^-9 of |dS| |k|, above 2 ulp of the difference.)
+    (2, 24, 1, 24),
+    (4, 200, 65, 97),      # a second block of one head, a last tile of one key
+    (160, 192, 17, 48),    # more items than SMs, two 16-head steps of which one has a single head
+])
+def test_grad_at_the_edges_of_tiles_and_head_blocks(S1, S2, N1, K, dtype):
+    """D = 512 kernel (48-key tiles, blocks of 64 heads): same rule as everywhere (2 ulp of the io dtype
+    given the same forward state)."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_grad_triton
+    q, k, qr, kr, do = sfa_grad_inputs(91, 1, S1, S2, N1, 512, 64, dtype)
+    idx = sparse_indices(1091, 1, S1, S2, K, 1, 3)
+    scale = 1.0 / math.sqrt(576.0)
+    out, mx, sm = sparse_flash_attention_oracle(q, k, idx, qr, kr, scale, [S1], [S2], sparse_mode=3,
+                                                return_softmax_lse=True, dtype=dtype)
+    dt = tdtype(dtype)
+    tk = dev(k, dt)
+    got = sparse_flash_attention_grad_triton(dev(q, dt), tk, tk, dev(idx), dev(do, dt), dev(out, dt), dev(mx), dev(sm),
+                                             scale_value=scale, query_rope=dev(qr, dt), key_rope=dev(kr, dt), sparse_mode=3)
+    ref = sparse_flash_attention_grad_oracle(q, k, idx, do, out, mx, sm, qr, kr, scale, [S1], [S2], sparse_mode=3,
+                                             dtype=dtype)
+    _check(got, ref, dtype, S1)
