@@ -17,6 +17,7 @@
 #include "sfa_bwd_mma.cuh"
 #include "sfa_bwd_sm100.cuh"
 #include "sli_grad.cuh"
+#include "sli_sm100.cuh"
 
 namespace dsa {
 
@@ -372,7 +373,8 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status,
   d.p_buf = reinterpret_cast<float*>(ws + buf_bytes);
   d.loss_parts = reinterpret_cast<float*>(ws + 2 * buf_bytes);
   float* stats = reinterpret_cast<float*>((char*)d.loss_parts + align256((size_t)rows * 4));
-  d.dki_acc = reinterpret_cast<float*>((char*)stats + align256((size_t)rows * 8));
+  d.di_max = reinterpret_cast<float*>((char*)stats + align256((size_t)rows * 8));
+  d.dki_acc = reinterpret_cast<float*>((char*)d.di_max + align256((size_t)rows * 4));
   d.stats_given = (p->dense && p->softmax_max_index) ? 1 : 0;
   d.index_max = d.stats_given ? const_cast<float*>(p->softmax_max_index) : stats;
   d.index_sum = d.stats_given ? const_cast<float*>(p->softmax_sum_index) : stats + rows;
@@ -382,7 +384,6 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status,
   d.g = p->g; d.d_idx = p->d_idx; d.topk = slots; d.dtype_w = p->dtype_w;
   d.scale = p->scale;
   if (cudaMemsetAsync(d.dki_acc, 0, (size_t)key_elems * 4, st) != cudaSuccess) return DSA_ERR_CUDA;
-  if (rows > 0 && cudaMemsetAsync(d.di, 0, 2 * buf_bytes, st) != cudaSuccess) return DSA_ERR_CUDA;
   if (rows > 0) {
     const int stride = std::max(p->d + p->d_rope, p->d_idx) + kSliPad;
     // teacher blocks of 32 heads when a side has more than 16 (half the key gathers per row)
@@ -392,18 +393,22 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status,
     // gradient blocks of 32 heads for d_idx = 128 (both head tiles' dQI accumulators fit in registers)
     const int hg = (d.g > kSliHeads && p->d_idx == 128) ? 2 * kSliHeads : kSliHeads;
     const size_t smem_b = (size_t)(hg + kSliTeacherKeys) * (p->d_idx + kSliPad) * sizeof(T);
-    if (cudaFuncSetAttribute(sli_teacher_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(sli_teacher_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(sli_grad_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(sli_grad_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b) !=
-            cudaSuccess)
+    int sms = 0;
+    const bool tensor = sli_sm100_aligned(p);
+    if (tensor) {
+      const int rc = sli_sm100_prepare(&sms);
+      if (rc != DSA_OK) return rc;
+    }
+    // Which kernel does what: the tcgen05 kernels take the attention side when its query heads share one key
+    // head or have one each, the index side always, the gradients when d_idx = 128.
+    const bool att_mqa = tensor && d.n2 == 1, att_mha = tensor && p->dense && d.n2 == d.n1 && d.n2 > 1;
+    SliMhaArgs mha = {};
+    if (att_mha) mha = sli_mha_args(p, d, sms);
+    if ((att_mqa ? sli_score_needs_zero(d.n1) : !att_mha || mha.parts > 1) &&
+        cudaMemsetAsync(d.p_buf, 0, buf_bytes, st) != cudaSuccess)
       return DSA_ERR_CUDA;
     // Dense operator: the index scores of all visible keys are the lightning indexer's scores; when
-    // the shape is one the tcgen05 scoring kernel takes, it writes them (row stride = s2) and the
-    // CUDA-core pass below only does the attention side.
+    // the shape is one the tcgen05 scoring kernel takes, it writes them (row stride = s2).
     bool index_done = false;
     if (p->dense && p->s2 % 4 == 0 && status != nullptr) {
       DsaLiParams l = {};
@@ -423,10 +428,23 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status,
         index_done = true;
       }
     }
+    if (!index_done && !(tensor && !sli_score_needs_zero(d.g)) &&
+        cudaMemsetAsync(d.di, 0, buf_bytes, st) != cudaSuccess)
+      return DSA_ERR_CUDA;
+    if (tensor && !index_done) {
+      const int rc = sli_score_sm100_launch(p, d, false, status, sms, st);
+      if (rc != DSA_OK) return rc;
+      index_done = true;
+    }
+    if (att_mqa || att_mha) {
+      const int rc = att_mqa ? sli_score_sm100_launch(p, d, true, status, sms, st) : sli_mha_sm100_launch(p, mha, status, sms, st);
+      if (rc != DSA_OK) return rc;
+    }
     // Dense operator with fewer than 16 query heads per key head: blocks of 16 (row, head) pairs
     // share the keys they walk over; the per-row kernel then only does the index side, if any.
     const int grp = d.n1 / d.n2;
-    const bool pair_blocks = p->dense && grp < kSliHeads && kSliHeads % grp == 0;
+    const bool att_done = att_mqa || att_mha;
+    const bool pair_blocks = !att_done && p->dense && grp < kSliHeads && kSliHeads % grp == 0;
     if (pair_blocks) {
       if (cudaFuncSetAttribute(sli_dense_teacher_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem_d) != cudaSuccess)
@@ -438,23 +456,40 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status,
       count_launch();
     }
     SliGradDev dt = d;
-    if (pair_blocks) dt.lse_only = 1;   // index chunks only
-    const unsigned chunks_t =
-        (unsigned)((pair_blocks ? 0 : sli_att_chunks(d.n1, d.n2, hb)) + (index_done ? 0 : sli_idx_chunks(d.g, hb)));
+    if (att_done || pair_blocks) dt.lse_only = 1;   // index chunks only
+    const unsigned chunks_t = (unsigned)((att_done || pair_blocks ? 0 : sli_att_chunks(d.n1, d.n2, hb)) +
+                                         (index_done ? 0 : sli_idx_chunks(d.g, hb)));
     if (chunks_t > 0) {
+      if (cudaFuncSetAttribute(sli_teacher_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a) !=
+              cudaSuccess ||
+          cudaFuncSetAttribute(sli_teacher_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a) !=
+              cudaSuccess)
+        return DSA_ERR_CUDA;
       dim3 grid_t((unsigned)rows, chunks_t, 1);
       if (hb > kSliHeads) sli_teacher_kernel<T, 2><<<grid_t, kSliThreads, smem_a, st>>>(dt, stride);
       else sli_teacher_kernel<T, 1><<<grid_t, kSliThreads, smem_a, st>>>(dt, stride);
       if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
       count_launch();
     }
+    if (!(tensor && p->d_idx == 128 && p->dtype == DSA_DTYPE_FP16)) d.di_max = nullptr;
     sli_student_kernel<<<(unsigned)rows, kSliThreads, 0, st>>>(d);
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
-    dim3 grid((unsigned)rows, (unsigned)sli_idx_chunks(d.g, hg), 1);
-    if (hg > kSliHeads) sli_grad_kernel<T, 2><<<grid, kSliThreads, smem_b, st>>>(d);
-    else sli_grad_kernel<T, 1><<<grid, kSliThreads, smem_b, st>>>(d);
-    if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
-    count_launch(2);
+    count_launch();
+    if (tensor && p->d_idx == 128) {
+      const int rc = sli_grad_sm100_launch<T>(p, d, status, sms, st);
+      if (rc != DSA_OK) return rc;
+    } else {
+      if (cudaFuncSetAttribute(sli_grad_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b) !=
+              cudaSuccess ||
+          cudaFuncSetAttribute(sli_grad_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b) !=
+              cudaSuccess)
+        return DSA_ERR_CUDA;
+      dim3 grid((unsigned)rows, (unsigned)sli_idx_chunks(d.g, hg), 1);
+      if (hg > kSliHeads) sli_grad_kernel<T, 2><<<grid, kSliThreads, smem_b, st>>>(d);
+      else sli_grad_kernel<T, 1><<<grid, kSliThreads, smem_b, st>>>(d);
+      if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
+      count_launch();
+    }
   }
   const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((key_elems + 255) / 256, 148 * 16));
   sli_finalize_kernel<T><<<blocks, 256, 0, st>>>(d, key_elems, (int32_t)rows);
@@ -673,7 +708,7 @@ int dsa_sli_grad_workspace_bytes(const DsaSliGradParams* p, size_t* out_bytes) {
   if (!out_bytes) return DSA_ERR_NULL;
   const size_t rows = (size_t)p->batch * p->s1;
   *out_bytes = kWorkspaceHeader + 2 * align256(rows * (size_t)sli_slots(p) * 4) + align256(rows * 4) +
-               align256(rows * 8) + (size_t)p->batch * p->s2 * p->d_idx * 4;
+               align256(rows * 8) + align256(rows * 4) + (size_t)p->batch * p->s2 * p->d_idx * 4;
   return DSA_OK;
 }
 

@@ -49,6 +49,7 @@ struct SliGradDev {
   float* di;                // [rows, topk]  scratch, zeroed by the caller: index scores, then dI
   float* p_buf;             // [rows, topk]  scratch, zeroed by the caller: sum over heads of the attention probabilities
   float* loss_parts;        // [rows]        scratch
+  float* di_max;            // [rows]        scratch: largest |dI| of the row; null: not wanted
   float* dki_acc;           // [batch * s2, d_idx] scratch, zeroed by the caller
   int32_t batch, s1, s2, n1, n2, d, d_rope, g, d_idx, topk, dtype_w;
   int32_t stats_given;   // dense: index_max / index_sum come from the caller
@@ -376,21 +377,29 @@ __global__ void __launch_bounds__(kSliThreads) sli_student_kernel(SliGradDev p) 
   if (p.lse_only) return;
   if (dense && !(se > 0.f)) {           // the reference skips such rows: no gradient, no loss
     for (int k = tid; k < n; k += kSliThreads) di[k] = 0.f;
-    if (tid == 0) p.loss_parts[row] = 0.f;
+    if (tid == 0) {
+      p.loss_parts[row] = 0.f;
+      if (p.di_max != nullptr) p.di_max[row] = 0.f;
+    }
     return;
   }
   const float* pb = p.p_buf + (int64_t)row * p.topk;
   const float inv = dense ? 1.f / fmaxf(se, kSliEps) : 1.f / (se + kSliEps);
   const float inv_n1 = 1.f / (float)p.n1;
-  float kl = 0.f;
+  float kl = 0.f, top = 0.f;
   for (int k = tid; k < n; k += kSliThreads) {
     const float si = expf(di[k] - m) * inv, pk = pb[k] * inv_n1;
     di[k] = si - pk;
+    top = fmaxf(top, fabsf(si - pk));
     const float pc = fmaxf(pk, kSliEps), sc = fmaxf(si, kSliEps);
     kl += pc * (logf(pc) - logf(sc));
   }
   kl = sli_block_reduce(kl, red8, false);
   if (tid == 0) p.loss_parts[row] = kl;
+  if (p.di_max != nullptr) {
+    top = sli_block_reduce(top, red8, true);
+    if (tid == 0) p.di_max[row] = top;
+  }
 }
 
 // MT = 16-head tiles per block (HB = 16 MT heads; two tiles only for d_idx = 128, where the dQI

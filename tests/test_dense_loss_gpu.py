@@ -67,7 +67,10 @@ _CORE = [(1, 2, 64, 32, 32, d, g, di) for d in (128, 256, 512) for g in (32, 64,
                                                               (1, 64, 512, 64, 1, 512, 64, 128),
                                                               (2, 5, 80, 32, 16, 128, 32, 128),
                                                               (1, 7, 64, 16, 4, 128, 32, 128),
-                                                              (1, 40, 256, 32, 32, 128, 32, 128)])
+                                                              (1, 40, 256, 32, 32, 128, 32, 128),
+                                                              # tiles of 128 rows x 128 keys: whole, one past, odd key counts
+                                                              (1, 128, 256, 3, 3, 256, 8, 128),
+                                                              (2, 129, 385, 5, 5, 128, 24, 128)])
 @pytest.mark.parametrize("dtype", ["bf16", "fp16"])
 def test_dense_operators_against_the_oracle_on_the_reference_configurations(B, S1, S2, N1, N2, D, G, Di, dtype):
     """test_dense_loss_backward_triton.py:20-31 (every third of the 27 core configurations, the two

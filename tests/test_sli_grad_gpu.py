@@ -88,6 +88,21 @@ def test_sli_grad_against_the_oracle_on_the_reference_shapes(B, S1, S2, N1, D, G
     _check(ref, _run(q, k, qr, kr, qi, ki, w, si, sm_max, sm_sum, scale, dtype), dtype)
 
 
+@pytest.mark.parametrize("B,S1,S2,N1,D,G,Di,topk", [
+    (1, 3, 130, 8, 256, 8, 128, 127),       # one tile of keys not quite full, fewer heads than a product takes
+    (1, 3, 260, 136, 128, 72, 128, 129),    # one key past a tile, one head block past 128 / 64
+    (2, 5, 300, 40, 512, 24, 256, 256),     # whole tiles, index scores of four feature blocks
+    (1, 2, 1100, 128, 512, 64, 128, 1027),  # the largest head block, a row cut into parts
+])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_sli_grad_at_the_edges_of_key_tiles_and_head_blocks(B, S1, S2, N1, D, G, Di, topk, dtype):
+    q, k, qr, kr, qi, ki, w, si = sli_grad_inputs(17, B, S1, S2, N1, D, G, Di, topk, "causal_random", dtype=dtype)
+    scale = 1.0 / math.sqrt(D)
+    sm_max, sm_sum = softmax_stats(q, k, qr, kr, scale, dtype=dtype)
+    ref = sli_grad_kl_loss_oracle(q, k, qr, kr, qi, ki, w, si, sm_max, sm_sum, scale, dtype=dtype)
+    _check(ref, _run(q, k, qr, kr, qi, ki, w, si, sm_max, sm_sum, scale, dtype), dtype)
+
+
 def test_sli_grad_valid_lengths_no_rope_fp32_weights_and_out_of_range_indices():
     """Rows beyond the valid query length and rows without visible keys give zero gradients and no
     loss; indices outside [0, S2) are clipped like the reference clips them (:96); the rope parts are
