@@ -27,9 +27,9 @@ constexpr uint32_t kSlSmemMax = 232448;
 // pipe.  So one block takes up to 128 heads of the row (every gathered byte serves all of them), Q stays in
 // shared memory and the keys stream through a ring of 64-feature blocks (16 KB each: a whole tile of 147
 // KB would not fit beside 128 heads of Q).  Rows are cut into parts when there are few of them.
-// Warps: 0..7 epilogue (two groups on alternate accumulators), 8..11 gather, 12 MMA issuer, 13 Q and head
+// Warps: 0..7 epilogue (two groups on alternate accumulators), 8..15 gather, 16 MMA issuer, 17 Q and head
 // parameters.
-constexpr int kScThreads = 448, kScGatherWarp0 = 8, kScIssuer = 12, kScLoader = 13;
+constexpr int kScThreads = 576, kScGatherWarp0 = 8, kScGatherWarps = 8, kScIssuer = 16, kScLoader = 17;
 constexpr int kScMaxStages = 12;
 
 struct SliScoreArgs {
@@ -168,8 +168,10 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
       ++n_item;
     }
   } else if (warp < kScIssuer) {
-    // gather: lane = group of 4 keys; the four warps take the 64-feature blocks in turn
-    const int pw = warp - kScGatherWarp0;
+    // gather: pairs of warps take the 64-feature blocks in turn, a warp issues half of a block's 32 loads (a
+    // warp issues its lanes' loads one by one).  Pairs <= stages: a warp that waited for a ring slot one round
+    // ahead of another would take the round before for its own (the wait tells odd from even rounds only).
+    const int pair = (warp - kScGatherWarp0) >> 1, grp = ((warp - kScGatherWarp0) & 1) * 16 + (lane & 15);
     if (lane == 0) { ptx::prefetch_tmap(&tmap_ka); ptx::prefetch_tmap(&tmap_kb); }
     uint32_t gb = 0, ph = 1;
     int stage = 0;
@@ -181,7 +183,7 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
       int32_t rn[4];
       auto load = [&](int32_t t) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rn[i] = sli_key_row(a.p, idx_row, it.b, t * kSlKeys + lane * 4 + i, it.n, a.key_rows);
+        for (int i = 0; i < 4; ++i) rn[i] = sli_key_row(a.p, idx_row, it.b, t * kSlKeys + grp * 4 + i, it.n, a.key_rows);
       };
       load(it.t0);
       for (int32_t t = it.t0; t < it.t1 && ok; ++t) {
@@ -190,14 +192,16 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
         for (int i = 0; i < 4; ++i) r[i] = rn[i];
         load(t + 1);       // (past the row: nothing is read)
         for (int blk = 0; blk < a.nblk && ok; ++blk, ++gb) {
-          if ((int)(gb & 3) == pw) {
+          if ((int)(gb % (kScGatherWarps / 2)) == pair) {
             ok = wait(&empty[stage], ph);
             if (!ok) break;
-            if (lane == 0) ptx::mbar_arrive_expect_tx(&full[stage], kSlKBlk);
+            if (grp == 0 && lane == 0) ptx::mbar_arrive_expect_tx(&full[stage], kSlKBlk);
             __syncwarp();
-            unsigned char* dst = slsm + a.off_k + stage * kSlKBlk + lane * 512;
-            if (blk < a.nblk_a) ptx::tma_gather4_2d(dst, &tmap_ka, &full[stage], blk * 64, r[0], r[1], r[2], r[3]);
-            else ptx::tma_gather4_2d(dst, &tmap_kb, &full[stage], (blk - a.nblk_a) * 64, r[0], r[1], r[2], r[3]);
+            unsigned char* dst = slsm + a.off_k + stage * kSlKBlk + grp * 512;
+            if (lane < 16) {
+              if (blk < a.nblk_a) ptx::tma_gather4_2d(dst, &tmap_ka, &full[stage], blk * 64, r[0], r[1], r[2], r[3]);
+              else ptx::tma_gather4_2d(dst, &tmap_kb, &full[stage], (blk - a.nblk_a) * 64, r[0], r[1], r[2], r[3]);
+            }
             __syncwarp();
           }
           if (++stage == a.stages) { stage = 0; ph ^= 1; }
@@ -496,9 +500,15 @@ sli_mha_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid_c
 // without a conversion per element.  fp16: both are scaled by a power of two per row taken from the
 // row's largest magnitude.  dW = sum_k dI relu(S) is summed in fp32 registers.
 // Tensor memory: S 2 x 64 columns | dKI^T 2 x 128 | dQI^T 64.
-// Warps: 0..7 epilogue (lane quarter x 32 heads), 8..11 drain, 12..13 gather (one 64-feature block
-// each), 14 issuer, 15 QI loader, 16..19 w QI.
-constexpr int kSgThreads = 640, kSgDrainWarp0 = 8, kSgGatherWarp0 = 12, kSgIssuer = 14, kSgLoader = 15, kSgStager0 = 16;
+// Warps: 0..7 epilogue (lane quarter x 32 heads), 8..11 drain, 12..17 gather, 18 issuer, 19 QI loader,
+// 20..23 w QI.
+constexpr int kSgThreads = 768, kSgDrainWarp0 = 8, kSgGatherWarp0 = 12, kSgGatherWarps = 6, kSgIssuer = 18, kSgLoader = 19;
+constexpr int kSgStager0 = 20;
+// the epilogue and drain warps take the registers that the others give back
+constexpr int kSgLaunchRegs = 80, kSgRegsLow = 56, kSgRegsHigh = 104;
+static_assert((kSgRegsHigh - kSgLaunchRegs) * kSgGatherWarp0 <= (kSgLaunchRegs - kSgRegsLow) * (kSgThreads / 32 - kSgGatherWarp0),
+              "setmaxnreg: more registers requested than released");
+static_assert(kSgLaunchRegs * kSgThreads <= 65536, "register file");
 constexpr int kSgStages = 3;
 constexpr uint32_t kSgHBlk = 64 * 128;                             // 64 heads x 64 features
 constexpr uint32_t kSgOffQ = 0;                                    // 2 blocks
@@ -536,7 +546,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   constexpr bool kScaled = !kIsBf16<T>;
   extern __shared__ __align__(1024) unsigned char sgsm[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(sgsm + kSgOffBar);
-  uint64_t* k_full = bars;          // [3] gather -> issuer                               (tx bytes, two warps)
+  uint64_t* k_full = bars;          // [3] gather -> issuer                               (tx bytes)
   uint64_t* k_empty = bars + 3;     // [3] dQI of the tile done                           (commit)
   uint64_t* s_full = bars + 6;      // [2] scores -> epilogue                             (commit)
   uint64_t* s_empty = bars + 8;     // [2] scores read                                    (8 warps)
@@ -545,7 +555,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   uint64_t* d_full = bars + 12;     // [2] dKI^T -> drain                                 (commit)
   uint64_t* d_empty = bars + 14;    // [2] dKI^T read                                     (4 warps)
   uint64_t* q_full = bars + 16;     // QI landed                                          (tx bytes)
-  uint64_t* q_empty = bars + 17;    // last scores of the item done                       (commit)
+  uint64_t* q_empty = bars + 17;    // last scores of the item done, w QI taken           (commit, 4 warps)
   uint64_t* w_full = bars + 18;     // w QI stored                                        (4 warps)
   uint64_t* w_empty = bars + 19;    // last gradient products of the item done            (commit)
   uint64_t* dq_full = bars + 20;    // dQI^T complete                                     (commit)
@@ -561,7 +571,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool misaligned = (ptx::smem_u32(sgsm) & 1023u) != 0;
   if (threadIdx.x == 0) {
-    const int counts[23] = {2, 2, 2, 1, 1, 1, 1, 1, 8, 8, 8, 1, 1, 1, 4, 4, 1, 1, 4, 1, 1, 8, 8};
+    const int counts[23] = {1, 1, 1, 1, 1, 1, 1, 1, 8, 8, 8, 1, 1, 1, 4, 4, 1, 5, 4, 1, 1, 8, 8};
 #pragma unroll
     for (int i = 0; i < 23; ++i) ptx::mbar_init(&bars[i], counts[i]);
     *abort_flag = misaligned ? 1 : 0;
@@ -580,9 +590,13 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return ptx::mbar_wait_warp(bar, parity, abort_flag); };
   auto tiles_of = [&](int32_t n) -> int32_t { return (n + kSlKeys - 1) / kSlKeys; };
 
-  if (*abort_flag) {
+  // Each class of roles sits in its own branch, right under its setmaxnreg: the compiler budgets a
+  // branch by the setmaxnreg that dominates it.
+  if (warp < kSgGatherWarp0) {
+   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSgRegsHigh));
+   if (*abort_flag) {
     // nothing started
-  } else if (warp < kSgDrainWarp0) {
+   } else if (warp < kSgDrainWarp0) {
     // -------------------------------------------------------------------- E and dI E, dW; then dQI
     const int quarter = warp & 3, half = warp >> 2;
     const int key = quarter * 32 + lane;                  // within the tile
@@ -714,7 +728,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       }
       ++n_item;
     }
-  } else if (warp < kSgGatherWarp0) {
+   } else {
     // -------------------------------------------------------------------- drain: reductions of dKI^T
     const int quarter = warp & 3;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + kSgTmK;
@@ -753,9 +767,16 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         }
       }
     }
-  } else if (warp < kSgIssuer) {
-    // -------------------------------------------------------------------- gather: lane = group of 4 keys
-    const int blk = warp - kSgGatherWarp0;
+   }
+  } else {
+   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSgRegsLow));
+   if (*abort_flag) {
+    // nothing started
+   } else if (warp < kSgIssuer) {
+    // -------------------------------------------------------------------- gather: 32 groups of 4 keys x 2 blocks
+    const int o = (warp - kSgGatherWarp0) + kSgGatherWarps * lane;
+    const bool active = o < 64;
+    const int grp = o >> 1, blk = o & 1;
     if (lane == 0) ptx::prefetch_tmap(&tmap_k);
     uint32_t ph = 1;
     int stage = 0;
@@ -768,7 +789,8 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       int32_t rn[4];
       auto load = [&](int32_t t) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rn[i] = sli_key_row(a.p, idx_row, b, t * kSlKeys + lane * 4 + i, n, a.key_rows);
+        for (int i = 0; i < 4; ++i)
+          rn[i] = active ? sli_key_row(a.p, idx_row, b, t * kSlKeys + grp * 4 + i, n, a.key_rows) : a.key_rows;
       };
       load(0);
       for (int32_t t = 0; t < ntiles && ok; ++t) {
@@ -778,15 +800,16 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         load(t + 1);
         ok = wait(&k_empty[stage], ph);
         if (!ok) break;
-        if (lane == 0) ptx::mbar_arrive_expect_tx(&k_full[stage], kSlKBlk);
+        if (warp == kSgGatherWarp0 && lane == 0) ptx::mbar_arrive_expect_tx(&k_full[stage], 2 * kSlKBlk);
         __syncwarp();
-        ptx::tma_gather4_2d(sgsm + kSgOffK + (stage * 2 + blk) * kSlKBlk + lane * 512, &tmap_k, &k_full[stage], blk * 64,
-                            r[0], r[1], r[2], r[3]);
+        if (active)
+          ptx::tma_gather4_2d(sgsm + kSgOffK + (stage * 2 + blk) * kSlKBlk + grp * 512, &tmap_k, &k_full[stage], blk * 64,
+                              r[0], r[1], r[2], r[3]);
         __syncwarp();
         if (++stage == kSgStages) { stage = 0; ph ^= 1; }
       }
     }
-  } else if (warp == kSgIssuer) {
+   } else if (warp == kSgIssuer) {
     // -------------------------------------------------------------------- products: scores one tile ahead
     const uint64_t q_k = ptx::desc_kmajor_sw128(sm0 + kSgOffQ), k_k = ptx::desc_kmajor_sw128(sm0 + kSgOffK);
     const uint64_t k_m = ptx::desc_mnmajor_sw128(sm0 + kSgOffK, kSlKBlk, 1024);
@@ -857,7 +880,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       }
       ++n_item;
     }
-  } else if (warp == kSgLoader) {
+   } else if (warp == kSgLoader) {
     // -------------------------------------------------------------------- QI (heads past the last: zeros)
     uint32_t n_item = 0;
     bool ok = true;
@@ -876,8 +899,9 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       __syncwarp();
       ++n_item;
     }
-  } else {
+   } else {
     // -------------------------------------------------------------------- w QI, high and low part
+    // (same place in its block as QI: the operand's layout is QI's)
     const int th = threadIdx.x - kSgStager0 * 32;         // 0..127
     uint32_t n_item = 0;
     bool ok = true;
@@ -886,42 +910,40 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       int32_t b;
       if (sli_row_slots(a.p, row, &b) == 0) continue;
       const int32_t hn = min(64, g - h0);
-      const T* qi = (const T*)a.p.query_index + ((int64_t)row * g + h0) * 128;
+      ok = wait(q_full, n_item & 1);
+      if (!ok) break;
       int e = 0;
       if constexpr (kScaled) {
         // every warp takes the maximum over the whole item (so that no warp waits for another)
         float mx = 0.f;
-        for (int i = lane; i < hn * 16; i += 32) {
-          const uint4 x = reinterpret_cast<const uint4*>(qi)[i];
+#pragma unroll 2
+        for (int i = lane; i < 1024; i += 32) {           // 16-byte chunk of head (i / 8) % 64
+          const uint4 x = reinterpret_cast<const uint4*>(sgsm + kSgOffQ)[i];
+          const int h = (i >> 3) & 63;
           const T* xv = reinterpret_cast<const T*>(&x);
           float q = 0.f;
 #pragma unroll
           for (int u = 0; u < 8; ++u) q = fmaxf(q, fabsf(to_f32<T>(xv[u])));
-          mx = fmaxf(mx, q * fabsf(load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + (i >> 4))));
+          if (h < hn) mx = fmaxf(mx, q * fabsf(load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + h)));
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         e = sli_exponent(mx);
       }
       const float up = kScaled ? scalbnf(1.f, e) : 1.f;
-      uint4 x[8];
       float wv[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int c = th + 128 * i, h = c >> 4;           // 16-byte chunk c & 15 of head h
-        x[i] = make_uint4(0, 0, 0, 0);
-        wv[i] = 0.f;
-        if (h < hn) {
-          x[i] = reinterpret_cast<const uint4*>(qi)[c];
-          wv[i] = load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + h) * up;
-        }
+        const int h = ((th + 128 * i) >> 3) & 63;
+        wv[i] = h < hn ? load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + h) * up : 0.f;
       }
       ok = wait(w_empty, (n_item & 1) ^ 1);
       if (!ok) break;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int c = th + 128 * i, h = c >> 4, f = c & 15;
-        const T* xv = reinterpret_cast<const T*>(&x[i]);
+        const int c = th + 128 * i;
+        const uint4 x = reinterpret_cast<const uint4*>(sgsm + kSgOffQ)[c];
+        const T* xv = reinterpret_cast<const T*>(&x);
         uint32_t hw[4], lw[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -930,16 +952,20 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
           hw[u] = sli_bits<T>(a0) | (sli_bits<T>(a1) << 16);
           lw[u] = sli_bits<T>(from_f32<T>(v0 - to_f32<T>(a0))) | (sli_bits<T>(from_f32<T>(v1 - to_f32<T>(a1))) << 16);
         }
-        unsigned char* dst = sgsm + kSgOffW + (f >> 3) * kSgHBlk + h * 128 + (((f & 7) ^ (h & 7)) << 4);
-        *reinterpret_cast<uint4*>(dst) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-        *reinterpret_cast<uint4*>(dst + 2 * kSgHBlk) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+        uint4* dst = reinterpret_cast<uint4*>(sgsm + kSgOffW) + c;
+        dst[0] = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+        dst[2 * kSgHBlk / 16] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
       }
       if (kScaled && th == 0) w_exp[n_item & 1] = e;
       ptx::fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(w_full);
+      if (lane == 0) {
+        ptx::mbar_arrive(w_full);
+        ptx::mbar_arrive(q_empty);
+      }
       ++n_item;
     }
+   }
   }
 
   __syncwarp();
@@ -980,6 +1006,12 @@ inline int sli_sm100_prepare(int* sms_out) {
         cudaFuncSetAttribute(sli_grad_sm100_kernel<__nv_bfloat16>, attr, (int)kSgSmemBytes) != cudaSuccess ||
         cudaFuncSetAttribute(sli_grad_sm100_kernel<__half>, attr, (int)kSgSmemBytes) != cudaSuccess)
       return DSA_ERR_CUDA;
+    // (a build with another register count must not run: setmaxnreg.inc could block for good)
+    cudaFuncAttributes fa0, fa1;
+    if (cudaFuncGetAttributes(&fa0, sli_grad_sm100_kernel<__nv_bfloat16>) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa1, sli_grad_sm100_kernel<__half>) != cudaSuccess || fa0.numRegs != kSgLaunchRegs ||
+        fa1.numRegs != kSgLaunchRegs)
+      return DSA_ERR_CUDA;
     sm_count[dev].store(sms, std::memory_order_release);
   }
   *sms_out = sms;
@@ -1015,6 +1047,7 @@ inline int sli_score_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d
   // (the ring starts on a 1024-byte boundary: hp * 128 is a multiple of 2048)
   a.off_k = qbytes;
   a.stages = (int32_t)std::min<uint32_t>(kScMaxStages, (kSlSmemMax - tail - qbytes) / kSlKBlk);
+  if (a.stages < kScGatherWarps / 2) return DSA_ERR_TOO_LARGE;   // (nblk <= 9 leaves five)
   a.off_prm = a.off_k + a.stages * kSlKBlk;
   a.off_bar = a.off_prm + 2 * 128 * 8;
   const uint32_t smem = a.off_bar + 512;
