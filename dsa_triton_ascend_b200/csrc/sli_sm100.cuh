@@ -500,12 +500,12 @@ sli_mha_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid_c
 // without a conversion per element.  fp16: both are scaled by a power of two per row taken from the
 // row's largest magnitude.  dW = sum_k dI relu(S) is summed in fp32 registers.
 // Tensor memory: S 2 x 64 columns | dKI^T 2 x 128 | dQI^T 64.
-// Warps: 0..7 epilogue (lane quarter x 32 heads), 8..11 drain, 12..17 gather, 18 issuer, 19 QI loader,
-// 20..23 w QI.
-constexpr int kSgThreads = 768, kSgDrainWarp0 = 8, kSgGatherWarp0 = 12, kSgGatherWarps = 6, kSgIssuer = 18, kSgLoader = 19;
-constexpr int kSgStager0 = 20;
+// Warps: 0..7 epilogue (lane quarter x 32 heads), 8..15 drain (lane quarter x 64 keys), 16..19 gather, 20
+// issuer, 21 QI loader, 22..23 w QI.
+constexpr int kSgThreads = 768, kSgDrainWarp0 = 8, kSgGatherWarp0 = 16, kSgGatherWarps = 4, kSgIssuer = 20, kSgLoader = 21;
+constexpr int kSgStager0 = 22;
 // the epilogue and drain warps take the registers that the others give back
-constexpr int kSgLaunchRegs = 80, kSgRegsLow = 56, kSgRegsHigh = 104;
+constexpr int kSgLaunchRegs = 80, kSgRegsLow = 48, kSgRegsHigh = 96;
 static_assert((kSgRegsHigh - kSgLaunchRegs) * kSgGatherWarp0 <= (kSgLaunchRegs - kSgRegsLow) * (kSgThreads / 32 - kSgGatherWarp0),
               "setmaxnreg: more registers requested than released");
 static_assert(kSgLaunchRegs * kSgThreads <= 65536, "register file");
@@ -536,6 +536,10 @@ __device__ __forceinline__ int sli_exponent(float m) {
   return (m > 0.f && m < INFINITY) ? max(-100, min(100, 13 - ilogbf(m))) : 0;
 }
 
+__device__ __forceinline__ void red_add(float* addr, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
+}
+
 template <typename T>
 __device__ __forceinline__ uint32_t sli_bits(T v) { return (uint32_t)*reinterpret_cast<const uint16_t*>(&v); }
 
@@ -553,10 +557,10 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   uint64_t* e_full = bars + 10;     // E, dI E, rows and dI of the tile stored            (8 warps)
   uint64_t* e_empty = bars + 11;    // gradient products of the tile done                 (commit)
   uint64_t* d_full = bars + 12;     // [2] dKI^T -> drain                                 (commit)
-  uint64_t* d_empty = bars + 14;    // [2] dKI^T read                                     (4 warps)
+  uint64_t* d_empty = bars + 14;    // [2] dKI^T read                                     (8 warps)
   uint64_t* q_full = bars + 16;     // QI landed                                          (tx bytes)
-  uint64_t* q_empty = bars + 17;    // last scores of the item done, w QI taken           (commit, 4 warps)
-  uint64_t* w_full = bars + 18;     // w QI stored                                        (4 warps)
+  uint64_t* q_empty = bars + 17;    // last scores of the item done, w QI taken           (commit, 2 warps)
+  uint64_t* w_full = bars + 18;     // w QI stored                                        (2 warps)
   uint64_t* w_empty = bars + 19;    // last gradient products of the item done            (commit)
   uint64_t* dq_full = bars + 20;    // dQI^T complete                                     (commit)
   uint64_t* dq_empty = bars + 21;   // dQI^T read                                         (8 warps)
@@ -571,7 +575,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool misaligned = (ptx::smem_u32(sgsm) & 1023u) != 0;
   if (threadIdx.x == 0) {
-    const int counts[23] = {1, 1, 1, 1, 1, 1, 1, 1, 8, 8, 8, 1, 1, 1, 4, 4, 1, 5, 4, 1, 1, 8, 8};
+    const int counts[23] = {1, 1, 1, 1, 1, 1, 1, 1, 8, 8, 8, 1, 1, 1, 8, 8, 1, 3, 2, 1, 1, 8, 8};
 #pragma unroll
     for (int i = 0; i < 23; ++i) ptx::mbar_init(&bars[i], counts[i]);
     *abort_flag = misaligned ? 1 : 0;
@@ -730,39 +734,54 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     }
    } else {
     // -------------------------------------------------------------------- drain: reductions of dKI^T
-    const int quarter = warp & 3;
-    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + kSgTmK;
+    const int quarter = warp & 3, k0 = ((warp - kSgDrainWarp0) >> 2) * 64;
+    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + kSgTmK + k0;
     float* base = a.p.dki_acc + quarter * 32 + lane;
     uint32_t n_tile = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       int32_t b;
-      const int32_t ntiles = tiles_of(sli_row_slots(a.p, item / a.hchunks, &b));
+      const int32_t n = sli_row_slots(a.p, item / a.hchunks, &b), ntiles = tiles_of(n);
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
         const int buf = n_tile & 1;
-        const int4* rows4 = reinterpret_cast<const int4*>(rows_s + (n_tile & 3) * kSlKeys);
-        const float4* di4 = reinterpret_cast<const float4*>(di_s + (n_tile & 3) * kSlKeys);
+        const int4* rows4 = reinterpret_cast<const int4*>(rows_s + (n_tile & 3) * kSlKeys + k0);
+        const float4* di4 = reinterpret_cast<const float4*>(di_s + (n_tile & 3) * kSlKeys + k0);
         ok = wait(&d_full[buf], (n_tile >> 1) & 1);
         if (!ok) break;
         ptx::tc_fence_after();
+        const bool whole = n - t * kSlKeys >= kSlKeys;
 #pragma unroll 1
-        for (int c = 0; c < kSlKeys; c += 32) {
-          float v[32];
-          ptx::tmem_ld_x32(lane_addr + buf * kSlKeys + c, reinterpret_cast<uint32_t*>(v));
+        for (int c = 0; c < 64; c += 16) {
+          float v[16];
+          int4 r[4];
+          ptx::tmem_ld_x16(lane_addr + buf * kSlKeys + c, reinterpret_cast<uint32_t*>(v));
+#pragma unroll
+          for (int k = 0; k < 4; ++k) r[k] = rows4[c / 4 + k];
+          float4 d[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) d[k] = di4[c / 4 + k];
           ptx::tmem_ld_wait();
-          if (c == kSlKeys - 32) {
+          if (c == 48) {
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&d_empty[buf]);
           }
+          if (whole) {
 #pragma unroll
-          for (int k = 0; k < 32; k += 4) {
-            const int4 r = rows4[(c + k) / 4];
-            const float4 d = di4[(c + k) / 4];
-            red_add_if(r.x >= 0, base + (int64_t)r.x * 128, v[k] * d.x);
-            red_add_if(r.y >= 0, base + (int64_t)r.y * 128, v[k + 1] * d.y);
-            red_add_if(r.z >= 0, base + (int64_t)r.z * 128, v[k + 2] * d.z);
-            red_add_if(r.w >= 0, base + (int64_t)r.w * 128, v[k + 3] * d.w);
+            for (int k = 0; k < 4; ++k) {
+              red_add(base + (int64_t)r[k].x * 128, v[4 * k] * d[k].x);
+              red_add(base + (int64_t)r[k].y * 128, v[4 * k + 1] * d[k].y);
+              red_add(base + (int64_t)r[k].z * 128, v[4 * k + 2] * d[k].z);
+              red_add(base + (int64_t)r[k].w * 128, v[4 * k + 3] * d[k].w);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              red_add_if(r[k].x >= 0, base + (int64_t)r[k].x * 128, v[4 * k] * d[k].x);
+              red_add_if(r[k].y >= 0, base + (int64_t)r[k].y * 128, v[4 * k + 1] * d[k].y);
+              red_add_if(r[k].z >= 0, base + (int64_t)r[k].z * 128, v[4 * k + 2] * d[k].z);
+              red_add_if(r[k].w >= 0, base + (int64_t)r[k].w * 128, v[4 * k + 3] * d[k].w);
+            }
           }
         }
       }
@@ -902,7 +921,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
    } else {
     // -------------------------------------------------------------------- w QI, high and low part
     // (same place in its block as QI: the operand's layout is QI's)
-    const int th = threadIdx.x - kSgStager0 * 32;         // 0..127
+    const int th = threadIdx.x - kSgStager0 * 32;         // 0..63
     uint32_t n_item = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
@@ -931,23 +950,18 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         e = sli_exponent(mx);
       }
       const float up = kScaled ? scalbnf(1.f, e) : 1.f;
-      float wv[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int h = ((th + 128 * i) >> 3) & 63;
-        wv[i] = h < hn ? load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + h) * up : 0.f;
-      }
       ok = wait(w_empty, (n_item & 1) ^ 1);
       if (!ok) break;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int c = th + 128 * i;
+#pragma unroll 2
+      for (int i = 0; i < 16; ++i) {
+        const int c = th + 64 * i, h = (c >> 3) & 63;     // 16-byte chunk c: of head h
+        const float w = h < hn ? load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + h) * up : 0.f;
         const uint4 x = reinterpret_cast<const uint4*>(sgsm + kSgOffQ)[c];
         const T* xv = reinterpret_cast<const T*>(&x);
         uint32_t hw[4], lw[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const float v0 = to_f32<T>(xv[2 * u]) * wv[i], v1 = to_f32<T>(xv[2 * u + 1]) * wv[i];
+          const float v0 = to_f32<T>(xv[2 * u]) * w, v1 = to_f32<T>(xv[2 * u + 1]) * w;
           const T a0 = from_f32<T>(v0), a1 = from_f32<T>(v1);
           hw[u] = sli_bits<T>(a0) | (sli_bits<T>(a1) << 16);
           lw[u] = sli_bits<T>(from_f32<T>(v0 - to_f32<T>(a0))) | (sli_bits<T>(from_f32<T>(v1 - to_f32<T>(a1))) << 16);
