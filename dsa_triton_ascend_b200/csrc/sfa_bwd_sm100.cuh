@@ -674,8 +674,7 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   f.rows = d.rows;
   f.sparse_count = d.sparse_count; f.sparse_block_size = d.sparse_block_size;
   const int64_t slots = (int64_t)p->sparse_count * p->sparse_block_size;
-  sfa_compact_kernel<<<(d.rows + 3) / 4, 128, 0, st>>>(f, nvalid, key_list, 1, (int32_t)slots, (int32_t)p->key_rows,
-                                                      redo, redo + d.rows, status);
+  sfa_compact_launch(f, nvalid, key_list, 1, (int32_t)slots, (int32_t)p->key_rows, redo, redo + d.rows, status, st);
   const int64_t pairs = (int64_t)d.rows * p->n1;
   sfa_bwd_delta_kernel<T><<<(unsigned)((pairs + 7) / 8), 256, 0, st>>>((const T*)p->d_out, (const T*)p->out, delta, bound,
                                                                       pairs, p->n1);
