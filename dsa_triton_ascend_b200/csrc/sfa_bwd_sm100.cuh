@@ -26,8 +26,8 @@
 //     scaled by 2^13, dS by a power of two per item that keeps |dS| <= scale * (|dO| |v| + |delta|)
 //     (Cauchy-Schwarz over the item's heads and all keys, taken by the pre-pass) below 2^13.
 //
-// Measured, B1 S1 512 S2 4096 N1 64 k 2048, bf16: 1.29 ms for the operator call (sfa_bwd_mma_kernel: 4.63
-// ms); 4092 rows x 128 heads: 7.6 ms (32.2 ms).  ncu: 3.4 TB/s of reductions, tensor pipe 22 % busy, the
+// Measured, B1 S1 512 S2 4096 N1 64 k 2048, bf16: 1.26 ms for the operator call (sfa_bwd_mma_kernel: 4.63
+// ms); 4092 rows x 128 heads: 7.1 ms (32.2 ms).  ncu: 3.4 TB/s of reductions, tensor pipe 22 % busy, the
 // load / store unit's data pipe - which a reduction of one line holds for 4.5 cycles - 66 % (77 % while
 // every SM has work).
 //
@@ -87,6 +87,9 @@ struct SfaBwdArgs {
   int32_t key_rows;
 };
 
+__device__ __forceinline__ void red_add(float* addr, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
+}
 __device__ __forceinline__ void red_add_if(bool on, float* addr, float v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p red.global.add.f32 [%0], %1;\n\t}\n" ::"l"(addr),
                "f"(v), "r"((int)on)
@@ -388,13 +391,23 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
           float* base = is_v ? a.p.dv_acc + m * 128 + f : a.p.dk_acc + (m - 4) * 128 + f;
           const float down = kScaled ? (is_v ? 1.f / 8192.f : dk_down) : 1.f;
           // one instruction = 32 features of one key = one full line
+          if (nv.x - t * kBwdBK >= kBwdBK) {                 // whole tile: no predicates
 #pragma unroll
-          for (int kb = 0; kb < kBwdBK; kb += 4) {
-            const int4 kr = rows4[kb / 4];
-            const int32_t r[4] = {kr.x, kr.y, kr.z, kr.w};
+            for (int kb = 0; kb < kBwdBK; kb += 4) {
+              const int4 kr = rows4[kb / 4];
+              const int32_t r[4] = {kr.x, kr.y, kr.z, kr.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              red_add_if(r[i] < a.key_rows, base + (int64_t)r[i] * width, kScaled ? v[kb + i] * down : v[kb + i]);
+              for (int i = 0; i < 4; ++i) red_add(base + (int64_t)r[i] * width, kScaled ? v[kb + i] * down : v[kb + i]);
+            }
+          } else {
+#pragma unroll
+            for (int kb = 0; kb < kBwdBK; kb += 4) {
+              const int4 kr = rows4[kb / 4];
+              const int32_t r[4] = {kr.x, kr.y, kr.z, kr.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                red_add_if(r[i] < a.key_rows, base + (int64_t)r[i] * width, kScaled ? v[kb + i] * down : v[kb + i]);
+            }
           }
         }
       }

@@ -536,10 +536,6 @@ __device__ __forceinline__ int sli_exponent(float m) {
   return (m > 0.f && m < INFINITY) ? max(-100, min(100, 13 - ilogbf(m))) : 0;
 }
 
-__device__ __forceinline__ void red_add(float* addr, float v) {
-  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
-}
-
 template <typename T>
 __device__ __forceinline__ uint32_t sli_bits(T v) { return (uint32_t)*reinterpret_cast<const uint16_t*>(&v); }
 
