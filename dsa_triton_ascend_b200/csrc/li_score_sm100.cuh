@@ -328,33 +328,37 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
       if (!ok) break;
       ++n_item;
-      // first key row of this lane's load of tile t
+      // First key rows of the loads of the `batch` tiles from t on: lane = tile * nsub + load.  One round of
+      // block-table look-ups serves them all, fetched a batch ahead (64 sequences x 2 rows x 41k keys: 174 us
+      // with a look-up per tile and one polling lane, 150 us = 4.5 TB/s).
+      const int batch = 32 / nsub;
       auto sub_row = [&](int32_t t) -> int32_t {
-        const int32_t p = t * kLiKeys + lane * a.sub_rows;
-        if (!paged) return (int32_t)item.krow0 + p;
+        const int32_t tile = t + lane / nsub;
+        const int32_t p = tile * kLiKeys + (lane % nsub) * a.sub_rows;
         const int32_t bi = p / sq.block_size;
-        if (lane >= nsub || bi >= sq.max_blocks) return a.krow_oob;
+        if (tile >= t1 || bi >= sq.max_blocks) return a.krow_oob;
         const int32_t blk = sq.block_table[(int64_t)item.b * sq.max_blocks + bi];
         if (blk < 0) return a.krow_oob;
         const int64_t r = (int64_t)blk * sq.block_size + (p - bi * sq.block_size);
         return r < (int64_t)a.krow_oob ? (int32_t)r : a.krow_oob;
       };
-      int32_t cur = sub_row(t0);
+      int32_t cur = sub_row(t0), nxt = cur;
+      int k = 0;                                   // tile within the batch
       for (int32_t t = t0; t < t1; ++t) {
-        const int32_t nxt = (t + 1 < t1) ? sub_row(t + 1) : 0;
-        if (lane == 0) ok = ptx::mbar_wait(&empty[s], (use & 1) ^ 1, abort_flag);
-        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        if (k == 0) nxt = sub_row(t + batch);      // (past the item: nothing is read)
+        // every lane polls (see ptx::mbar_wait_warp)
+        ok = ptx::mbar_wait_warp(&empty[s], (use & 1) ^ 1, abort_flag);
         if (!ok) break;
         if (lane == 0) ptx::mbar_arrive_expect_tx(&full[s], kLiKStage);
         for (int u = 0; u < nsub; ++u) {
-          const int32_t r = __shfl_sync(0xffffffffu, cur, u);
+          const int32_t r = __shfl_sync(0xffffffffu, cur, k * nsub + u);
           if (lane == 0) {
             unsigned char* dst = li_smem + li_stage_off(s) + u * a.sub_rows * 128;
             ptx::tma_load_2d(dst, &tmap_k, &full[s], 0, r);
             ptx::tma_load_2d(dst + kLiKBlock, &tmap_k, &full[s], 64, r);
           }
         }
-        cur = nxt;
+        if (++k == batch) { k = 0; cur = nxt; }
         if (++s == stages) { s = 0; ++use; }
       }
     }
@@ -448,6 +452,30 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           if (!ok) break;
           if (acc) ++n_use1; else ++n_use0;
           ptx::tc_fence_after();
+          if (kDense && item.nrows <= 2) {
+            // decode: one row per column half, so that all eight warps share the tile's two rows
+            // (64 sequences x 2 rows x 41k keys: 177.0 us with both rows on four of the warps, 174.5 us; 8 sequences x 1
+            // row: 15.1 and 13.7 us)
+            uint32_t r[64];
+            const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + acc * 256 + chalf * 64;
+            ptx::tmem_ld_x32(taddr, r);
+            ptx::tmem_ld_x32(taddr + 32, r + 32);
+            ptx::tmem_ld_wait();
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&tempty[acc]);
+            if (chalf < item.nrows) {
+              const float* w = w_s + chalf * kLiHeads;
+              float sa = 0.f, sb = 0.f;
+#pragma unroll
+              for (int g = 0; g < kLiHeads; g += 2) {
+                sa = fmaf(fmaxf(__uint_as_float(r[g]), 0.f), w[g], sa);
+                sb = fmaf(fmaxf(__uint_as_float(r[g + 1]), 0.f), w[g + 1], sb);
+              }
+              if (pos < vis[chalf]) a.scores[(int64_t)(row0 + chalf) * a.ld + pos] = sa + sb + 0.f;
+            }
+            continue;
+          }
           const int tok0 = h * kLiHalf + chalf * 2;
           // (rows that do not exist are computed as well and dropped by the `vis` test below: making
           // the loads conditional cost the full-size case 45 %)
