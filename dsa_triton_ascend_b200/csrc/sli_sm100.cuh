@@ -500,13 +500,16 @@ sli_mha_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid_c
 // without a conversion per element.  fp16: both are scaled by a power of two per row taken from the
 // row's largest magnitude.  dW = sum_k dI relu(S) is summed in fp32 registers.
 // Tensor memory: S 2 x 64 columns | dKI^T 2 x 128 | dQI^T 64.
-// Warps: 0..7 epilogue (lane quarter x 32 heads), 8..15 drain (lane quarter x 64 keys), 16..19 gather, 20
-// issuer, 21 QI loader, 22..23 w QI.
-constexpr int kSgThreads = 768, kSgDrainWarp0 = 8, kSgGatherWarp0 = 16, kSgGatherWarps = 4, kSgIssuer = 20, kSgLoader = 21;
-constexpr int kSgStager0 = 22;
+// Warps: 0..7 epilogue (lane quarter x 32 heads), 8..15 drain (lane quarter x 64 keys), 16..23 gather, 24
+// issuer of S / dKI, 25 issuer of dQI, 26..27 QI and w QI.  (A thread issues a product of 64 columns only every
+// 60-90 cycles, and a gather warp its lanes' loads one by one, ~180 cycles each: one issuer and four gather
+// warps took 3300 and 3000 cycles a tile.)
+constexpr int kSgThreads = 896, kSgDrainWarp0 = 8, kSgGatherWarp0 = 16, kSgGatherWarps = 8, kSgIssueA = 24, kSgIssueB = 25;
+constexpr int kSgStager0 = 26;
 // the epilogue and drain warps take the registers that the others give back
-constexpr int kSgLaunchRegs = 80, kSgRegsLow = 48, kSgRegsHigh = 96;
-static_assert((kSgRegsHigh - kSgLaunchRegs) * kSgGatherWarp0 <= (kSgLaunchRegs - kSgRegsLow) * (kSgThreads / 32 - kSgGatherWarp0),
+constexpr int kSgLaunchRegs = 72, kSgRegsLow = 48, kSgRegsDrain = 80, kSgRegsEpi = 96;
+static_assert((kSgRegsEpi - kSgLaunchRegs) * kSgDrainWarp0 + (kSgRegsDrain - kSgLaunchRegs) * (kSgGatherWarp0 - kSgDrainWarp0) <=
+                  (kSgLaunchRegs - kSgRegsLow) * (kSgThreads / 32 - kSgGatherWarp0),
               "setmaxnreg: more registers requested than released");
 static_assert(kSgLaunchRegs * kSgThreads <= 65536, "register file");
 constexpr int kSgStages = 3;
@@ -551,7 +554,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   uint64_t* s_full = bars + 6;      // [2] scores -> epilogue                             (commit)
   uint64_t* s_empty = bars + 8;     // [2] scores read                                    (8 warps)
   uint64_t* e_full = bars + 10;     // E, dI E, rows and dI of the tile stored            (8 warps)
-  uint64_t* e_empty = bars + 11;    // gradient products of the tile done                 (commit)
+  uint64_t* e_empty = bars + 11;    // gradient products of the tile done                 (commits A, B)
   uint64_t* d_full = bars + 12;     // [2] dKI^T -> drain                                 (commit)
   uint64_t* d_empty = bars + 14;    // [2] dKI^T read                                     (8 warps)
   uint64_t* q_full = bars + 16;     // QI landed                                          (tx bytes)
@@ -571,13 +574,13 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool misaligned = (ptx::smem_u32(sgsm) & 1023u) != 0;
   if (threadIdx.x == 0) {
-    const int counts[23] = {1, 1, 1, 1, 1, 1, 1, 1, 8, 8, 8, 1, 1, 1, 8, 8, 1, 3, 2, 1, 1, 8, 8};
+    const int counts[23] = {1, 1, 1, 1, 1, 1, 1, 1, 8, 8, 8, 2, 1, 1, 8, 8, 1, 3, 2, 1, 1, 8, 8};
 #pragma unroll
     for (int i = 0; i < 23; ++i) ptx::mbar_init(&bars[i], counts[i]);
     *abort_flag = misaligned ? 1 : 0;
     ptx::mbar_fence_init();
   }
-  if (warp == kSgIssuer) {
+  if (warp == kSgIssueA) {
     ptx::tmem_alloc(tmem_slot, 512);
     ptx::tmem_relinquish();
   }
@@ -592,11 +595,9 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
 
   // Each class of roles sits in its own branch, right under its setmaxnreg: the compiler budgets a
   // branch by the setmaxnreg that dominates it.
-  if (warp < kSgGatherWarp0) {
-   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSgRegsHigh));
-   if (*abort_flag) {
-    // nothing started
-   } else if (warp < kSgDrainWarp0) {
+  if (warp < kSgDrainWarp0) {
+   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSgRegsEpi));
+   if (!*abort_flag) {
     // -------------------------------------------------------------------- E and dI E, dW; then dQI
     const int quarter = warp & 3, half = warp >> 2;
     const int key = quarter * 32 + lane;                  // within the tile
@@ -728,7 +729,10 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       }
       ++n_item;
     }
-   } else {
+   }
+  } else if (warp < kSgGatherWarp0) {
+   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSgRegsDrain));
+   if (!*abort_flag) {
     // -------------------------------------------------------------------- drain: reductions of dKI^T
     const int quarter = warp & 3, k0 = ((warp - kSgDrainWarp0) >> 2) * 64;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + kSgTmK + k0;
@@ -787,7 +791,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSgRegsLow));
    if (*abort_flag) {
     // nothing started
-   } else if (warp < kSgIssuer) {
+   } else if (warp < kSgIssueA) {
     // -------------------------------------------------------------------- gather: 32 groups of 4 keys x 2 blocks
     const int o = (warp - kSgGatherWarp0) + kSgGatherWarps * lane;
     const bool active = o < 64;
@@ -824,15 +828,13 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         if (++stage == kSgStages) { stage = 0; ph ^= 1; }
       }
     }
-   } else if (warp == kSgIssuer) {
-    // -------------------------------------------------------------------- products: scores one tile ahead
+   } else if (warp == kSgIssueA) {
+    // -------------------------------------------------------------------- issuer A: scores one tile ahead, then dKI
     const uint64_t q_k = ptx::desc_kmajor_sw128(sm0 + kSgOffQ), k_k = ptx::desc_kmajor_sw128(sm0 + kSgOffK);
-    const uint64_t k_m = ptx::desc_mnmajor_sw128(sm0 + kSgOffK, kSlKBlk, 1024);
     const uint64_t w_m = ptx::desc_mnmajor_sw128(sm0 + kSgOffW, kSgHBlk, 1024);
     const uint64_t e_k = ptx::desc_kmajor_sw128(sm0 + kSgOffE);
-    const uint64_t de_m = ptx::desc_mnmajor_sw128(sm0 + kSgOffE + kSlKBlk, 0, 1024);
     uint32_t n_s = 0, n_g = 0, n_item = 0, ph_s = 0;
-    int st_s = 0, st_g = 0;
+    int st_s = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       const int32_t row = item / a.hchunks, h0 = (item - row * a.hchunks) * 64;
@@ -861,7 +863,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         }
         if (t > 0) {
           const int buf = n_g & 1;
-          if (t == 1) ok = wait(w_full, n_item & 1) && wait(dq_empty, (n_item & 1) ^ 1);
+          if (t == 1) ok = wait(w_full, n_item & 1);
           ok = ok && wait(e_full, n_g & 1) && wait(&d_empty[buf], ((n_g >> 1) & 1) ^ 1);
           if (!ok) break;
           ptx::tc_fence_after();
@@ -875,48 +877,53 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
               }
             }
             ptx::mma_commit(&d_full[buf]);
-#pragma unroll
-            for (int s = 0; s < 8; ++s)
-#pragma unroll
-              for (int lo = 0; lo < 2; ++lo)
-                ptx::mma_ss(tmem + kSgTmQ, k_m + ((st_g * 2 * kSlKBlk + s * 2048) >> 4),
-                            de_m + ((lo * kSlKBlk + s * 2048) >> 4), a.idesc_q, (t > 1 || s > 0 || lo > 0) ? 1u : 0u);
-            ptx::mma_commit(&k_empty[st_g]);
             ptx::mma_commit(e_empty);
-            if (t == ntiles) {
-              ptx::mma_commit(dq_full);
-              ptx::mma_commit(w_empty);
-            }
+            if (t == ntiles) ptx::mma_commit(w_empty);
           }
           __syncwarp();
           ++n_g;
-          if (++st_g == kSgStages) st_g = 0;
         }
       }
       ++n_item;
     }
-   } else if (warp == kSgLoader) {
-    // -------------------------------------------------------------------- QI (heads past the last: zeros)
-    uint32_t n_item = 0;
+   } else if (warp == kSgIssueB) {
+    // -------------------------------------------------------------------- issuer B: dQI
+    const uint64_t k_m = ptx::desc_mnmajor_sw128(sm0 + kSgOffK, kSlKBlk, 1024);
+    const uint64_t de_m = ptx::desc_mnmajor_sw128(sm0 + kSgOffE + kSlKBlk, 0, 1024);
+    uint32_t n_tile = 0, n_item = 0;
+    int stage = 0;
     bool ok = true;
-    if (lane == 0) ptx::prefetch_tmap(&tmap_q);
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hchunks, h0 = (item - row * a.hchunks) * 64;
       int32_t b;
-      if (sli_row_slots(a.p, row, &b) == 0) continue;
-      ok = wait(q_empty, (n_item & 1) ^ 1);
-      if (!ok) break;
-      if (lane == 0) {
-        ptx::mbar_arrive_expect_tx(q_full, 2 * kSgHBlk);
-        ptx::tma_load_3d(sgsm + kSgOffQ, &tmap_q, q_full, 0, h0, row);
-        ptx::tma_load_3d(sgsm + kSgOffQ + kSgHBlk, &tmap_q, q_full, 64, h0, row);
+      const int32_t ntiles = tiles_of(sli_row_slots(a.p, item / a.hchunks, &b));
+      if (ntiles == 0) continue;
+      ok = wait(dq_empty, (n_item & 1) ^ 1);
+      for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
+        // (E is there, so the scores of its keys are: the tile has landed)
+        ok = wait(e_full, n_tile & 1);
+        if (!ok) break;
+        ptx::tc_fence_after();
+        if (ptx::elect_one()) {
+          ptx::fence_proxy_async_smem();
+#pragma unroll
+          for (int s = 0; s < 8; ++s)
+#pragma unroll
+            for (int lo = 0; lo < 2; ++lo)
+              ptx::mma_ss(tmem + kSgTmQ, k_m + ((stage * 2 * kSlKBlk + s * 2048) >> 4),
+                          de_m + ((lo * kSlKBlk + s * 2048) >> 4), a.idesc_q, (t > 0 || s > 0 || lo > 0) ? 1u : 0u);
+          ptx::mma_commit(&k_empty[stage]);
+          ptx::mma_commit(e_empty);
+          if (t == ntiles - 1) ptx::mma_commit(dq_full);
+        }
+        __syncwarp();
+        if (++stage == kSgStages) stage = 0;
       }
-      __syncwarp();
       ++n_item;
     }
    } else {
-    // -------------------------------------------------------------------- w QI, high and low part
-    // (same place in its block as QI: the operand's layout is QI's)
+    // -------------------------------------------------------------------- QI (heads past the last: zeros), then
+    // w QI, high and low part (same place in its block as QI: the operand's layout is QI's)
+    if (warp == kSgStager0 && lane == 0) ptx::prefetch_tmap(&tmap_q);
     const int th = threadIdx.x - kSgStager0 * 32;         // 0..63
     uint32_t n_item = 0;
     bool ok = true;
@@ -925,6 +932,16 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       int32_t b;
       if (sli_row_slots(a.p, row, &b) == 0) continue;
       const int32_t hn = min(64, g - h0);
+      if (warp == kSgStager0) {
+        ok = wait(q_empty, (n_item & 1) ^ 1);
+        if (!ok) break;
+        if (lane == 0) {
+          ptx::mbar_arrive_expect_tx(q_full, 2 * kSgHBlk);
+          ptx::tma_load_3d(sgsm + kSgOffQ, &tmap_q, q_full, 0, h0, row);
+          ptx::tma_load_3d(sgsm + kSgOffQ + kSgHBlk, &tmap_q, q_full, 64, h0, row);
+        }
+        __syncwarp();
+      }
       ok = wait(q_full, n_item & 1);
       if (!ok) break;
       int e = 0;
@@ -984,7 +1001,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   }
   ptx::tc_fence_before();
   __syncthreads();
-  if (warp == kSgIssuer) {
+  if (warp == kSgIssueA) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, 512);
   }
