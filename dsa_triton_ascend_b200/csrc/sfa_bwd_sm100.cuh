@@ -625,6 +625,9 @@ inline int64_t sfa_bwd_rows(const DsaSfaGradParams* p) {
 }
 inline bool sfa_bwd_sm100_eligible(const DsaSfaGradParams* p) {
   if (p->d != 512 || p->d_rope != 64 || p->kernel == DSA_KERNEL_PORTABLE) return false;
+  // (fewer than 16 heads fill one 16-head block of the mma.sync kernel, which needs no lists beside its
+  // accumulators; a block of 64 heads would be mostly padding)
+  if (p->n1 < 16) return false;
   if (((uintptr_t)p->query | (uintptr_t)p->query_rope | (uintptr_t)p->key | (uintptr_t)p->key_rope |
        (uintptr_t)p->d_out | (uintptr_t)p->out) & 15u)
     return false;
