@@ -373,8 +373,8 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status,
   d.p_buf = reinterpret_cast<float*>(ws + buf_bytes);
   d.loss_parts = reinterpret_cast<float*>(ws + 2 * buf_bytes);
   float* stats = reinterpret_cast<float*>((char*)d.loss_parts + align256((size_t)rows * 4));
-  d.di_max = reinterpret_cast<float*>((char*)stats + align256((size_t)rows * 8));
-  d.dki_acc = reinterpret_cast<float*>((char*)d.di_max + align256((size_t)rows * 4));
+  d.di_max = stats;    // (takes the place of a row's index maximum, which nobody reads once its dI is written)
+  d.dki_acc = reinterpret_cast<float*>((char*)stats + align256((size_t)rows * 8));
   d.stats_given = (p->dense && p->softmax_max_index) ? 1 : 0;
   d.index_max = d.stats_given ? const_cast<float*>(p->softmax_max_index) : stats;
   d.index_sum = d.stats_given ? const_cast<float*>(p->softmax_sum_index) : stats + rows;
@@ -708,7 +708,7 @@ int dsa_sli_grad_workspace_bytes(const DsaSliGradParams* p, size_t* out_bytes) {
   if (!out_bytes) return DSA_ERR_NULL;
   const size_t rows = (size_t)p->batch * p->s1;
   *out_bytes = kWorkspaceHeader + 2 * align256(rows * (size_t)sli_slots(p) * 4) + align256(rows * 4) +
-               align256(rows * 8) + align256(rows * 4) + (size_t)p->batch * p->s2 * p->d_idx * 4;
+               align256(rows * 8) + (size_t)p->batch * p->s2 * p->d_idx * 4;
   return DSA_OK;
 }
 
