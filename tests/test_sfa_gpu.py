@@ -378,3 +378,22 @@ def test_sfa_rows_whose_scores_outgrow_the_first_tile_are_exact(dtype, boost, K)
     finally:
         sfa.set_kernel("auto")
     _compare(host(got[0]), host(got[1]), host(got[2]), ref[0], ref[1], ref[2], dtype)
+
+
+@pytest.mark.parametrize("K", [4, 2048, 2052, 4096])
+def test_the_pre_pass_by_blocks_lists_what_the_pre_pass_by_warps_lists(K):
+    """Few rows of 16-byte aligned indices are compacted by one block per row; a further column of -1 makes the
+    rows unaligned (one warp per row) and changes nothing else: the outputs agree bit for bit."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_triton
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(torch.bfloat16)
+    S1, S2 = 40, 5000     # (with fewer rows their lists are split, and where depends on the number of columns)
+    q, k, qr, kr = r(1, S1, 16, 512), r(1, S2, 1, 512), r(1, S1, 16, 64), r(1, S2, 1, 64)
+    idx = torch.stack([torch.randperm(S2, generator=gen, device="cuda")[:K] for _ in range(S1)]).int()
+    idx[torch.rand(S1, K, generator=gen, device="cuda") < 0.3] = -1
+    idx[3] = -1
+    wide = torch.cat([idx, torch.full((S1, 1), -1, dtype=torch.int32, device="cuda")], 1)
+    a, b = (sparse_flash_attention_triton(q, k, k, i.view(1, S1, 1, -1), scale_value=0.04, query_rope=qr, key_rope=kr,
+                                          sparse_mode=0, return_softmax_lse=True) for i in (idx, wide))
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)

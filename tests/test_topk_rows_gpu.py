@@ -87,3 +87,16 @@ def test_constructed_rows_fp16():
     exp_i, exp_v = _expected(values, K)
     np.testing.assert_array_equal(got_i, exp_i)
     np.testing.assert_array_equal(got_v, exp_v)
+
+
+def test_a_row_whose_sampled_scores_mislead_is_counted_again():
+    """Rows of 16384 keys or more count only the bins that a sample of 512 positions puts the best K in; a row
+    whose sampled positions hold its only large scores has fewer than K keys there."""
+    S2, K = 20000, 2048
+    rng = np.random.RandomState(5)
+    v = _bf16(rng.randn(S2))
+    v[(np.arange(512) * S2) >> 9] = _bf16(8.0 + np.abs(rng.randn(512)))
+    got_i, got_v = _run(v[None], K)
+    exp_i, exp_v = _expected(v[None], K)
+    np.testing.assert_array_equal(got_i, exp_i)
+    np.testing.assert_array_equal(got_v + 0.0, exp_v + 0.0)
