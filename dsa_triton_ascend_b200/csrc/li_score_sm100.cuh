@@ -228,11 +228,32 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     // count of chunks per group.  The static round-robin over this list leaves the CTAs within one
     // chunk of each other, where the (chunk, group) grid leaves them with whatever mix of full,
     // partial and empty chunks the sequence lengths produce.
-    if (threadIdx.x == 0) {
-      int64_t total = 0;
-      for (int g = 0; g < a.groups; ++g) total += cum_s[g + 1];
+    if (warp == 0) {
+      int32_t mine = 0;
+      for (int g = lane; g < a.groups; g += 32) mine += cum_s[g + 1];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+      const int64_t total = mine;
       int64_t ct = (total + 8ll * grid - 1) / (8ll * grid);
+      if (a.stages == kLiStages) {
+        // Groups of up to eight rows load 128 KB of Q per chunk, about three tiles' time that nothing hides: the
+        // chunk size with the least rounds x (tiles + 3), a lane per candidate (512 rows x 4096 keys: 60 us with
+        // eight tiles per chunk, 52 us with sixteen)
+        const int32_t unit = (int32_t)((total + 16ll * grid - 1) / (16ll * grid));
+        const int32_t cand = max(8, unit * (lane + 1));
+        int32_t chunks = 0;
+        for (int g = 0; g < a.groups; ++g) chunks += (cum_s[g + 1] + cand - 1) / cand;
+        const uint64_t cost = (uint64_t)((chunks + grid - 1) / grid) * (uint64_t)(cand + 3);
+        uint64_t best = cost * 32 + lane;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const uint64_t other = __shfl_xor_sync(0xffffffffu, best, o);
+          best = other < best ? other : best;
+        }
+        ct = max(8, unit * ((int32_t)(best & 31) + 1));
+      }
       if (ct < 8) ct = 8;
+     if (lane == 0) {
       int32_t acc = 0;
       cum_s[0] = 0;
       for (int g = 0; g < a.groups; ++g) {
@@ -240,6 +261,7 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         cum_s[g + 1] = acc;
       }
       cum_s[kLiDenseGroups + 1] = (int32_t)ct;
+     }
     }
     __syncthreads();
   }
