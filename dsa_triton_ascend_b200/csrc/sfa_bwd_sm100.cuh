@@ -79,7 +79,7 @@ struct SfaBwdArgs {
   SfaGradDev p;
   int32_t* status;
   const int2* nvalid;        // [rows] .x slots that take part, .y first entry in key_list
-  const int32_t* key_list;   // [rows, slots] their key rows, front-packed
+  const int32_t* key_list;   // [rows, slots] their key rows, front-packed, all in [0, key_rows)
   const float* delta;        // [rows, n1]
   const float* bound;        // fp16: [0] largest key norm, [4 + 2 row] largest |dO|, [5 + 2 row] largest |delta|
   uint32_t idesc_s, idesc_q, idesc_d;
@@ -391,7 +391,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
           float* base = is_v ? a.p.dv_acc + m * 128 + f : a.p.dk_acc + (m - 4) * 128 + f;
           const float down = kScaled ? (is_v ? 1.f / 8192.f : dk_down) : 1.f;
           // one instruction = 32 features of one key = one full line
-          if (nv.x - t * kBwdBK >= kBwdBK) {                 // whole tile: no predicates
+          if (nv.x - t * kBwdBK >= kBwdBK) {                 // whole tile of existing rows: no predicates
 #pragma unroll
             for (int kb = 0; kb < kBwdBK; kb += 4) {
               const int4 kr = rows4[kb / 4];
@@ -690,7 +690,8 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   f.rows = d.rows;
   f.sparse_count = d.sparse_count; f.sparse_block_size = d.sparse_block_size;
   const int64_t slots = (int64_t)p->sparse_count * p->sparse_block_size;
-  sfa_compact_launch(f, nvalid, key_list, 1, (int32_t)slots, (int32_t)p->key_rows, redo, redo + d.rows, status, st);
+  // (slots without a row are left out: the reductions of a whole tile go to every listed row unchecked)
+  sfa_compact_launch(f, nvalid, key_list, 1, (int32_t)slots, (int32_t)p->key_rows, -1, redo, redo + d.rows, status, st);
   const int64_t pairs = (int64_t)d.rows * p->n1;
   sfa_bwd_delta_kernel<T><<<(unsigned)((pairs + 7) / 8), 256, 0, st>>>((const T*)p->d_out, (const T*)p->out, delta, bound,
                                                                       pairs, p->n1);

@@ -149,13 +149,14 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi, int is_bf16) {
 }
 
 // Pre-pass: one warp per query row.  Writes the physical KV rows of the slots that take part, in
-// slot order, and their count.  A slot whose paged block is absent inside the valid length takes
-// part as a zero row, like the reference's un-paged cache
-// (sparse_flash_attention_triton.py:1012-1033): it gets the row number `oob_row` (= the number of
-// KV rows), which the gather loads as zeros.
+// slot order, and their count.  A slot whose paged block is absent inside the valid length (or whose row
+// lies past the KV tensor) gets the row number `absent`.  Forward: the number of KV rows, which the gather
+// loads as zeros - the slot takes part as a zero row, like the reference's un-paged cache
+// (sparse_flash_attention_triton.py:1012-1033).  Backward: -1, the slot is left out (it has no row to carry a
+// gradient to, and the list then names existing rows only).
 __global__ void __launch_bounds__(128) sfa_compact_kernel(SfaDev p, int2* __restrict__ nvalid,
                                                           int32_t* __restrict__ key_list, int32_t split,
-                                                          int32_t part_keys, int32_t oob_row,
+                                                          int32_t part_keys, int32_t kv_rows, int32_t absent,
                                                           int32_t* __restrict__ redo,
                                                           int32_t* __restrict__ redo_count,
                                                           int32_t* __restrict__ status) {
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(128) sfa_compact_kernel(SfaDev p, int2* __rest
           if (tok >= 0 && tok < ri.threshold && tok < ri.act_k &&
               (p.seq.layout_k == DSA_LAYOUT_PA_BSND || tok < p.seq.s2)) {
             r = key_row(p.seq, ri, (int32_t)tok);
-            if (r < 0 || r >= oob_row) r = oob_row;
+            if (r < 0 || r >= kv_rows) r = absent;
           }
           prow[u][e] = (int32_t)r;
         }
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(128) sfa_compact_kernel(SfaDev p, int2* __rest
         const int32_t tok = sfa_slot_token(p, ri, idx_row, j);
         if (tok >= 0) {
           prow = key_row(p.seq, ri, tok);
-          if (prow < 0 || prow >= oob_row) prow = oob_row;
+          if (prow < 0 || prow >= kv_rows) prow = absent;
         }
       }
       const uint32_t m = __ballot_sync(0xffffffffu, prow >= 0);
@@ -256,7 +257,7 @@ inline bool sfa_compact_by_blocks(const SfaDev& p) {
 }
 __global__ void __launch_bounds__(256) sfa_compact_block_kernel(SfaDev p, int2* __restrict__ nvalid,
                                                                 int32_t* __restrict__ key_list, int32_t split,
-                                                                int32_t part_keys, int32_t oob_row,
+                                                                int32_t part_keys, int32_t kv_rows, int32_t absent,
                                                                 int32_t* __restrict__ redo,
                                                                 int32_t* __restrict__ redo_count,
                                                                 int32_t* __restrict__ status) {
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(256) sfa_compact_block_kernel(SfaDev p, int2* 
           if (tok >= 0 && tok < ri.threshold && tok < ri.act_k &&
               (p.seq.layout_k == DSA_LAYOUT_PA_BSND || tok < p.seq.s2)) {
             r = key_row(p.seq, ri, (int32_t)tok);
-            if (r < 0 || r >= oob_row) r = oob_row;
+            if (r < 0 || r >= kv_rows) r = absent;
           }
           prow[u][e] = (int32_t)r;
         }
@@ -333,13 +334,14 @@ __global__ void __launch_bounds__(256) sfa_compact_block_kernel(SfaDev p, int2* 
                                                            (int32_t)((int64_t)row * slots + threadIdx.x * part_keys));
 }
 inline void sfa_compact_launch(const SfaDev& d, int2* nvalid, int32_t* key_list, int32_t split, int32_t part_keys,
-                               int32_t oob_row, int32_t* redo, int32_t* redo_count, int32_t* status, cudaStream_t st) {
+                               int32_t kv_rows, int32_t absent, int32_t* redo, int32_t* redo_count, int32_t* status,
+                               cudaStream_t st) {
   if (sfa_compact_by_blocks(d))
-    sfa_compact_block_kernel<<<d.rows, 256, 0, st>>>(d, nvalid, key_list, split, part_keys, oob_row, redo, redo_count,
-                                                    status);
+    sfa_compact_block_kernel<<<d.rows, 256, 0, st>>>(d, nvalid, key_list, split, part_keys, kv_rows, absent, redo,
+                                                    redo_count, status);
   else
-    sfa_compact_kernel<<<(d.rows + 3) / 4, 128, 0, st>>>(d, nvalid, key_list, split, part_keys, oob_row, redo, redo_count,
-                                                        status);
+    sfa_compact_kernel<<<(d.rows + 3) / 4, 128, 0, st>>>(d, nvalid, key_list, split, part_keys, kv_rows, absent, redo,
+                                                        redo_count, status);
 }
 
 // Development aid, compiled only with -DDSA_SFA_PROFILE: cycle sums per role of the first cluster
@@ -1193,7 +1195,8 @@ inline int sfa_sm100_launch(const DsaSfaParams* p, const SfaDev& d, int32_t* sta
   int32_t* redo = reinterpret_cast<int32_t*>((char*)scratch + w.redo);
   int32_t* redo_list = reinterpret_cast<int32_t*>((char*)scratch + w.redo_list);
   int32_t* redo_count = reinterpret_cast<int32_t*>((char*)scratch + w.redo_count);
-  sfa_compact_launch(d, nvalid, key_list, split, part_keys, (int32_t)p->key_rows, redo, redo_count, status, st);
+  sfa_compact_launch(d, nvalid, key_list, split, part_keys, (int32_t)p->key_rows, (int32_t)p->key_rows, redo, redo_count,
+                     status, st);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
   SfaSm100Args a;

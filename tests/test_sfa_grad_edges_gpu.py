@@ -1,0 +1,49 @@
+"""Attention backward where its inputs leave the ordinary: selected keys that do not exist, keys and heads whose
+values are far from the others', rows without statistics.  Each call is compared with one that has to give the
+same result, or with the numpy oracle."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle.compare import sfa_grad_acceptance_rule
+from tests.util import host, tdtype
+
+pytestmark = pytest.mark.gpu
+NAMES = ("d_query", "d_key", "d_value", "d_query_rope", "d_key_rope")
+
+
+def _randn(seed, *shape, dtype, scale=0.3):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device="cuda") * scale).to(dtype)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("N1,K", [(64, 160), (16, 160), (64, 161)])   # 161: rows off their 16-byte boundaries
+def test_selected_keys_past_the_key_tensor_take_no_part(N1, K, dtype):
+    """TND key lengths that overrun the tensor: a slot that names a row which does not exist is as good as an
+    unused one (-1), in whole tiles of keys too."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_grad_triton
+    dt = tdtype(dtype)
+    T1, T2, ends_q, ends_k = 6, 100, [2, 6], [60, 200]       # keys 40.. of the second sequence do not exist
+    q, qr = _randn(1, T1, N1, 512, dtype=dt), _randn(2, T1, N1, 64, dtype=dt)
+    k, kr = _randn(3, T2, 1, 512, dtype=dt), _randn(4, T2, 1, 64, dtype=dt)
+    do, out = _randn(5, T1, N1, 512, dtype=dt), _randn(6, T1, N1, 512, dtype=dt)
+    mx, sm = torch.zeros(1, T1, N1, device="cuda"), torch.full((1, T1, N1), 150.0, device="cuda")
+    rng = np.random.RandomState(7)
+    idx = np.full((T1, 1, K), -1, np.int32)
+    for t in range(T1):
+        n = 60 if t < 2 else 140
+        idx[t, 0, :n] = rng.permutation(n)
+    exists = idx.copy()
+    exists[2:][exists[2:] >= 40] = -1
+    kw = dict(scale_value=1.0 / 24.0, query_rope=qr, key_rope=kr, actual_seq_lengths_query=ends_q,
+              actual_seq_lengths_kv=ends_k, layout="TND", sparse_mode=0)
+    got = sparse_flash_attention_grad_triton(q, k, k, torch.from_numpy(idx).cuda(), do, out, mx, sm, **kw)
+    ref = sparse_flash_attention_grad_triton(q, k, k, torch.from_numpy(exists).cuda(), do, out, mx, sm, **kw)
+    for n, a, b in zip(NAMES, got, ref):
+        if n.startswith("d_query"):
+            assert torch.equal(a, b), n
+        else:                       # (reductions arrive in any order: one rounding of the output apart)
+            sfa_grad_acceptance_rule(host(a), host(b), dtype, name=n, ulps=1.0)
