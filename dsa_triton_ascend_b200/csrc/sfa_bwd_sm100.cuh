@@ -23,8 +23,8 @@
 //     the layout the score product uses.
 //   * P and dS are fp32 values that enter their products as a high and a low io-dtype part
 //     (x = hi + lo up to 2^-16 relative for bf16, 2^-22 for fp16), as in sfa_bwd_mma_kernel.  fp16: P is
-//     scaled by 2^13, dS by a power of two per item that keeps |dS| <= scale * (|dO| |v| + |delta|)
-//     (Cauchy-Schwarz over the item's heads and all keys, taken by the pre-pass) below 2^13.
+//     scaled by 2^13, dS by a power of two per row that keeps |dS| <= scale * (|dO| |v| + |delta|)
+//     (Cauchy-Schwarz over the row's heads and selected keys, taken by small kernels in front) below 2^13.
 //
 // Measured, B1 S1 512 S2 4096 N1 64 k 2048, bf16: 1.26 ms for the operator call (sfa_bwd_mma_kernel: 4.63
 // ms); 4092 rows x 128 heads: 7.1 ms (32.2 ms).  ncu: 3.4 TB/s of reductions, tensor pipe 22 % busy, the
@@ -81,7 +81,7 @@ struct SfaBwdArgs {
   const int2* nvalid;        // [rows] .x slots that take part, .y first entry in key_list
   const int32_t* key_list;   // [rows, slots] their key rows, front-packed, all in [0, key_rows)
   const float* delta;        // [rows, n1]
-  const float* bound;        // fp16: [0] largest key norm, [4 + 2 row] largest |dO|, [5 + 2 row] largest |delta|
+  const int32_t* exps;       // fp16: [rows] exponent of the power of two that the row's dS is scaled by
   uint32_t idesc_s, idesc_q, idesc_d;
   int32_t items, hblocks;    // rows * hblocks
   int32_t key_rows;
@@ -127,39 +127,56 @@ __global__ void __launch_bounds__(256) sfa_bwd_delta_kernel(const T* __restrict_
     delta[i] = s;
     if (bound != nullptr) {   // (non-negative floats order like their bit patterns)
       const int64_t row = i / n1;
-      atomicMax(reinterpret_cast<int*>(bound + 4 + 2 * row), __float_as_int(sqrtf(n)));
-      atomicMax(reinterpret_cast<int*>(bound + 5 + 2 * row), __float_as_int(fabsf(s)));
+      atomicMax(reinterpret_cast<int*>(bound + 2 * row), __float_as_int(sqrtf(n)));
+      atomicMax(reinterpret_cast<int*>(bound + 2 * row + 1), __float_as_int(fabsf(s)));
     }
   }
 }
 
-// fp16: largest norm of the value part of a key.
+// fp16: norm of the value part of each key, a warp per key.
 template <typename T>
-__global__ void __launch_bounds__(256) sfa_bwd_key_norm_kernel(const T* __restrict__ key, float* __restrict__ bound,
+__global__ void __launch_bounds__(256) sfa_bwd_key_norm_kernel(const T* __restrict__ key, float* __restrict__ norms,
                                                                int64_t key_rows) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  float best = 0.f;
-  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < key_rows; r += (int64_t)gridDim.x * 8) {
-    float n = 0.f;
+  if (r >= key_rows) return;
+  float n = 0.f;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const uint4 a = reinterpret_cast<const uint4*>(key + r * 512)[lane + 32 * u];
-      const T* av = reinterpret_cast<const T*>(&a);
+  for (int u = 0; u < 2; ++u) {
+    const uint4 a = reinterpret_cast<const uint4*>(key + r * 512)[lane + 32 * u];
+    const T* av = reinterpret_cast<const T*>(&a);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { const float x = to_f32<T>(av[e]); n = fmaf(x, x, n); }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    best = fmaxf(best, n);
+    for (int e = 0; e < 8; ++e) { const float x = to_f32<T>(av[e]); n = fmaf(x, x, n); }
   }
-  if (lane == 0) atomicMax(reinterpret_cast<int*>(bound), __float_as_int(sqrtf(best)));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+  if (lane == 0) norms[r] = sqrtf(n);
 }
 
-// fp16: exponent of the power of two that dS of a row is scaled by.
-__device__ __forceinline__ int sfa_bwd_exponent(const SfaBwdArgs& a, int32_t row) {
-  const float b = a.p.scale * (a.bound[4 + 2 * row] * a.bound[0] + a.bound[5 + 2 * row]);
-  if (!(fabsf(b) > 0.f) || !(fabsf(b) < INFINITY)) return 0;
-  return max(-100, min(100, 12 - ilogbf(fabsf(b))));
+// fp16: the row's exponent, a block per row.  Only the keys that the row selected count: what a key tensor
+// holds elsewhere (padding past the valid lengths, keys of other sequences) may be anything.
+__global__ void __launch_bounds__(256) sfa_bwd_exponent_kernel(const int2* __restrict__ nvalid,
+                                                               const int32_t* __restrict__ key_list,
+                                                               const float* __restrict__ norms,
+                                                               const float* __restrict__ bound,
+                                                               int32_t* __restrict__ exps, float scale) {
+  __shared__ float red[8];
+  const int32_t row = blockIdx.x;
+  const int2 nv = nvalid[row];
+  const int32_t* list = key_list + nv.y;
+  float m = 0.f;
+#pragma unroll 8
+  for (int32_t j = threadIdx.x; j < nv.x; j += 256) m = fmaxf(m, norms[list[j]]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w]);
+    const float b = fabsf(scale) * fmaf(bound[2 * row], m, bound[2 * row + 1]);
+    exps[row] = b > 0.f && b < INFINITY ? max(-100, min(100, 12 - ilogbf(b))) : 0;
+  }
 }
 
 template <typename T>
@@ -249,7 +266,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
             c0 = a.delta[hi_];
           }
         }
-        if constexpr (kScaled) up = is_s ? 8192.f : scalbnf(1.f, sfa_bwd_exponent(a, row));
+        if constexpr (kScaled) up = is_s ? 8192.f : scalbnf(1.f, a.exps[row]);
         for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
           const uint32_t ph = n_tile & 1;
           ok = wait(s_full, ph);
@@ -316,7 +333,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
       }
       // dQ^T tile m: this thread's feature is m * 128 + quarter * 32 + lane, a column is a head
       float down = 1.f;
-      if constexpr (kScaled) { if (ntiles > 0) down = scalbnf(1.f, -sfa_bwd_exponent(a, row)); }
+      if constexpr (kScaled) { if (ntiles > 0) down = scalbnf(1.f, -a.exps[row]); }
       const int32_t hn = min(kBwdHeads, n1 - h0);
 #pragma unroll 1
       for (int m = half; m < 5; m += 2) {
@@ -364,7 +381,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
       const int2 nv = a.nvalid[row];
       const int32_t ntiles = tiles_of(nv.x);
       float dk_down = 1.f;
-      if constexpr (kScaled) { if (ntiles > 0) dk_down = scalbnf(1.f, -sfa_bwd_exponent(a, row)); }
+      if constexpr (kScaled) { if (ntiles > 0) dk_down = scalbnf(1.f, -a.exps[row]); }
       for (int32_t t = 0; t < ntiles && ok; ++t) {
         const int4* rows4 = reinterpret_cast<const int4*>(rows_s + rbuf * kBwdBK);
         rbuf = rbuf == 2 ? 0 : rbuf + 1;
@@ -636,17 +653,20 @@ inline bool sfa_bwd_sm100_eligible(const DsaSfaGradParams* p) {
   if (rows < 1 || rows * ((p->n1 + kBwdHeads - 1) / kBwdHeads) >= (1ll << 31)) return false;
   return rows * p->sparse_count * p->sparse_block_size < (1ll << 31);    // key_list offsets are int32
 }
-// Workspace: header | dk / dv accumulators | bounds (fp16) - zeroed before the call - | nvalid |
-// delta | redo flags and count of the pre-pass (unused) | key_list
-struct SfaBwdWs { size_t acc, bound, zeroed, nvalid, delta, redo, key_list, total; };
+// Workspace: header | dk / dv accumulators | fp16: bounds of the rows - zeroed before the call - | fp16: exponents of
+// the rows, norms of the keys | nvalid | delta | redo flags and count of the pre-pass (unused) | key_list
+struct SfaBwdWs { size_t acc, bound, zeroed, exps, norms, nvalid, delta, redo, key_list, total; };
 inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   const size_t rows = (size_t)sfa_bwd_rows(p);
   SfaBwdWs w;
   w.acc = header;
   w.bound = w.acc + up((size_t)p->key_rows * (size_t)(2 * p->d + p->d_rope) * sizeof(float));
-  w.zeroed = w.bound + (p->dtype == DSA_DTYPE_FP16 ? up((rows * 2 + 4) * 4) : 0);
-  w.nvalid = w.zeroed;
+  const bool fp16 = p->dtype == DSA_DTYPE_FP16;
+  w.zeroed = w.bound + (fp16 ? up(rows * 2 * 4) : 0);
+  w.exps = w.zeroed;
+  w.norms = w.exps + (fp16 ? up(rows * 4) : 0);
+  w.nvalid = w.norms + (fp16 ? up((size_t)p->key_rows * 4) : 0);
   w.delta = w.nvalid + up(rows * 8);
   w.redo = w.delta + up(rows * p->n1 * 4);
   w.key_list = w.redo + up(rows * 4) + 256;
@@ -683,6 +703,8 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   int32_t* key_list = (int32_t*)(ws + w.key_list);
   float* delta = (float*)(ws + w.delta);
   float* bound = bf16 ? nullptr : (float*)(ws + w.bound);
+  int32_t* exps = (int32_t*)(ws + w.exps);
+  float* norms = (float*)(ws + w.norms);
   int32_t* redo = (int32_t*)(ws + w.redo);
   SfaDev f = {};
   f.seq = d.seq;
@@ -695,15 +717,16 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   const int64_t pairs = (int64_t)d.rows * p->n1;
   sfa_bwd_delta_kernel<T><<<(unsigned)((pairs + 7) / 8), 256, 0, st>>>((const T*)p->d_out, (const T*)p->out, delta, bound,
                                                                       pairs, p->n1);
-  if (!bf16)
-    sfa_bwd_key_norm_kernel<T><<<(unsigned)std::min<int64_t>((p->key_rows + 7) / 8, sms * 4), 256, 0, st>>>(
-        (const T*)p->key, bound, p->key_rows);
+  if (!bf16) {
+    sfa_bwd_key_norm_kernel<T><<<(unsigned)((p->key_rows + 7) / 8), 256, 0, st>>>((const T*)p->key, norms, p->key_rows);
+    sfa_bwd_exponent_kernel<<<d.rows, 256, 0, st>>>(nvalid, key_list, norms, bound, exps, p->scale);
+  }
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
-  count_launch(bf16 ? 2 : 3);
+  count_launch(bf16 ? 2 : 4);
   SfaBwdArgs a;
   a.p = d;
   a.status = status;
-  a.nvalid = nvalid; a.key_list = key_list; a.delta = delta; a.bound = bound;
+  a.nvalid = nvalid; a.key_list = key_list; a.delta = delta; a.exps = exps;
   const uint32_t fmt = bf16 ? 1u : 0u;
   a.idesc_s = ptx::idesc_f16(fmt, 128, kBwdBK, 0, 0);
   a.idesc_q = ptx::idesc_f16(fmt, 128, kBwdHeads, 1, 1);

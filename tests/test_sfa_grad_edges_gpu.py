@@ -47,3 +47,38 @@ def test_selected_keys_past_the_key_tensor_take_no_part(N1, K, dtype):
             assert torch.equal(a, b), n
         else:                       # (reductions arrive in any order: one rounding of the output apart)
             sfa_grad_acceptance_rule(host(a), host(b), dtype, name=n, ulps=1.0)
+
+
+def _fp16_case(seed, S1, S2, N1, K, valid, do_scale):
+    """BSND inputs of which keys 0..valid-1 are in use, and forward statistics that fit them."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_triton
+    dt = torch.float16
+    q, qr = _randn(seed, 1, S1, N1, 512, dtype=dt), _randn(seed + 1, 1, S1, N1, 64, dtype=dt)
+    k, kr = _randn(seed + 2, 1, S2, 1, 512, dtype=dt), _randn(seed + 3, 1, S2, 1, 64, dtype=dt)
+    do = _randn(seed + 4, 1, S1, N1, 512, dtype=dt, scale=do_scale)
+    rng = np.random.RandomState(seed)
+    idx = torch.from_numpy(np.stack([rng.permutation(valid)[:K] for _ in range(S1)]).astype(np.int32)).cuda()
+    kw = dict(scale_value=1.0 / 24.0, query_rope=qr, key_rope=kr, actual_seq_lengths_kv=[valid], sparse_mode=0)
+    idx = idx.view(1, S1, 1, K)
+    out, mx, sm = sparse_flash_attention_triton(q, k, k, idx, return_softmax_lse=True, **kw)
+    return q, k, idx, do, out, mx, sm, kw
+
+
+@pytest.mark.parametrize("do_scale", [0.3, 1e-3])
+@pytest.mark.parametrize("what", [1e3, 65504.0, math.inf, math.nan])
+def test_fp16_gradients_do_not_depend_on_keys_that_nobody_selected(what, do_scale):
+    """Large, infinite or undefined values in padding rows and in one visible, unselected key change nothing: d_query
+    stays the same bit for bit, the scattered gradients up to the order of their sums."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_grad_triton
+    q, k, idx, do, out, mx, sm, kw = _fp16_case(21, 5, 300, 64, 100, 260, do_scale)
+    idx[idx == 11] = -1
+    ref = sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)
+    foreign = k.clone()
+    foreign[:, 260:] = what
+    foreign[:, 11] = what
+    got = sparse_flash_attention_grad_triton(q, foreign, foreign, idx, do, out, mx, sm, **kw)
+    for n, a, b in zip(NAMES, got, ref):
+        if n.startswith("d_query"):
+            assert torch.equal(a, b), n
+        else:
+            sfa_grad_acceptance_rule(host(a), host(b), "fp16", name=n, ulps=1.0)
