@@ -23,8 +23,8 @@
 //     the layout the score product uses.
 //   * P and dS are fp32 values that enter their products as a high and a low io-dtype part
 //     (x = hi + lo up to 2^-16 relative for bf16, 2^-22 for fp16), as in sfa_bwd_mma_kernel.  fp16: P is
-//     scaled by 2^13, dS by a power of two per row that keeps |dS| <= scale * (|dO| |v| + |delta|)
-//     (Cauchy-Schwarz over the row's heads and selected keys, taken by small kernels in front) below 2^13.
+//     scaled by 2^13, dS by a power of two per item that keeps |dS| <= scale * (|dO| |v| + |delta|)
+//     (Cauchy-Schwarz over the item's heads and selected keys, taken by small kernels in front) below 2^13.
 //
 // Measured, B1 S1 512 S2 4096 N1 64 k 2048, bf16: 1.26 ms for the operator call (sfa_bwd_mma_kernel: 4.63
 // ms); 4092 rows x 128 heads: 7.1 ms (32.2 ms).  ncu: 3.4 TB/s of reductions, tensor pipe 22 % busy, the
@@ -81,7 +81,7 @@ struct SfaBwdArgs {
   const int2* nvalid;        // [rows] .x slots that take part, .y first entry in key_list
   const int32_t* key_list;   // [rows, slots] their key rows, front-packed, all in [0, key_rows)
   const float* delta;        // [rows, n1]
-  const int32_t* exps;       // fp16: [rows] exponent of the power of two that the row's dS is scaled by
+  const int32_t* exps;       // fp16: [items] exponent of the power of two that the item's dS is scaled by
   uint32_t idesc_s, idesc_q, idesc_d;
   int32_t items, hblocks;    // rows * hblocks
   int32_t key_rows;
@@ -96,11 +96,12 @@ __device__ __forceinline__ void red_add_if(bool on, float* addr, float v) {
                : "memory");
 }
 
-// delta = dO . O per (row, head), one warp each; for fp16 also the row's largest |dO| and |delta|.
+// delta = dO . O per (row, head), one warp each; for fp16 also the item's largest |dO| and |delta|.  A head
+// with an Inf or NaN in either is left out: its own gradients are lost, those of the other heads keep their scale.
 template <typename T>
 __global__ void __launch_bounds__(256) sfa_bwd_delta_kernel(const T* __restrict__ d_out, const T* __restrict__ out,
                                                             float* __restrict__ delta, float* __restrict__ bound,
-                                                            int64_t total, int32_t n1) {
+                                                            int64_t total, int32_t n1, int32_t hblocks) {
   const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= total) return;
@@ -125,15 +126,16 @@ __global__ void __launch_bounds__(256) sfa_bwd_delta_kernel(const T* __restrict_
   }
   if (lane == 0) {
     delta[i] = s;
-    if (bound != nullptr) {   // (non-negative floats order like their bit patterns)
-      const int64_t row = i / n1;
-      atomicMax(reinterpret_cast<int*>(bound + 2 * row), __float_as_int(sqrtf(n)));
-      atomicMax(reinterpret_cast<int*>(bound + 2 * row + 1), __float_as_int(fabsf(s)));
+    if (bound != nullptr && n < INFINITY && fabsf(s) < INFINITY) {
+      // (non-negative floats order like their bit patterns)
+      const int64_t row = i / n1, item = row * hblocks + (i - row * n1) / kBwdHeads;
+      atomicMax(reinterpret_cast<int*>(bound + 2 * item), __float_as_int(sqrtf(n)));
+      atomicMax(reinterpret_cast<int*>(bound + 2 * item + 1), __float_as_int(fabsf(s)));
     }
   }
 }
 
-// fp16: norm of the value part of each key, a warp per key.
+// fp16: norm of the value part of each key, a warp per key; 0 where it is not finite (as for heads above).
 template <typename T>
 __global__ void __launch_bounds__(256) sfa_bwd_key_norm_kernel(const T* __restrict__ key, float* __restrict__ norms,
                                                                int64_t key_rows) {
@@ -150,16 +152,16 @@ __global__ void __launch_bounds__(256) sfa_bwd_key_norm_kernel(const T* __restri
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-  if (lane == 0) norms[r] = sqrtf(n);
+  if (lane == 0) norms[r] = n < INFINITY ? sqrtf(n) : 0.f;
 }
 
-// fp16: the row's exponent, a block per row.  Only the keys that the row selected count: what a key tensor
+// fp16: the exponents of a row's items, a block per row.  Only the keys that the row selected count: what a key tensor
 // holds elsewhere (padding past the valid lengths, keys of other sequences) may be anything.
 __global__ void __launch_bounds__(256) sfa_bwd_exponent_kernel(const int2* __restrict__ nvalid,
                                                                const int32_t* __restrict__ key_list,
                                                                const float* __restrict__ norms,
                                                                const float* __restrict__ bound,
-                                                               int32_t* __restrict__ exps, float scale) {
+                                                               int32_t* __restrict__ exps, int32_t hblocks, float scale) {
   __shared__ float red[8];
   const int32_t row = blockIdx.x;
   const int2 nv = nvalid[row];
@@ -171,11 +173,12 @@ __global__ void __launch_bounds__(256) sfa_bwd_exponent_kernel(const int2* __res
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
-  if (threadIdx.x == 0) {
 #pragma unroll
-    for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w]);
-    const float b = fabsf(scale) * fmaf(bound[2 * row], m, bound[2 * row + 1]);
-    exps[row] = b > 0.f && b < INFINITY ? max(-100, min(100, 12 - ilogbf(b))) : 0;
+  for (int w = 0; w < 8; ++w) m = fmaxf(m, red[w]);
+  for (int32_t h = threadIdx.x; h < hblocks; h += 256) {
+    const int64_t item = (int64_t)row * hblocks + h;
+    const float b = fabsf(scale) * fmaf(bound[2 * item], m, bound[2 * item + 1]);
+    exps[item] = b > 0.f && b < INFINITY ? max(-100, min(100, 12 - ilogbf(b))) : 0;
   }
 }
 
@@ -266,7 +269,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
             c0 = a.delta[hi_];
           }
         }
-        if constexpr (kScaled) up = is_s ? 8192.f : scalbnf(1.f, a.exps[row]);
+        if constexpr (kScaled) up = is_s ? 8192.f : scalbnf(1.f, a.exps[item]);
         for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
           const uint32_t ph = n_tile & 1;
           ok = wait(s_full, ph);
@@ -333,7 +336,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
       }
       // dQ^T tile m: this thread's feature is m * 128 + quarter * 32 + lane, a column is a head
       float down = 1.f;
-      if constexpr (kScaled) { if (ntiles > 0) down = scalbnf(1.f, -a.exps[row]); }
+      if constexpr (kScaled) { if (ntiles > 0) down = scalbnf(1.f, -a.exps[item]); }
       const int32_t hn = min(kBwdHeads, n1 - h0);
 #pragma unroll 1
       for (int m = half; m < 5; m += 2) {
@@ -381,7 +384,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
       const int2 nv = a.nvalid[row];
       const int32_t ntiles = tiles_of(nv.x);
       float dk_down = 1.f;
-      if constexpr (kScaled) { if (ntiles > 0) dk_down = scalbnf(1.f, -a.exps[row]); }
+      if constexpr (kScaled) { if (ntiles > 0) dk_down = scalbnf(1.f, -a.exps[item]); }
       for (int32_t t = 0; t < ntiles && ok; ++t) {
         const int4* rows4 = reinterpret_cast<const int4*>(rows_s + rbuf * kBwdBK);
         rbuf = rbuf == 2 ? 0 : rbuf + 1;
@@ -653,8 +656,8 @@ inline bool sfa_bwd_sm100_eligible(const DsaSfaGradParams* p) {
   if (rows < 1 || rows * ((p->n1 + kBwdHeads - 1) / kBwdHeads) >= (1ll << 31)) return false;
   return rows * p->sparse_count * p->sparse_block_size < (1ll << 31);    // key_list offsets are int32
 }
-// Workspace: header | dk / dv accumulators | fp16: bounds of the rows - zeroed before the call - | fp16: exponents of
-// the rows, norms of the keys | nvalid | delta | redo flags and count of the pre-pass (unused) | key_list
+// Workspace: header | dk / dv accumulators | fp16: bounds of the items - zeroed before the call - | fp16: exponents
+// of the items, norms of the keys | nvalid | delta | redo flags and count of the pre-pass (unused) | key_list
 struct SfaBwdWs { size_t acc, bound, zeroed, exps, norms, nvalid, delta, redo, key_list, total; };
 inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
@@ -663,9 +666,10 @@ inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
   w.acc = header;
   w.bound = w.acc + up((size_t)p->key_rows * (size_t)(2 * p->d + p->d_rope) * sizeof(float));
   const bool fp16 = p->dtype == DSA_DTYPE_FP16;
-  w.zeroed = w.bound + (fp16 ? up(rows * 2 * 4) : 0);
+  const size_t items = rows * ((p->n1 + kBwdHeads - 1) / kBwdHeads);
+  w.zeroed = w.bound + (fp16 ? up(items * 2 * 4) : 0);
   w.exps = w.zeroed;
-  w.norms = w.exps + (fp16 ? up(rows * 4) : 0);
+  w.norms = w.exps + (fp16 ? up(items * 4) : 0);
   w.nvalid = w.norms + (fp16 ? up((size_t)p->key_rows * 4) : 0);
   w.delta = w.nvalid + up(rows * 8);
   w.redo = w.delta + up(rows * p->n1 * 4);
@@ -715,11 +719,13 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   // (slots without a row are left out: the reductions of a whole tile go to every listed row unchecked)
   sfa_compact_launch(f, nvalid, key_list, 1, (int32_t)slots, (int32_t)p->key_rows, -1, redo, redo + d.rows, status, st);
   const int64_t pairs = (int64_t)d.rows * p->n1;
+  const int32_t hblocks = (p->n1 + kBwdHeads - 1) / kBwdHeads;
   sfa_bwd_delta_kernel<T><<<(unsigned)((pairs + 7) / 8), 256, 0, st>>>((const T*)p->d_out, (const T*)p->out, delta, bound,
-                                                                      pairs, p->n1);
+                                                                      pairs, p->n1, hblocks);
   if (!bf16) {
     sfa_bwd_key_norm_kernel<T><<<(unsigned)((p->key_rows + 7) / 8), 256, 0, st>>>((const T*)p->key, norms, p->key_rows);
-    sfa_bwd_exponent_kernel<<<d.rows, 256, 0, st>>>(nvalid, key_list, norms, bound, exps, p->scale);
+    sfa_bwd_exponent_kernel<<<d.rows, 256, 0, st>>>(nvalid, key_list, norms, bound, exps, hblocks,
+                                                   p->scale);
   }
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch(bf16 ? 2 : 4);
@@ -731,7 +737,7 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   a.idesc_s = ptx::idesc_f16(fmt, 128, kBwdBK, 0, 0);
   a.idesc_q = ptx::idesc_f16(fmt, 128, kBwdHeads, 1, 1);
   a.idesc_d = ptx::idesc_f16(fmt, 128, kBwdBK, 1, 0);
-  a.hblocks = (p->n1 + kBwdHeads - 1) / kBwdHeads;
+  a.hblocks = hblocks;
   a.items = d.rows * a.hblocks;
   a.key_rows = (int32_t)p->key_rows;
   CUtensorMap tkn, tkr, tq, tqr, tdo;

@@ -82,3 +82,36 @@ def test_fp16_gradients_do_not_depend_on_keys_that_nobody_selected(what, do_scal
             assert torch.equal(a, b), n
         else:
             sfa_grad_acceptance_rule(host(a), host(b), "fp16", name=n, ulps=1.0)
+
+
+@pytest.mark.parametrize("where", ["d_out", "out"])
+@pytest.mark.parametrize("what", [math.inf, math.nan])
+def test_fp16_heads_do_not_lose_their_scale_to_a_head_without_finite_values(what, where):
+    """An Inf or NaN in d_out or out of one head: d_query of every other head is the same, bit for bit, as without
+    that head (its d_out zero)."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_grad_triton
+    q, k, idx, do, out, mx, sm, kw = _fp16_case(31, 5, 260, 80, 100, 260, 1e-3)
+    bad = 3
+    do[:, :, bad] = 0
+    ref = sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)
+    do, out = do.clone(), out.clone()
+    if where == "d_out":
+        do[:, :, bad, 7] = what
+    else:
+        do[:, :, bad, 7] = 1e-3
+        out[:, :, bad, 7] = what
+    got = sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)
+    others = [h for h in range(80) if h != bad]
+    assert torch.equal(got[0][:, :, others], ref[0][:, :, others])
+    assert torch.equal(got[3][:, :, others], ref[3][:, :, others])
+
+
+def test_fp16_head_blocks_scale_apart():
+    """d_out of one head four orders larger: heads of other 64-head blocks keep their d_query bit for bit."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_grad_triton
+    q, k, idx, do, out, mx, sm, kw = _fp16_case(41, 5, 260, 80, 100, 260, 1e-3)
+    ref = sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)
+    loud = do.clone()
+    loud[:, :, 70] *= 1e4
+    got = sparse_flash_attention_grad_triton(q, k, k, idx, loud, out, mx, sm, **kw)
+    assert torch.equal(got[0][:, :, :64], ref[0][:, :, :64]) and torch.equal(got[3][:, :, :64], ref[3][:, :, :64])
