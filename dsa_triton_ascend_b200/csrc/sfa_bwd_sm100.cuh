@@ -96,20 +96,27 @@ __device__ __forceinline__ void red_add_if(bool on, float* addr, float v) {
                : "memory");
 }
 
-// delta = dO . O per (row, head), one warp each; for fp16 also the item's largest |dO| and |delta|.  A head
-// with an Inf or NaN in either is left out: its own gradients are lost, those of the other heads keep their scale.
+// delta = dO . O per (row, head), one warp each; for fp16 also the item's largest |dO| and |delta|, and, by the
+// warps past the last pair, the norm of the value part of each key.  A head with an Inf or NaN in either is left
+// out of the bounds (its own gradients are lost, those of the other heads keep their scale), and the norm of a
+// key that is not finite is 0.
 template <typename T>
 __global__ void __launch_bounds__(256) sfa_bwd_delta_kernel(const T* __restrict__ d_out, const T* __restrict__ out,
                                                             float* __restrict__ delta, float* __restrict__ bound,
-                                                            int64_t total, int32_t n1, int32_t hblocks) {
+                                                            int64_t total, int32_t n1, int32_t hblocks,
+                                                            const T* __restrict__ key, float* __restrict__ norms,
+                                                            int64_t key_rows) {
   const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (i >= total) return;
+  const bool pair = i < total;
+  if (!pair && i - total >= key_rows) return;
+  const T* x_row = pair ? d_out + i * 512 : key + (i - total) * 512;
+  const T* y_row = pair ? out + i * 512 : x_row;
   float s = 0.f, n = 0.f;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    const uint4 a = reinterpret_cast<const uint4*>(d_out + i * 512)[lane + 32 * u];
-    const uint4 b = reinterpret_cast<const uint4*>(out + i * 512)[lane + 32 * u];
+    const uint4 a = reinterpret_cast<const uint4*>(x_row)[lane + 32 * u];
+    const uint4 b = reinterpret_cast<const uint4*>(y_row)[lane + 32 * u];
     const T* av = reinterpret_cast<const T*>(&a);
     const T* bv = reinterpret_cast<const T*>(&b);
 #pragma unroll
@@ -124,35 +131,18 @@ __global__ void __launch_bounds__(256) sfa_bwd_delta_kernel(const T* __restrict_
     s += __shfl_xor_sync(0xffffffffu, s, o);
     n += __shfl_xor_sync(0xffffffffu, n, o);
   }
-  if (lane == 0) {
-    delta[i] = s;
-    if (bound != nullptr && n < INFINITY && fabsf(s) < INFINITY) {
-      // (non-negative floats order like their bit patterns)
-      const int64_t row = i / n1, item = row * hblocks + (i - row * n1) / kBwdHeads;
-      atomicMax(reinterpret_cast<int*>(bound + 2 * item), __float_as_int(sqrtf(n)));
-      atomicMax(reinterpret_cast<int*>(bound + 2 * item + 1), __float_as_int(fabsf(s)));
-    }
+  if (lane != 0) return;
+  if (!pair) {
+    norms[i - total] = n < INFINITY ? sqrtf(n) : 0.f;
+    return;
   }
-}
-
-// fp16: norm of the value part of each key, a warp per key; 0 where it is not finite (as for heads above).
-template <typename T>
-__global__ void __launch_bounds__(256) sfa_bwd_key_norm_kernel(const T* __restrict__ key, float* __restrict__ norms,
-                                                               int64_t key_rows) {
-  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (r >= key_rows) return;
-  float n = 0.f;
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const uint4 a = reinterpret_cast<const uint4*>(key + r * 512)[lane + 32 * u];
-    const T* av = reinterpret_cast<const T*>(&a);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) { const float x = to_f32<T>(av[e]); n = fmaf(x, x, n); }
+  delta[i] = s;
+  if (bound != nullptr && n < INFINITY && fabsf(s) < INFINITY) {
+    // (non-negative floats order like their bit patterns)
+    const int64_t row = i / n1, item = row * hblocks + (i - row * n1) / kBwdHeads;
+    atomicMax(reinterpret_cast<int*>(bound + 2 * item), __float_as_int(sqrtf(n)));
+    atomicMax(reinterpret_cast<int*>(bound + 2 * item + 1), __float_as_int(fabsf(s)));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-  if (lane == 0) norms[r] = n < INFINITY ? sqrtf(n) : 0.f;
 }
 
 // fp16: the exponents of a row's items, a block per row.  Only the keys that the row selected count: what a key tensor
@@ -720,15 +710,13 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   sfa_compact_launch(f, nvalid, key_list, 1, (int32_t)slots, (int32_t)p->key_rows, -1, redo, redo + d.rows, status, st);
   const int64_t pairs = (int64_t)d.rows * p->n1;
   const int32_t hblocks = (p->n1 + kBwdHeads - 1) / kBwdHeads;
-  sfa_bwd_delta_kernel<T><<<(unsigned)((pairs + 7) / 8), 256, 0, st>>>((const T*)p->d_out, (const T*)p->out, delta, bound,
-                                                                      pairs, p->n1, hblocks);
-  if (!bf16) {
-    sfa_bwd_key_norm_kernel<T><<<(unsigned)((p->key_rows + 7) / 8), 256, 0, st>>>((const T*)p->key, norms, p->key_rows);
-    sfa_bwd_exponent_kernel<<<d.rows, 256, 0, st>>>(nvalid, key_list, norms, bound, exps, hblocks,
-                                                   p->scale);
-  }
+  const int64_t norm_rows = bf16 ? 0 : p->key_rows;
+  sfa_bwd_delta_kernel<T><<<(unsigned)((pairs + norm_rows + 7) / 8), 256, 0, st>>>(
+      (const T*)p->d_out, (const T*)p->out, delta, bound, pairs, p->n1, hblocks, (const T*)p->key, norms, norm_rows);
+  if (!bf16)
+    sfa_bwd_exponent_kernel<<<d.rows, 256, 0, st>>>(nvalid, key_list, norms, bound, exps, hblocks, p->scale);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
-  count_launch(bf16 ? 2 : 4);
+  count_launch(bf16 ? 2 : 3);
   SfaBwdArgs a;
   a.p = d;
   a.status = status;
