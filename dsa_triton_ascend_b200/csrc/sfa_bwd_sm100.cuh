@@ -252,13 +252,15 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
         float c0 = 0.f, c1 = 0.f, up = 1.f;                 // S: max, 1 / sum; dP: delta
         if (head) {
           if (is_s) {
+            c0 = a.p.softmax_max[hi_];
             const float l = a.p.softmax_sum[hi_];
-            c0 = l > 0.f ? a.p.softmax_max[hi_] : INFINITY;   // (no sum: P = 0)
             c1 = l > 0.f ? 1.f / l : 0.f;
           } else {
             c0 = a.delta[hi_];
           }
         }
+        // (a head without a sum, or past the last one, has P = 0 whatever its scores are)
+        const int32_t nlive = !is_s || c1 > 0.f ? nvalid : 0;
         if constexpr (kScaled) up = is_s ? 8192.f : scalbnf(1.f, a.exps[item]);
         for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
           const uint32_t ph = n_tile & 1;
@@ -281,8 +283,12 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(s_empty);
-          const int32_t cnt = nvalid - t * kBwdBK - kk0;    // valid keys among this warp's 24
+          const int32_t cnt = nlive - t * kBwdBK - kk0;     // keys among this warp's 24 that take part
           if (is_s) {
+            // (exp of a sum beside 1 / sum: against 64 bits P is off by 1.7e-7 (rms), expf(..) / sum by 1.1e-7.  Its
+            // share shows in neither the fp32 sums of d_key - fp16, 64 heads, k 1024: 8.1e-7 and 7.8e-7, most of
+            // it from the 512-feature score products - nor in the results, 2.0692e-4 and 2.0692e-4 from their one
+            // rounding; four S warps have this tile's exponentials to themselves, and expf takes 1262 us to 1584.)
 #pragma unroll
             for (int k = 0; k < 24; ++k)
               v[k] = k < cnt ? ex2(fmaf(v[k], a.p.scale, -c0) * 1.4426950408889634f) * c1 : 0.f;

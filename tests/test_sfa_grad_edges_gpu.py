@@ -115,3 +115,50 @@ def test_fp16_head_blocks_scale_apart():
     loud[:, :, 70] *= 1e4
     got = sparse_flash_attention_grad_triton(q, k, k, idx, loud, out, mx, sm, **kw)
     assert torch.equal(got[0][:, :, :64], ref[0][:, :, :64]) and torch.equal(got[3][:, :, :64], ref[3][:, :, :64])
+
+
+def test_a_head_without_a_sum_has_no_probabilities():
+    """softmax_sum = 0 and scores that overflow to +Inf: the head contributes nothing, as if its query were zero."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_grad_triton
+    bf, S1, S2, N1, K, dead = torch.bfloat16, 3, 120, 20, 100, 5
+    q, qr = _randn(51, 1, S1, N1, 512, dtype=bf), _randn(52, 1, S1, N1, 64, dtype=bf)
+    k, kr = _randn(53, 1, S2, 1, 512, dtype=bf), _randn(54, 1, S2, 1, 64, dtype=bf)
+    do, out = _randn(55, 1, S1, N1, 512, dtype=bf), _randn(56, 1, S1, N1, 512, dtype=bf)
+    # feature 0: 1e20 in the dead head's query and in key 3 (score 1e40); no other head uses it
+    q[..., 0], do[..., 0], k[..., 0] = 0, 0, 0
+    k[:, 3, 0, 0] = 1e20
+    q[:, :, dead, 0] = 1e20
+    mx, sm = torch.zeros(1, 1, S1, N1, device="cuda"), torch.full((1, 1, S1, N1), 100.0, device="cuda")
+    sm[..., dead] = 0
+    idx = torch.arange(K, dtype=torch.int32, device="cuda").expand(1, S1, 1, K).contiguous()
+    kw = dict(scale_value=1.0 / 24.0, query_rope=qr, key_rope=kr, sparse_mode=0)
+    got = sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)
+    still = q.clone()
+    still[:, :, dead] = 0
+    ref = sparse_flash_attention_grad_triton(still, k, k, idx, do, out, mx, sm, **kw)
+    for n, a, b in zip(NAMES, got, ref):
+        if n.startswith("d_query"):
+            assert torch.equal(a, b) and (a[:, :, dead] == 0).all(), n
+        else:
+            sfa_grad_acceptance_rule(host(a), host(b), "bf16", name=n, ulps=1.0)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+def test_heads_past_the_last_one_add_nothing_to_d_value(dtype):
+    """17 heads in a block of 64, and a key of -Inf score (probability 0 in every head): d_value stays finite and
+    is what it is without that key."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_grad_triton
+    dt, S1, S2, N1, K = tdtype(dtype), 3, 120, 17, 100
+    q, qr = _randn(61, 1, S1, N1, 512, dtype=dt), _randn(62, 1, S1, N1, 64, dtype=dt)
+    k, kr = _randn(63, 1, S2, 1, 512, dtype=dt), _randn(64, 1, S2, 1, 64, dtype=dt)
+    do, out = _randn(65, 1, S1, N1, 512, dtype=dt), _randn(66, 1, S1, N1, 512, dtype=dt)
+    q[..., 0], k[..., 0] = -1, 0
+    mx, sm = torch.zeros(1, 1, S1, N1, device="cuda"), torch.full((1, 1, S1, N1), 100.0, device="cuda")
+    idx = torch.arange(K, dtype=torch.int32, device="cuda").expand(1, S1, 1, K).clone()
+    kw = dict(scale_value=1.0 / 24.0, query_rope=qr, key_rope=kr, sparse_mode=0)
+    far = k.clone()
+    far[:, 3, 0, 0] = math.inf
+    got = sparse_flash_attention_grad_triton(q, far, far, idx, do, out, mx, sm, **kw)[2]
+    idx[..., 3] = -1
+    ref = sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)[2]
+    sfa_grad_acceptance_rule(host(got), host(ref), dtype, name="d_value", ulps=1.0)
