@@ -266,7 +266,7 @@ static int sfa_grad_mma_launch(const SfaGradDev& d, int n1, cudaStream_t st) {
 }
 
 template <typename T>
-static int sfa_grad_launch(const DsaSfaGradParams* p, char* ws, const SfaBwdWs& w, cudaStream_t st) {
+static int sfa_grad_launch(const DsaSfaGradParams* p, bool tensor, char* ws, const SfaBwdWs& w, cudaStream_t st) {
   SfaGradDev d;
   float* acc = reinterpret_cast<float*>(ws + w.acc);
   d.seq.seq_q = p->seq_q; d.seq.seq_k = p->seq_k; d.seq.block_table = nullptr;
@@ -289,9 +289,9 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, char* ws, const SfaBwdWs& 
   if (d.rows > 0) {
     const unsigned gy = (unsigned)((p->n1 + kSfaGradHeads - 1) / kSfaGradHeads);
     dim3 grid((unsigned)d.rows, gy, 1);
-    // D = 512 on tcgen05; other head dims (and tensors off their 16-byte boundaries) on mma.sync; on
-    // request the CUDA-core kernel
-    if (sfa_bwd_sm100_eligible(p)) {
+    // D = 512 with 16 heads or more on tcgen05; other shapes (and calls with the smaller workspace) on mma.sync;
+    // on request the CUDA-core kernel
+    if (tensor) {
       const int rc = sfa_bwd_sm100_launch<T>(p, d, ws, w, st);
       if (rc != DSA_OK) return rc;
     } else if (p->kernel != DSA_KERNEL_PORTABLE) {
@@ -308,7 +308,7 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, char* ws, const SfaBwdWs& 
       sfa_bwd_simt_kernel<T><<<grid, kSfaGradThreads, smem, st>>>(d);
     }
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
-    if (!sfa_bwd_sm100_eligible(p)) count_launch();
+    if (!tensor) count_launch();
   }
   if (p->key_rows > 0) {
     const int64_t total = p->key_rows * (int64_t)(2 * p->d + p->d_rope);
@@ -642,26 +642,34 @@ int dsa_sfa_forward(const DsaSfaParams* p, void* workspace, size_t workspace_byt
 // ---------------------------------------------------------------------------------------------
 // Attention backward
 // ---------------------------------------------------------------------------------------------
+static size_t sfa_grad_least_bytes(const DsaSfaGradParams* p) {
+  return kWorkspaceHeader + (size_t)p->key_rows * (size_t)(2 * p->d + p->d_rope) * sizeof(float);
+}
+
+int dsa_sfa_grad_uses_tensor_path(const DsaSfaGradParams* p) {
+  if (sfa_grad_validate(p) != DSA_OK) return 0;
+  return sfa_bwd_sm100_shape(p) && sfa_bwd_sm100_aligned(p) ? 1 : 0;
+}
+
 int dsa_sfa_grad_workspace_bytes(const DsaSfaGradParams* p, size_t* out_bytes) {
   int st = sfa_grad_validate(p);
   if (st != DSA_OK) return st;
   if (!out_bytes) return DSA_ERR_NULL;
-  const SfaBwdWs w = sfa_bwd_ws_layout(p, kWorkspaceHeader);
-  *out_bytes = sfa_bwd_sm100_eligible(p) ? w.total : w.zeroed;
+  *out_bytes = sfa_bwd_sm100_shape(p) ? sfa_bwd_ws_layout(p, kWorkspaceHeader).total : sfa_grad_least_bytes(p);
   return DSA_OK;
 }
 
 int dsa_sfa_grad(const DsaSfaGradParams* p, void* workspace, size_t workspace_bytes, void* stream) {
   int st = sfa_grad_validate(p);
   if (st != DSA_OK) return st;
-  size_t need = 0;
-  dsa_sfa_grad_workspace_bytes(p, &need);
-  if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255u) != 0) return DSA_ERR_WORKSPACE;
+  const size_t least = sfa_grad_least_bytes(p);
+  if (!workspace || workspace_bytes < least || ((uintptr_t)workspace & 255u) != 0) return DSA_ERR_WORKSPACE;
   cudaStream_t cs = (cudaStream_t)stream;
   const SfaBwdWs w = sfa_bwd_ws_layout(p, kWorkspaceHeader);
-  if (cudaMemsetAsync(workspace, 0, w.zeroed, cs) != cudaSuccess) return DSA_ERR_CUDA;
-  if (p->dtype == DSA_DTYPE_BF16) return sfa_grad_launch<__nv_bfloat16>(p, (char*)workspace, w, cs);
-  return sfa_grad_launch<__half>(p, (char*)workspace, w, cs);
+  const bool tensor = dsa_sfa_grad_uses_tensor_path(p) && workspace_bytes >= w.total;
+  if (cudaMemsetAsync(workspace, 0, tensor ? w.zeroed : least, cs) != cudaSuccess) return DSA_ERR_CUDA;
+  if (p->dtype == DSA_DTYPE_BF16) return sfa_grad_launch<__nv_bfloat16>(p, tensor, (char*)workspace, w, cs);
+  return sfa_grad_launch<__half>(p, tensor, (char*)workspace, w, cs);
 }
 
 static int dense_lse_validate(const DsaDenseLseParams* p) {

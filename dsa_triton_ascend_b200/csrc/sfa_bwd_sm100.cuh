@@ -639,18 +639,20 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
 inline int64_t sfa_bwd_rows(const DsaSfaGradParams* p) {
   return p->layout_q == DSA_LAYOUT_TND ? (int64_t)p->s1 : (int64_t)p->batch * p->s1;
 }
-inline bool sfa_bwd_sm100_eligible(const DsaSfaGradParams* p) {
+// The shapes this kernel takes, given the larger workspace and 16-byte aligned tensors.
+inline bool sfa_bwd_sm100_shape(const DsaSfaGradParams* p) {
   if (p->d != 512 || p->d_rope != 64 || p->kernel == DSA_KERNEL_PORTABLE) return false;
   // (fewer than 16 heads fill one 16-head block of the mma.sync kernel, which needs no lists beside its
   // accumulators; a block of 64 heads would be mostly padding)
   if (p->n1 < 16) return false;
-  if (((uintptr_t)p->query | (uintptr_t)p->query_rope | (uintptr_t)p->key | (uintptr_t)p->key_rope |
-       (uintptr_t)p->d_out | (uintptr_t)p->out) & 15u)
-    return false;
   if (p->key_rows < 1 || p->key_rows >= (1ll << 31) - 1) return false;
   const int64_t rows = sfa_bwd_rows(p);
   if (rows < 1 || rows * ((p->n1 + kBwdHeads - 1) / kBwdHeads) >= (1ll << 31)) return false;
   return rows * p->sparse_count * p->sparse_block_size < (1ll << 31);    // key_list offsets are int32
+}
+inline bool sfa_bwd_sm100_aligned(const DsaSfaGradParams* p) {
+  return (((uintptr_t)p->query | (uintptr_t)p->query_rope | (uintptr_t)p->key | (uintptr_t)p->key_rope |
+           (uintptr_t)p->d_out | (uintptr_t)p->out) & 15u) == 0;
 }
 // Workspace: header | dk / dv accumulators | fp16: bounds of the items - zeroed before the call - | fp16: exponents
 // of the items, norms of the keys | nvalid | delta | redo flags and count of the pre-pass (unused) | key_list

@@ -18,13 +18,14 @@ from ._host import (INT64_MAX, current_stream, dtype_code, max_len_from_cumulati
 
 _VALID_D = (128, 256, 512)
 _D_ROPE = 64
+_HEADER = 256      # status header of every workspace
 
 
 _kernel = _cabi.KERNEL_AUTO
 
 
 def set_kernel(kind):
-    """"auto" / "tensor" (mma.sync kernel) or "portable" (CUDA-core kernel)."""
+    """"auto" / "tensor" (tensor-core kernels) or "portable" (CUDA-core kernel)."""
     global _kernel
     _kernel = {"auto": _cabi.KERNEL_AUTO, "portable": _cabi.KERNEL_PORTABLE, "tensor": _cabi.KERNEL_TENSOR}[kind]
 
@@ -158,7 +159,11 @@ def sparse_flash_attention_grad_triton(
         nbytes = ctypes.c_size_t(0)
         _cabi.check(_cabi.lib.dsa_sfa_grad_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)),
                     "sparse_flash_attention_grad")
-        ws = workspace(nbytes.value, dev)
+        try:
+            ws = workspace(nbytes.value, dev)
+        except torch.cuda.OutOfMemoryError:
+            # header and accumulators alone: the mma.sync kernel
+            ws = workspace(_HEADER + p.key_rows * (2 * D + d_rope) * 4, dev)
         _cabi.check(_cabi.lib.dsa_sfa_grad(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
                     "sparse_flash_attention_grad")
         note_launch("sparse_flash_attention_grad", ws, dev)

@@ -152,7 +152,7 @@ int dsa_sfa_forward(const DsaSfaParams* p, void* workspace, size_t workspace_byt
  */
 typedef struct DsaSfaGradParams {
   uint32_t struct_size; /* sizeof(DsaSfaGradParams) */
-  int32_t kernel;       /* DSA_KERNEL_AUTO / _TENSOR: mma.sync kernel; _PORTABLE: CUDA-core kernel */
+  int32_t kernel;       /* DSA_KERNEL_AUTO / _TENSOR: tensor-core kernels; _PORTABLE: CUDA-core kernel */
   const void* query;      /* [rows, n1, d]      */
   const void* query_rope; /* [rows, n1, d_rope] */
   const void* key;        /* BSND [batch, s2, 1, d] | TND [T2, 1, d] */
@@ -177,9 +177,15 @@ typedef struct DsaSfaGradParams {
   int64_t key_rows; /* batch*s2 (BSND) or T2 (TND) */
 } DsaSfaGradParams;
 
-/* Workspace: a status header plus fp32 accumulators key_rows * (2*d + d_rope) * 4 bytes. */
+/* 1 when the call, given the workspace that dsa_sfa_grad_workspace_bytes() names, runs on the tcgen05 kernel:
+ * d = 512, 16 heads or more, operands on 16-byte boundaries, kernel not DSA_KERNEL_PORTABLE. */
+int dsa_sfa_grad_uses_tensor_path(const DsaSfaGradParams* p);
+/* Workspace: a status header (256 bytes) plus fp32 accumulators key_rows * (2*d + d_rope) * 4 bytes are enough
+ * for every call.  For the shapes of the tcgen05 kernel the size named here also covers its scratch, mostly the
+ * rows' key lists (rows * sparse_count * sparse_block_size * 4 bytes); dsa_sfa_grad() with less than that
+ * runs such a call on the mma.sync kernel: the same results, 3.7 times the time at 512 rows x 64 heads. */
 int dsa_sfa_grad_workspace_bytes(const DsaSfaGradParams* p, size_t* out_bytes);
-/* Enqueue the backward on `stream`: clears the accumulators, runs the gradient kernel and the
+/* Enqueue the backward on `stream`: clears the accumulators, runs the gradient kernels and the
  * conversion of the accumulators to the io dtype. */
 int dsa_sfa_grad(const DsaSfaGradParams* p, void* workspace, size_t workspace_bytes, void* stream);
 

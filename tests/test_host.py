@@ -300,3 +300,31 @@ def test_length_lists_are_uploaded_once():
     d, host_d = _host.seq_tensor(t, "cpu")
     assert d.tolist() == [1, 2] and host_d == [1, 2]
     assert _host.seq_tensor(None, "cpu") == (None, None)
+
+
+def test_sfa_grad_workspace_and_kernel_choice():
+    """The least workspace (header and accumulators) is accepted for every shape and one byte less is not; the size
+    that is named does not depend on how the pointers are aligned; the tcgen05 kernel starts at 16 heads of D = 512."""
+    from dsa_triton_ascend_b200 import _cabi
+    n = ctypes.c_size_t(0)
+    g = _cabi.DsaSfaGradParams()
+    g.struct_size = ctypes.sizeof(g)
+    for f in ("query", "query_rope", "key", "key_rope", "sparse_indices", "d_out", "out", "softmax_max",
+              "softmax_sum", "d_query", "d_query_rope", "d_key", "d_key_rope", "d_value"):
+        setattr(g, f, 256)
+    g.batch, g.s1, g.s2, g.d_rope = 1, 4, 64, 64
+    g.sparse_count, g.sparse_block_size, g.sparse_mode, g.key_rows = 16, 1, 3, 64
+    for d, heads, dtype, tensor in ((512, 64, 0, 1), (512, 16, 1, 1), (512, 15, 1, 0), (256, 64, 0, 0), (128, 16, 1, 0)):
+        g.d, g.n1, g.dtype, g.kernel = d, heads, dtype, 0
+        least = 256 + 64 * (2 * d + 64) * 4
+        assert _cabi.lib.dsa_sfa_grad_uses_tensor_path(ctypes.byref(g)) == tensor
+        assert _cabi.lib.dsa_sfa_grad_workspace_bytes(ctypes.byref(g), ctypes.byref(n)) == 0
+        full = n.value
+        assert (full >= least + 4 * 16 * 4) if tensor else (full == least)
+        assert _cabi.lib.dsa_sfa_grad(ctypes.byref(g), 256, least - 1, None) == -4
+        g.d_out = 264
+        assert _cabi.lib.dsa_sfa_grad_uses_tensor_path(ctypes.byref(g)) == 0
+        assert _cabi.lib.dsa_sfa_grad_workspace_bytes(ctypes.byref(g), ctypes.byref(n)) == 0 and n.value == full
+        g.d_out, g.kernel = 256, 1
+        assert _cabi.lib.dsa_sfa_grad_uses_tensor_path(ctypes.byref(g)) == 0
+        assert _cabi.lib.dsa_sfa_grad_workspace_bytes(ctypes.byref(g), ctypes.byref(n)) == 0 and n.value == least

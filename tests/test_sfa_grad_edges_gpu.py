@@ -162,3 +162,32 @@ def test_heads_past_the_last_one_add_nothing_to_d_value(dtype):
     idx[..., 3] = -1
     ref = sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)[2]
     sfa_grad_acceptance_rule(host(got), host(ref), dtype, name="d_value", ulps=1.0)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+def test_the_documented_least_workspace_is_enough(dtype, monkeypatch):
+    """Header and accumulators alone (what the wrapper falls back to when the larger workspace cannot be had): the
+    mma.sync kernel runs, with the same results up to the rounding of the outputs."""
+    from dsa_triton_ascend_b200 import _host
+    from dsa_triton_ascend_b200 import sparse_flash_attention_grad as module
+    dt, S1, S2, N1, K = tdtype(dtype), 5, 120, 64, 100
+    q, qr = _randn(71, 1, S1, N1, 512, dtype=dt), _randn(72, 1, S1, N1, 64, dtype=dt)
+    k, kr = _randn(73, 1, S2, 1, 512, dtype=dt), _randn(74, 1, S2, 1, 64, dtype=dt)
+    do, out = _randn(75, 1, S1, N1, 512, dtype=dt), _randn(76, 1, S1, N1, 512, dtype=dt)
+    mx, sm = torch.zeros(1, 1, S1, N1, device="cuda"), torch.full((1, 1, S1, N1), 100.0, device="cuda")
+    idx = torch.arange(K, dtype=torch.int32, device="cuda").expand(1, S1, 1, K).contiguous()
+    kw = dict(scale_value=1.0 / 24.0, query_rope=qr, key_rope=kr, sparse_mode=0)
+    ref = module.sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)
+    asked = []
+
+    def scarce(nbytes, device):
+        asked.append(int(nbytes))
+        if len(asked) == 1:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return _host.workspace(nbytes, device)
+
+    monkeypatch.setattr(module, "workspace", scarce)
+    got = module.sparse_flash_attention_grad_triton(q, k, k, idx, do, out, mx, sm, **kw)
+    assert len(asked) == 2 and asked[1] == 256 + S2 * (2 * 512 + 64) * 4 < asked[0]
+    for n, a, b in zip(NAMES, got, ref):
+        sfa_grad_acceptance_rule(host(a), host(b), dtype, name=n, ulps=1.0)
