@@ -65,6 +65,13 @@ def ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
+def packed(t):
+    """`t` contiguous and on a 16-byte boundary (a view into a flat buffer may start anywhere): the kernels load
+    keys and heads 16 bytes at a time."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def workspace(nbytes, device):
     # torch's caching allocator returns 512-byte aligned blocks; the library wants 256.
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)

@@ -24,6 +24,8 @@ namespace dsa {
 constexpr size_t kWorkspaceHeader = 256;  // bytes reserved at the start of every workspace (status word)
 
 static inline int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
+// Every attention and loss kernel gathers keys 16 bytes at a time.
+static inline bool off16(const void* a, const void* b = nullptr) { return (((uintptr_t)a | (uintptr_t)b) & 15u) != 0; }
 
 static int li_validate(const DsaLiParams* p) {
   if (p == nullptr) return DSA_ERR_NULL;
@@ -161,6 +163,7 @@ static int sfa_validate(const DsaSfaParams* p) {
   if (p->layout_kv == DSA_LAYOUT_PA_BSND && (!p->block_table || p->block_size < 1 || p->max_blocks < 1 || !p->seq_k))
     return DSA_ERR_VALUE;
   if (p->kernel < DSA_KERNEL_AUTO || p->kernel > DSA_KERNEL_TENSOR) return DSA_ERR_VALUE;
+  if (off16(p->key, p->key_rope)) return DSA_ERR_VALUE;
   return DSA_OK;
 }
 
@@ -241,6 +244,7 @@ static int sfa_grad_validate(const DsaSfaGradParams* p) {
   if (p->layout_kv == DSA_LAYOUT_TND && (!p->seq_k || !p->seq_k_cumulative)) return DSA_ERR_VALUE;
   if (p->kernel != DSA_KERNEL_AUTO && p->kernel != DSA_KERNEL_PORTABLE && p->kernel != DSA_KERNEL_TENSOR)
     return DSA_ERR_UNSUPPORTED;
+  if (off16(p->key, p->key_rope)) return DSA_ERR_VALUE;
   return DSA_OK;
 }
 
@@ -290,11 +294,12 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, bool tensor, char* ws, con
     const unsigned gy = (unsigned)((p->n1 + kSfaGradHeads - 1) / kSfaGradHeads);
     dim3 grid((unsigned)d.rows, gy, 1);
     // D = 512 with 16 heads or more on tcgen05; other shapes (and calls with the smaller workspace) on mma.sync;
-    // on request the CUDA-core kernel
+    // on request, or with a query or d_out off its 16-byte boundary, the CUDA-core kernel
+    const bool mma = p->kernel != DSA_KERNEL_PORTABLE && !off16(p->query, p->query_rope) && !off16(p->d_out);
     if (tensor) {
       const int rc = sfa_bwd_sm100_launch<T>(p, d, ws, w, st);
       if (rc != DSA_OK) return rc;
-    } else if (p->kernel != DSA_KERNEL_PORTABLE) {
+    } else if (mma) {
       int rc;
       if (p->d == 512) rc = sfa_grad_mma_launch<T, 512>(d, p->n1, st);
       else if (p->d == 256) rc = sfa_grad_mma_launch<T, 256>(d, p->n1, st);
@@ -350,6 +355,7 @@ static int sli_grad_validate(const DsaSliGradParams* p) {
     if (p->topk < 1) return DSA_ERR_VALUE;
   }
   if (p->kernel != DSA_KERNEL_AUTO && p->kernel != DSA_KERNEL_PORTABLE) return DSA_ERR_UNSUPPORTED;
+  if (off16(p->key, p->d_rope ? p->key_rope : nullptr) || off16(p->key_index)) return DSA_ERR_VALUE;
   return DSA_OK;
 }
 
@@ -682,6 +688,7 @@ static int dense_lse_validate(const DsaDenseLseParams* p) {
   if (p->d_idx != 128 && p->d_idx != 256 && p->d_idx != 512) return DSA_ERR_VALUE;
   if (p->batch < 1 || p->s1 < 0 || p->s2 < 1 || p->g < 1) return DSA_ERR_VALUE;
   if ((int64_t)p->batch * p->s1 > 0x7FFFFFFF) return DSA_ERR_TOO_LARGE;
+  if (off16(p->key_index)) return DSA_ERR_VALUE;
   return DSA_OK;
 }
 

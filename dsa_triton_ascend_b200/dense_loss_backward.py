@@ -12,7 +12,8 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import INT64_MAX, current_stream, dtype_code, note_launch, ptr, require_cuda, seq_tensor, workspace
+from ._host import (INT64_MAX, current_stream, dtype_code, note_launch, packed, ptr, require_cuda, seq_tensor,
+                    workspace)
 
 SUPPORTED_D = (128, 256, 512)
 
@@ -56,7 +57,7 @@ def npu_dense_lightning_indexer_softmax_lse_triton(query_index, key_index, weigh
     dev = query_index.device
     B, S1, G, Di = query_index.shape
     S2 = key_index.shape[1]
-    query_index, key_index, weights = query_index.contiguous(), key_index.contiguous(), weights.contiguous()
+    query_index, key_index, weights = packed(query_index), packed(key_index), weights.contiguous()
     seq_q, _ = seq_tensor(actual_seq_qlen, dev)
     seq_k, _ = seq_tensor(actual_seq_klen, dev)
     mx = torch.empty(B, 1, S1, dtype=torch.float32, device=dev)
@@ -151,11 +152,11 @@ def dense_loss_backward_triton(query, key, query_index, key_index, weights, soft
                  softmax_sum_index, query_rope, key_rope)
     dev = query.device
 
-    query, key = query.contiguous(), key.contiguous()
-    query_index, key_index, weights = query_index.contiguous(), key_index.contiguous(), weights.contiguous()
+    query, key = packed(query), packed(key)
+    query_index, key_index, weights = packed(query_index), packed(key_index), weights.contiguous()
     softmax_max, softmax_sum = softmax_max.contiguous(), softmax_sum.contiguous()
     if d_rope:
-        query_rope, key_rope = query_rope.contiguous(), key_rope.contiguous()
+        query_rope, key_rope = packed(query_rope), packed(key_rope)
     seq_q, _ = seq_tensor(actual_seq_qlen, dev)
     seq_k, _ = seq_tensor(actual_seq_klen, dev)
     G, Di = query_index.shape[2], query_index.shape[3]

@@ -12,8 +12,8 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, dtype_code, max_len_from_cumulative, note_launch, ptr,
-                    require_cuda, seq_tensor, workspace)
+from ._host import (INT64_MAX, current_stream, dtype_code, max_len_from_cumulative, note_launch, packed,
+                    ptr, require_cuda, seq_tensor, workspace)
 
 _VALID_D = (128, 256, 512)
 _D_ROPE = 64
@@ -136,8 +136,7 @@ def sparse_flash_attention_triton(
         raise ValueError("query, key, query_rope and key_rope must share a dtype")
     require_cuda(query, key, sparse_indices, query_rope, key_rope, block_table)
 
-    query, query_rope = query.contiguous(), query_rope.contiguous()
-    key, key_rope = key.contiguous(), key_rope.contiguous()
+    query, query_rope, key, key_rope = packed(query), packed(query_rope), packed(key), packed(key_rope)
     sparse_indices = sparse_indices.to(torch.int32).contiguous()
     topk = sparse_indices.shape[-1]
     rows = s1 if is_tnd_q else B * s1

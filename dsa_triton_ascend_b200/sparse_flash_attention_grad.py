@@ -13,8 +13,8 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, dtype_code, max_len_from_cumulative, note_launch, ptr,
-                    require_cuda, seq_tensor, workspace)
+from ._host import (INT64_MAX, current_stream, dtype_code, max_len_from_cumulative, note_launch, packed,
+                    ptr, require_cuda, seq_tensor, workspace)
 
 _VALID_D = (128, 256, 512)
 _D_ROPE = 64
@@ -120,9 +120,8 @@ def sparse_flash_attention_grad_triton(
         raise ValueError(f"softmax_max / softmax_sum must have shape {stat_shape}")
     require_cuda(query, key, sparse_indices, d_out, out, softmax_max, softmax_sum, query_rope, key_rope)
 
-    query, query_rope = query.contiguous(), query_rope.contiguous()
-    key, key_rope = key.contiguous(), key_rope.contiguous()
-    d_out, out = d_out.contiguous(), out.contiguous()
+    query, query_rope, key, key_rope = packed(query), packed(query_rope), packed(key), packed(key_rope)
+    d_out, out = packed(d_out), packed(out)
     softmax_max = softmax_max.to(torch.float32).contiguous()
     softmax_sum = softmax_sum.to(torch.float32).contiguous()
     sparse_indices = sparse_indices.to(torch.int32).contiguous()

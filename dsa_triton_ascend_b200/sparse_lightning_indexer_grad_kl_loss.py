@@ -13,7 +13,8 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import INT64_MAX, current_stream, dtype_code, note_launch, ptr, require_cuda, seq_tensor, workspace
+from ._host import (INT64_MAX, current_stream, dtype_code, note_launch, packed, ptr, require_cuda, seq_tensor,
+                    workspace)
 
 
 def sparse_lightning_indexer_grad_kl_loss_triton(
@@ -79,10 +80,10 @@ def sparse_lightning_indexer_grad_kl_loss_triton(
                  query_rope, key_rope)
     dev = query.device
 
-    query, key = query.contiguous(), key.contiguous()
-    query_index, key_index, weights = query_index.contiguous(), key_index.contiguous(), weights.contiguous()
+    query, key = packed(query), packed(key)
+    query_index, key_index, weights = packed(query_index), packed(key_index), weights.contiguous()
     if d_rope:
-        query_rope, key_rope = query_rope.contiguous(), key_rope.contiguous()
+        query_rope, key_rope = packed(query_rope), packed(key_rope)
     sparse_indices = sparse_indices.to(torch.int32).contiguous()
     softmax_max = softmax_max.to(torch.float32).contiguous()
     softmax_sum = softmax_sum.to(torch.float32).contiguous()

@@ -12,6 +12,9 @@
  * without synchronising.  All functions return 0 on success and a negative DSA_ERR_*
  * code otherwise; none throws, exits or allocates device memory (except the entry point
  * explicitly documented to own static device scratch).
+ * The attention and loss calls gather keys 16 bytes at a time: key, key_rope and key_index start on 16-byte
+ * boundaries (DSA_ERR_VALUE otherwise).  The tcgen05 kernels ask that of the queries, d_out and out as well;
+ * without it another kernel runs.
  */
 #ifndef DSA_B200_H_
 #define DSA_B200_H_
@@ -48,8 +51,8 @@ extern "C" {
 
 #define DSA_KERNEL_AUTO 0     /* tensor-core path when the shape is eligible, else portable */
 #define DSA_KERNEL_PORTABLE 1 /* any-shape kernels (mma.sync / CUDA cores)                    */
-#define DSA_KERNEL_TENSOR 2   /* tensor-core path (tcgen05 forward, mma.sync backward);
-                                 DSA_ERR_UNSUPPORTED when the shape is not eligible         */
+#define DSA_KERNEL_TENSOR 2   /* tensor-core path; forward calls: DSA_ERR_UNSUPPORTED when the shape is
+                                 not eligible (the attention backward takes every legal shape) */
 
 #define DSA_PHASE_SCORE 1
 #define DSA_PHASE_TOPK 2

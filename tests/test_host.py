@@ -328,3 +328,37 @@ def test_sfa_grad_workspace_and_kernel_choice():
         g.d_out, g.kernel = 256, 1
         assert _cabi.lib.dsa_sfa_grad_uses_tensor_path(ctypes.byref(g)) == 0
         assert _cabi.lib.dsa_sfa_grad_workspace_bytes(ctypes.byref(g), ctypes.byref(n)) == 0 and n.value == least
+
+
+def test_keys_off_their_16_byte_boundaries_are_refused():
+    """The attention and loss kernels gather keys 16 bytes at a time (the Python wrappers copy such tensors)."""
+    from dsa_triton_ascend_b200 import _cabi
+    n = ctypes.c_size_t(0)
+
+    def params(cls, **kw):
+        p = cls()
+        p.struct_size = ctypes.sizeof(p)
+        for name, kind in cls._fields_:
+            if kind is ctypes.c_void_p and name not in ("seq_q", "seq_k", "block_table"):
+                setattr(p, name, 256)
+        for name, v in kw.items():
+            setattr(p, name, v)
+        return p
+
+    shape = dict(batch=1, s1=4, s2=64)
+    cases = [
+        ("dsa_sfa", params(_cabi.DsaSfaParams, n1=16, d=512, d_rope=64, sparse_count=16, sparse_block_size=1,
+                           sparse_mode=3, key_rows=64, **shape), ("key", "key_rope")),
+        ("dsa_sfa_grad", params(_cabi.DsaSfaGradParams, n1=16, d=512, d_rope=64, sparse_count=16, sparse_block_size=1,
+                                sparse_mode=3, key_rows=64, **shape), ("key", "key_rope")),
+        ("dsa_sli_grad", params(_cabi.DsaSliGradParams, n1=16, n2=1, d=512, d_rope=64, g=16, d_idx=128, topk=16,
+                                **shape), ("key", "key_rope", "key_index")),
+        ("dsa_dense_li_lse", params(_cabi.DsaDenseLseParams, g=16, d_idx=128, **shape), ("key_index",)),
+    ]
+    for name, p, fields in cases:
+        size = getattr(_cabi.lib, name + "_workspace_bytes")
+        assert size(ctypes.byref(p), ctypes.byref(n)) == 0, name
+        for f in fields:
+            setattr(p, f, 256 + 8)
+            assert size(ctypes.byref(p), ctypes.byref(n)) == -3, (name, f)
+            setattr(p, f, 256)

@@ -169,3 +169,44 @@ def test_a_device_wait_that_runs_out_is_reported_and_leaves_the_gpu_usable():
                                       return_value=True)
     li_reference_rule(host(idx), host(val), ri, rv)
     pkg.check_status()
+
+
+def _shifted(t):
+    """The same values one element into a flat buffer: contiguous, off its 16-byte boundary."""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    out = buf[1:].view(t.shape)
+    out.copy_(t)
+    assert out.data_ptr() % 16 != 0
+    return out
+
+
+@pytest.mark.parametrize("heads", [64, 8])
+def test_tensors_off_their_16_byte_boundaries_give_the_same_results(heads):
+    """Attention forward and backward, sparse and dense losses and the dense statistics, every 16-bit operand of
+    which is a view that starts 2 bytes past a boundary."""
+    from dsa_triton_ascend_b200 import (dense_lightning_indexer_softmax_lse_triton, dense_loss_backward_triton,
+                                        sparse_flash_attention_grad_triton, sparse_flash_attention_triton,
+                                        sparse_lightning_indexer_grad_kl_loss_triton)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    draw = lambda *s: (torch.randn(*s, generator=g, device="cuda") * 0.3).to(torch.bfloat16)   # noqa: E731
+    S1, S2, K = 5, 96, 48
+    q, qr, do = draw(1, S1, heads, 512), draw(1, S1, heads, 64), draw(1, S1, heads, 512)
+    k, kr = draw(1, S2, 1, 512), draw(1, S2, 1, 64)
+    qi, ki, w = draw(1, S1, heads, 128), draw(1, S2, 1, 128), draw(1, S1, heads).abs()
+    idx = torch.stack([torch.randperm(S2 - S1, generator=g, device="cuda")[:K] for _ in range(S1)])
+    idx = idx.to(torch.int32).view(1, S1, 1, K)
+
+    def all_of(f):
+        a = dict(scale_value=1.0 / 24.0, query_rope=f(qr), key_rope=f(kr))
+        out, mx, sm = sparse_flash_attention_triton(f(q), f(k), f(k), idx, return_softmax_lse=True, sparse_mode=3, **a)
+        grads = sparse_flash_attention_grad_triton(f(q), f(k), f(k), idx, f(do), f(out), mx, sm, sparse_mode=3, **a)
+        loss = sparse_lightning_indexer_grad_kl_loss_triton(f(q), f(k), f(qi), f(ki), f(w), idx, mx, sm, **a)
+        top, total = dense_lightning_indexer_softmax_lse_triton(f(qi), f(ki), f(w))
+        dense = dense_loss_backward_triton(f(q), f(k), f(qi), f(ki), f(w), mx, sm, top, total, 1.0 / 24.0,
+                                           query_rope=f(qr), key_rope=f(kr))
+        return [out, mx, sm, *grads, *loss, top, total, *dense]
+
+    for i, (a, b) in enumerate(zip(all_of(_shifted), all_of(lambda t: t))):
+        # (one bf16 rounding apart where sums are reductions in any order, and the loss, an fp32 sum)
+        torch.testing.assert_close(a.float(), b.float(), rtol=2.0 ** -7, atol=1e-6 * float(b.float().abs().max() + 1),
+                                   msg=lambda m: f"output {i}: {m}")
