@@ -49,7 +49,7 @@ constexpr uint32_t kLiOffW = kLiOffK + kLiStages * kLiKStage;
 constexpr uint32_t kLiOffBar = kLiOffW + kLiTok * kLiHeads * 4;
 constexpr int kLiDenseGroups = 128;   // most row groups of the dense chunked mode (its table sits behind the barriers)
 constexpr uint32_t kLiOffCum = kLiOffBar + 256;
-constexpr uint32_t kLiSmemBytes = kLiOffCum + (kLiDenseGroups + 2) * 4;
+constexpr uint32_t kLiSmemBytes = kLiOffCum + (kLiDenseGroups + 3) * 4;
 // Byte offset of key stage s: stages 3 and 4 live in the second half of the Q buffer.
 __host__ __device__ constexpr uint32_t li_stage_off(uint32_t s) {
   return s < (uint32_t)kLiStages ? kLiOffK + s * kLiKStage : 2 * kLiQBlock + (s - kLiStages) * kLiKStage;
@@ -114,7 +114,8 @@ __device__ __forceinline__ LiItem li_group(const LiSm100Args& a, int32_t i) {
   return it;
 }
 // `cum` (shared memory, dense mode only): cum[g] = chunks with keys of the row groups before g,
-// cum[groups] = their total, cum[kLiDenseGroups + 1] = key tiles per chunk.
+// cum[groups] = their total, cum[kLiDenseGroups + 1 / + 2] = key tiles per chunk of a group of
+// up to four / of more rows.
 template <bool kDense>
 __device__ __forceinline__ LiItem li_item(const LiSm100Args& a, int32_t i, const int32_t* cum) {
   if constexpr (kDense) {
@@ -157,7 +158,7 @@ __device__ __forceinline__ bool li_item_range(const LiSm100Args& a, const LiItem
     mx = max(mx, v);
   }
   const int32_t tiles = (mx + kLiKeys - 1) / kLiKeys;
-  const int32_t ct = kDense ? cum[kLiDenseGroups + 1] : a.chunk_tiles;
+  const int32_t ct = kDense ? cum[kLiDenseGroups + 1 + (it.nrows > kLiHalf ? 1 : 0)] : a.chunk_tiles;
   *t0 = it.chunk * ct;
   *t1 = min(tiles, *t0 + ct);
   return *t1 > *t0;
@@ -211,13 +212,14 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     ptx::tmem_relinquish();
   }
   if constexpr (kDense) {
-    // li_dense_setup: key tiles of every row group (every CTA builds the same list)
+    // li_dense_setup: key tiles of every row group (every CTA builds the same list), times two, plus one for
+    // groups of more than four rows
     for (int g = threadIdx.x; g < a.groups; g += kLiThreads) {
       const LiItem it = li_group(a, g);
       int32_t mx = 0;
       if (it.row0 >= 0)
         for (int t = 0; t < it.nrows; ++t) mx = max(mx, row_info(a.p.seq, it.row0 + t).visible);
-      cum_s[g + 1] = (mx + kLiKeys - 1) / kLiKeys;
+      cum_s[g + 1] = (mx + kLiKeys - 1) / kLiKeys * 2 + (it.nrows > kLiHalf ? 1 : 0);
     }
   }
   ptx::tc_fence_before();
@@ -225,43 +227,78 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   ptx::tc_fence_after();
   if constexpr (kDense) {
     // chunk size: about eight chunks of real work per CTA, at least 8 tiles each; then the running
-    // count of chunks per group.  The static round-robin over this list leaves the CTAs within one
+    // count of chunks per group (one warp: the whole set-up is in front of the first load).  The static round-robin over this list leaves the CTAs within one
     // chunk of each other, where the (chunk, group) grid leaves them with whatever mix of full,
     // partial and empty chunks the sequence lengths produce.
     if (warp == 0) {
-      int32_t mine = 0;
-      for (int g = lane; g < a.groups; g += 32) mine += cum_s[g + 1];
+      int32_t few = 0, many = 0;              // tiles of groups of up to four / of more rows
+      for (int g = lane; g < a.groups; g += 32) {
+        const int32_t c = cum_s[g + 1];
+        if (c & 1) many += c >> 1; else few += c >> 1;
+      }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-      const int64_t total = mine;
-      int64_t ct = (total + 8ll * grid - 1) / (8ll * grid);
+      for (int o = 16; o > 0; o >>= 1) {
+        few += __shfl_xor_sync(0xffffffffu, few, o);
+        many += __shfl_xor_sync(0xffffffffu, many, o);
+      }
+      const int32_t total = few + many;
+      int32_t ct[2];                          // tiles per chunk of a group of up to four / of more rows
+      ct[0] = ct[1] = max(8, (total + 8 * grid - 1) / (8 * grid));
       if (a.stages == kLiStages) {
-        // Groups of up to eight rows load 128 KB of Q per chunk, about three tiles' time that nothing hides: the
-        // chunk size with the least rounds x (tiles + 3), a lane per candidate (512 rows x 4096 keys: 60 us with
-        // eight tiles per chunk, 52 us with sixteen)
-        const int32_t unit = (int32_t)((total + 16ll * grid - 1) / (16ll * grid));
-        const int32_t cand = max(8, unit * (lane + 1));
-        int32_t chunks = 0;
-        for (int g = 0; g < a.groups; ++g) chunks += (cum_s[g + 1] + cand - 1) / cand;
-        const uint64_t cost = (uint64_t)((chunks + grid - 1) / grid) * (uint64_t)(cand + 3);
+        // Calls whose groups may have eight rows (prefill, TND).  A tile of eight rows takes twice the time of one of
+        // up to four, so chunks of such groups have half the tiles; loading Q (128 KB for eight rows) takes about
+        // three of their tiles' time, which nothing hides; and a round lasts as long as its longest chunk.  A
+        // lane per candidate, the size with the least rounds x (tiles + Q) wins: 512 rows x 4096 keys, eight tiles
+        // per chunk 58.2 us, sixteen 47.2 us; TND, 64 sequences of 16K-65K keys, a row each: 181.8 -> 147.4 us;
+        // 60 sequences of one row beside one of 200 rows: 102.8 us with one size for both kinds, 79.8 us.
+        const int32_t weight = few + 2 * many;
+        const int32_t unit = (weight + 16 * grid - 1) / (16 * grid);
+        const int32_t cf = max(8, unit * (lane + 1)), cm = max(8, unit * (lane + 1) / 2);
+        const float inv_f = 1.f / (float)cf, inv_m = 1.f / (float)cm;
+        float count = 0.f;
+#pragma unroll 8
+        for (int g = 0; g < a.groups; ++g) {
+          // tiles / size rounded up: less a quarter of a tile plus a half, rounded to nearest (exact up to 2^20 tiles)
+          const int32_t c = cum_s[g + 1];
+          count += (fmaf((float)(c >> 1) - 0.25f, (c & 1) ? inv_m : inv_f, 0.5f) + 8388608.f) - 8388608.f;
+        }
+        const int32_t chunks = (int32_t)count;
+        const int32_t longest = max(few > 0 ? cf + 3 : 0, many > 0 ? 2 * cm + 6 : 0);
+        const uint64_t cost = (uint64_t)((chunks + grid - 1) / grid) * (uint64_t)longest;
         uint64_t best = cost * 32 + lane;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
           const uint64_t other = __shfl_xor_sync(0xffffffffu, best, o);
           best = other < best ? other : best;
         }
-        ct = max(8, unit * ((int32_t)(best & 31) + 1));
+        ct[0] = __shfl_sync(0xffffffffu, cf, (int)(best & 31));
+        ct[1] = __shfl_sync(0xffffffffu, cm, (int)(best & 31));
       }
-      if (ct < 8) ct = 8;
-     if (lane == 0) {
-      int32_t acc = 0;
-      cum_s[0] = 0;
-      for (int g = 0; g < a.groups; ++g) {
-        acc += (int32_t)((cum_s[g + 1] + ct - 1) / ct);
-        cum_s[g + 1] = acc;
+      // running count, four groups per lane
+      static_assert(kLiDenseGroups == 128, "four groups per lane");
+      int32_t n[4], sum = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int g = 4 * lane + i;
+        const int32_t c = g < a.groups ? cum_s[g + 1] : 0, size = (c & 1) ? ct[1] : ct[0];
+        sum += ((c >> 1) + size - 1) / size;
+        n[i] = sum;
       }
-      cum_s[kLiDenseGroups + 1] = (int32_t)ct;
-     }
+      int32_t before = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int32_t t = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += t;
+      }
+      before -= sum;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (4 * lane + i < a.groups) cum_s[4 * lane + i + 1] = before + n[i];
+      if (lane == 0) {
+        cum_s[0] = 0;
+        cum_s[kLiDenseGroups + 1] = ct[0];
+        cum_s[kLiDenseGroups + 2] = ct[1];
+      }
     }
     __syncthreads();
   }
