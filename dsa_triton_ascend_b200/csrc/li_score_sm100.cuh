@@ -328,8 +328,8 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    // Lane 0 issues; the other lanes only help with the block table of a paged cache (lane u looks
-    // up the u-th whole-block load of a tile, one tile ahead of its use).
+    // Lane 0 issues; with a paged cache all lanes look up block-table entries (one round serves the loads of
+    // several tiles) and wait for the ring together.
     if (lane == 0) {
       ptx::prefetch_tmap(&tmap_q);
       ptx::prefetch_tmap(&tmap_k);
@@ -595,7 +595,8 @@ inline bool li_sm100_eligible(const DsaLiParams* p) {
     if (p->block_table == nullptr || p->max_blocks < 1) return false;
   }
   // fewer than 64 heads run with zero rows and zero weights in the spare slots: the time of 64 heads whatever
-  // their number, which the CUDA-core kernel does not reach at any (512 x 512, 8 heads: 109 us, here 16 us)
+  // their number.  The CUDA-core kernel, whose time hardly falls with the heads, is slower even with one (512 x
+  // 512: 107 us, here 15 us; 64 x 512: 27 and 14 us; one decode row over 2048 keys: 16 and 13 us)
   if (p->n1 > kLiHeads || p->n2 != 1 || p->d != kLiDim) return false;
   if (p->s1 < 1 || p->s2 < 1) return false;
   if (((uintptr_t)p->query & 15u) || ((uintptr_t)p->key & 15u)) return false;

@@ -1,5 +1,6 @@
-"""The tcgen05 scoring kernel where its dispatch and its lists of work have edges, against the CUDA-core kernel: batches
-that mix row groups of one and of eight rows."""
+"""The tcgen05 scoring kernel where its dispatch and its lists of work have edges, against the CUDA-core kernel: few
+and odd head counts, paged caches whose block-table look-ups take several rounds, batches that mix row groups of
+one and of eight rows."""
 import numpy as np
 import pytest
 import torch
@@ -39,6 +40,25 @@ def _paged(rng, draw, lens, bs):
         table[b, :n] = perm[at:at + n]
         at += n
     return draw(sum(need), bs, 1, 128), torch.from_numpy(table).cuda()
+
+
+@pytest.mark.parametrize("heads", [1, 3, 8, 15])
+@pytest.mark.parametrize("layout,bs", [("BSND", 0), ("TND", 0), ("PA_BSND", 16), ("PA_BSND", 32), ("PA_BSND", 64),
+                                       ("PA_BSND", 128)])
+def test_few_heads(heads, layout, bs):
+    rng, draw = np.random.RandomState(heads), _draw(heads)
+    if layout == "BSND":
+        _compare(draw(2, 9, heads, 128), draw(2, 700, 1, 128), draw(2, 9, heads).float(), sparse_count=64)
+    elif layout == "TND":
+        _compare(draw(14, heads, 128), draw(1500, 1, 128), draw(14, heads).float(), sparse_count=64,
+                 layout_query="TND", layout_key="TND", actual_seq_lengths_query=[1, 13, 14],
+                 actual_seq_lengths_key=[600, 613, 1500])
+    else:
+        # (one round of look-ups serves 32 loads: 512 to 4096 keys)
+        lens = [5000, 130, 4097]
+        k, table = _paged(rng, draw, lens, bs)
+        _compare(draw(3, 2, heads, 128), k, draw(3, 2, heads).float(), sparse_count=64, layout_key="PA_BSND",
+                 block_table=table, actual_seq_lengths_key=lens)
 
 
 @pytest.mark.parametrize("rows", [[1] * 20, [1, 1, 60, 1, 3, 1, 9], [70, 8, 33], [1] * 100, [5, 1, 1, 1, 1, 1]])
