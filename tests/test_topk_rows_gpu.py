@@ -89,9 +89,9 @@ def test_constructed_rows_fp16():
     np.testing.assert_array_equal(got_v, exp_v)
 
 
-def test_a_row_whose_sampled_scores_mislead_is_counted_again():
-    """Rows of 16384 keys or more count only the bins that a sample of 512 positions puts the best K in; a row
-    whose sampled positions hold its only large scores has fewer than K keys there."""
+def test_a_row_whose_sampled_scores_mislead():
+    """A sample of 512 positions sets the scale of the bins; here the sampled positions hold the row's only large
+    scores, so that all other keys share the bins at the far end."""
     S2, K = 20000, 2048
     rng = np.random.RandomState(5)
     v = _bf16(rng.randn(S2))
