@@ -248,11 +248,17 @@ __global__ void __launch_bounds__(128) sfa_compact_kernel(SfaDev p, int2* __rest
 }
 
 // The same for few rows: one block of 8 warps per row, so that a row of 2048 slots is one round of index loads
-// and block-table look-ups instead of four (decode, 8 rows: 16.6 -> 3.8 us, 128 rows: 18.1 -> 4.8 us; the warps of a large call hide
-// that latency behind each other).  Token-wise indices whose rows start on 16-byte boundaries only.
-constexpr int32_t kSfaBlockCompactRows = 4096;
+// and block-table look-ups instead of four (decode, 8 rows: 16.6 -> 3.8 us, 128 rows: 18.1 -> 4.8 us).  Token-wise
+// indices whose rows start on 16-byte boundaries only.
+// Where the line lies: in a call of many rows the warps of the other kernel hide that latency behind each other,
+// and blocks that are mostly idle cost more.  us with a block / a warp per row, unpaged keys:
+//   64 slots:   384 rows 3.0 / 3.3,   512 3.4 / 3.4,   1024 5.1 / 3.6,   4095 14.6 / 4.8
+//   1024 slots: 512 rows 3.7 / 5.3,   1024 5.6 / 5.8,  1536 7.2 / 6.1,   4095 16.0 / 9.3
+//   2048 slots: 1024 rows 6.4 / 9.4,  2048 10.8 / 12.3, 3072 14.7 / 14.3, 4095 18.7 / 16.3
+//   4096 slots: 2048 rows 19.0 / 22.6, 3072 25.9 / 27.0, 4095 33.3 / 31.1
 inline bool sfa_compact_by_blocks(const SfaDev& p) {
-  return p.rows < kSfaBlockCompactRows && p.sparse_block_size == 1 && (p.sparse_count & 3) == 0 &&
+  const int32_t slots = std::min(p.sparse_count, 4096), rows = std::min(3072, std::max(512, slots + slots / 4));
+  return p.rows <= rows && p.sparse_block_size == 1 && (p.sparse_count & 3) == 0 &&
          ((uintptr_t)p.sparse_indices & 15) == 0;
 }
 __global__ void __launch_bounds__(256) sfa_compact_block_kernel(SfaDev p, int2* __restrict__ nvalid,

@@ -397,3 +397,22 @@ def test_the_pre_pass_by_blocks_lists_what_the_pre_pass_by_warps_lists(K):
                                           sparse_mode=0, return_softmax_lse=True) for i in (idx, wide))
     for x, y in zip(a, b):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("K,line", [(64, 512), (600, 750)])
+def test_the_pre_pass_on_either_side_of_its_line(K, line):
+    """With one row more than the line every row is compacted by a warp: the other rows' outputs stay as they are."""
+    from dsa_triton_ascend_b200 import sparse_flash_attention_triton
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(torch.bfloat16)   # noqa: E731
+    S1, S2 = line + 1, 1500
+    q, k, qr, kr = r(1, S1, 16, 512), r(1, S2, 1, 512), r(1, S1, 16, 64), r(1, S2, 1, 64)
+    idx = torch.stack([torch.randperm(S2, generator=gen, device="cuda")[:K] for _ in range(S1)]).int()
+    idx[torch.rand(S1, K, generator=gen, device="cuda") < 0.3] = -1
+    idx[3] = -1
+    both = [sparse_flash_attention_triton(q[:, :n].contiguous(), k, k, idx[:n].view(1, n, 1, K), scale_value=0.04,
+                                          query_rope=qr[:, :n].contiguous(), key_rope=kr, sparse_mode=0,
+                                          return_softmax_lse=True) for n in (line, line + 1)]
+    assert torch.equal(both[0][0], both[1][0][:, :line])
+    for x, y in zip(both[0][1:], both[1][1:]):
+        assert torch.equal(x, y[:, :, :line])
