@@ -1,5 +1,5 @@
-// Sparse flash attention backward on tcgen05 tensor cores for D = 512 (+ 64 rope), one KV head, any
-// head count, BSND / TND, token- or block-wise indices.  Same math as sfa_bwd_mma_kernel
+// Sparse flash attention backward on tcgen05 tensor cores for D = 512 (+ 64 rope), one KV head, 16
+// heads or more, BSND / TND, token- or block-wise indices.  Same math as sfa_bwd_mma_kernel
 // (sparse_flash_attention_grad_triton.py:100-470, golden sparse_flash_attention_grad_numpy.py:96-135):
 //     S  = q . k^T          dP = dO . k_nope^T
 //     P  = exp(S * scale - max) / sum       dS = P * (dP - delta) * scale
@@ -642,8 +642,10 @@ inline int64_t sfa_bwd_rows(const DsaSfaGradParams* p) {
 // The shapes this kernel takes, given the larger workspace and 16-byte aligned tensors.
 inline bool sfa_bwd_sm100_shape(const DsaSfaGradParams* p) {
   if (p->d != 512 || p->d_rope != 64 || p->kernel == DSA_KERNEL_PORTABLE) return false;
-  // (fewer than 16 heads fill one 16-head block of the mma.sync kernel, which needs no lists beside its
-  // accumulators; a block of 64 heads would be mostly padding)
+  // Fewer than 16 heads: the workspace that dsa_sfa_grad_workspace_bytes names for them is the accumulators alone,
+  // a documented figure that callers size from, and this kernel does not fit in it.  Time is not the reason: 512
+  // rows x 2048 of 4096 keys, 1 / 8 / 15 heads: mma.sync 1814 / 1818 / 1838 us, this kernel 1185 / 1185 / 1187; at 16
+  // and 32 heads 1838 and 2655 us against 1187 and 1220.
   if (p->n1 < 16) return false;
   if (p->key_rows < 1 || p->key_rows >= (1ll << 31) - 1) return false;
   const int64_t rows = sfa_bwd_rows(p);

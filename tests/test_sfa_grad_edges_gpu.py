@@ -1,14 +1,17 @@
 """Attention backward where its inputs leave the ordinary: selected keys that do not exist, keys and heads whose
 values are far from the others', rows without statistics.  Each call is compared with one that has to give the
 same result, or with the numpy oracle."""
+import ctypes
 import math
 
 import numpy as np
 import pytest
 import torch
 
+from oracle import sparse_flash_attention_grad_oracle, sparse_flash_attention_oracle
 from oracle.compare import sfa_grad_acceptance_rule
-from tests.util import host, tdtype
+from oracle.inputs import sfa_grad_inputs, sparse_indices
+from tests.util import dev, host, tdtype
 
 pytestmark = pytest.mark.gpu
 NAMES = ("d_query", "d_key", "d_value", "d_query_rope", "d_key_rope")
@@ -191,3 +194,33 @@ def test_the_documented_least_workspace_is_enough(dtype, monkeypatch):
     assert len(asked) == 2 and asked[1] == 256 + S2 * (2 * 512 + 64) * 4 < asked[0]
     for n, a, b in zip(NAMES, got, ref):
         sfa_grad_acceptance_rule(host(a), host(b), dtype, name=n, ulps=1.0)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("N1,tensor", [(15, 0), (16, 1), (17, 1)])
+@pytest.mark.parametrize("S2", [23, 24, 25, 48, 49])
+def test_the_first_tile_and_the_first_head_block(S2, N1, tensor, dtype):
+    """The last row sees S2 keys (half of the tcgen05 kernel's softmax warps have none up to 24, a tile is 48), on
+    either side of the head count at which that kernel begins; 2 ulp of the io dtype, as everywhere."""
+    from dsa_triton_ascend_b200 import _cabi, sparse_flash_attention_grad_triton
+    p = _cabi.DsaSfaGradParams()
+    p.struct_size = ctypes.sizeof(p)
+    for name, kind in p._fields_:
+        if kind is ctypes.c_void_p and name not in ("seq_q", "seq_k"):
+            setattr(p, name, 256)
+    p.batch, p.s1, p.s2, p.n1, p.d, p.d_rope, p.key_rows = 1, 2, S2, N1, 512, 64, S2
+    p.sparse_count, p.sparse_block_size, p.sparse_mode = S2, 1, 3
+    assert _cabi.lib.dsa_sfa_grad_uses_tensor_path(ctypes.byref(p)) == tensor
+    q, k, qr, kr, do = sfa_grad_inputs(S2, 1, 2, S2, N1, 512, 64, dtype)
+    idx = sparse_indices(1000 + S2, 1, 2, S2, S2, 1, 3)
+    out, mx, sm = sparse_flash_attention_oracle(q, k, idx, qr, kr, 1.0 / 24.0, [2], [S2], sparse_mode=3,
+                                                return_softmax_lse=True, dtype=dtype)
+    dt = tdtype(dtype)
+    tk = dev(k, dt)
+    got = sparse_flash_attention_grad_triton(dev(q, dt), tk, tk, dev(idx), dev(do, dt), dev(out, dt), dev(mx), dev(sm),
+                                             scale_value=1.0 / 24.0, query_rope=dev(qr, dt), key_rope=dev(kr, dt),
+                                             sparse_mode=3)
+    ref = sparse_flash_attention_grad_oracle(q, k, idx, do, out, mx, sm, qr, kr, 1.0 / 24.0, [2], [S2], sparse_mode=3,
+                                             dtype=dtype)
+    for n, a, b in zip(NAMES, got, ref):
+        sfa_grad_acceptance_rule(host(a), b, dtype, name=n)

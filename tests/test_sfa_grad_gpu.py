@@ -243,8 +243,8 @@ def test_grad_untouched_rows_are_zero_and_repeat_runs_agree():
     (160, 192, 17, 48),    # more items than SMs, two 16-head steps of which one has a single head
 ])
 def test_grad_at_the_edges_of_tiles_and_head_blocks(S1, S2, N1, K, dtype):
-    """D = 512 kernel (48-key tiles, blocks of 64 heads): same rule as everywhere (2 ulp of the io dtype
-    given the same forward state)."""
+    """D = 512 kernels (tcgen05: 48-key tiles, blocks of 64 heads; the one-head case: mma.sync): same rule as
+    everywhere (2 ulp of the io dtype given the same forward state)."""
     from dsa_triton_ascend_b200 import sparse_flash_attention_grad_triton
     q, k, qr, kr, do = sfa_grad_inputs(91, 1, S1, S2, N1, 512, 64, dtype)
     idx = sparse_indices(1091, 1, S1, S2, K, 1, 3)
