@@ -46,8 +46,10 @@ struct SliGradDev {
   void* d_weights;          // [rows, g], dtype_w
   void* d_key_index;        // [batch * s2, d_idx]
   float* loss;              // [1]
-  float* di;                // [rows, topk]  scratch, zeroed by the caller: index scores, then dI
-  float* p_buf;             // [rows, topk]  scratch, zeroed by the caller: sum over heads of the attention probabilities
+  // Scratch of which a row's first n slots are defined (n: sli_row_slots), the others may hold anything.  Kernels
+  // that add into them (the mma.sync kernels, several head chunks or parts) get them zeroed by the caller.
+  float* di;                // [rows, topk]  index scores, then dI
+  float* p_buf;             // [rows, topk]  sum over heads of the attention probabilities
   float* loss_parts;        // [rows]        scratch
   float* di_max;            // [rows]        scratch: largest |dI| of the row; null: not wanted
   float* dki_acc;           // [batch * s2, d_idx] scratch, zeroed by the caller

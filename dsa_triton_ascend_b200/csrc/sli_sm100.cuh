@@ -64,7 +64,9 @@ __device__ __forceinline__ int32_t sli_key_row(const SliGradDev& p, const int32_
   return j < n ? b * p.s2 + sli_slot_key(p, idx_row, j) : none;
 }
 
-template <bool ATT>
+// PAD: the last chunk of attention heads is not full.  Q of the missing ones is zero, their scores are NaN beside an
+// infinite key; compiled apart because the test costs the others 1 % (2048 rows x 128 heads: 1658 -> 1674 us).
+template <bool ATT, bool PAD>
 __global__ void __launch_bounds__(kScThreads, 1)
 sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid_constant__ CUtensorMap tmap_kb,
                        const __grid_constant__ CUtensorMap tmap_qa, const __grid_constant__ CUtensorMap tmap_qb,
@@ -124,6 +126,7 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
       const float2* pm = prm + mb * 128;
       ok = wait(&m_full[mb], (n_item >> 1) & 1);
       float* out_row = a.out + (int64_t)it.row * a.p.topk;
+      const int32_t hn = PAD ? min(a.hp, a.heads - it.h0) : a.hp;
       for (int32_t t = it.t0; t < it.t1 && ok; ++t, ++n_tile) {
         if ((int)(n_tile & 1) != wg) continue;
         ok = wait(&s_full[wg], (n_tile >> 1) & 1);
@@ -141,6 +144,10 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s_empty[wg]);
+          }
+          if (PAD && c + 32 > hn) {
+#pragma unroll
+            for (int h = 0; h < 32; ++h) v[h] = c + h < hn ? v[h] : 0.f;
           }
 #pragma unroll
           for (int h = 0; h < 32; h += 2) {
@@ -1027,8 +1034,9 @@ inline int sli_sm100_prepare(int* sms_out) {
     // (idempotent: two threads that get here together do the same thing)
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1 ||
-        cudaFuncSetAttribute(sli_score_sm100_kernel<true>, attr, (int)kSlSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(sli_score_sm100_kernel<false>, attr, (int)kSlSmemMax) != cudaSuccess ||
+        cudaFuncSetAttribute(sli_score_sm100_kernel<true, false>, attr, (int)kSlSmemMax) != cudaSuccess ||
+        cudaFuncSetAttribute(sli_score_sm100_kernel<true, true>, attr, (int)kSlSmemMax) != cudaSuccess ||
+        cudaFuncSetAttribute(sli_score_sm100_kernel<false, false>, attr, (int)kSlSmemMax) != cudaSuccess ||
         cudaFuncSetAttribute(sli_mha_sm100_kernel, attr, (int)kMhSmemBytes) != cudaSuccess ||
         cudaFuncSetAttribute(sli_grad_sm100_kernel<__nv_bfloat16>, attr, (int)kSgSmemBytes) != cudaSuccess ||
         cudaFuncSetAttribute(sli_grad_sm100_kernel<__half>, attr, (int)kSgSmemBytes) != cudaSuccess)
@@ -1090,8 +1098,9 @@ inline int sli_score_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d
                           bf16))
     return DSA_ERR_CUDA;
   const int grid = std::min(a.items, sms);
-  if (att) sli_score_sm100_kernel<true><<<grid, kScThreads, smem, st>>>(tka, tkb, tqa, tqb, a);
-  else sli_score_sm100_kernel<false><<<grid, kScThreads, smem, st>>>(tka, tkb, tqa, tqb, a);
+  if (!att) sli_score_sm100_kernel<false, false><<<grid, kScThreads, smem, st>>>(tka, tkb, tqa, tqb, a);
+  else if (a.heads % a.hp) sli_score_sm100_kernel<true, true><<<grid, kScThreads, smem, st>>>(tka, tkb, tqa, tqb, a);
+  else sli_score_sm100_kernel<true, false><<<grid, kScThreads, smem, st>>>(tka, tkb, tqa, tqb, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
   return DSA_OK;

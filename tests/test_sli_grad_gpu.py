@@ -156,3 +156,26 @@ def test_sli_grad_agrees_with_autograd_of_the_kl_loss():
         a, b = host(a), b.numpy()
         assert np.abs(a - b).max() <= 3e-3 * np.abs(b).max() + 1e-6, f"{name}: {np.abs(a - b).max()} vs {np.abs(b).max()}"
     assert abs(float(got[3][0]) - clamped) <= 1e-3 * abs(clamped)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_heads_past_the_last_one_add_nothing_beside_an_infinite_key(dense):
+    """17 attention heads (padded to 32) and a key whose score is -Inf in each of them: its probability is 0, as for
+    a key of score -5000."""
+    from dsa_triton_ascend_b200 import dense_loss_backward_triton, sparse_lightning_indexer_grad_kl_loss_triton
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: (torch.randn(*s, generator=gen, device="cuda") * 0.3).to(torch.bfloat16)   # noqa: E731
+    S1, S2, N1, G, K = 4, 150, 17, 8, 140
+    q, k, qi, ki, w = r(1, S1, N1, 128), r(1, S2, 1, 128), r(1, S1, G, 128), r(1, S2, 1, 128), r(1, S1, G).abs()
+    q[..., 0], k[..., 0] = -1, 0
+    mx, sm = torch.zeros(1, 1, S1, N1, device="cuda"), torch.full((1, 1, S1, N1), 150.0, device="cuda")
+    idx = torch.arange(K, dtype=torch.int32, device="cuda").expand(1, S1, 1, K).contiguous()
+    out = []
+    for far in (math.inf, 6e4):
+        k[:, 5, 0, 0] = far
+        args = (q, k, qi, ki, w)
+        out.append(dense_loss_backward_triton(*args, mx, sm, scale_value=1.0 / 12.0) if dense else
+                   sparse_lightning_indexer_grad_kl_loss_triton(*args, idx, mx, sm, scale_value=1.0 / 12.0))
+    for a, b in zip(*out):
+        assert torch.isfinite(a).all()
+        torch.testing.assert_close(a.float(), b.float(), rtol=2.0 ** -7, atol=1e-6)
