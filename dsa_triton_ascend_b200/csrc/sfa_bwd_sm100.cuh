@@ -5,11 +5,11 @@
 //     P  = exp(S * scale - max) / sum       dS = P * (dP - delta) * scale
 //     dQ += dS . k          dK += dS^T . q  dV += P^T . dO
 //
-// What bounds it: the scatter-adds.  A selected (row, key) pair adds 1088 fp32 values to d_key /
-// d_value, 4.6 GB for 512 rows x 2048 keys x 64 heads, and the L2 takes whole-line fp32 reductions at
+// What it is built around: the scatter-adds.  A selected (row, key) pair adds 1088 fp32 values to d_key /
+// d_value, 4.56 GB for 512 rows x 2048 keys x 64 heads, and the L2 takes whole-line fp32 reductions at
 // 6.2 TB/s (lanes that cover 32-byte sectors only: 3.7 TB/s) whichever instruction brings them (scalar,
 // 16-byte or bulk).  So a block covers 64 heads - every reduction then carries 64 heads - and everything
-// else is arranged to hide behind the stream of reductions:
+// else is arranged to run beside the stream of reductions:
 //
 //   * A work item is (query row, 64 heads).  Q and dO stay in shared memory for the whole row (136 KB),
 //     keys come 48 at a time (TMA gather4, 54 KB, one buffer).
@@ -26,10 +26,13 @@
 //     scaled by 2^13, dS by a power of two per item that keeps |dS| <= scale * (|dO| |v| + |delta|)
 //     (Cauchy-Schwarz over the item's heads and selected keys, taken by small kernels in front) below 2^13.
 //
-// Measured, B1 S1 512 S2 4096 N1 64 k 2048, bf16: 1.26 ms for the operator call (sfa_bwd_mma_kernel: 4.63
-// ms); 4092 rows x 128 heads: 7.1 ms (32.2 ms).  ncu: 3.4 TB/s of reductions, tensor pipe 22 % busy, the
-// load / store unit's data pipe - which a reduction of one line holds for 4.5 cycles - 66 % (77 % while
-// every SM has work).
+// Measured, whole operator call: B1 S1 512 S2 4096 N1 64 k 2048 1.26 ms in bf16, 1.29 ms in fp16
+// (sfa_bwd_mma_kernel: 4.63 ms); 4092 rows x 128 heads in bf16 7.6 ms (32.2 ms).  ncu, the first of them, this kernel alone: 1.27
+// ms, 3.6 TB/s of reductions, tensor pipe 28 %, L2 41 %, load / store data pipe 33 %.  No unit is full: what is
+// left is the chain of a tile (S -> P -> dS -> products; P is made by four warps, and expf(..) / sum in the place of their
+// exp2 and product takes the call to 1.58 ms), the reload of Q / dO between items, and the last of the four
+// rounds that 512 items make on 148 SMs.
+// ptxas spills 20 bytes (bf16) and 88 bytes (fp16) of a thread's 72 registers.
 //
 // Tensor memory: dQ^T 5 x 64 columns | S, dP 48 | rope part of S 48 | drain ring 2 x 48.
 // Warps (896 threads): 0..7 softmax (lane quarter = warp & 3: quarters 0, 1 hold S of heads 0..63,

@@ -494,9 +494,10 @@ sli_mha_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid_c
 }
 
 // ---- gradients -----------------------------------------------------------------------------------
-// What bounds it: the scatter-adds of dKI (512 B per (row, key): 2300 cycles of the load / store unit
+// What it is built around: the scatter-adds of dKI (512 B per (row, key): 2300 cycles of the load / store unit
 // per 128 keys, 4.5 per line; all SMs together 6.2 TB/s), against 1300 cycles of tensor pipe and 1170 of
-// gather.  So a work item is (query row, 64 index heads), which makes every reduction carry all heads
+// gather.  ncu, 512 rows x 2048 keys, 64 heads: 174 us, 3.1 TB/s of reductions, load / store data pipe 41 %, tensor
+// pipe 29 % (dense over 3840 keys a row: 286 us, 3.5 TB/s, 44 %, 33 %).  So a work item is (query row, 64 index heads), which makes every reduction carry all heads
 // of up to 64, and as in sfa_bwd_sm100.cuh the gradient products run with FEATURES on the lanes, so that a
 // reduction instruction is one full line.  Per tile of 128 gathered keys (M = the first named):
 //     S   [keys, heads]     = K . QI^T                              E = S > 0
@@ -505,7 +506,8 @@ sli_mha_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid_c
 // E is exact in 16 bits.  w QI (once per row) and dI (once per key) enter as a high and a low io-dtype part
 // (x = hi + lo up to 2^-16 relative for bf16, 2^-22 for fp16), dI E is then two masked copies of the parts
 // without a conversion per element.  fp16: both are scaled by a power of two per row taken from the
-// row's largest magnitude.  dW = sum_k dI relu(S) is summed in fp32 registers.
+// row's largest magnitude (sli_grad_kernel scales dI per 64 keys; all terms meet in one sum, whose error the row's largest
+// decides either way).  dW = sum_k dI relu(S) is summed in fp32 registers.
 // Tensor memory: S 2 x 64 columns | dKI^T 2 x 128 | dQI^T 64.
 // Warps: 0..7 epilogue (lane quarter x 32 heads), 8..15 drain (lane quarter x 64 keys), 16..23 gather, 24
 // issuer of S / dKI, 25 issuer of dQI, 26..27 QI and w QI.  (A thread issues a product of 64 columns only every
