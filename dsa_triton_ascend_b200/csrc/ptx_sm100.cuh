@@ -229,6 +229,17 @@ __device__ __forceinline__ void tma_gather4_2d(void* dst, const CUtensorMap* m, 
       : "memory");
 }
 
+// ---- cp.async -------------------------------------------------------------------------------------
+// 16 bytes of global memory into shared memory; `bytes` (0 or 16) of them are read, the rest is zero.
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// One arrival of this thread on the barrier once all its earlier cp.async copies have landed (counted in the
+// barrier's expected arrivals: nothing is added to them here).
+__device__ __forceinline__ void cp_async_mbar_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // ---- tcgen05: tensor memory ---------------------------------------------------------------------
 // One warp allocates `cols` (power of two, 32..512) columns; the base address lands in *dst_smem.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t cols) {

@@ -18,13 +18,15 @@
 // shared-memory offsets, the score product needs identical features at an offset and the value
 // product identical keys.
 //
-// Data movement.  Only the K block is gathered from L2: TMA tile::gather4 loads into the
-// 128-byte-swizzled MMA layout, issued by six producer warps from a front-packed list of physical
-// KV rows that a pre-pass kernel writes.  The SM's TMA unit is the scarce resource here (it
-// saturates at one 512-byte gather4 per ~18 cycles, bulk copies included), so the V block is not
-// gathered a second time: four copier warps build it from the K block, which already holds this
-// CTA's 32 keys with all columns - plain loads / stores for the columns this CTA owns, st.async
-// into the peer's shared memory for the columns the peer owns.
+// Data movement.  Both blocks are gathered from L2 with 16-byte cp.async copies straight into the 128-byte-swizzled
+// MMA layout, K by six producer warps and V by four, from a front-packed list of physical KV rows that a pre-pass
+// kernel writes; a copy's completion is an arrival on the slot's barrier, so that no warp waits for its own copies.
+// An SM takes 72 B/clk this way (12 warps with 16 KB in flight each); TMA tile::gather4 takes one 512-byte load per
+// 16.5 cycles (31 B/clk), whatever else the SM does.  The 32 keys that both blocks share are loaded twice: building
+// V from the K block instead (loads, stores and st.async to the peer) holds the K slot until the copy is done
+// and costs the shared memory 512 cycles of traffic per tile against 256.  attend 15360 tokens x 128 heads, top-k
+// 2048, in turn with the version that gathered K with gather4 and copied V: 8130 -> 7167 us; 1471 ragged tokens x
+// 64 heads, indexer included: 629 -> 570 us.
 //
 // Accumulator layout of a pair MMA with M = 128 (measured): lanes 0..63 hold a CTA's rows with the
 // first half of N, lanes 64..127 the same rows with the second half.  So TMEM lane L of CTA c
@@ -47,7 +49,7 @@
 //
 // Warps (768 threads): 0..5 K gather producers, 6 Q loader, 8..10 QK^T issuers (issuer i owns
 // feature blocks 3i..3i+2 and a partial S: one thread issues a short N = 64 MMA only every 60-90
-// cycles), 11 PV issuer, 12..15 V copiers, 16..19 / 20..23 softmax groups.  MMAs are issued by the
+// cycles), 11 PV issuer, 12..15 V gather, 16..19 / 20..23 softmax groups.  MMAs are issued by the
 // even CTA only; in the odd CTA the issuer warps relay "my operand has landed" to the even CTA's
 // barriers instead.  All waits are bounded; a wait that gives up sets the status word.
 #pragma once
@@ -71,7 +73,7 @@ constexpr int kSfaKWarps = 6;        // warps 0..5: two per issuer
 constexpr int kSfaQWarp = 6;         // Q loader (warp 7 idle)
 constexpr int kSfaQkWarp0 = 8;       // warps 8..10
 constexpr int kSfaPvWarp = 11;
-constexpr int kSfaCopyWarp0 = 12;    // warps 12..15
+constexpr int kSfaVWarp0 = 12;    // warps 12..15
 constexpr int kSfaSoftWarp0 = 16;    // warps 16..19 (group 0), 20..23 (group 1)
 constexpr int kSfaDv = 512;
 constexpr int kSfaMaxSlots = 8192;   // sparse_count * sparse_block_size served by this kernel
@@ -97,12 +99,10 @@ static_assert(kSfaSmemBytes <= 232448, "shared memory");
 // setmaxnreg.inc only ever gets registers that warps of the SAME CTA have released and blocks (for
 // good) until it has them: what the softmax warps ask for must fit into what the others give back.
 constexpr int kSfaLaunchRegs = 80;   // 65536 / 768 threads, rounded down to a multiple of 8
-constexpr int kSfaRegsLow = 56;      // warps 0..11
-constexpr int kSfaRegsCopy = 104;    // warps 12..15 (a tile's 16 chunks of 16 bytes sit in registers)
+constexpr int kSfaRegsLow = 56;      // warps 0..15
 constexpr int kSfaRegsHigh = 104;    // warps 16..23
-static_assert((kSfaRegsHigh - kSfaLaunchRegs) * (kSfaThreads / 32 - kSfaSoftWarp0) +
-                      (kSfaRegsCopy - kSfaLaunchRegs) * (kSfaSoftWarp0 - kSfaCopyWarp0) <=
-                  (kSfaLaunchRegs - kSfaRegsLow) * kSfaCopyWarp0,
+static_assert((kSfaRegsHigh - kSfaLaunchRegs) * (kSfaThreads / 32 - kSfaSoftWarp0) <=
+                  (kSfaLaunchRegs - kSfaRegsLow) * kSfaSoftWarp0,
               "setmaxnreg: more registers requested than released");
 static_assert(kSfaLaunchRegs * kSfaThreads <= 65536, "register file");
 
@@ -125,6 +125,7 @@ struct SfaSm100Args {
   // normalised fp32 partial output with its own maximum and sum, merged by sfa_merge_kernel.
   int32_t split, part_keys;
   int32_t items;            // rows * split
+  int32_t kv_rows;          // of the KV tensor: a listed row past them (an absent page) loads zeros
   float* part_o;            // [items, 128, 512] fp32 (split > 1)
   float* part_m;            // [items, 128] maximum of the scaled scores of the part (natural log units)
   float* part_l;            // [items, 128] sum of exp(score - maximum); 0 marks an empty part
@@ -368,8 +369,7 @@ __device__ long long g_sfa_prof[128];
 // prefill instantiation carries none of it.
 template <bool kSplit>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSfaThreads, 1)
-sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_constant__ CUtensorMap tmap_kr,
-                     const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_qr,
+sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_qr,
                      const SfaSm100Args a) {
   extern __shared__ __align__(1024) unsigned char sfa_sm[];
   unsigned char* q_s = sfa_sm + kSfaOffQ;
@@ -382,11 +382,11 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
   uint64_t* bars = reinterpret_cast<uint64_t*>(sfa_sm + kSfaOffBar);
   // K barriers are indexed [slot * 3 + issuer]: every issuer's three feature blocks are handed over
   // and released on their own.
-  uint64_t* k_full = bars;         // [6] gather -> QK issuer / relay, copiers              (tx bytes)
-  uint64_t* k_empty = bars + 6;    // [6] blocks read by the issuer's MMAs (commit) and by the four copier warps -> K producers
+  uint64_t* k_full = bars;         // [6] gather -> QK issuer / relay                       (64 lanes' copies)
+  uint64_t* k_empty = bars + 6;    // [6] blocks read by the issuer's MMAs -> K producers   (commit, both CTAs)
   uint64_t* k_ready = bars + 12;   // [6] even CTA only: the odd CTA's blocks have landed
-  uint64_t* v_full = bars + 18;    // [2] own copier warps (4 arrivals + 1 arming) and the peer's st.async bytes -> PV issuer / relay
-  uint64_t* v_empty = bars + 20;   // [2] PV of the tile done -> copiers                     (commit, both CTAs)
+  uint64_t* v_full = bars + 18;    // [2] gather -> PV issuer / relay                       (128 lanes' copies)
+  uint64_t* v_empty = bars + 20;   // [2] PV of the tile done -> V gather                    (commit, both CTAs)
   uint64_t* v_ready = bars + 22;   // [2] even CTA only: the odd CTA's V slot is complete
   uint64_t* s_full = bars + 24;    // [2] all three partial products done -> softmax group   (commit x 3, both CTAs)
   uint64_t* s_empty = bars + 26;   // [2] even CTA only: the group's warps of both CTAs hold S in registers
@@ -414,10 +414,10 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
   const bool misaligned = (ptx::smem_u32(sfa_sm) & 1023u) != 0;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 6; ++i) {
-      ptx::mbar_init(&k_full[i], 1); ptx::mbar_init(&k_empty[i], 5); ptx::mbar_init(&k_ready[i], 1);
+      ptx::mbar_init(&k_full[i], 64); ptx::mbar_init(&k_empty[i], 1); ptx::mbar_init(&k_ready[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(&v_full[i], 5); ptx::mbar_init(&v_empty[i], 1); ptx::mbar_init(&v_ready[i], 1);
+      ptx::mbar_init(&v_full[i], 128); ptx::mbar_init(&v_empty[i], 1); ptx::mbar_init(&v_ready[i], 1);
       ptx::mbar_init(&s_full[i], kSfaQkLanes); ptx::mbar_init(&s_empty[i], 8);
       ptx::mbar_init(&p_full[i], 8); ptx::mbar_init(&p_empty[i], 1);
     }
@@ -450,30 +450,27 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
   auto item_tiles = [&](int32_t item) -> int32_t { return (a.nvalid[item].x + kSfaBK - 1) / kSfaBK; };
 
   // Registers: kSfaLaunchRegs per thread at launch; producers and issuers give some back, the
-  // copier and softmax warps take them (whole warpgroups of four warps change together).  Each
+  // softmax warps take them (whole warpgroups of four warps change together).  Each
   // class of roles sits in its own branch, right under its setmaxnreg: the compiler budgets a
   // branch by the setmaxnreg that dominates it.
-  if (warp < kSfaCopyWarp0) {
+  if (warp < kSfaVWarp0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSfaRegsLow));
     if (*abort_flag) {
       // nothing started: fall through to the teardown
     } else if (warp < kSfaKWarps) {
       // ------------------------------------------------------------------ K gather producers
-      // Two warps per QK^T issuer: 8 row groups (4 of this CTA's 32 keys each) x the issuer's 3
-      // column blocks = 24 gather4 loads of 512 bytes per tile, dealt out over the two warps.  The
-      // lanes of a warp issue one after the other (~100 cycles per load), warps issue in parallel
-      // until the SM's TMA unit saturates at one load per ~18 cycles.
+      // Two warps per QK^T issuer: 16 of this CTA's 32 keys each x the issuer's 3 column blocks = 12 copies per lane
+      // and tile (one instruction: 4 keys x 128 bytes).
       const int qi = warp >> 1;                          // the issuer this warp feeds
-      const int gw = warp & 1;
-      const int o = gw + 2 * lane;
-      const bool active = o < 24;
-      const int grp = o / 3, blk = 3 * qi + (o - grp * 3);
-      const int key0 = (int)rank * kSfaHalfBK + grp * 4;   // first key (within the tile) of this load
-      const int32_t x = blk < 8 ? blk * 64 : 0;
-      unsigned char* slot0 = k_s + blk * kSfaKBlk + grp * 512;
+      const int key_w = (warp & 1) * 16 + (lane >> 3);   // this lane's keys of the CTA's 32: key_w + 4 j
+      const int key0 = (int)rank * kSfaHalfBK + key_w;   // .. of the tile
+      const int ch = lane & 7;
+      const uint32_t dst0 = ptx::smem_u32(k_s) + 3 * qi * kSfaKBlk + key_w * 128 + ((ch ^ (key_w & 7)) << 4);
+      const uint32_t dst1 = ptx::smem_u32(k_s) + 3 * qi * kSfaKBlk + (key_w + 4) * 128 + ((ch ^ ((key_w + 4) & 7)) << 4);
+      const unsigned char* kn = (const unsigned char*)a.p.key + qi * 384 + ch * 16;
+      const unsigned char* kr = (const unsigned char*)a.p.key_rope + ch * 16;
       uint64_t* full = k_full + qi;                      // slot s: full[s * 3]
       uint64_t* empty = k_empty + qi;
-      if (lane == 0) { ptx::prefetch_tmap(&tmap_kn); ptx::prefetch_tmap(&tmap_kr); }
       // The row numbers of a tile come from global memory (the pre-pass list); they are fetched one
       // tile ahead so that their latency never sits between a freed slot and the gather.
       struct TilePos { int32_t item, t, ntiles, nvalid, off; };
@@ -484,20 +481,13 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
         }
         return TilePos{a.items, 0, 0, 0, 0};
       };
-      // (the four keys of a load are consecutive entries of the list: one 16-byte load when the
-      // row's list starts on a 16-byte boundary, except in a row's last tile, where keys past the
-      // end re-read the tile's first key and are masked by the softmax)
+      // (in a row's last tile keys past the end re-read the tile's first key and are masked by the softmax)
       auto load_rows = [&](const TilePos& tp, int32_t* r) {
-        if (!active || tp.item >= a.items) { r[0] = r[1] = r[2] = r[3] = 0; return; }
+        if (tp.item >= a.items) { r[0] = r[1] = r[2] = r[3] = 0; return; }
         const int32_t* list = a.key_list + tp.off + tp.t * kSfaBK;
-        if ((tp.t + 1) * kSfaBK <= tp.nvalid && (tp.off & 3) == 0) {
-          const int4 v = *reinterpret_cast<const int4*>(list + key0);
-          r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
-        } else {
-          const int32_t left = tp.nvalid - tp.t * kSfaBK;
+        const int32_t left = tp.nvalid - tp.t * kSfaBK;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) r[i] = list[key0 + i < left ? key0 + i : 0];
-        }
+        for (int j = 0; j < 4; ++j) r[j] = list[key0 + 4 * j < left ? key0 + 4 * j : 0];
       };
       uint32_t n_tile = 0;
       bool ok = true;
@@ -511,20 +501,23 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
         load_rows(nxt, rn);
         const uint32_t s = n_tile & 1, use = n_tile >> 1;
         SFA_PROF(0);
-        // every lane polls (see ptx::mbar_wait_warp): the gather below is issued for the lanes one
-        // after the other and must find the warp converged.  Like every wait of this kernel it
-        // spins without suspending: waking from a suspended try_wait costs hundreds of cycles at
+        // every lane polls (see ptx::mbar_wait_warp).  Like every wait of this kernel it spins without suspending: waking from a suspended try_wait costs hundreds of cycles at
         // every hand-over (826 vs 640 TFLOP/s on a 4096-token, top-2048 case).
         ok = ptx::mbar_spin_warp(&empty[s * 3], (use & 1) ^ 1, abort_flag);
         if (!ok) break;
         SFA_PROF(1);
-        if (gw == 0 && lane == 0) ptx::mbar_arrive_expect_tx(&full[s * 3], kSfaKSub);
-        __syncwarp();
-        if (active) {
-          if (blk == 8) ptx::tma_gather4_2d(slot0 + s * kSfaKSlot, &tmap_kr, &full[s * 3], 0, rc[0], rc[1], rc[2], rc[3]);
-          else ptx::tma_gather4_2d(slot0 + s * kSfaKSlot, &tmap_kn, &full[s * 3], x, rc[0], rc[1], rc[2], rc[3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          // a row past the cache (an absent page) loads zeros
+          const uint32_t bytes = rc[j] < a.kv_rows ? 16u : 0u;
+          const int64_t row = rc[j] < a.kv_rows ? rc[j] : 0;
+          const uint32_t dst = ((j & 1) ? dst1 : dst0) + s * kSfaKSlot + (j >> 1) * 1024;
+          const unsigned char* src = kn + row * (kSfaDv * 2);
+          ptx::cp_async_16(dst, src, bytes);
+          ptx::cp_async_16(dst + kSfaKBlk, src + 128, bytes);
+          ptx::cp_async_16(dst + 2 * kSfaKBlk, qi == 2 ? kr + row * 128 : src + 256, bytes);
         }
-        __syncwarp();
+        ptx::cp_async_mbar_arrive(&full[s * 3]);
         SFA_PROF(2);
         ++n_tile;
         cur = nxt;
@@ -599,9 +592,12 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
           if (!ok) break;
           SFA_PROF(1);
           if (rank != 0) {
-            // relaxed: the blocks were written by the TMA unit and are complete once the barrier
-            // says so; nothing of this thread's own has to be published
-            if (ptx::elect_one()) ptx::mbar_arrive_remote_relaxed(k_ready_lead + kb * 8, 0u);
+            // the blocks were written through the generic proxy: order them before the tensor core's reads of this
+            // CTA's shared memory, then tell the issuer; nothing of this thread's own has to be published
+            if (ptx::elect_one()) {
+              ptx::fence_proxy_async_smem();
+              ptx::mbar_arrive_remote_relaxed(k_ready_lead + kb * 8, 0u);
+            }
             __syncwarp();
             continue;
           }
@@ -612,6 +608,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
           SFA_PROF(3);
           ptx::tc_fence_after();
           if (ptx::elect_one()) {
+            ptx::fence_proxy_async_smem();   // (the copies went through the generic proxy)
 #pragma unroll
             for (int f = 0; f < 3; ++f) {
 #pragma unroll
@@ -654,8 +651,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
           if (!ok) break;
           SFA_PROF(1);
           if (rank != 0) {
-            // the peer's rows arrived through the generic proxy: order them before the tensor core's
-            // reads of this CTA's shared memory, then tell the issuer
+            // (as the K relays)
             if (ptx::elect_one()) {
               ptx::fence_proxy_async_smem();
               ptx::mbar_arrive_remote_relaxed(v_ready_lead + b * 8, 0u);
@@ -670,7 +666,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
           SFA_PROF(3);
           ptx::tc_fence_after();
           if (ptx::elect_one()) {
-            ptx::fence_proxy_async_smem();   // the V rows the peer stored into this CTA (generic proxy)
+            ptx::fence_proxy_async_smem();   // (the copies went through the generic proxy)
 #pragma unroll
             for (int ks = 0; ks < kSfaBK / 16; ++ks) {
               const uint64_t ad = ptx::desc_kmajor_sw128(p_addr + b * kSfaPBuf + ks * 32);
@@ -692,76 +688,53 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
       SFA_PROF_STORE(3, lane == 0);
     }
   } else if (warp < kSfaSoftWarp0) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSfaRegsCopy));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSfaRegsLow));
     if (!*abort_flag) {
-      // ------------------------------------------------------------------ V copiers
-      // These 128 threads copy the four column blocks of the K slot that this CTA owns as value
-      // columns into its own V slot (plain loads and stores) and the four that the peer owns into
-      // the peer's V slot (st.async: the bytes are counted on the peer's barrier when they land,
-      // the sender does not wait), rows 32*rank.. of every block; 16 chunks of 16 bytes per thread.
-      // Byte offsets inside 4 KB are kept, so the 128-byte swizzle pattern carries over.
-      const int tid = (warp - kSfaCopyWarp0) * 32 + lane;
-      const uint32_t peer = rank ^ 1u;
-      const uint32_t v_peer = ptx::map_to_rank(v_s, peer);
-      const uint32_t v_full_peer = ptx::map_to_rank(v_full, peer);
+      // ------------------------------------------------------------------ V gather
+      // 16 of the tile's 64 keys per warp x the four column blocks that this CTA owns as value columns: 16 copies per
+      // lane and tile (one instruction: 4 keys x 128 bytes).
+      const int key_w = (warp - kSfaVWarp0) * 16 + (lane >> 3), ch = lane & 7;      // this lane's keys: key_w + 4 j
+      const uint32_t dst0 = ptx::smem_u32(v_s) + key_w * 128 + ((ch ^ (key_w & 7)) << 4);
+      const uint32_t dst1 = ptx::smem_u32(v_s) + (key_w + 4) * 128 + ((ch ^ ((key_w + 4) & 7)) << 4);
+      const unsigned char* kn = (const unsigned char*)a.p.key + rank * 256 + ch * 16;
       uint32_t n_tile = 0;
       bool ok = true;
       SFA_PROF_DECL;
       for (int32_t item = cluster_id; item < a.items && ok; item += n_clusters) {
-        const int32_t ntiles = item_tiles(item);
+        const int2 nv = a.nvalid[item];
+        const int32_t ntiles = (nv.x + kSfaBK - 1) / kSfaBK;
+        const int32_t* list = a.key_list + nv.y;
+        int32_t rn[4];
+        auto load_rows = [&](int32_t t) {
+          const int32_t left = nv.x - t * kSfaBK;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) rn[j] = left > 0 ? list[t * kSfaBK + (key_w + 4 * j < left ? key_w + 4 * j : 0)] : 0;
+        };
+        load_rows(0);
         for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
           const uint32_t b = n_tile & 1, use = n_tile >> 1;
-          SFA_PROF(0);
-          ok = ptx::mbar_spin_warp(&k_full[b * 3], use & 1, abort_flag) &&
-               ptx::mbar_spin_warp(&k_full[b * 3 + 1], use & 1, abort_flag) &&
-               ptx::mbar_spin_warp(&k_full[b * 3 + 2], use & 1, abort_flag);
-          if (!ok) break;
-          SFA_PROF(1);
-          // The tile's 16 chunks go into registers first and the K slot is handed back at once: its
-          // refill must not wait for the V slot, which is only free when the value product two
-          // tiles back has completed (the registers act as a third V stage).
-          const unsigned char* ksrc = k_s + b * kSfaKSlot;
-          uint4 v[16];
+          int32_t r[4];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            // i < 8: the four blocks this CTA owns (local copy), i >= 8: the four the peer owns (remote)
-            const int owner = i < 8 ? (int)rank : (int)peer;
-            const int q = (i & 7) * 128 + tid;                  // 0..1023: chunk within the four blocks
-            const int pblk = q >> 8, within = q & 255;
-            const int fblk = 4 * (pblk >> 1) + 2 * owner + (pblk & 1);
-            v[i] = *reinterpret_cast<const uint4*>(ksrc + fblk * kSfaKBlk + within * 16);
-          }
-          // The slot goes back to the TMA unit: reads through the generic proxy (the loads above)
-          // and the writes of the next gather through the async proxy are only ordered by a proxy
-          // fence.  Without it the gather was seen to overtake these loads (outputs changed from
-          // run to run once the hand-overs of this kernel got fast).
-          ptx::fence_proxy_async_smem();
-          __syncwarp();
-          if (lane < 3) ptx::mbar_arrive(&k_empty[b * 3 + lane]);
-          SFA_PROF(2);
-          // V slot b is free in both CTAs once the product that read it has completed
+          for (int j = 0; j < 4; ++j) r[j] = rn[j];
+          load_rows(t + 1);
+          SFA_PROF(0);
           ok = ptx::mbar_spin_warp(&v_empty[b], (use & 1) ^ 1, abort_flag);
           if (!ok) break;
-          SFA_PROF(3);
-          // the peer's half of my V slot: 16 KB of transaction bytes
-          if (tid == 0) ptx::mbar_arrive_expect_tx(&v_full[b], kSfaVSlot / 2);
-          const uint32_t vdst = b * kSfaVSlot + rank * kSfaKBlk;     // rows 32*rank.. of a V block
+          SFA_PROF(1);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int q = (i & 7) * 128 + tid;
-            const int pblk = q >> 8, within = q & 255;
-            const uint32_t off = vdst + pblk * kSfaVBlk + within * 16;
-            if (i >= 8) ptx::st_async_v4(v_peer + off, v[i], v_full_peer + b * 8);
-            else *reinterpret_cast<uint4*>(v_s + off) = v[i];
+          for (int j = 0; j < 4; ++j) {
+            // a row past the cache (an absent page) loads zeros
+            const uint32_t bytes = r[j] < a.kv_rows ? 16u : 0u;
+            const unsigned char* src = kn + (int64_t)(r[j] < a.kv_rows ? r[j] : 0) * (kSfaDv * 2);
+            const uint32_t dst = ((j & 1) ? dst1 : dst0) + b * kSfaVSlot + (j >> 1) * 1024;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ptx::cp_async_16(dst + q * kSfaVBlk, src + (q >> 1) * 512 + (q & 1) * 128, bytes);
           }
-          // the local rows are made visible to the tensor core's reads before the arrival says so
-          ptx::fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&v_full[b]);
-          SFA_PROF(4);
+          ptx::cp_async_mbar_arrive(&v_full[b]);
+          SFA_PROF(2);
         }
       }
-      SFA_PROF_STORE(1, tid == 0);
+      SFA_PROF_STORE(1, warp == kSfaVWarp0 && lane == 0);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSfaRegsHigh));
@@ -1217,6 +1190,7 @@ inline int sfa_sm100_launch(const DsaSfaParams* p, const SfaDev& d, int32_t* sta
   a.split = split;
   a.part_keys = part_keys;
   a.items = d.rows * split;
+  a.kv_rows = (int32_t)p->key_rows;
   a.part_m = reinterpret_cast<float*>((char*)scratch + w.part_m);
   a.part_l = reinterpret_cast<float*>((char*)scratch + w.part_l);
   a.part_o = reinterpret_cast<float*>((char*)scratch + w.part_o);
@@ -1225,17 +1199,15 @@ inline int sfa_sm100_launch(const DsaSfaParams* p, const SfaDev& d, int32_t* sta
   a.redo_count = redo_count;
   int clusters = sms / 2;
   if (clusters > a.items) clusters = a.items;
-  CUtensorMap tkn, tkr, tq, tqr;
-  if (!make_tmap_gather4_16bit(&tkn, p->key, (uint64_t)p->key_rows, 512, 1024, 64, bf16)) return DSA_ERR_CUDA;
-  if (!make_tmap_gather4_16bit(&tkr, p->key_rope, (uint64_t)p->key_rows, 64, 128, 64, bf16)) return DSA_ERR_CUDA;
+  CUtensorMap tq, tqr;
   if (!make_tmap_3d_16bit(&tq, p->query, (uint64_t)d.rows, (uint64_t)p->n1, 512, 1024, (uint64_t)p->n1 * 1024,
                           kSfaCtaHeads, 64, bf16))
     return DSA_ERR_CUDA;
   if (!make_tmap_3d_16bit(&tqr, p->query_rope, (uint64_t)d.rows, (uint64_t)p->n1, 64, 128, (uint64_t)p->n1 * 128,
                           kSfaCtaHeads, 64, bf16))
     return DSA_ERR_CUDA;
-  if (split > 1) sfa_fwd_sm100_kernel<true><<<clusters * 2, kSfaThreads, kSfaSmemBytes, st>>>(tkn, tkr, tq, tqr, a);
-  else sfa_fwd_sm100_kernel<false><<<clusters * 2, kSfaThreads, kSfaSmemBytes, st>>>(tkn, tkr, tq, tqr, a);
+  if (split > 1) sfa_fwd_sm100_kernel<true><<<clusters * 2, kSfaThreads, kSfaSmemBytes, st>>>(tq, tqr, a);
+  else sfa_fwd_sm100_kernel<false><<<clusters * 2, kSfaThreads, kSfaSmemBytes, st>>>(tq, tqr, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
   if (split > 1) {
