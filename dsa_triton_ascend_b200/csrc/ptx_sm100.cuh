@@ -185,6 +185,23 @@ __device__ __forceinline__ bool mbar_spin_warp_impl(uint64_t* bar, uint32_t pari
 __device__ __forceinline__ bool mbar_spin_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return mbar_spin_warp_impl<false>(bar, parity, abort_flag);
 }
+// For a loop that one thread runs by itself (an issuer): no votes, nothing to re-converge.
+__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  for (uint32_t i = 0; i < (kWaitPolls << 6); ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, P;\n\t}\n"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((i & 1023u) == 1023u && *abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
 __device__ __forceinline__ bool mbar_spin_cluster_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return mbar_spin_warp_impl<true>(bar, parity, abort_flag);
 }

@@ -21,20 +21,23 @@ constexpr uint32_t kSlKBlk = kSlKeys * 128;        // 128 keys x 64 features
 constexpr uint32_t kSlSmemMax = 232448;
 
 // ---- scores --------------------------------------------------------------------------------------
-// What bounds it: bringing the keys.  A row's selected keys are its own, so each (row, key) pair is a
-// gather of 2 (D + Dr) bytes, and the SM's TMA unit takes one gather4 (512 B) per ~18 cycles: 5200
-// cycles per 128-key tile of 1152 B keys, against 1150 (64 heads) or 2300 (128 heads) cycles of tensor
-// pipe.  So one block takes up to 128 heads of the row (every gathered byte serves all of them), Q stays in
-// shared memory and the keys stream through a ring of 64-feature blocks (16 KB each: a whole tile of 147
-// KB would not fit beside 128 heads of Q).  Rows are cut into parts when there are few of them.
-// Warps: 0..7 epilogue (two groups on alternate accumulators), 8..15 gather, 16 MMA issuer, 17 Q and head
+// What bounds it: the hand-overs between gather, issuers and epilogue (512 rows x 2048 keys x 64 heads: 150 us; with a
+// quarter of the products and no global reads still 117).  A row's selected keys are its own, so each (row, key) pair
+// is a gather of 2 (D + Dr) bytes; cp.async copies bring 72 B/clk of them to an SM, TMA gather4 31 (one 512-byte
+// load per 16.5 cycles).  A block takes up to 128 heads of the row (every gathered byte serves all of them), Q stays
+// in shared memory and the keys stream through a ring of 64-feature blocks (16 KB each: a whole tile of 147 KB would
+// not fit beside 128 heads of Q).  Rows are cut into parts when there are few of them.
+// With gather4 and one issuer, and with the copies and two (attention / index side): 512 rows x 64 heads 191 / 67 us
+// -> 150 / 56, 2048 rows x 128 heads, fp16: 838 / 253 -> 680 / 202.
+// Warps: 0..7 epilogue (two groups on alternate accumulators), 8..15 gather, 16, 17 MMA issuers, 18 Q and head
 // parameters.
-constexpr int kScThreads = 576, kScGatherWarp0 = 8, kScGatherWarps = 8, kScIssuer = 16, kScLoader = 17;
+constexpr int kScThreads = 608, kScGatherWarp0 = 8, kScGatherWarps = 8, kScIssuer = 16, kScLoader = 18;
 constexpr int kScMaxStages = 12;
 
 struct SliScoreArgs {
   SliGradDev p;
   int32_t* status;
+  const void *ka, *kb;       // the keys' first tensor, and the rope's
   float* out;                // [rows, topk]
   int32_t heads;             // of this side
   int32_t nblk, nblk_a;      // 64-feature blocks in all / of the first tensor (the others: rope)
@@ -68,17 +71,16 @@ __device__ __forceinline__ int32_t sli_key_row(const SliGradDev& p, const int32_
 // infinite key; compiled apart because the test costs the others 1 % (2048 rows x 128 heads: 1658 -> 1674 us).
 template <bool ATT, bool PAD>
 __global__ void __launch_bounds__(kScThreads, 1)
-sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid_constant__ CUtensorMap tmap_kb,
-                       const __grid_constant__ CUtensorMap tmap_qa, const __grid_constant__ CUtensorMap tmap_qb,
+sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_qa, const __grid_constant__ CUtensorMap tmap_qb,
                        const SliScoreArgs a) {
   extern __shared__ __align__(1024) unsigned char slsm[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(slsm + a.off_bar);
-  uint64_t* full = bars;                       // [stages] gather -> issuer        (tx bytes)
+  uint64_t* full = bars;                       // [stages] gather -> its issuer    (64 lanes' copies)
   uint64_t* empty = bars + kScMaxStages;       // [stages] products done -> gather (commit)
-  uint64_t* s_full = bars + 2 * kScMaxStages;  // [2] scores -> epilogue           (commit)
+  uint64_t* s_full = bars + 2 * kScMaxStages;  // [2] scores -> epilogue           (both issuers' commits)
   uint64_t* s_empty = s_full + 2;              // [2] scores read                  (4 warps)
   uint64_t* q_full = s_full + 4;               // Q landed                         (tx bytes)
-  uint64_t* q_empty = s_full + 5;              // last product of the item         (commit)
+  uint64_t* q_empty = s_full + 5;              // last products of the item        (both issuers' commits)
   uint64_t* m_full = s_full + 6;               // [2] head parameters stored       (loader)
   uint64_t* m_empty = s_full + 8;              // [2] head parameters read         (8 warps)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 10);
@@ -88,20 +90,20 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool misaligned = (ptx::smem_u32(slsm) & 1023u) != 0;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kScMaxStages; ++i) { ptx::mbar_init(&full[i], 1); ptx::mbar_init(&empty[i], 1); }
+    for (int i = 0; i < kScMaxStages; ++i) { ptx::mbar_init(&full[i], 64); ptx::mbar_init(&empty[i], 1); }
     for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(&s_full[i], 1);
+      ptx::mbar_init(&s_full[i], 2);
       ptx::mbar_init(&s_empty[i], 4);
       ptx::mbar_init(&m_full[i], 1);
       ptx::mbar_init(&m_empty[i], 8);
     }
     ptx::mbar_init(q_full, 1);
-    ptx::mbar_init(q_empty, 1);
+    ptx::mbar_init(q_empty, 2);
     *abort_flag = misaligned ? 1 : 0;
     ptx::mbar_fence_init();
   }
   if (warp == kScIssuer) {
-    ptx::tmem_alloc(tmem_slot, 256);
+    ptx::tmem_alloc(tmem_slot, 512);
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before();
@@ -111,12 +113,13 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
   const uint32_t sm0 = ptx::smem_u32(slsm);
   const uint32_t qblk = (uint32_t)a.hp * 128;
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return ptx::mbar_wait_warp(bar, parity, abort_flag); };
+  auto spin = [&](uint64_t* bar, uint32_t parity) -> bool { return ptx::mbar_spin(bar, parity, abort_flag); };
 
   if (*abort_flag) {
     // nothing started
   } else if (warp < kScGatherWarp0) {
     const int wg = warp >> 2, quarter = warp & 3;
-    const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + wg * 128;
+    const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + wg * 256;
     uint32_t n_tile = 0, n_item = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
@@ -136,10 +139,16 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
 #pragma unroll 1
         for (int c = 0; c < a.hp; c += 32) {
           const bool two = c + 16 < a.hp;
-          float v[32];
+          float v[32], u[32];
           ptx::tmem_ld_x16(base + c, reinterpret_cast<uint32_t*>(v));
-          if (two) ptx::tmem_ld_x16(base + c + 16, reinterpret_cast<uint32_t*>(v + 16));
+          ptx::tmem_ld_x16(base + 128 + c, reinterpret_cast<uint32_t*>(u));
+          if (two) {
+            ptx::tmem_ld_x16(base + c + 16, reinterpret_cast<uint32_t*>(v + 16));
+            ptx::tmem_ld_x16(base + 128 + c + 16, reinterpret_cast<uint32_t*>(u + 16));
+          }
           ptx::tmem_ld_wait();
+#pragma unroll
+          for (int h = 0; h < 32; ++h) v[h] += u[h];
           if (c + 32 >= a.hp) {
             ptx::tc_fence_before();
             __syncwarp();
@@ -175,79 +184,96 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
       ++n_item;
     }
   } else if (warp < kScIssuer) {
-    // gather: pairs of warps take the 64-feature blocks in turn, a warp issues half of a block's 32 loads (a
-    // warp issues its lanes' loads one by one).  Pairs <= stages: a warp that waited for a ring slot one round
-    // ahead of another would take the round before for its own (the wait tells odd from even rounds only).
-    const int pair = (warp - kScGatherWarp0) >> 1, grp = ((warp - kScGatherWarp0) & 1) * 16 + (lane & 15);
-    if (lane == 0) { ptx::prefetch_tmap(&tmap_ka); ptx::prefetch_tmap(&tmap_kb); }
-    uint32_t gb = 0, ph = 1;
-    int stage = 0;
+    // gather: pairs of warps take the 64-feature blocks in turn, a warp half of a block's keys (16 copies per lane, an
+    // instruction is 4 keys x 128 bytes).  Pairs <= stages: a warp that waited for a ring slot one round ahead of
+    // another would take the round before for its own (the wait tells odd from even rounds only).
+    const int pair = (warp - kScGatherWarp0) >> 1, key_w = ((warp - kScGatherWarp0) & 1) * 64 + (lane >> 3), ch = lane & 7;
+    const uint32_t dst0 = sm0 + a.off_k + key_w * 128 + ((ch ^ (key_w & 7)) << 4);
+    const uint32_t dst1 = sm0 + a.off_k + (key_w + 4) * 128 + ((ch ^ ((key_w + 4) & 7)) << 4);
+    const unsigned char *ka = (const unsigned char*)a.ka + ch * 16, *kb = (const unsigned char*)a.kb + ch * 16;
+    // (the pair's block of the ring: `blk` of the current tile; it and `stage` move on by kPairs.  The wait suspends:
+    // eight polling warps take the issuers' issue slots, 150 -> 155 us)
+    constexpr int kPairs = kScGatherWarps / 2;
+    uint32_t ph = 1;
+    int stage = pair, blk = pair;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       const SliItem it = sli_score_item(a, item);
       if (it.t1 <= it.t0) continue;
       const int32_t* idx_row = a.p.sparse_indices ? a.p.sparse_indices + (int64_t)it.row * a.p.topk : nullptr;
-      int32_t rn[4];
+      int32_t rn[16];
       auto load = [&](int32_t t) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rn[i] = sli_key_row(a.p, idx_row, it.b, t * kSlKeys + grp * 4 + i, it.n, a.key_rows);
+        for (int i = 0; i < 16; ++i) {        // (no branch, or each load would wait for the one before it)
+          const int32_t j = min(t * kSlKeys + key_w + 4 * i, it.n - 1);
+          rn[i] = idx_row ? idx_row[j] : j;
+        }
       };
       load(it.t0);
       for (int32_t t = it.t0; t < it.t1 && ok; ++t) {
-        int32_t r[4];
+        int32_t r[16];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = rn[i];
-        load(t + 1);       // (past the row: nothing is read)
-        for (int blk = 0; blk < a.nblk && ok; ++blk, ++gb) {
-          if ((int)(gb % (kScGatherWarps / 2)) == pair) {
-            ok = wait(&empty[stage], ph);
-            if (!ok) break;
-            if (grp == 0 && lane == 0) ptx::mbar_arrive_expect_tx(&full[stage], kSlKBlk);
-            __syncwarp();
-            unsigned char* dst = slsm + a.off_k + stage * kSlKBlk + grp * 512;
-            if (lane < 16) {
-              if (blk < a.nblk_a) ptx::tma_gather4_2d(dst, &tmap_ka, &full[stage], blk * 64, r[0], r[1], r[2], r[3]);
-              else ptx::tma_gather4_2d(dst, &tmap_kb, &full[stage], (blk - a.nblk_a) * 64, r[0], r[1], r[2], r[3]);
-            }
-            __syncwarp();
-          }
-          if (++stage == a.stages) { stage = 0; ph ^= 1; }
+        for (int i = 0; i < 16; ++i)          // (slots past the row's last: -1)
+          r[i] = t * kSlKeys + key_w + 4 * i < it.n ? it.b * a.p.s2 + min(max(rn[i], 0), a.p.s2 - 1) : -1;
+        if (t + 1 < it.t1) load(t + 1);
+        for (; blk < a.nblk; blk += kPairs) {
+          ok = wait(&empty[stage], ph);
+          if (!ok) break;
+          const unsigned char* src = blk < a.nblk_a ? ka + blk * 128 : kb + (blk - a.nblk_a) * 128;
+          const uint32_t pitch = (uint32_t)(blk < a.nblk_a ? a.nblk_a : a.nblk - a.nblk_a) * 128;
+          const uint32_t off = stage * kSlKBlk;
+#pragma unroll
+          for (int i = 0; i < 16; ++i)        // (slots past the row's last load zeros)
+            ptx::cp_async_16(((i & 1) ? dst1 : dst0) + off + (i >> 1) * 1024, src + (uint64_t)max(r[i], 0) * pitch,
+                             r[i] >= 0 ? 16u : 0u);
+          ptx::cp_async_mbar_arrive(&full[stage]);
+          stage += kPairs;
+          if (stage >= a.stages) { stage -= a.stages; ph ^= 1; }
         }
+        blk -= a.nblk;
       }
     }
-  } else if (warp == kScIssuer) {
-    const uint64_t q_d = ptx::desc_kmajor_sw128(sm0), k_d = ptx::desc_kmajor_sw128(sm0 + a.off_k);
-    uint32_t n_tile = 0, n_item = 0, ph = 0;
-    int stage = 0;
-    bool ok = true;
-    for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const SliItem it = sli_score_item(a, item);
-      if (it.t1 <= it.t0) continue;
-      ok = wait(q_full, n_item & 1);
-      for (int32_t t = it.t0; t < it.t1 && ok; ++t, ++n_tile) {
-        const int buf = n_tile & 1;
-        ok = wait(&s_empty[buf], ((n_tile >> 1) & 1) ^ 1);
-        for (int blk = 0; blk < a.nblk && ok; ++blk) {
-          ok = wait(&full[stage], ph);
+  } else if (warp < kScLoader) {
+    // Two issuers, one thread each, take the ring's even and odd blocks into accumulators of their own (the epilogue
+    // adds them): one thread needs about 560 cycles for a block's four products, twice what the tensor core does.
+    // The number of stages is even, so that a stage has one reader: one that waited for a stage whose block before
+    // belongs to the other would take the round before for its own.
+    if (lane == 0) {
+      const uint64_t q_d = ptx::desc_kmajor_sw128(sm0), k_d = ptx::desc_kmajor_sw128(sm0 + a.off_k);
+      const int me = warp - kScIssuer;
+      uint32_t n_tile = 0, n_item = 0, ph = 0;
+      int stage = me, first = me;              // first: my first block of the tile
+      bool ok = true;
+      for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+        const SliItem it = sli_score_item(a, item);
+        if (it.t1 <= it.t0) continue;
+        ok = spin(q_full, n_item & 1);
+        for (int32_t t = it.t0; t < it.t1 && ok; ++t, ++n_tile) {
+          const int buf = n_tile & 1;
+          ok = spin(&s_empty[buf], ((n_tile >> 1) & 1) ^ 1);
           if (!ok) break;
           ptx::tc_fence_after();
-          if (ptx::elect_one()) {
+          const uint32_t acc = tmem + buf * 256 + me * 128;
+          for (int blk = first; blk < a.nblk; blk += 2) {
+            ok = spin(&full[stage], ph);
+            if (!ok) break;
+            ptx::fence_proxy_async_smem();     // (the copies went through the generic proxy)
+            const uint64_t kd = k_d + ((stage * kSlKBlk) >> 4), qd = q_d + ((blk * qblk) >> 4);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              ptx::mma_ss(tmem + buf * 128, k_d + ((stage * kSlKBlk) >> 4) + i * 2, q_d + ((blk * qblk) >> 4) + i * 2,
-                          a.idesc, (blk > 0 || i > 0) ? 1u : 0u);
+            for (int i = 0; i < 4; ++i) ptx::mma_ss(acc, kd + i * 2, qd + i * 2, a.idesc, (blk > first || i > 0) ? 1u : 0u);
             ptx::mma_commit(&empty[stage]);
-            if (blk == a.nblk - 1) {
-              ptx::mma_commit(&s_full[buf]);
-              if (t == it.t1 - 1) ptx::mma_commit(q_empty);
-            }
+            stage += 2;
+            if (stage >= a.stages) { stage = me; ph ^= 1; }
           }
-          __syncwarp();
-          if (++stage == a.stages) { stage = 0; ph ^= 1; }
+          if (!ok) break;
+          first ^= a.nblk & 1;
+          ptx::mma_commit(&s_full[buf]);
+          if (t == it.t1 - 1) ptx::mma_commit(q_empty);
         }
+        ++n_item;
       }
-      ++n_item;
     }
+    __syncwarp();
   } else if (warp == kScLoader) {
     if (lane == 0) { ptx::prefetch_tmap(&tmap_qa); ptx::prefetch_tmap(&tmap_qb); }
     uint32_t n_item = 0;
@@ -295,7 +321,7 @@ sli_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid
   __syncthreads();
   if (warp == kScIssuer) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem, 256);
+    ptx::tmem_dealloc(tmem, 512);
   }
   if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, misaligned ? 2 : 1);
 }
@@ -1083,26 +1109,25 @@ inline int sli_score_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d
   const uint32_t qbytes = (uint32_t)a.nblk * a.hp * 128, tail = 2 * 128 * 8 + 512;
   // (the ring starts on a 1024-byte boundary: hp * 128 is a multiple of 2048)
   a.off_k = qbytes;
-  a.stages = (int32_t)std::min<uint32_t>(kScMaxStages, (kSlSmemMax - tail - qbytes) / kSlKBlk);
-  if (a.stages < kScGatherWarps / 2) return DSA_ERR_TOO_LARGE;   // (nblk <= 9 leaves five)
+  a.stages = (int32_t)std::min<uint32_t>(kScMaxStages, (kSlSmemMax - tail - qbytes) / kSlKBlk) & ~1;
+  if (a.stages < kScGatherWarps / 2 || a.nblk < 2) return DSA_ERR_TOO_LARGE;   // (nblk: 2 to 9, nine leave four)
   a.off_prm = a.off_k + a.stages * kSlKBlk;
   a.off_bar = a.off_prm + 2 * 128 * 8;
   const uint32_t smem = a.off_bar + 512;
   const void *ka = att ? p->key : p->key_index, *kb = wb ? p->key_rope : ka;
   const void *qa = att ? p->query : p->query_index, *qb = wb ? p->query_rope : qa;
   const int wkb = wb ? wb : wa;
-  CUtensorMap tka, tkb, tqa, tqb;
-  if (!make_tmap_gather4_16bit(&tka, ka, (uint64_t)a.key_rows, wa, wa * 2, 64, bf16) ||
-      !make_tmap_gather4_16bit(&tkb, kb, (uint64_t)a.key_rows, wkb, wkb * 2, 64, bf16) ||
-      !make_tmap_3d_16bit(&tqa, qa, (uint64_t)rows, (uint64_t)a.heads, wa, wa * 2, (uint64_t)a.heads * wa * 2, a.hp, 64,
+  a.ka = ka; a.kb = kb;
+  CUtensorMap tqa, tqb;
+  if (!make_tmap_3d_16bit(&tqa, qa, (uint64_t)rows, (uint64_t)a.heads, wa, wa * 2, (uint64_t)a.heads * wa * 2, a.hp, 64,
                           bf16) ||
       !make_tmap_3d_16bit(&tqb, qb, (uint64_t)rows, (uint64_t)a.heads, wkb, wkb * 2, (uint64_t)a.heads * wkb * 2, a.hp, 64,
                           bf16))
     return DSA_ERR_CUDA;
   const int grid = std::min(a.items, sms);
-  if (!att) sli_score_sm100_kernel<false, false><<<grid, kScThreads, smem, st>>>(tka, tkb, tqa, tqb, a);
-  else if (a.heads % a.hp) sli_score_sm100_kernel<true, true><<<grid, kScThreads, smem, st>>>(tka, tkb, tqa, tqb, a);
-  else sli_score_sm100_kernel<true, false><<<grid, kScThreads, smem, st>>>(tka, tkb, tqa, tqb, a);
+  if (!att) sli_score_sm100_kernel<false, false><<<grid, kScThreads, smem, st>>>(tqa, tqb, a);
+  else if (a.heads % a.hp) sli_score_sm100_kernel<true, true><<<grid, kScThreads, smem, st>>>(tqa, tqb, a);
+  else sli_score_sm100_kernel<true, false><<<grid, kScThreads, smem, st>>>(tqa, tqb, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
   return DSA_OK;
