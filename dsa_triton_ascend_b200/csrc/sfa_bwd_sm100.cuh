@@ -12,7 +12,8 @@
 // else is arranged to run beside the stream of reductions:
 //
 //   * A work item is (query row, 64 heads).  Q and dO stay in shared memory for the whole row (136 KB),
-//     keys come 48 at a time (TMA gather4, 54 KB, one buffer).
+//     keys come 48 at a time (cp.async, 54 KB, one buffer: 1.26 -> 1.22 ms and 7.54 -> 7.37 ms for the calls below
+//     against TMA gather4, which takes 3700 cycles from a free buffer to a full one, the copies 1700).
 //   * Q and dO are stacked: feature block f of both forms one 128-row A operand, so that ONE product
 //     with the key tile yields S (lanes 0..63) and dP (lanes 64..127).  The rope part of S goes to
 //     columns of its own (its lower 64 rows are whatever follows in shared memory; nobody reads them).
@@ -26,13 +27,12 @@
 //     scaled by 2^13, dS by a power of two per item that keeps |dS| <= scale * (|dO| |v| + |delta|)
 //     (Cauchy-Schwarz over the item's heads and selected keys, taken by small kernels in front) below 2^13.
 //
-// Measured, whole operator call: B1 S1 512 S2 4096 N1 64 k 2048 1.26 ms in bf16, 1.29 ms in fp16
-// (sfa_bwd_mma_kernel: 4.63 ms); 4092 rows x 128 heads in bf16 7.6 ms (32.2 ms).  ncu, the first of them, this kernel alone: 1.27
-// ms, 3.6 TB/s of reductions, tensor pipe 28 %, L2 41 %, load / store data pipe 33 %.  No unit is full: what is
-// left is the chain of a tile (S -> P -> dS -> products; P is made by four warps, and expf(..) / sum in the place of their
-// exp2 and product takes the call to 1.58 ms), the reload of Q / dO between items, and the last of the four
-// rounds that 512 items make on 148 SMs.
-// ptxas spills 20 bytes (bf16) and 88 bytes (fp16) of a thread's 72 registers.
+// Measured, whole operator call: B1 S1 512 S2 4096 N1 64 k 2048 in bf16 1.22 ms (sfa_bwd_mma_kernel: 4.63 ms); 4092
+// rows x 128 heads in bf16 7.4 ms under the power cap (32.2 ms).  A tile of 48 keys takes 12 400 cycles: its reductions alone would take
+// 8400, its products 8000.  What is left is the chain of a tile (keys 1700, S 2200, P and dS 5500, of which 1600 wait
+// for dK of the tile before, dQ 2100) beside the chain of the dV / dK tiles (issue 6400, ring slots 3100), the reload
+// of Q / dO between items, and the last of the four rounds that 512 items make on 148 SMs.
+// ptxas spills 16 bytes (bf16) and 60 bytes (fp16) of a thread's 72 registers.
 //
 // Tensor memory: dQ^T 5 x 64 columns | S, dP 48 | rope part of S 48 | drain ring 2 x 48.
 // Warps (896 threads): 0..7 softmax (lane quarter = warp & 3: quarters 0, 1 hold S of heads 0..63,
@@ -66,7 +66,7 @@ constexpr uint32_t kBwdOffX = kBwdOffP + 4 * kBwdPMat;            // P as fp32 [
 constexpr uint32_t kBwdOffBar = kBwdOffX + kBwdBK * kBwdHeads * 4;
 constexpr uint32_t kBwdOffRows = kBwdOffBar + 256;               // int32 [3][48]: key rows of the last tiles
 constexpr uint32_t kBwdSmemBytes = kBwdOffRows + 3 * kBwdBK * 4;
-constexpr uint32_t kBwdQBytes = 8 * kBwdQdBlk + kBwdHBlk, kBwdKBytes = 9 * kBwdKBlk;
+constexpr uint32_t kBwdQBytes = 8 * kBwdQdBlk + kBwdHBlk;
 static_assert(kBwdOffK % 1024 == 0 && kBwdOffP % 1024 == 0, "operand alignment");
 static_assert(kBwdSmemBytes <= 232448, "shared memory");
 // the drain warps take the registers that the gather, issuer and loader warps give back
@@ -177,13 +177,12 @@ __global__ void __launch_bounds__(256) sfa_bwd_exponent_kernel(const int2* __res
 
 template <typename T>
 __global__ void __launch_bounds__(kBwdThreads, 1)
-sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_constant__ CUtensorMap tmap_kr,
-                     const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_qr,
+sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_qr,
                      const __grid_constant__ CUtensorMap tmap_do, const SfaBwdArgs a) {
   constexpr bool kScaled = !kIsBf16<T>;
   extern __shared__ __align__(1024) unsigned char bwd_sm[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(bwd_sm + kBwdOffBar);
-  uint64_t* k_full = bars;          // gather -> issuer A                                 (tx bytes)
+  uint64_t* k_full = bars;          // gather -> issuer A                                 (128 lanes' copies, rows_s)
   uint64_t* k_empty = bars + 1;     // dQ of the tile done -> gather                      (commit A)
   uint64_t* q_full = bars + 2;      // Q, dO landed -> issuer A (issuer B follows it)     (tx bytes)
   uint64_t* q_empty = bars + 3;     // both issuers through with the item -> loader       (commits A, B)
@@ -207,7 +206,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
   const int32_t n1 = a.p.n1;
   const bool misaligned = (ptx::smem_u32(bwd_sm) & 1023u) != 0;
   if (threadIdx.x == 0) {
-    const int counts[25] = {1, 1, 1, 2, 1, 8, 4, 1, 4, 2, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 4, 4, 1, 8};
+    const int counts[25] = {4 * 32 + 1, 1, 1, 2, 1, 8, 4, 1, 4, 2, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 4, 4, 1, 8};
 #pragma unroll
     for (int i = 0; i < 25; ++i) ptx::mbar_init(&bars[i], counts[i]);
     *abort_flag = misaligned ? 1 : 0;
@@ -437,12 +436,12 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
    if (*abort_flag) {
     // nothing started
    } else if (warp < kBwdIssueA) {
-    // -------------------------------------------------------------------- K gather: 12 groups of 4 keys x 9 blocks
-    const int o = (warp - kBwdGatherWarp0) + kBwdGatherWarps * lane;
-    const bool active = o < 108;
-    const int grp = o / 9, blk = o - grp * 9;
-    unsigned char* dst = bwd_sm + kBwdOffK + blk * kBwdKBlk + grp * 512;
-    if (lane == 0) { ptx::prefetch_tmap(&tmap_kn); ptx::prefetch_tmap(&tmap_kr); }
+    // -------------------------------------------------------------------- K gather: four warps take 12 keys each, 9
+    // blocks (27 copies per lane, an instruction is 4 keys x 128 bytes); the fifth writes the drain warps' row numbers
+    const int gw = warp - kBwdGatherWarp0;
+    const int ch = lane & 7, key_w = gw * 12 + (lane >> 3);          // this lane's keys: key_w + 4 j
+    const unsigned char* kn = (const unsigned char*)a.p.key + ch * 16;
+    const unsigned char* kr = (const unsigned char*)a.p.key_rope + ch * 16;
     uint32_t n_tile = 0;
     int rbuf = 0;
     bool ok = true;
@@ -450,42 +449,47 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
       const int2 nv = a.nvalid[item / a.hblocks];
       const int32_t ntiles = tiles_of(nv.x);
       const int32_t* list = a.key_list + nv.y;
-      int32_t rn[4], dn0 = 0, dn1 = 0;
+      int32_t rn[3] = {0, 0, 0};
       auto load = [&](int32_t t) {
         const int32_t left = nv.x - t * kBwdBK;
+        if (left <= 0) return;
+        if (gw < 4) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          rn[i] = active && left > 0 ? list[t * kBwdBK + (grp * 4 + i < left ? grp * 4 + i : 0)] : 0;
-        if (warp == kBwdGatherWarp0) {
-          dn0 = lane < left ? list[t * kBwdBK + lane] : a.key_rows;
-          dn1 = lane < 16 && 32 + lane < left ? list[t * kBwdBK + 32 + lane] : a.key_rows;
+          for (int j = 0; j < 3; ++j) rn[j] = list[t * kBwdBK + (key_w + 4 * j < left ? key_w + 4 * j : 0)];
+        } else {
+          rn[0] = lane < left ? list[t * kBwdBK + lane] : a.key_rows;
+          rn[1] = lane < 16 && 32 + lane < left ? list[t * kBwdBK + 32 + lane] : a.key_rows;
         }
       };
       load(0);
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
-        int32_t r[4];
+        int32_t r[3];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = rn[i];
-        const int32_t d0 = dn0, d1 = dn1;
+        for (int j = 0; j < 3; ++j) r[j] = rn[j];
         load(t + 1);
         ok = wait(k_empty, (n_tile & 1) ^ 1);
         if (!ok) break;
-        if (warp == kBwdGatherWarp0) {
+        if (gw < 4) {
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const int key = key_w + 4 * j;
+            const uint32_t dst = sm0 + kBwdOffK + key * 128 + ((ch ^ (key & 7)) << 4);
+            const unsigned char* src = kn + (int64_t)r[j] * 1024;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) ptx::cp_async_16(dst + b * kBwdKBlk, src + b * 128, 16u);
+            ptx::cp_async_16(dst + 8 * kBwdKBlk, kr + (int64_t)r[j] * 128, 16u);
+          }
+          ptx::cp_async_mbar_arrive(k_full);
+        } else {
           // The drain warps' row numbers (past the keys: no such key).  Three buffers: tile t + 3 is gathered
           // after dQ of tile t + 2, i.e. after every dK^T tile of t + 1 was issued and so after every drain
           // group has left tile t behind.
-          rows_s[rbuf * kBwdBK + lane] = d0;
-          if (lane < 16) rows_s[rbuf * kBwdBK + 32 + lane] = d1;
+          rows_s[rbuf * kBwdBK + lane] = r[0];
+          if (lane < 16) rows_s[rbuf * kBwdBK + 32 + lane] = r[1];
           rbuf = rbuf == 2 ? 0 : rbuf + 1;
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_expect_tx(k_full, kBwdKBytes);
+          if (lane == 0) ptx::mbar_arrive(k_full);
         }
-        __syncwarp();
-        if (active) {
-          if (blk == 8) ptx::tma_gather4_2d(dst, &tmap_kr, k_full, 0, r[0], r[1], r[2], r[3]);
-          else ptx::tma_gather4_2d(dst, &tmap_kn, k_full, blk * 64, r[0], r[1], r[2], r[3]);
-        }
-        __syncwarp();
       }
     }
    } else if (warp == kBwdIssueA) {
@@ -506,6 +510,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kn, const __grid_c
         if (!ok) break;
         ptx::tc_fence_after();
         if (ptx::elect_one()) {
+          ptx::fence_proxy_async_smem();   // (the copies went through the generic proxy)
 #pragma unroll
           for (int i = 0; i < 4; ++i)
             ptx::mma_ss(tmem + kBwdTmR, qr_k + i * 2, k_k + ((8 * kBwdKBlk) >> 4) + i * 2, a.idesc_s, i ? 1u : 0u);
@@ -741,10 +746,8 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   a.hblocks = hblocks;
   a.items = d.rows * a.hblocks;
   a.key_rows = (int32_t)p->key_rows;
-  CUtensorMap tkn, tkr, tq, tqr, tdo;
-  if (!make_tmap_gather4_16bit(&tkn, p->key, (uint64_t)p->key_rows, 512, 1024, 64, bf16) ||
-      !make_tmap_gather4_16bit(&tkr, p->key_rope, (uint64_t)p->key_rows, 64, 128, 64, bf16) ||
-      !make_tmap_3d_16bit(&tq, p->query, (uint64_t)d.rows, (uint64_t)p->n1, 512, 1024, (uint64_t)p->n1 * 1024, kBwdHeads,
+  CUtensorMap tq, tqr, tdo;
+  if (!make_tmap_3d_16bit(&tq, p->query, (uint64_t)d.rows, (uint64_t)p->n1, 512, 1024, (uint64_t)p->n1 * 1024, kBwdHeads,
                           64, bf16) ||
       !make_tmap_3d_16bit(&tqr, p->query_rope, (uint64_t)d.rows, (uint64_t)p->n1, 64, 128, (uint64_t)p->n1 * 128,
                           kBwdHeads, 64, bf16) ||
@@ -752,7 +755,7 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
                           kBwdHeads, 64, bf16))
     return DSA_ERR_CUDA;
   const int grid = std::min(a.items, sms);
-  sfa_bwd_sm100_kernel<T><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tkn, tkr, tq, tqr, tdo, a);
+  sfa_bwd_sm100_kernel<T><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tqr, tdo, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
   return DSA_OK;
