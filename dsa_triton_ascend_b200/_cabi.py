@@ -16,6 +16,7 @@ DTYPE_BF16, DTYPE_FP16, DTYPE_FP32 = 0, 1, 2
 RANK_IO_DTYPE, RANK_FP32 = 0, 1
 KERNEL_AUTO, KERNEL_PORTABLE, KERNEL_TENSOR = 0, 1, 2
 PHASE_SCORE, PHASE_TOPK, PHASE_ALL = 1, 2, 3
+OUT_ZEROS = 2   # return_value / return_lse: zeros in the place of the results
 
 ERR_VALUE = -3
 

@@ -1,5 +1,6 @@
 """Host-side helpers shared by the two operator wrappers: dtype/length handling, workspace
 and stream plumbing.  torch is used for device memory and streams only."""
+import contextlib
 import functools
 import os
 
@@ -77,8 +78,22 @@ def workspace(nbytes, device):
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
 
+# (torch.cuda.current_stream builds a Stream object around the handle: 2-4 us of a call that takes 30)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def current_stream(device):
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_no_guard = contextlib.nullcontext()
+
+
+def device_guard(device):
+    """Context in which `device` is the current CUDA device; nothing to enter when it is already."""
+    return _no_guard if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 # ---- device status ----------------------------------------------------------------------------------

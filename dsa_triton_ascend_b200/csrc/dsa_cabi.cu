@@ -74,7 +74,10 @@ static LiDev li_dev(const DsaLiParams* p) {
   d.out_indices = p->out_indices; d.out_values = p->out_values;
   d.dtype_w = p->dtype_w; d.n1 = p->n1; d.n2 = p->n2; d.d = p->d;
   d.rows = (int32_t)li_rows(p);
-  d.sparse_count = p->sparse_count; d.rank_mode = p->rank_mode; d.return_value = p->return_value;
+  d.sparse_count = p->sparse_count; d.rank_mode = p->rank_mode;
+  d.return_value = p->return_value == DSA_OUT_ZEROS ? 0 : p->return_value;
+  d.zero_values = p->return_value == DSA_OUT_ZEROS && p->out_values != nullptr;
+  d.cta_status = nullptr; d.status = nullptr; d.n_cta_status = 0;
   return d;
 }
 
@@ -84,8 +87,10 @@ static bool li_takes_tensor_path(const DsaLiParams* p) {
 }
 
 template <typename T>
-static int li_launch(const DsaLiParams* p, float* scores, cudaStream_t st, int32_t* status = nullptr) {
+static int li_launch(const DsaLiParams* p, float* scores, cudaStream_t st, int32_t* status = nullptr,
+                     bool clear_status = false) {
   LiDev d = li_dev(p);
+  if (clear_status) { d.cta_status = (uint8_t*)status + 64; d.status = status; }
   const int64_t ld = li_score_ld(p);
   const int64_t rown = (int64_t)d.rows * p->n2;
   if (rown == 0) return DSA_OK;
@@ -182,7 +187,8 @@ static SfaDev sfa_dev(const DsaSfaParams* p) {
   d.rows = p->layout_q == DSA_LAYOUT_TND ? p->s1 : p->batch * p->s1;
   d.n1 = p->n1; d.d = p->d; d.d_rope = p->d_rope;
   d.sparse_count = p->sparse_count; d.sparse_block_size = p->sparse_block_size;
-  d.return_lse = p->return_lse;
+  d.return_lse = p->return_lse == DSA_OUT_ZEROS ? 0 : p->return_lse;
+  d.zero_lse = p->return_lse == DSA_OUT_ZEROS;
   d.scale = p->scale;
   return d;
 }
@@ -191,6 +197,10 @@ template <typename T>
 static int sfa_launch_simt(const DsaSfaParams* p, cudaStream_t st) {
   SfaDev d = sfa_dev(p);
   if (d.rows == 0) return DSA_OK;
+  const size_t stat_bytes = (size_t)d.rows * p->n1 * sizeof(float);
+  if (d.zero_lse && (cudaMemsetAsync(p->softmax_max, 0, stat_bytes, st) != cudaSuccess ||
+                     cudaMemsetAsync(p->softmax_sum, 0, stat_bytes, st) != cudaSuccess))
+    return DSA_ERR_CUDA;
   const size_t smem = (size_t)(kSfaSimtHeads + kSfaSimtKeys) * (p->d + p->d_rope + kSfaSimtPad) * sizeof(T);
   if (cudaFuncSetAttribute(sfa_fwd_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
@@ -612,10 +622,12 @@ int dsa_li_forward(const DsaLiParams* p, void* workspace, size_t workspace_bytes
   if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255u) != 0) return DSA_ERR_WORKSPACE;
   if (p->kernel == DSA_KERNEL_TENSOR && !dsa_li_uses_tensor_path(p)) return DSA_ERR_UNSUPPORTED;
   cudaStream_t cs = (cudaStream_t)stream;
-  if (cudaMemsetAsync(workspace, 0, kWorkspaceHeader, cs) != cudaSuccess) return DSA_ERR_CUDA;
+  // (with both phases on the tensor path the kernels write the status word themselves)
+  const bool own = p->phases == DSA_PHASE_ALL && p->s2 > 0 && li_rows(p) > 0 && li_takes_tensor_path(p);
+  if (!own && cudaMemsetAsync(workspace, 0, kWorkspaceHeader, cs) != cudaSuccess) return DSA_ERR_CUDA;
   float* scores = reinterpret_cast<float*>((char*)workspace + kWorkspaceHeader);
-  if (p->dtype_qk == DSA_DTYPE_BF16) return li_launch<__nv_bfloat16>(p, scores, cs, (int32_t*)workspace);
-  return li_launch<__half>(p, scores, cs, (int32_t*)workspace);
+  if (p->dtype_qk == DSA_DTYPE_BF16) return li_launch<__nv_bfloat16>(p, scores, cs, (int32_t*)workspace, own);
+  return li_launch<__half>(p, scores, cs, (int32_t*)workspace, own);
 }
 
 int dsa_sfa_workspace_bytes(const DsaSfaParams* p, size_t* out_bytes) {

@@ -19,6 +19,12 @@ struct LiDev {
   int32_t n1, n2, d;
   int32_t rows;  // number of query rows (batch * s1 or T1)
   int32_t sparse_count, rank_mode, return_value;
+  int32_t zero_values;       // the values are not wanted: the top-k kernel stores zeros
+  // The scoring kernel's CTAs leave a status byte each, which the top-k kernel folds into the status word (that saves
+  // the call a memset in front of its first kernel); null: the scoring kernel sets the word, which starts at zero.
+  uint8_t* cta_status;
+  int32_t* status;
+  int32_t n_cta_status;
 };
 
 constexpr int kSimtKeys = 128;   // keys per block (one per thread)

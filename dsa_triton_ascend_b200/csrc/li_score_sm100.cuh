@@ -189,7 +189,10 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const int32_t cta = blockIdx.x, grid = gridDim.x;
 
   if ((ptx::smem_u32(li_smem) & 1023u) != 0) {  // the swizzled tiles need a 1024-byte aligned base
-    if (threadIdx.x == 0) atomicExch(a.status, 2);
+    if (threadIdx.x == 0) {
+      if (a.p.cta_status) a.p.cta_status[cta] = 2;
+      else atomicExch(a.status, 2);
+    }
     return;
   }
   if (threadIdx.x == 0) {
@@ -583,8 +586,13 @@ li_score_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, 512);
   }
-  if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, 1);
+  if (threadIdx.x == 0) {
+    if (a.p.cta_status) a.p.cta_status[cta] = *abort_flag ? 1 : 0;
+    else if (*abort_flag) atomicExch(a.status, 1);
+  }
 }
+
+constexpr int kLiStatusBytes = 192;   // of the 256-byte header, after 64 bytes that start with the status word
 
 // Host side: eligibility, tensor maps, launch.
 inline bool li_sm100_eligible(const DsaLiParams* p) {
@@ -606,7 +614,7 @@ inline bool li_sm100_eligible(const DsaLiParams* p) {
   return true;
 }
 
-inline int li_sm100_launch(const DsaLiParams* p, const LiDev& d, float* scores, int64_t ld, int32_t* status,
+inline int li_sm100_launch(const DsaLiParams* p, LiDev& d, float* scores, int64_t ld, int32_t* status,
                            cudaStream_t st) {
   // SM count per device, set up once per device (safe from several host threads)
   static std::atomic<int> sm_count[64];
@@ -638,7 +646,6 @@ inline int li_sm100_launch(const DsaLiParams* p, const LiDev& d, float* scores, 
   if (!make_tmap_2d_16bit(&tk, p->key, (uint64_t)p->key_rows, kLiDim, kLiDim * 2, sub_rows, 64, bf16))
     return DSA_ERR_CUDA;
   LiSm100Args a;
-  a.p = d;
   a.scores = scores;
   a.ld = ld;
   a.status = status;
@@ -672,6 +679,14 @@ inline int li_sm100_launch(const DsaLiParams* p, const LiDev& d, float* scores, 
   a.dense = (a.nchunks > 1 && groups <= kLiDenseGroups) ? 1 : 0;
   if (a.dense) a.items = groups * ((tiles_max + 7) / 8);      // upper bound: chunks are at least 8 tiles
   const int grid = a.items < sms ? a.items : sms;
+  if (d.cta_status != nullptr) {
+    d.n_cta_status = grid;
+    if (grid > kLiStatusBytes) {               // (no such device so far)
+      d.cta_status = nullptr;
+      if (cudaMemsetAsync(status, 0, sizeof(int32_t), st) != cudaSuccess) return DSA_ERR_CUDA;
+    }
+  }
+  a.p = d;
   if (a.dense) li_score_sm100_kernel<true><<<grid, kLiThreads, kLiSmemBytes, st>>>(tq, tk, a);
   else li_score_sm100_kernel<false><<<grid, kLiThreads, kLiSmemBytes, st>>>(tq, tk, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;

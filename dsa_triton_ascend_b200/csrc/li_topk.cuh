@@ -54,6 +54,27 @@ __device__ __forceinline__ uint32_t bins_exclusive_prefix(uint32_t v, uint32_t* 
   return base + inc - v;
 }
 
+// What every top-k kernel does beside the selection: zeros in the place of values that are not wanted, and (the first
+// block) the scoring kernel's status bytes folded into the status word.
+template <typename T>
+__device__ __forceinline__ void li_row_extras(const LiDev& p, int32_t rown) {
+  if (p.zero_values) {
+    const int32_t K = p.sparse_count;
+    T* ov = (T*)p.out_values + (int64_t)rown * K;
+    if ((K & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out_values) & 15) == 0) {
+      for (int i = threadIdx.x; i < K / 8; i += kTopkThreads) reinterpret_cast<uint4*>(ov)[i] = make_uint4(0, 0, 0, 0);
+    } else {
+      for (int i = threadIdx.x; i < K; i += kTopkThreads) ov[i] = from_f32<T>(0.f);
+    }
+  }
+  if (rown == 0 && p.cta_status != nullptr && threadIdx.x < 32) {
+    uint32_t v = 0;
+    for (int i = threadIdx.x; i < p.n_cta_status; i += 32) v = max(v, (uint32_t)p.cta_status[i]);
+    v = __reduce_max_sync(0xffffffffu, v);
+    if (threadIdx.x == 0) *p.status = (int32_t)v;
+  }
+}
+
 // grid = rows * n2; block = 512 threads; dynamic smem = sort_cap * 8 + kTopkKeyCache * 4 bytes.
 template <typename T, bool kRank16>
 __global__ void __launch_bounds__(kTopkThreads) li_topk_kernel(LiDev p, const float* __restrict__ scores,
@@ -75,6 +96,7 @@ __global__ void __launch_bounds__(kTopkThreads) li_topk_kernel(LiDev p, const fl
   const int32_t nsel = min(n, K);
   int32_t* oi = p.out_indices + (int64_t)rown * K;
   T* ov = (p.return_value && p.out_values != nullptr) ? (T*)p.out_values + (int64_t)rown * K : nullptr;
+  li_row_extras<T>(p, rown);
 
   for (int i = nsel + tid; i < K; i += kTopkThreads) {
     oi[i] = -1;
@@ -278,6 +300,7 @@ __global__ void __launch_bounds__(kTopkThreads) li_topk_fast_kernel(LiDev p, con
   const int32_t nsel = min(n, K);
   int32_t* oi = p.out_indices + (int64_t)rown * K;
   T* ov = (p.return_value && p.out_values != nullptr) ? (T*)p.out_values + (int64_t)rown * K : nullptr;
+  li_row_extras<T>(p, rown);
 
   if (nsel == 0) {
     for (int i = tid; i < K; i += kTopkThreads) {
@@ -538,6 +561,7 @@ __global__ void __launch_bounds__(kTopkThreads, 4) li_topk_bins_kernel(LiDev p, 
   const int32_t nsel = min(n, K);
   int32_t* oi = p.out_indices + (int64_t)rown * K;
   T* ov = (p.return_value && p.out_values != nullptr) ? (T*)p.out_values + (int64_t)rown * K : nullptr;
+  li_row_extras<T>(p, rown);
   if (nsel == 0) {
     for (int i = tid; i < K; i += kTopkThreads) {
       oi[i] = -1;
@@ -825,6 +849,7 @@ __global__ void __launch_bounds__(kTopkThreads, 2) li_topk_bins_stream_kernel(Li
   const int32_t nsel = min(n, K);
   int32_t* oi = p.out_indices + (int64_t)rown * K;
   T* ov = (p.return_value && p.out_values != nullptr) ? (T*)p.out_values + (int64_t)rown * K : nullptr;
+  li_row_extras<T>(p, rown);
   if (nsel == 0) {
     for (int i = tid; i < K; i += kTopkThreads) {
       oi[i] = -1;

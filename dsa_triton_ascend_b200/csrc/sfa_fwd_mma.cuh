@@ -24,6 +24,7 @@ struct SfaDev {
   float* softmax_sum;
   int32_t rows, n1, d, d_rope;
   int32_t sparse_count, sparse_block_size, return_lse;
+  int32_t zero_lse;            // the statistics are not wanted: the pre-pass stores zeros
   float scale;
 };
 

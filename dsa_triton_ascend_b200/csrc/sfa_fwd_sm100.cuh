@@ -169,6 +169,8 @@ __global__ void __launch_bounds__(128) sfa_compact_kernel(SfaDev p, int2* __rest
   if (blockIdx.x == 0 && threadIdx.x < 64) status[threadIdx.x] = 0;
   if (row >= p.rows) return;
   if (lane == 0) redo[row] = 0;
+  if (p.zero_lse)
+    for (int32_t h = lane; h < p.n1; h += 32) p.softmax_max[(int64_t)row * p.n1 + h] = p.softmax_sum[(int64_t)row * p.n1 + h] = 0.f;
   const RowInfo ri = row_info(p.seq, row);
   const int32_t slots = p.sparse_count * p.sparse_block_size;
   const int32_t* idx_row = p.sparse_indices + (int64_t)row * p.sparse_count;
@@ -274,6 +276,8 @@ __global__ void __launch_bounds__(256) sfa_compact_block_kernel(SfaDev p, int2* 
   if (row == 0 && threadIdx.x == 0) *redo_count = 0;
   if (row == 0 && threadIdx.x < 64) status[threadIdx.x] = 0;   // (workspace header, as above)
   if (threadIdx.x == 0) redo[row] = 0;
+  if (p.zero_lse)
+    for (int32_t h = threadIdx.x; h < p.n1; h += 256) p.softmax_max[(int64_t)row * p.n1 + h] = p.softmax_sum[(int64_t)row * p.n1 + h] = 0.f;
   const RowInfo ri = row_info(p.seq, row);
   const int32_t slots = p.sparse_count;
   const int32_t* idx_row = p.sparse_indices + (int64_t)row * slots;

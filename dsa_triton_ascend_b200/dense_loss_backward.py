@@ -12,8 +12,8 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, dtype_code, note_launch, packed, ptr, require_cuda, seq_tensor,
-                    workspace)
+from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, note_launch, packed, ptr, require_cuda,
+                    seq_tensor, workspace)
 
 SUPPORTED_D = (128, 256, 512)
 
@@ -70,7 +70,7 @@ def npu_dense_lightning_indexer_softmax_lse_triton(query_index, key_index, weigh
     p.dtype = dtype_code(query_index, (torch.bfloat16, torch.float16), "query_index")
     p.dtype_w = dtype_code(weights, (torch.bfloat16, torch.float16, torch.float32), "weights")
     p.batch, p.s1, p.s2, p.g, p.d_idx = B, S1, S2, G, Di
-    with torch.cuda.device(dev):
+    with device_guard(dev):
         nbytes = ctypes.c_size_t(0)
         _cabi.check(_cabi.lib.dsa_dense_li_lse_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)),
                     "dense_lightning_indexer_softmax_lse")
@@ -182,7 +182,7 @@ def dense_loss_backward_triton(query, key, query_index, key_index, weights, soft
     p.dense, p.n2 = 1, N2
     p.softmax_max_index, p.softmax_sum_index = ptr(softmax_max_index), ptr(softmax_sum_index)
 
-    with torch.cuda.device(dev):
+    with device_guard(dev):
         nbytes = ctypes.c_size_t(0)
         _cabi.check(_cabi.lib.dsa_sli_grad_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)), "dense_loss_backward")
         ws = workspace(nbytes.value, dev)

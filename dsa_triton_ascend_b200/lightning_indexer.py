@@ -21,7 +21,7 @@ import os
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, dtype_code, max_len_from_cumulative, note_launch, ptr,
+from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, max_len_from_cumulative, note_launch, ptr,
                     require_cuda, seq_tensor, workspace)
 
 _RANK_MODES = {"io_dtype": _cabi.RANK_IO_DTYPE, "fp32": _cabi.RANK_FP32}
@@ -115,7 +115,7 @@ def _build_params(query, key, weights, actual_seq_lengths_query, actual_seq_leng
     query, key, weights = query.contiguous(), key.contiguous(), weights.contiguous()
     rows = s1 if is_tnd else B * s1
     idx = torch.empty((rows, N2, sparse_count), dtype=torch.int32, device=dev)
-    val = torch.empty((rows, N2, sparse_count), dtype=query.dtype, device=dev) if return_value else None
+    val = torch.empty((rows, N2, sparse_count), dtype=query.dtype, device=dev)
 
     p = _cabi.DsaLiParams()
     p.struct_size = ctypes.sizeof(_cabi.DsaLiParams)
@@ -132,7 +132,7 @@ def _build_params(query, key, weights, actual_seq_lengths_query, actual_seq_leng
     p.block_size, p.max_blocks = block_size, max_blocks
     p.sparse_count, p.sparse_mode = int(sparse_count), int(sparse_mode)
     p.rank_mode = _RANK_MODES[_rank_mode]
-    p.return_value = 1 if return_value else 0
+    p.return_value = 1 if return_value else _cabi.OUT_ZEROS
     p.phases = _cabi.PHASE_ALL
     p.key_rows = key.numel() // (N2 * D)
     keep = (query, key, weights, seq_q, seq_k, block_table, idx, val)
@@ -182,7 +182,7 @@ def lightning_indexer_triton(
         query, key, weights, actual_seq_lengths_query, actual_seq_lengths_key, block_table,
         layout_query, layout_key, sparse_count, sparse_mode, return_value, max_seqlen_key)
     dev = query.device
-    with torch.cuda.device(dev):
+    with device_guard(dev):
         nbytes = ctypes.c_size_t(0)
         _cabi.check(_cabi.lib.dsa_li_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)), "lightning_indexer")
         ws = workspace(nbytes.value, dev)
@@ -190,9 +190,7 @@ def lightning_indexer_triton(
                     "lightning_indexer")
         note_launch("lightning_indexer", ws, dev)
     del keep
-    indices = idx.view(out_shape)
-    values = val.view(out_shape) if val is not None else torch.zeros(out_shape, dtype=query.dtype, device=dev)
-    return indices, values
+    return idx.view(out_shape), val.view(out_shape)
 
 
 class LightningIndexerTriton(torch.nn.Module):

@@ -12,7 +12,7 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, dtype_code, max_len_from_cumulative, note_launch, packed,
+from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, max_len_from_cumulative, note_launch, packed,
                     ptr, require_cuda, seq_tensor, workspace)
 
 _VALID_D = (128, 256, 512)
@@ -143,11 +143,8 @@ def sparse_flash_attention_triton(
 
     out = torch.empty_like(query)
     stat_shape = (1, s1, N1) if is_tnd_q else (B, 1, s1, N1)
-    if return_softmax_lse:
-        sm_max = torch.empty(stat_shape, dtype=torch.float32, device=dev)
-        sm_sum = torch.empty(stat_shape, dtype=torch.float32, device=dev)
-    else:
-        sm_max = sm_sum = None
+    sm_max = torch.empty(stat_shape, dtype=torch.float32, device=dev)
+    sm_sum = torch.empty(stat_shape, dtype=torch.float32, device=dev)
 
     p = _cabi.DsaSfaParams()
     p.struct_size = ctypes.sizeof(_cabi.DsaSfaParams)
@@ -165,12 +162,12 @@ def sparse_flash_attention_triton(
     p.block_size, p.max_blocks = pa_block, max_blocks
     p.sparse_count, p.sparse_block_size = topk, sparse_block_size
     p.sparse_mode = sparse_mode
-    p.return_lse = 1 if return_softmax_lse else 0
+    p.return_lse = 1 if return_softmax_lse else _cabi.OUT_ZEROS
     p.scale = float(scale_value)
     p.key_rows = key.numel() // D
 
     if rows > 0:
-        with torch.cuda.device(dev):
+        with device_guard(dev):
             nbytes = ctypes.c_size_t(0)
             _cabi.check(_cabi.lib.dsa_sfa_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)),
                         "sparse_flash_attention")
@@ -178,9 +175,6 @@ def sparse_flash_attention_triton(
             _cabi.check(_cabi.lib.dsa_sfa_forward(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
                         "sparse_flash_attention")
             note_launch("sparse_flash_attention", ws, dev)
-    if not return_softmax_lse:
-        sm_max = torch.zeros(stat_shape, dtype=torch.float32, device=dev)
-        sm_sum = torch.zeros(stat_shape, dtype=torch.float32, device=dev)
     return out, sm_max, sm_sum
 
 

@@ -13,7 +13,7 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, dtype_code, max_len_from_cumulative, note_launch, packed,
+from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, max_len_from_cumulative, note_launch, packed,
                     ptr, require_cuda, seq_tensor, workspace)
 
 _VALID_D = (128, 256, 512)
@@ -154,7 +154,7 @@ def sparse_flash_attention_grad_triton(
     p.scale = float(scale_value)
     p.key_rows = key.numel() // D
 
-    with torch.cuda.device(dev):
+    with device_guard(dev):
         nbytes = ctypes.c_size_t(0)
         _cabi.check(_cabi.lib.dsa_sfa_grad_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)),
                     "sparse_flash_attention_grad")

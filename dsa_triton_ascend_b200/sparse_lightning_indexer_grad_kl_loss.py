@@ -13,8 +13,8 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, dtype_code, note_launch, packed, ptr, require_cuda, seq_tensor,
-                    workspace)
+from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, note_launch, packed, ptr, require_cuda,
+                    seq_tensor, workspace)
 
 
 def sparse_lightning_indexer_grad_kl_loss_triton(
@@ -110,7 +110,7 @@ def sparse_lightning_indexer_grad_kl_loss_triton(
     p.g, p.d_idx, p.topk = G, Di, topk
     p.scale = float(scale_value)
 
-    with torch.cuda.device(dev):
+    with device_guard(dev):
         nbytes = ctypes.c_size_t(0)
         _cabi.check(_cabi.lib.dsa_sli_grad_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)),
                     "sparse_lightning_indexer_grad_kl_loss")

@@ -54,6 +54,10 @@ extern "C" {
 #define DSA_KERNEL_TENSOR 2   /* tensor-core path; forward calls: DSA_ERR_UNSUPPORTED when the shape is
                                  not eligible (the attention backward takes every legal shape) */
 
+/* return_value / return_lse: 0 the buffer is not written (it may be NULL), 1 the results, or zeros in their place
+   (what the reference's wrappers return for outputs that were not asked for) without a fill of the caller's */
+#define DSA_OUT_ZEROS 2
+
 #define DSA_PHASE_SCORE 1
 #define DSA_PHASE_TOPK 2
 #define DSA_PHASE_ALL 3
@@ -79,7 +83,7 @@ typedef struct DsaLiParams {
   const int32_t* seq_k; /* [batch] lengths, or cumulative ends when seq_k_cumulative; NULL = s2 */
   const int32_t* block_table; /* PA only: [batch, max_blocks], -1 = no block                  */
   int32_t* out_indices; /* [rows, n2, sparse_count]                                           */
-  void* out_values;     /* [rows, n2, sparse_count] in dtype_qk; may be NULL if !return_value */
+  void* out_values;     /* [rows, n2, sparse_count] in dtype_qk; may be NULL if !return_value (see DSA_OUT_ZEROS) */
   int32_t layout_q;     /* DSA_LAYOUT_BSND | DSA_LAYOUT_TND                                    */
   int32_t layout_k;     /* DSA_LAYOUT_*                                                        */
   int32_t dtype_qk;     /* DSA_DTYPE_BF16 | DSA_DTYPE_FP16                                     */
