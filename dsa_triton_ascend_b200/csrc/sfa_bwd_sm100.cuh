@@ -27,12 +27,12 @@
 //     scaled by 2^13, dS by a power of two per item that keeps |dS| <= scale * (|dO| |v| + |delta|)
 //     (Cauchy-Schwarz over the item's heads and selected keys, taken by small kernels in front) below 2^13.
 //
-// Measured, whole operator call: B1 S1 512 S2 4096 N1 64 k 2048 in bf16 1.22 ms (sfa_bwd_mma_kernel: 4.63 ms); 4092
-// rows x 128 heads in bf16 7.4 ms under the power cap (32.2 ms).  A tile of 48 keys takes 12 400 cycles: its reductions alone would take
-// 8400, its products 8000.  What is left is the chain of a tile (keys 1700, S 2200, P and dS 5500, of which 1600 wait
-// for dK of the tile before, dQ 2100) beside the chain of the dV / dK tiles (issue 6400, ring slots 3100), the reload
-// of Q / dO between items, and the last of the four rounds that 512 items make on 148 SMs.
-// ptxas spills 16 bytes (bf16) and 60 bytes (fp16) of a thread's 72 registers.
+// Measured, whole operator call: B1 S1 512 S2 4096 N1 64 k 2048 in bf16 1.14 ms (sfa_bwd_mma_kernel: 4.63 ms); 4092
+// rows x 128 heads in bf16 7.3 ms under the power cap (32.2 ms).  A tile of 48 keys takes 12 400 cycles: its
+// reductions alone would take 8400, its products 8000.  What is left is the chain of a tile (keys 1700, S 2200, P and
+// dS 5500, of which 1600 wait for dK of the tile before, dQ 2100) beside the chain of the dV / dK tiles (issue 6400,
+// ring slots 3100), and the reload of Q / dO between items.
+// ptxas spills 0 bytes (bf16) and 32 bytes (fp16) of a thread's 72 registers.
 //
 // Tensor memory: dQ^T 5 x 64 columns | S, dP 48 | rope part of S 48 | drain ring 2 x 48.
 // Warps (896 threads): 0..7 softmax (lane quarter = warp & 3: quarters 0, 1 hold S of heads 0..63,
@@ -86,9 +86,35 @@ struct SfaBwdArgs {
   const float* delta;        // [rows, n1]
   const int32_t* exps;       // fp16: [items] exponent of the power of two that the item's dS is scaled by
   uint32_t idesc_s, idesc_q, idesc_d;
-  int32_t items, hblocks;    // rows * hblocks
+  int32_t items, hblocks;    // rows * hblocks, the last ones cut into parts (SfaBwdSplit)
+  int32_t full, parts;
+  float* dq_part;            // [items - full][64 heads][576]
   int32_t key_rows;
 };
+struct BwdItem { int32_t base, row, h0, slot; int2 nv; };
+// Work item `i`: its (row, 64 heads), its share of the row's list, and its place in dq_part (-1: the whole row).
+__device__ __forceinline__ BwdItem bwd_item(const SfaBwdArgs& a, int32_t i) {
+  BwdItem it;
+  it.base = i;
+  it.slot = i - a.full;
+  int32_t part = 0;
+  if (it.slot >= 0) {
+    const int32_t r = it.slot / a.parts;
+    part = it.slot - r * a.parts;
+    it.base = a.full + r;
+  } else {
+    it.slot = -1;
+  }
+  it.row = it.base / a.hblocks;
+  it.h0 = (it.base - it.row * a.hblocks) * kBwdHeads;
+  it.nv = a.nvalid[it.row];
+  if (it.slot >= 0) {
+    const int32_t tiles = (it.nv.x + kBwdBK - 1) / kBwdBK, per = (tiles + a.parts - 1) / a.parts * kBwdBK;
+    it.nv.x = max(0, min(per, it.nv.x - part * per));
+    it.nv.y += part * per;
+  }
+  return it;
+}
 
 __device__ __forceinline__ void red_add(float* addr, float v) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
@@ -246,8 +272,8 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint32_t n_tile = 0, n_item = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hblocks, h0 = (item - row * a.hblocks) * kBwdHeads;
-      const int32_t nvalid = a.nvalid[row].x, ntiles = tiles_of(nvalid);
+      const BwdItem it = bwd_item(a, item);
+      const int32_t row = it.row, h0 = it.h0, nvalid = it.nv.x, ntiles = tiles_of(nvalid);
       const bool head = h0 + hl < n1;
       const int64_t hi_ = (int64_t)row * n1 + h0 + hl;
       if (ntiles > 0) {
@@ -263,7 +289,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
         // (a head without a sum, or past the last one, has P = 0 whatever its scores are)
         const int32_t nlive = !is_s || c1 > 0.f ? nvalid : 0;
-        if constexpr (kScaled) up = is_s ? 8192.f : scalbnf(1.f, a.exps[item]);
+        if constexpr (kScaled) up = is_s ? 8192.f : scalbnf(1.f, a.exps[it.base]);
         for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
           const uint32_t ph = n_tile & 1;
           ok = wait(s_full, ph);
@@ -334,7 +360,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       }
       // dQ^T tile m: this thread's feature is m * 128 + quarter * 32 + lane, a column is a head
       float down = 1.f;
-      if constexpr (kScaled) { if (ntiles > 0) down = scalbnf(1.f, -a.exps[item]); }
+      if constexpr (kScaled) { if (ntiles > 0) down = scalbnf(1.f, -a.exps[it.base]); }
       const int32_t hn = min(kBwdHeads, n1 - h0);
 #pragma unroll 1
       for (int m = half; m < 5; m += 2) {
@@ -354,9 +380,16 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
             for (int i = 0; i < 16; ++i) o[i] = 0.f;
           }
+          if (it.slot < 0) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (c + i < hn) dst[(int64_t)(c + i) * step] = from_f32<T>(o[i] * down);
+            for (int i = 0; i < 16; ++i)
+              if (c + i < hn) dst[(int64_t)(c + i) * step] = from_f32<T>(o[i] * down);
+          } else {
+            float* part = a.dq_part + ((int64_t)it.slot * kBwdHeads + c) * 576 + m * 128 + f;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (c + i < hn) part[i * 576] = o[i] * down;
+          }
         }
       }
       if (ntiles > 0) {
@@ -378,11 +411,11 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     int turn = 0, rbuf = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hblocks;
-      const int2 nv = a.nvalid[row];
+      const BwdItem it = bwd_item(a, item);
+      const int2 nv = it.nv;
       const int32_t ntiles = tiles_of(nv.x);
       float dk_down = 1.f;
-      if constexpr (kScaled) { if (ntiles > 0) dk_down = scalbnf(1.f, -a.exps[item]); }
+      if constexpr (kScaled) { if (ntiles > 0) dk_down = scalbnf(1.f, -a.exps[it.base]); }
       for (int32_t t = 0; t < ntiles && ok; ++t) {
         const int4* rows4 = reinterpret_cast<const int4*>(rows_s + rbuf * kBwdBK);
         rbuf = rbuf == 2 ? 0 : rbuf + 1;
@@ -446,7 +479,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     int rbuf = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int2 nv = a.nvalid[item / a.hblocks];
+      const int2 nv = bwd_item(a, item).nv;
       const int32_t ntiles = tiles_of(nv.x);
       const int32_t* list = a.key_list + nv.y;
       int32_t rn[3] = {0, 0, 0};
@@ -501,7 +534,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint32_t n_tile = 0, n_item = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t ntiles = tiles_of(a.nvalid[item / a.hblocks].x);
+      const int32_t ntiles = tiles_of(bwd_item(a, item).nv.x);
       if (ntiles == 0) continue;
       ok = wait(q_full, n_item & 1);
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
@@ -554,10 +587,10 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     int turn = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hblocks, h0 = (item - row * a.hblocks) * kBwdHeads;
-      const int32_t ntiles = tiles_of(a.nvalid[row].x);
+      const BwdItem it = bwd_item(a, item);
+      const int32_t ntiles = tiles_of(it.nv.x);
       if (ntiles == 0) continue;
-      const int steps = (min(kBwdHeads, n1 - h0) + 15) / 16;       // 16-head steps with real heads
+      const int steps = (min(kBwdHeads, n1 - it.h0) + 15) / 16;       // 16-head steps with real heads
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
         const uint32_t ph = n_tile & 1;
 #pragma unroll 1
@@ -598,8 +631,9 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     bool ok = true;
     if (lane == 0) { ptx::prefetch_tmap(&tmap_q); ptx::prefetch_tmap(&tmap_qr); ptx::prefetch_tmap(&tmap_do); }
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hblocks, h0 = (item - row * a.hblocks) * kBwdHeads;
-      if (a.nvalid[row].x == 0) continue;
+      const BwdItem it = bwd_item(a, item);
+      const int32_t row = it.row, h0 = it.h0;
+      if (it.nv.x == 0) continue;
       if (lane == 0) {
         ok = ptx::mbar_wait(q_empty, (n_item & 1) ^ 1, abort_flag);
         if (ok) {
@@ -615,7 +649,8 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         // the other lanes pull the next item's rows into L2
         const int32_t next = item + gridDim.x;
         if (next < a.items) {
-          const int32_t nrow = next / a.hblocks, nh0 = (next - nrow * a.hblocks) * kBwdHeads;
+          const BwdItem nx = bwd_item(a, next);
+          const int32_t nrow = nx.row, nh0 = nx.h0;
           const int64_t off = ((int64_t)nrow * n1 + nh0) * 1024;
           for (int32_t i = lane - 1; i < min(kBwdHeads, n1 - nh0) * 8; i += 31) {
             ptx::prefetch_l2((const unsigned char*)a.p.query + off + (int64_t)i * 128);
@@ -643,7 +678,38 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, misaligned ? 2 : 1);
 }
 
+// d_query of the rows that were cut into parts: the parts' sums in their order, rounded once.
+template <typename T>
+__global__ void __launch_bounds__(192) sfa_bwd_dq_kernel(const float* __restrict__ dq_part, T* __restrict__ d_query,
+                                                         T* __restrict__ d_query_rope, int32_t full, int32_t parts,
+                                                         int32_t hblocks, int32_t n1) {
+  const int32_t base = full + blockIdx.x, row = base / hblocks, hl = blockIdx.y;
+  const int32_t h = (base - row * hblocks) * kBwdHeads + hl;
+  if (h >= n1) return;
+  const float* src = dq_part + ((int64_t)blockIdx.x * parts * kBwdHeads + hl) * 576;
+#pragma unroll
+  for (int u = 0; u < 3; ++u) {
+    const int f = threadIdx.x + u * 192;
+    float v = src[f];
+    for (int32_t q = 1; q < parts; ++q) v += src[(int64_t)q * kBwdHeads * 576 + f];
+    const int64_t i = (int64_t)row * n1 + h;
+    if (f < 512) d_query[i * 512 + f] = from_f32<T>(v);
+    else d_query_rope[i * 64 + f - 512] = from_f32<T>(v);
+  }
+}
+
 // ---- host side ---------------------------------------------------------------------------------
+// Items of the last round: a round lasts as long as its longest item, so where half of the SMs or more would idle in
+// it, its items are cut into 2 to 4 parts of 8 tiles or more, whose d_query is added up afterwards.  512 rows x 64
+// heads, 2048 of 4096 keys: 4 rounds -> 3.5, 1222 -> 1135 us.  148 SMs are assumed (the workspace is sized from it); any other
+// number is still correct.
+struct SfaBwdSplit { int32_t full, parts, items; };
+inline SfaBwdSplit sfa_bwd_split(int64_t items, int64_t slots) {
+  const int64_t sms = 148, rest = items % sms;
+  const int64_t parts = rest == 0 ? 1 : std::min<int64_t>(std::min<int64_t>(4, sms / rest), slots / (8 * kBwdBK));
+  if (parts < 2) return SfaBwdSplit{(int32_t)items, 1, (int32_t)items};
+  return SfaBwdSplit{(int32_t)(items - rest), (int32_t)parts, (int32_t)(items - rest + rest * parts)};
+}
 inline int64_t sfa_bwd_rows(const DsaSfaGradParams* p) {
   return p->layout_q == DSA_LAYOUT_TND ? (int64_t)p->s1 : (int64_t)p->batch * p->s1;
 }
@@ -665,8 +731,9 @@ inline bool sfa_bwd_sm100_aligned(const DsaSfaGradParams* p) {
            (uintptr_t)p->d_out | (uintptr_t)p->out) & 15u) == 0;
 }
 // Workspace: header | dk / dv accumulators | fp16: bounds of the items - zeroed before the call - | fp16: exponents
-// of the items, norms of the keys | nvalid | delta | redo flags and count of the pre-pass (unused) | key_list
-struct SfaBwdWs { size_t acc, bound, zeroed, exps, norms, nvalid, delta, redo, key_list, total; };
+// of the items, norms of the keys | nvalid | delta | redo flags and count of the pre-pass (unused) | d_query of parts
+// of rows | key_list
+struct SfaBwdWs { size_t acc, bound, zeroed, exps, norms, nvalid, delta, redo, dq_part, key_list, total; };
 inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   const size_t rows = (size_t)sfa_bwd_rows(p);
@@ -681,7 +748,9 @@ inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
   w.nvalid = w.norms + (fp16 ? up((size_t)p->key_rows * 4) : 0);
   w.delta = w.nvalid + up(rows * 8);
   w.redo = w.delta + up(rows * p->n1 * 4);
-  w.key_list = w.redo + up(rows * 4) + 256;
+  w.dq_part = w.redo + up(rows * 4) + 256;
+  const SfaBwdSplit sp = sfa_bwd_split((int64_t)items, (int64_t)p->sparse_count * p->sparse_block_size);
+  w.key_list = w.dq_part + (size_t)(sp.items - sp.full) * kBwdHeads * 576 * 4;
   w.total = w.key_list + rows * p->sparse_count * p->sparse_block_size * 4;
   return w;
 }
@@ -744,7 +813,9 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   a.idesc_q = ptx::idesc_f16(fmt, 128, kBwdHeads, 1, 1);
   a.idesc_d = ptx::idesc_f16(fmt, 128, kBwdBK, 1, 0);
   a.hblocks = hblocks;
-  a.items = d.rows * a.hblocks;
+  const SfaBwdSplit sp = sfa_bwd_split((int64_t)d.rows * hblocks, slots);
+  a.items = sp.items; a.full = sp.full; a.parts = sp.parts;
+  a.dq_part = (float*)(ws + w.dq_part);
   a.key_rows = (int32_t)p->key_rows;
   CUtensorMap tq, tqr, tdo;
   if (!make_tmap_3d_16bit(&tq, p->query, (uint64_t)d.rows, (uint64_t)p->n1, 512, 1024, (uint64_t)p->n1 * 1024, kBwdHeads,
@@ -758,6 +829,12 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   sfa_bwd_sm100_kernel<T><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tqr, tdo, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
+  if (sp.parts > 1) {
+    sfa_bwd_dq_kernel<T><<<dim3((unsigned)((sp.items - sp.full) / sp.parts), (unsigned)std::min(p->n1, kBwdHeads)), 192, 0, st>>>(
+        a.dq_part, (T*)p->d_query, (T*)p->d_query_rope, sp.full, sp.parts, hblocks, p->n1);
+    if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
+    count_launch();
+  }
   return DSA_OK;
 }
 

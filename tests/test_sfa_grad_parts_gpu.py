@@ -1,0 +1,48 @@
+"""Attention backward where the last round of work items is cut into parts: against the CUDA-core kernel, which takes
+every row as a whole."""
+import pytest
+import torch
+
+from dsa_triton_ascend_b200 import check_status, sparse_flash_attention_grad_triton, sparse_flash_attention_triton
+from dsa_triton_ascend_b200 import sparse_flash_attention_grad as grad
+
+pytestmark = pytest.mark.gpu
+
+
+# items of 64 heads left for the last round of 148: 2 (four parts), 52 (two parts), 2 of two head blocks
+# (the second of 16 heads), 49 (three parts, short rows: parts without keys), 75 (whole: more than half a round)
+@pytest.mark.parametrize("q_lens,k_lens,heads", [([150], [1200], 16), ([200], [1200], 64), ([75], [1300], 80),
+                                                 ([20, 177], [20, 1000], 16), ([223], [1200], 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_parts_add_up(q_lens, k_lens, heads, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(sum(q_lens) + heads)
+    rows, keys, count = sum(q_lens), sum(k_lens), 1152
+
+    def normal(*shape):
+        return (torch.randn(shape, generator=gen, device="cuda") * 0.3).to(dtype)
+
+    q, qr, k, kr = normal(rows, heads, 512), normal(rows, heads, 64), normal(keys, 1, 512), normal(keys, 1, 64)
+    d_out = normal(rows, heads, 512)
+    ends_q, ends_k = ([sum(v[:i + 1]) for i in range(len(v))] for v in (q_lens, k_lens))
+    idx = torch.stack([torch.randperm(max(k_lens), generator=gen, device="cuda")[:count] if max(k_lens) >= count else
+                       torch.nn.functional.pad(torch.randperm(max(k_lens), generator=gen, device="cuda"),
+                                               (0, count - max(k_lens)), value=-1) for _ in range(rows)])
+    idx = idx.to(torch.int32).view(rows, 1, count)
+    kw = dict(scale_value=576 ** -0.5, query_rope=qr, key_rope=kr, actual_seq_lengths_query=ends_q,
+              actual_seq_lengths_kv=ends_k, sparse_mode=3)
+    out, mx, sm = sparse_flash_attention_triton(q, k, k, idx, layout_query="TND", layout_kv="TND",
+                                                return_softmax_lse=True, **kw)
+    args = (q, k, k, idx, d_out, out, mx, sm)
+    got = sparse_flash_attention_grad_triton(*args, layout="TND", **kw)
+    again = sparse_flash_attention_grad_triton(*args, layout="TND", **kw)
+    check_status()
+    grad.set_kernel("portable")
+    try:
+        want = sparse_flash_attention_grad_triton(*args, layout="TND", **kw)
+    finally:
+        grad.set_kernel("auto")
+    # each side rounds an fp32 sum once: 2^-9 (bf16) or 2^-12 (fp16) of a value at most
+    bound = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    for g, w in zip(got, want):
+        assert (g.double() - w.double()).norm() <= bound * w.double().norm()
+    assert torch.equal(got[0], again[0]) and torch.equal(got[3], again[3])     # d_query, d_query_rope: no atomics
