@@ -111,21 +111,21 @@ static int li_launch(const DsaLiParams* p, float* scores, cudaStream_t st, int32
     if (p->s2 <= kTopkThreads * kTopkFastKeys && p->sparse_count <= kTopkThreads * 4) {
       // register / shuffle kernel: rows of up to 8192 keys, up to 2048 outputs
       const int e = p->sparse_count <= kTopkThreads ? 1 : (p->sparse_count <= 2 * kTopkThreads ? 2 : 4);
-#define DSA_TOPK_FAST(R, E) li_topk_fast_kernel<T, R, E><<<(unsigned)rown, kTopkThreads, 0, st>>>(d, scores, ld)
+#define DSA_TOPK_FAST(R, E) launch_after(li_topk_fast_kernel<T, R, E>, dim3((unsigned)rown), dim3(kTopkThreads), 0, st, d, scores, ld)
       if (rank16) {
         // io-dtype ranking: one histogram on a linear scale selects and orders
-        if (e == 1) li_topk_bins_kernel<T, 1><<<(unsigned)rown, kTopkThreads, 0, st>>>(d, scores, ld);
-        else if (e == 2) li_topk_bins_kernel<T, 2><<<(unsigned)rown, kTopkThreads, 0, st>>>(d, scores, ld);
-        else li_topk_bins_kernel<T, 4><<<(unsigned)rown, kTopkThreads, 0, st>>>(d, scores, ld);
+        if (e == 1) launch_after(li_topk_bins_kernel<T, 1>, dim3((unsigned)rown), dim3(kTopkThreads), 0, st, d, scores, ld);
+        else if (e == 2) launch_after(li_topk_bins_kernel<T, 2>, dim3((unsigned)rown), dim3(kTopkThreads), 0, st, d, scores, ld);
+        else launch_after(li_topk_bins_kernel<T, 4>, dim3((unsigned)rown), dim3(kTopkThreads), 0, st, d, scores, ld);
       }
       else { if (e == 1) DSA_TOPK_FAST(false, 1); else if (e == 2) DSA_TOPK_FAST(false, 2); else DSA_TOPK_FAST(false, 4); }
 #undef DSA_TOPK_FAST
     } else if (rank16 && p->sparse_count <= kTopkThreads * 4) {
       // longer rows, io-dtype ranking: the same histogram selection, streaming the row twice
       const int e = p->sparse_count <= kTopkThreads ? 1 : (p->sparse_count <= 2 * kTopkThreads ? 2 : 4);
-      if (e == 1) li_topk_bins_stream_kernel<T, 1><<<(unsigned)rown, kTopkThreads, 0, st>>>(d, scores, ld);
-      else if (e == 2) li_topk_bins_stream_kernel<T, 2><<<(unsigned)rown, kTopkThreads, 0, st>>>(d, scores, ld);
-      else li_topk_bins_stream_kernel<T, 4><<<(unsigned)rown, kTopkThreads, 0, st>>>(d, scores, ld);
+      if (e == 1) launch_after(li_topk_bins_stream_kernel<T, 1>, dim3((unsigned)rown), dim3(kTopkThreads), 0, st, d, scores, ld);
+      else if (e == 2) launch_after(li_topk_bins_stream_kernel<T, 2>, dim3((unsigned)rown), dim3(kTopkThreads), 0, st, d, scores, ld);
+      else launch_after(li_topk_bins_stream_kernel<T, 4>, dim3((unsigned)rown), dim3(kTopkThreads), 0, st, d, scores, ld);
     } else {
       int32_t cap = 1;
       while (cap < p->sparse_count) cap <<= 1;
@@ -134,11 +134,11 @@ static int li_launch(const DsaLiParams* p, float* scores, cudaStream_t st, int32
       if (rank16) {
         e = cudaFuncSetAttribute(li_topk_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return DSA_ERR_CUDA;
-        li_topk_kernel<T, true><<<(unsigned)rown, kTopkThreads, smem, st>>>(d, scores, ld, cap);
+        launch_after(li_topk_kernel<T, true>, dim3((unsigned)rown), dim3(kTopkThreads), smem, st, d, scores, ld, cap);
       } else {
         e = cudaFuncSetAttribute(li_topk_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return DSA_ERR_CUDA;
-        li_topk_kernel<T, false><<<(unsigned)rown, kTopkThreads, smem, st>>>(d, scores, ld, cap);
+        launch_after(li_topk_kernel<T, false>, dim3((unsigned)rown), dim3(kTopkThreads), smem, st, d, scores, ld, cap);
       }
     }
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;

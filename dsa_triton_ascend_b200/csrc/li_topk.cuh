@@ -90,6 +90,8 @@ __global__ void __launch_bounds__(kTopkThreads) li_topk_kernel(LiDev p, const fl
   const uint32_t lt = (1u << (tid & 31)) - 1u;
   const int32_t rown = blockIdx.x;
   const int32_t row = rown / p.n2;
+  grid_dep_launch();
+  grid_dep_wait();
   const RowInfo ri = row_info(p.seq, row);
   const int32_t n = ri.visible;
   const int32_t K = p.sparse_count;
@@ -294,6 +296,8 @@ __global__ void __launch_bounds__(kTopkThreads) li_topk_fast_kernel(LiDev p, con
   const int tid = threadIdx.x;
   const int32_t rown = blockIdx.x;
   const int32_t row = rown / p.n2;
+  grid_dep_launch();
+  grid_dep_wait();
   const RowInfo ri = row_info(p.seq, row);
   const int32_t n = ri.visible;
   const int32_t K = p.sparse_count;
@@ -555,6 +559,8 @@ __global__ void __launch_bounds__(kTopkThreads, 4) li_topk_bins_kernel(LiDev p, 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t rown = blockIdx.x;
   const int32_t row = rown / p.n2;
+  grid_dep_launch();
+  grid_dep_wait();
   const RowInfo ri = row_info(p.seq, row);
   const int32_t n = ri.visible;
   const int32_t K = p.sparse_count;
@@ -843,6 +849,8 @@ __global__ void __launch_bounds__(kTopkThreads, 2) li_topk_bins_stream_kernel(Li
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t rown = blockIdx.x;
   const int32_t row = rown / p.n2;
+  grid_dep_launch();
+  grid_dep_wait();
   const RowInfo ri = row_info(p.seq, row);
   const int32_t n = ri.visible;
   const int32_t K = p.sparse_count;

@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(kSfaSimtThreads) sfa_fwd_mma_kernel(SfaDev p) 
 template <typename T>
 __global__ void __launch_bounds__(kSfaSimtThreads) sfa_redo_kernel(SfaDev p, const int32_t* __restrict__ redo_list,
                                                                    const int32_t* __restrict__ redo_count) {
+  grid_dep_wait();
   const int32_t chunks = (p.n1 + kSfaSimtHeads - 1) / kSfaSimtHeads;
   const int64_t work = (int64_t)min(*redo_count, p.rows) * chunks;
   for (int64_t i = blockIdx.x; i < work; i += gridDim.x) {

@@ -163,6 +163,8 @@ __global__ void __launch_bounds__(128) sfa_compact_kernel(SfaDev p, int2* __rest
                                                           int32_t* __restrict__ status) {
   const int lane = threadIdx.x & 31;
   const int32_t row = blockIdx.x * 4 + (threadIdx.x >> 5);
+  grid_dep_launch();
+  grid_dep_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) *redo_count = 0;
   // the workspace header (status word of the call) starts at zero: cleared here instead of by a
   // memset node of its own in front of the operator's launches
@@ -273,6 +275,8 @@ __global__ void __launch_bounds__(256) sfa_compact_block_kernel(SfaDev p, int2* 
   __shared__ int32_t counts[2][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t row = blockIdx.x;
+  grid_dep_launch();
+  grid_dep_wait();
   if (row == 0 && threadIdx.x == 0) *redo_count = 0;
   if (row == 0 && threadIdx.x < 64) status[threadIdx.x] = 0;   // (workspace header, as above)
   if (threadIdx.x == 0) redo[row] = 0;
@@ -348,11 +352,11 @@ inline void sfa_compact_launch(const SfaDev& d, int2* nvalid, int32_t* key_list,
                                int32_t kv_rows, int32_t absent, int32_t* redo, int32_t* redo_count, int32_t* status,
                                cudaStream_t st) {
   if (sfa_compact_by_blocks(d))
-    sfa_compact_block_kernel<<<d.rows, 256, 0, st>>>(d, nvalid, key_list, split, part_keys, kv_rows, absent, redo,
-                                                    redo_count, status);
+    launch_after(sfa_compact_block_kernel, dim3(d.rows), dim3(256), 0, st, d, nvalid, key_list, split, part_keys, kv_rows,
+                 absent, redo, redo_count, status);
   else
-    sfa_compact_kernel<<<(d.rows + 3) / 4, 128, 0, st>>>(d, nvalid, key_list, split, part_keys, kv_rows, absent, redo,
-                                                        redo_count, status);
+    launch_after(sfa_compact_kernel, dim3((d.rows + 3) / 4), dim3(128), 0, st, d, nvalid, key_list, split, part_keys,
+                 kv_rows, absent, redo, redo_count, status);
 }
 
 // Development aid, compiled only with -DDSA_SFA_PROFILE: cycle sums per role of the first cluster
@@ -448,6 +452,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   // the peer's barriers must exist before anything is sent to it
   ptx::cluster_arrive();
   ptx::cluster_wait();
+  grid_dep_wait();      // (nothing before this touches global memory)
   const uint32_t tmem = *tmem_slot;
 
   const int32_t n1 = a.p.n1;                   // real heads (<= 128); rows past them carry zero queries
@@ -1047,6 +1052,7 @@ __global__ void __launch_bounds__(256) sfa_merge_kernel(SfaDev p, int32_t split,
                                                         const float* __restrict__ part_m,
                                                         const float* __restrict__ part_l, int32_t is_bf16) {
   const int32_t row = blockIdx.x;
+  grid_dep_wait();
   {
     const int32_t h = blockIdx.y * 2 + threadIdx.x / (kSfaDv / 4), c4 = threadIdx.x % (kSfaDv / 4);
     if (h >= p.n1) return;
@@ -1210,12 +1216,13 @@ inline int sfa_sm100_launch(const DsaSfaParams* p, const SfaDev& d, int32_t* sta
   if (!make_tmap_3d_16bit(&tqr, p->query_rope, (uint64_t)d.rows, (uint64_t)p->n1, 64, 128, (uint64_t)p->n1 * 128,
                           kSfaCtaHeads, 64, bf16))
     return DSA_ERR_CUDA;
-  if (split > 1) sfa_fwd_sm100_kernel<true><<<clusters * 2, kSfaThreads, kSfaSmemBytes, st>>>(tq, tqr, a);
-  else sfa_fwd_sm100_kernel<false><<<clusters * 2, kSfaThreads, kSfaSmemBytes, st>>>(tq, tqr, a);
+  launch_after(split > 1 ? sfa_fwd_sm100_kernel<true> : sfa_fwd_sm100_kernel<false>, dim3(clusters * 2), dim3(kSfaThreads),
+               kSfaSmemBytes, st, tq, tqr, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
   if (split > 1) {
-    sfa_merge_kernel<<<dim3(d.rows, (p->n1 + 1) / 2), 256, 0, st>>>(d, split, a.part_o, a.part_m, a.part_l, a.is_bf16);
+    launch_after(sfa_merge_kernel, dim3(d.rows, (p->n1 + 1) / 2), dim3(256), 0, st, d, split, a.part_o, a.part_m, a.part_l,
+                 a.is_bf16);
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
     count_launch();
   }
@@ -1224,8 +1231,8 @@ inline int sfa_sm100_launch(const DsaSfaParams* p, const SfaDev& d, int32_t* sta
     const size_t smem = (size_t)(kSfaSimtHeads + kSfaSimtKeys) * (p->d + p->d_rope + kSfaSimtPad) * 2;
     const int64_t work = (int64_t)d.rows * ((p->n1 + kSfaSimtHeads - 1) / kSfaSimtHeads);
     const unsigned blocks = (unsigned)std::min<int64_t>(work, (int64_t)sms * 2);
-    if (bf16) sfa_redo_kernel<__nv_bfloat16><<<blocks, kSfaSimtThreads, smem, st>>>(d, redo_list, redo_count);
-    else sfa_redo_kernel<__half><<<blocks, kSfaSimtThreads, smem, st>>>(d, redo_list, redo_count);
+    launch_after(bf16 ? sfa_redo_kernel<__nv_bfloat16> : sfa_redo_kernel<__half>, dim3(blocks), dim3(kSfaSimtThreads), smem,
+                 st, d, redo_list, redo_count);
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
     count_launch();
   }
