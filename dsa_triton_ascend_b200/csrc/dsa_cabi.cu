@@ -492,7 +492,8 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status,
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
     count_launch();
     if (tensor && p->d_idx == 128) {
-      const int rc = sli_grad_sm100_launch<T>(p, d, status, sms, st);
+      float* part = reinterpret_cast<float*>((char*)d.dki_acc + align256((size_t)key_elems * 4));
+      const int rc = sli_grad_sm100_launch<T>(p, d, part, status, sms, st);
       if (rc != DSA_OK) return rc;
     } else {
       if (cudaFuncSetAttribute(sli_grad_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b) !=
@@ -735,7 +736,7 @@ int dsa_sli_grad_workspace_bytes(const DsaSliGradParams* p, size_t* out_bytes) {
   if (!out_bytes) return DSA_ERR_NULL;
   const size_t rows = (size_t)p->batch * p->s1;
   *out_bytes = kWorkspaceHeader + 2 * align256(rows * (size_t)sli_slots(p) * 4) + align256(rows * 4) +
-               align256(rows * 8) + (size_t)p->batch * p->s2 * p->d_idx * 4;
+               align256(rows * 8) + align256((size_t)p->batch * p->s2 * p->d_idx * 4) + sli_grad_part_bytes(p);
   return DSA_OK;
 }
 

@@ -61,12 +61,6 @@ __device__ __forceinline__ SliItem sli_score_item(const SliScoreArgs& a, int32_t
   return it;
 }
 
-// Key row of slot j of a row; past its n slots a row that does not exist (TMA fills zeros).
-__device__ __forceinline__ int32_t sli_key_row(const SliGradDev& p, const int32_t* idx_row, int32_t b, int32_t j, int32_t n,
-                                               int32_t none) {
-  return j < n ? b * p.s2 + sli_slot_key(p, idx_row, j) : none;
-}
-
 // PAD: the last chunk of attention heads is not full.  Q of the missing ones is zero, their scores are NaN beside an
 // infinite key; compiled apart because the test costs the others 1 % (2048 rows x 128 heads: 1658 -> 1674 us).
 template <bool ATT, bool PAD>
@@ -561,13 +555,47 @@ constexpr uint32_t kSgSmemBytes = kSgOffBar + 256;
 static_assert(kSgSmemBytes <= kSlSmemMax, "shared memory");
 constexpr uint32_t kSgTmS = 0, kSgTmK = 128, kSgTmQ = 384;
 
+constexpr int kSgPart = 64 * 128 + 64;
+
 struct SliGradArgs {
   SliGradDev p;
   int32_t* status;
   const float* di_max;       // [rows] largest |dI| of the row (fp16)
   int32_t hchunks, items, key_rows;
+  int32_t full, parts;
+  float* part;               // [items - full][kSgPart]: dQI of 64 heads x 128 features (before w), dW of 64 heads
   uint32_t idesc_s, idesc_k, idesc_q;
 };
+
+// Work item: (row, 64 heads) or, in the last round, a part of its slots (SliGradSplit): slots off .. off + n - 1.
+struct SliGradItem { int32_t row, h0, b, n, off, slot; };
+__device__ __forceinline__ SliGradItem sli_grad_item(const SliGradArgs& a, int32_t i) {
+  SliGradItem it;
+  it.slot = i - a.full;
+  int32_t base = i, part = 0;
+  if (it.slot >= 0) {
+    const int32_t r = it.slot / a.parts;
+    part = it.slot - r * a.parts;
+    base = a.full + r;
+  } else {
+    it.slot = -1;
+  }
+  it.row = base / a.hchunks;
+  it.h0 = (base - it.row * a.hchunks) * 64;
+  it.n = sli_row_slots(a.p, it.row, &it.b);
+  it.off = 0;
+  if (it.slot >= 0) {
+    const int32_t tiles = (it.n + kSlKeys - 1) / kSlKeys, per = (tiles + a.parts - 1) / a.parts * kSlKeys;
+    it.off = part * per;
+    it.n = max(0, min(per, it.n - it.off));
+  }
+  return it;
+}
+// Key row of the item's j-th slot; past its n slots `none` (a row that does not exist: TMA fills zeros).
+__device__ __forceinline__ int32_t sli_key_row(const SliGradDev& p, const int32_t* idx_row, const SliGradItem& it, int32_t j,
+                                               int32_t none) {
+  return j < it.n ? it.b * p.s2 + sli_slot_key(p, idx_row, it.off + j) : none;
+}
 
 // Exponent of the power of two that brings magnitudes up to `m` below 2^14.
 __device__ __forceinline__ int sli_exponent(float m) {
@@ -641,19 +669,23 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     uint32_t n_tile = 0, n_item = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hchunks, h0 = (item - row * a.hchunks) * 64;
-      int32_t b;
-      const int32_t n = sli_row_slots(a.p, row, &b), ntiles = tiles_of(n);
+      const SliGradItem it = sli_grad_item(a, item);
+      const int32_t row = it.row, h0 = it.h0, n = it.n, ntiles = tiles_of(n);
       const int32_t hn = min(32, g - h0 - half * 32);     // this warp's heads that exist
+      float* part = it.slot >= 0 ? a.part + (int64_t)it.slot * kSgPart : nullptr;
       T* dq = (T*)a.p.d_query_index + ((int64_t)row * g + h0 + half * 32) * 128 + key;
       if (ntiles == 0) {
-        for (int h = 0; h < hn; ++h) dq[h * 128] = from_f32<T>(0.f);
-        if (quarter == 0 && lane < hn)
+        for (int h = 0; h < hn; ++h) {
+          if (part) part[(half * 32 + h) * 128 + key] = 0.f;
+          else dq[h * 128] = from_f32<T>(0.f);
+        }
+        if (part) { if (quarter == 0) part[64 * 128 + half * 32 + lane] = 0.f; }
+        else if (quarter == 0 && lane < hn)
           store_weight(a.p.d_weights, a.p.dtype_w, (int64_t)row * g + h0 + half * 32 + lane, 0.f);
         continue;
       }
       const int32_t* idx_row = a.p.sparse_indices ? a.p.sparse_indices + (int64_t)row * a.p.topk : nullptr;
-      const float* di_row = a.p.di + (int64_t)row * a.p.topk;
+      const float* di_row = a.p.di + (int64_t)row * a.p.topk + it.off;
       float up = 1.f, down = 1.f, w_down = 1.f;
       if constexpr (kScaled) {
         const int e = sli_exponent(a.di_max[row]);
@@ -667,7 +699,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
 #pragma unroll
       for (int h = 0; h < 32; ++h) dw[h] = 0.f;
       float d_next = key < n ? di_row[key] : 0.f;
-      int32_t r_next = sli_key_row(a.p, idx_row, b, key, n, -1);
+      int32_t r_next = sli_key_row(a.p, idx_row, it, key, -1);
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
         const int buf = n_tile & 1;
         const float d = d_next;
@@ -675,7 +707,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         {
           const int32_t j = (t + 1) * kSlKeys + key;
           d_next = j < n ? di_row[j] : 0.f;
-          r_next = sli_key_row(a.p, idx_row, b, j, n, -1);
+          r_next = sli_key_row(a.p, idx_row, it, j, -1);
         }
         const float du = kScaled ? d * up : d;
         const T hi = from_f32<T>(du), lo = from_f32<T>(du - to_f32<T>(hi));
@@ -739,8 +771,9 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       if (!ok) break;
       if (quarter == 0 && lane < hn) {
         const int h = half * 32 + lane;
-        store_weight(a.p.d_weights, a.p.dtype_w, (int64_t)row * g + h0 + h,
-                     (dwb[h] + dwb[64 + h]) + (dwb[128 + h] + dwb[192 + h]));
+        const float sum = (dwb[h] + dwb[64 + h]) + (dwb[128 + h] + dwb[192 + h]);
+        if (part) part[64 * 128 + h] = sum;
+        else store_weight(a.p.d_weights, a.p.dtype_w, (int64_t)row * g + h0 + h, sum);
       }
       ok = wait(dq_full, n_item & 1);
       if (!ok) break;
@@ -758,8 +791,11 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
 #pragma unroll
         for (int h = 0; h < 16; ++h)
           if (c + h < hn) {
-            const float w = load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + half * 32 + c + h);
-            dq[(c + h) * 128] = from_f32<T>((kScaled ? v[h] * down : v[h]) * w);
+            const float x = kScaled ? v[h] * down : v[h];
+            if (part) part[(half * 32 + c + h) * 128 + key] = x;
+            else
+              dq[(c + h) * 128] =
+                  from_f32<T>(x * load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + half * 32 + c + h));
           }
       }
       ++n_item;
@@ -775,8 +811,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     uint32_t n_tile = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      int32_t b;
-      const int32_t n = sli_row_slots(a.p, item / a.hchunks, &b), ntiles = tiles_of(n);
+      const int32_t n = sli_grad_item(a, item).n, ntiles = tiles_of(n);
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
         const int buf = n_tile & 1;
         const int4* rows4 = reinterpret_cast<const int4*>(rows_s + (n_tile & 3) * kSlKeys + k0);
@@ -836,15 +871,14 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     int stage = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hchunks;
-      int32_t b;
-      const int32_t n = sli_row_slots(a.p, row, &b), ntiles = tiles_of(n);
-      const int32_t* idx_row = a.p.sparse_indices ? a.p.sparse_indices + (int64_t)row * a.p.topk : nullptr;
+      const SliGradItem it = sli_grad_item(a, item);
+      const int32_t ntiles = tiles_of(it.n);
+      const int32_t* idx_row = a.p.sparse_indices ? a.p.sparse_indices + (int64_t)it.row * a.p.topk : nullptr;
       int32_t rn[4];
       auto load = [&](int32_t t) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          rn[i] = active ? sli_key_row(a.p, idx_row, b, t * kSlKeys + grp * 4 + i, n, a.key_rows) : a.key_rows;
+          rn[i] = active ? sli_key_row(a.p, idx_row, it, t * kSlKeys + grp * 4 + i, a.key_rows) : a.key_rows;
       };
       load(0);
       for (int32_t t = 0; t < ntiles && ok; ++t) {
@@ -872,11 +906,10 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     int st_s = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hchunks, h0 = (item - row * a.hchunks) * 64;
-      int32_t b;
-      const int32_t ntiles = tiles_of(sli_row_slots(a.p, row, &b));
+      const SliGradItem it = sli_grad_item(a, item);
+      const int32_t ntiles = tiles_of(it.n);
       if (ntiles == 0) continue;
-      const int steps = (min(64, g - h0) + 15) / 16;
+      const int steps = (min(64, g - it.h0) + 15) / 16;
       ok = wait(q_full, n_item & 1);
       for (int32_t t = 0; t <= ntiles && ok; ++t) {
         if (t < ntiles) {
@@ -929,8 +962,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     int stage = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      int32_t b;
-      const int32_t ntiles = tiles_of(sli_row_slots(a.p, item / a.hchunks, &b));
+      const int32_t ntiles = tiles_of(sli_grad_item(a, item).n);
       if (ntiles == 0) continue;
       ok = wait(dq_empty, (n_item & 1) ^ 1);
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
@@ -963,9 +995,9 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     uint32_t n_item = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t row = item / a.hchunks, h0 = (item - row * a.hchunks) * 64;
-      int32_t b;
-      if (sli_row_slots(a.p, row, &b) == 0) continue;
+      const SliGradItem it = sli_grad_item(a, item);
+      const int32_t row = it.row, h0 = it.h0;
+      if (it.n == 0) continue;
       const int32_t hn = min(64, g - h0);
       if (warp == kSgStager0) {
         ok = wait(q_empty, (n_item & 1) ^ 1);
@@ -1043,7 +1075,42 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, misaligned ? 2 : 1);
 }
 
+// dQI and dW of the items that were cut into parts: the parts' sums in their order.  A block per item, 128 features.
+template <typename T>
+__global__ void __launch_bounds__(128) sli_grad_parts_kernel(SliGradDev p, const float* __restrict__ part, int32_t full,
+                                                             int32_t parts, int32_t hchunks) {
+  const int32_t base = full + blockIdx.x, row = base / hchunks, h0 = (base - row * hchunks) * 64, hn = min(64, p.g - h0);
+  const float* src = part + (int64_t)blockIdx.x * parts * kSgPart;
+  const int64_t i0 = (int64_t)row * p.g + h0;
+  for (int32_t h = blockIdx.y; h < hn; h += gridDim.y) {
+    float v = src[h * 128 + threadIdx.x];
+    for (int32_t q = 1; q < parts; ++q) v += src[(int64_t)q * kSgPart + h * 128 + threadIdx.x];
+    ((T*)p.d_query_index)[(i0 + h) * 128 + threadIdx.x] = from_f32<T>(v * load_weight(p.weights, p.dtype_w, i0 + h));
+    if (threadIdx.x == 0) {
+      float w = src[64 * 128 + h];
+      for (int32_t q = 1; q < parts; ++q) w += src[(int64_t)q * kSgPart + 64 * 128 + h];
+      store_weight(p.d_weights, p.dtype_w, i0 + h, w);
+    }
+  }
+}
+
 // ---- host side -----------------------------------------------------------------------------------
+// Gradient items of a last round that would leave half of the SMs idle or more: cut into 2 to 4 parts of 4 tiles or more (as
+// sfa_bwd_split).  Whole calls of 512 rows, 64 heads: dense over 4096 keys 508 -> 495 us, 2048 selected keys 381 -> 377.
+struct SliGradSplit { int32_t full, parts, items; };
+inline SliGradSplit sli_grad_split(int64_t items, int64_t slots) {
+  const int64_t sms = 148, rest = items % sms;
+  const int64_t parts = rest == 0 ? 1 : std::min<int64_t>(std::min<int64_t>(4, sms / rest), slots / (4 * kSlKeys));
+  if (parts < 2) return SliGradSplit{(int32_t)items, 1, (int32_t)items};
+  return SliGradSplit{(int32_t)(items - rest), (int32_t)parts, (int32_t)(items - rest + rest * parts)};
+}
+// Bytes that the parts leave their sums in, after the dKI accumulators of the workspace.
+inline size_t sli_grad_part_bytes(const DsaSliGradParams* p) {
+  if (p->d_idx != 128) return 0;
+  const SliGradSplit sp = sli_grad_split((int64_t)p->batch * p->s1 * ((p->g + 63) / 64), p->dense ? p->s2 : p->topk);
+  return (size_t)(sp.items - sp.full) * kSgPart * sizeof(float);
+}
+
 // Workspaces of the operator reach these kernels with 16-byte aligned rows; what is asked for here is what
 // TMA wants of the caller's tensors.
 inline bool sli_sm100_aligned(const DsaSliGradParams* p) {
@@ -1167,7 +1234,8 @@ inline int sli_mha_sm100_launch(const DsaSliGradParams* p, SliMhaArgs a, int32_t
 }
 
 template <typename T>
-inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d, int32_t* status, int sms, cudaStream_t st) {
+inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d, float* part, int32_t* status, int sms,
+                                 cudaStream_t st) {
   const bool bf16 = p->dtype == DSA_DTYPE_BF16;
   const int64_t rows = (int64_t)p->batch * p->s1;
   SliGradArgs a;
@@ -1176,7 +1244,9 @@ inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d,
   a.di_max = d.di_max;
   a.hchunks = (p->g + 63) / 64;
   if (rows * a.hchunks >= (1ll << 31)) return DSA_ERR_TOO_LARGE;
-  a.items = (int32_t)(rows * a.hchunks);
+  const SliGradSplit sp = sli_grad_split(rows * a.hchunks, p->dense ? p->s2 : p->topk);
+  a.items = sp.items; a.full = sp.full; a.parts = sp.parts;
+  a.part = part;
   a.key_rows = (int32_t)((int64_t)p->batch * p->s2);
   const uint32_t fmt = bf16 ? 1u : 0u;
   a.idesc_s = ptx::idesc_f16(fmt, 128, 64, 0, 0);
@@ -1189,6 +1259,12 @@ inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d,
   sli_grad_sm100_kernel<T><<<std::min(a.items, sms), kSgThreads, kSgSmemBytes, st>>>(tk, tq, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
+  if (sp.parts > 1) {
+    sli_grad_parts_kernel<T><<<dim3((unsigned)((sp.items - sp.full) / sp.parts), 8), 128, 0, st>>>(d, part, sp.full, sp.parts,
+                                                                                                  a.hchunks);
+    if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
+    count_launch();
+  }
   return DSA_OK;
 }
 
