@@ -69,34 +69,6 @@ __device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void st_cluster_v4(uint32_t raddr, float a, float b, float c, float d) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(raddr), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
-__device__ __forceinline__ void st_cluster_v4_b32(uint32_t raddr, uint4 v) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(raddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
-               : "memory");
-}
-// Asynchronous 16-byte store into another CTA of the cluster; when the bytes have landed they are
-// counted as transaction bytes on an mbarrier of the destination CTA (no wait on the sender side).
-__device__ __forceinline__ void st_async_v4(uint32_t raddr, uint4 v, uint32_t raddr_bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-               ::"r"(raddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(raddr_bar)
-               : "memory");
-}
-// Arrive on an mbarrier of another CTA of the cluster; orders this thread's earlier (remote) writes.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t raddr_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(raddr_bar) : "memory");
-}
-// Bulk copy of `bytes` (multiple of 16) from this CTA's shared memory into another CTA of the
-// cluster; completion is counted as transaction bytes on an mbarrier of the destination CTA.
-__device__ __forceinline__ void bulk_copy_to_peer(uint32_t raddr_dst, const void* src, uint32_t bytes,
-                                                  uint32_t raddr_bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(raddr_dst), "r"(smem_u32(src)), "r"(bytes), "r"(raddr_bar)
-      : "memory");
-}
 // Remote arrive that publishes nothing (it only says "I have finished reading"): relaxed, so it
 // does not wait for this thread's outstanding writes.  `dep` ties the instruction to a value that
 // depends on the loads it must not overtake.
