@@ -601,11 +601,12 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           if (!ok) break;
           SFA_PROF(1);
           if (rank != 0) {
-            // the blocks were written through the generic proxy: order them before the tensor core's reads of this
-            // CTA's shared memory, then tell the issuer; nothing of this thread's own has to be published
+            // The blocks were written by 64 lanes' copies through the generic proxy.  This thread has seen them land
+            // (k_full); it orders them before the tensor core's reads of this CTA's shared memory and releases
+            // them, with that fence, to the issuer in the other CTA.
             if (ptx::elect_one()) {
               ptx::fence_proxy_async_smem();
-              ptx::mbar_arrive_remote_relaxed(k_ready_lead + kb * 8, 0u);
+              ptx::mbar_arrive_remote_release(k_ready_lead + kb * 8);
             }
             __syncwarp();
             continue;
@@ -663,7 +664,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             // (as the K relays)
             if (ptx::elect_one()) {
               ptx::fence_proxy_async_smem();
-              ptx::mbar_arrive_remote_relaxed(v_ready_lead + b * 8, 0u);
+              ptx::mbar_arrive_remote_release(v_ready_lead + b * 8);
             }
             __syncwarp();
             continue;
