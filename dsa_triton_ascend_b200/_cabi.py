@@ -114,6 +114,7 @@ EXPORTS = (
     "dsa_sfa_workspace_bytes", "dsa_sfa_forward", "dsa_sfa_uses_tensor_path",
     "dsa_li_forward_static", "dsa_li_static_scratch_bytes", "dsa_selftest_wait_timeout",
     "dsa_kernel_launch_count", "dsa_sfa_grad_workspace_bytes", "dsa_sfa_grad", "dsa_sfa_grad_uses_tensor_path",
+    "dsa_sfa_grad_workspace_bytes_uncut",
     "dsa_sli_grad_workspace_bytes", "dsa_sli_grad", "dsa_dense_li_lse_workspace_bytes", "dsa_dense_li_lse",
 )
 
@@ -138,8 +139,9 @@ def _load():
         f = getattr(lib, f"dsa_{name}_uses_tensor_path")
         f.argtypes = [_c.POINTER(ptype)]
         f.restype = _c.c_int
-    lib.dsa_sfa_grad_workspace_bytes.argtypes = [_c.POINTER(DsaSfaGradParams), _c.POINTER(_c.c_size_t)]
-    lib.dsa_sfa_grad_workspace_bytes.restype = _c.c_int
+    for f in (lib.dsa_sfa_grad_workspace_bytes, lib.dsa_sfa_grad_workspace_bytes_uncut):
+        f.argtypes = [_c.POINTER(DsaSfaGradParams), _c.POINTER(_c.c_size_t)]
+        f.restype = _c.c_int
     lib.dsa_sfa_grad_uses_tensor_path.argtypes = [_c.POINTER(DsaSfaGradParams)]
     lib.dsa_sfa_grad_uses_tensor_path.restype = _c.c_int
     lib.dsa_sfa_grad.argtypes = [_c.POINTER(DsaSfaGradParams), _c.c_void_p, _c.c_size_t, _c.c_void_p]

@@ -280,7 +280,8 @@ static int sfa_grad_mma_launch(const SfaGradDev& d, int n1, cudaStream_t st) {
 }
 
 template <typename T>
-static int sfa_grad_launch(const DsaSfaGradParams* p, bool tensor, char* ws, const SfaBwdWs& w, cudaStream_t st) {
+static int sfa_grad_launch(const DsaSfaGradParams* p, bool tensor, char* ws, size_t ws_bytes, const SfaBwdWs& w,
+                           cudaStream_t st) {
   SfaGradDev d;
   float* acc = reinterpret_cast<float*>(ws + w.acc);
   d.seq.seq_q = p->seq_q; d.seq.seq_k = p->seq_k; d.seq.block_table = nullptr;
@@ -307,7 +308,7 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, bool tensor, char* ws, con
     // on request, or with a query or d_out off its 16-byte boundary, the CUDA-core kernel
     const bool mma = p->kernel != DSA_KERNEL_PORTABLE && !off16(p->query, p->query_rope) && !off16(p->d_out);
     if (tensor) {
-      const int rc = sfa_bwd_sm100_launch<T>(p, d, ws, w, st);
+      const int rc = sfa_bwd_sm100_launch<T>(p, d, ws, ws_bytes, w, st);
       if (rc != DSA_OK) return rc;
     } else if (mma) {
       int rc;
@@ -678,6 +679,14 @@ int dsa_sfa_grad_workspace_bytes(const DsaSfaGradParams* p, size_t* out_bytes) {
   return DSA_OK;
 }
 
+int dsa_sfa_grad_workspace_bytes_uncut(const DsaSfaGradParams* p, size_t* out_bytes) {
+  int st = sfa_grad_validate(p);
+  if (st != DSA_OK) return st;
+  if (!out_bytes) return DSA_ERR_NULL;
+  *out_bytes = sfa_bwd_sm100_shape(p) ? sfa_bwd_ws_layout(p, kWorkspaceHeader).uncut : sfa_grad_least_bytes(p);
+  return DSA_OK;
+}
+
 int dsa_sfa_grad(const DsaSfaGradParams* p, void* workspace, size_t workspace_bytes, void* stream) {
   int st = sfa_grad_validate(p);
   if (st != DSA_OK) return st;
@@ -685,10 +694,10 @@ int dsa_sfa_grad(const DsaSfaGradParams* p, void* workspace, size_t workspace_by
   if (!workspace || workspace_bytes < least || ((uintptr_t)workspace & 255u) != 0) return DSA_ERR_WORKSPACE;
   cudaStream_t cs = (cudaStream_t)stream;
   const SfaBwdWs w = sfa_bwd_ws_layout(p, kWorkspaceHeader);
-  const bool tensor = dsa_sfa_grad_uses_tensor_path(p) && workspace_bytes >= w.total;
+  const bool tensor = dsa_sfa_grad_uses_tensor_path(p) && workspace_bytes >= w.uncut;
   if (cudaMemsetAsync(workspace, 0, tensor ? w.zeroed : least, cs) != cudaSuccess) return DSA_ERR_CUDA;
-  if (p->dtype == DSA_DTYPE_BF16) return sfa_grad_launch<__nv_bfloat16>(p, tensor, (char*)workspace, w, cs);
-  return sfa_grad_launch<__half>(p, tensor, (char*)workspace, w, cs);
+  if (p->dtype == DSA_DTYPE_BF16) return sfa_grad_launch<__nv_bfloat16>(p, tensor, (char*)workspace, workspace_bytes, w, cs);
+  return sfa_grad_launch<__half>(p, tensor, (char*)workspace, workspace_bytes, w, cs);
 }
 
 static int dense_lse_validate(const DsaDenseLseParams* p) {

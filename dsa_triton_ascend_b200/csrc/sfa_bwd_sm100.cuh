@@ -731,9 +731,11 @@ inline bool sfa_bwd_sm100_aligned(const DsaSfaGradParams* p) {
            (uintptr_t)p->d_out | (uintptr_t)p->out) & 15u) == 0;
 }
 // Workspace: header | dk / dv accumulators | fp16: bounds of the items - zeroed before the call - | fp16: exponents
-// of the items, norms of the keys | nvalid | delta | redo flags and count of the pre-pass (unused) | d_query of parts
-// of rows | key_list
-struct SfaBwdWs { size_t acc, bound, zeroed, exps, norms, nvalid, delta, redo, dq_part, key_list, total; };
+// of the items, norms of the keys | nvalid | delta | redo flags and count of the pre-pass (unused) | key_list | d_query
+// of parts of rows.  What lies before the parts (`uncut` bytes) grows with every size of the call, the parts come and
+// go with its last round: without room for them the rows stay whole, so that a workspace made for a larger call is
+// enough for a smaller one.
+struct SfaBwdWs { size_t acc, bound, zeroed, exps, norms, nvalid, delta, redo, key_list, uncut, dq_part, total; };
 inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   const size_t rows = (size_t)sfa_bwd_rows(p);
@@ -748,16 +750,17 @@ inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
   w.nvalid = w.norms + (fp16 ? up((size_t)p->key_rows * 4) : 0);
   w.delta = w.nvalid + up(rows * 8);
   w.redo = w.delta + up(rows * p->n1 * 4);
-  w.dq_part = w.redo + up(rows * 4) + 256;
+  w.key_list = w.redo + up(rows * 4) + 256;
+  w.uncut = w.key_list + rows * p->sparse_count * p->sparse_block_size * 4;
+  w.dq_part = up(w.uncut);
   const SfaBwdSplit sp = sfa_bwd_split((int64_t)items, (int64_t)p->sparse_count * p->sparse_block_size);
-  w.key_list = w.dq_part + (size_t)(sp.items - sp.full) * kBwdHeads * 576 * 4;
-  w.total = w.key_list + rows * p->sparse_count * p->sparse_block_size * 4;
+  w.total = sp.parts > 1 ? w.dq_part + (size_t)(sp.items - sp.full) * kBwdHeads * 576 * 4 : w.uncut;
   return w;
 }
 
 template <typename T>
-inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, char* ws, const SfaBwdWs& w,
-                                cudaStream_t st) {
+inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, char* ws, size_t ws_bytes,
+                                const SfaBwdWs& w, cudaStream_t st) {
   static std::atomic<int> sm_count[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DSA_ERR_CUDA;
@@ -813,7 +816,9 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   a.idesc_q = ptx::idesc_f16(fmt, 128, kBwdHeads, 1, 1);
   a.idesc_d = ptx::idesc_f16(fmt, 128, kBwdBK, 1, 0);
   a.hblocks = hblocks;
-  const SfaBwdSplit sp = sfa_bwd_split((int64_t)d.rows * hblocks, slots);
+  const int64_t whole = (int64_t)d.rows * hblocks;
+  const SfaBwdSplit sp = ws_bytes >= w.total ? sfa_bwd_split(whole, slots)
+                                             : SfaBwdSplit{(int32_t)whole, 1, (int32_t)whole};
   a.items = sp.items; a.full = sp.full; a.parts = sp.parts;
   a.dq_part = (float*)(ws + w.dq_part);
   a.key_rows = (int32_t)p->key_rows;

@@ -161,12 +161,25 @@ def sparse_flash_attention_grad_triton(
         try:
             ws = workspace(nbytes.value, dev)
         except torch.cuda.OutOfMemoryError:
-            # header and accumulators alone: the mma.sync kernel
-            ws = workspace(_HEADER + p.key_rows * (2 * D + d_rope) * 4, dev)
+            ws = _smaller_workspace(p, nbytes.value, dev)
         _cabi.check(_cabi.lib.dsa_sfa_grad(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
                     "sparse_flash_attention_grad")
         note_launch("sparse_flash_attention_grad", ws, dev)
     return d_query, d_key, d_value, d_query_rope, d_key_rope
+
+
+def _smaller_workspace(p, refused, dev):
+    """Without the parts of a last round if that is less; failing that header and accumulators alone, with which the
+    mma.sync kernel runs."""
+    nbytes = ctypes.c_size_t(0)
+    _cabi.check(_cabi.lib.dsa_sfa_grad_workspace_bytes_uncut(ctypes.byref(p), ctypes.byref(nbytes)),
+                "sparse_flash_attention_grad")
+    if nbytes.value < refused:
+        try:
+            return workspace(nbytes.value, dev)
+        except torch.cuda.OutOfMemoryError:
+            pass
+    return workspace(_HEADER + p.key_rows * (2 * p.d + p.d_rope) * 4, dev)
 
 
 class SparseFlashAttentionGradTriton(torch.nn.Module):

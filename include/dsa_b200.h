@@ -184,14 +184,20 @@ typedef struct DsaSfaGradParams {
   int64_t key_rows; /* batch*s2 (BSND) or T2 (TND) */
 } DsaSfaGradParams;
 
-/* 1 when the call, given the workspace that dsa_sfa_grad_workspace_bytes() names, runs on the tcgen05 kernel:
+/* 1 when the call, given the workspace that dsa_sfa_grad_workspace_bytes_uncut() names, runs on the tcgen05 kernel:
  * d = 512, 16 heads or more, operands on 16-byte boundaries, kernel not DSA_KERNEL_PORTABLE. */
 int dsa_sfa_grad_uses_tensor_path(const DsaSfaGradParams* p);
 /* Workspace: a status header (256 bytes) plus fp32 accumulators key_rows * (2*d + d_rope) * 4 bytes are enough
- * for every call.  For the shapes of the tcgen05 kernel the size named here also covers its scratch, mostly the
- * rows' key lists (rows * sparse_count * sparse_block_size * 4 bytes); dsa_sfa_grad() with less than that
- * runs such a call on the mma.sync kernel: the same results, 3.7 times the time at 512 rows x 64 heads. */
+ * for every call.  The tcgen05 kernel has scratch of its own: ..._uncut names the size with its key lists (rows *
+ * sparse_count * sparse_block_size * 4 bytes, mostly); it grows with every size of the call, so that a workspace
+ * made for the largest call is enough for the others.  dsa_sfa_grad() with less than that runs on the mma.sync kernel:
+ * the same results, 3.7 times the time at 512 rows x 64 heads.  The size named by dsa_sfa_grad_workspace_bytes() may
+ * hold up to 148 fp32 blocks of 64 x (d + d_rope) more (21.8 MB): with all of them, rows of a last round that would
+ * leave most SMs idle are cut into parts (1135 us against 1222 at 512 rows x 64 heads), whose d_query sums are
+ * added up.  That can change the last place of d_query and d_query_rope, by the number of rows and heads of the call;
+ * with less, a row's d_query does not depend on the other rows. */
 int dsa_sfa_grad_workspace_bytes(const DsaSfaGradParams* p, size_t* out_bytes);
+int dsa_sfa_grad_workspace_bytes_uncut(const DsaSfaGradParams* p, size_t* out_bytes);
 /* Enqueue the backward on `stream`: clears the accumulators, runs the gradient kernels and the
  * conversion of the accumulators to the io dtype. */
 int dsa_sfa_grad(const DsaSfaGradParams* p, void* workspace, size_t workspace_bytes, void* stream);
