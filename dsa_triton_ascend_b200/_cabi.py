@@ -114,7 +114,7 @@ EXPORTS = (
     "dsa_sfa_workspace_bytes", "dsa_sfa_forward", "dsa_sfa_uses_tensor_path",
     "dsa_li_forward_static", "dsa_li_static_scratch_bytes", "dsa_selftest_wait_timeout",
     "dsa_kernel_launch_count", "dsa_sfa_grad_workspace_bytes", "dsa_sfa_grad", "dsa_sfa_grad_uses_tensor_path",
-    "dsa_sfa_grad_workspace_bytes_uncut",
+    "dsa_sfa_grad_workspace_bytes_uncut", "dsa_sli_grad_workspace_bytes_uncut",
     "dsa_sli_grad_workspace_bytes", "dsa_sli_grad", "dsa_dense_li_lse_workspace_bytes", "dsa_dense_li_lse",
 )
 
@@ -146,8 +146,9 @@ def _load():
     lib.dsa_sfa_grad_uses_tensor_path.restype = _c.c_int
     lib.dsa_sfa_grad.argtypes = [_c.POINTER(DsaSfaGradParams), _c.c_void_p, _c.c_size_t, _c.c_void_p]
     lib.dsa_sfa_grad.restype = _c.c_int
-    lib.dsa_sli_grad_workspace_bytes.argtypes = [_c.POINTER(DsaSliGradParams), _c.POINTER(_c.c_size_t)]
-    lib.dsa_sli_grad_workspace_bytes.restype = _c.c_int
+    for f in (lib.dsa_sli_grad_workspace_bytes, lib.dsa_sli_grad_workspace_bytes_uncut):
+        f.argtypes = [_c.POINTER(DsaSliGradParams), _c.POINTER(_c.c_size_t)]
+        f.restype = _c.c_int
     lib.dsa_sli_grad.argtypes = [_c.POINTER(DsaSliGradParams), _c.c_void_p, _c.c_size_t, _c.c_void_p]
     lib.dsa_sli_grad.restype = _c.c_int
     lib.dsa_dense_li_lse_workspace_bytes.argtypes = [_c.POINTER(DsaDenseLseParams), _c.POINTER(_c.c_size_t)]

@@ -1,6 +1,7 @@
 """Host-side helpers shared by the two operator wrappers: dtype/length handling, workspace
 and stream plumbing.  torch is used for device memory and streams only."""
 import contextlib
+import ctypes
 import functools
 import os
 
@@ -76,6 +77,19 @@ def packed(t):
 def workspace(nbytes, device):
     # torch's caching allocator returns 512-byte aligned blocks; the library wants 256.
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
+
+
+def loss_workspace(p, device, what, allocate):
+    """Workspace of a loss call: the size that dsa_sli_grad() runs best with, or the least if that cannot be had."""
+    nbytes, least = ctypes.c_size_t(0), ctypes.c_size_t(0)
+    _cabi.check(_cabi.lib.dsa_sli_grad_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)), what)
+    try:
+        return allocate(nbytes.value, device)
+    except torch.cuda.OutOfMemoryError:
+        _cabi.check(_cabi.lib.dsa_sli_grad_workspace_bytes_uncut(ctypes.byref(p), ctypes.byref(least)), what)
+        if least.value == nbytes.value:
+            raise
+        return allocate(least.value, device)
 
 
 # (torch.cuda.current_stream builds a Stream object around the handle: 2-4 us of a call that takes 30)

@@ -373,7 +373,7 @@ static int sli_grad_validate(const DsaSliGradParams* p) {
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 template <typename T>
-static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status, cudaStream_t st) {
+static int sli_grad_launch(const DsaSliGradParams* p, char* ws, bool cut, int32_t* status, cudaStream_t st) {
   SliGradDev d;
   const int64_t rows = (int64_t)p->batch * p->s1;
   const int64_t key_elems = (int64_t)p->batch * p->s2 * p->d_idx;
@@ -493,7 +493,7 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, int32_t* status,
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
     count_launch();
     if (tensor && p->d_idx == 128) {
-      float* part = reinterpret_cast<float*>((char*)d.dki_acc + align256((size_t)key_elems * 4));
+      float* part = cut ? reinterpret_cast<float*>((char*)d.dki_acc + align256((size_t)key_elems * 4)) : nullptr;
       const int rc = sli_grad_sm100_launch<T>(p, d, part, status, sms, st);
       if (rc != DSA_OK) return rc;
     } else {
@@ -739,28 +739,35 @@ int dsa_dense_li_lse(const DsaDenseLseParams* p, void* workspace, size_t workspa
   return dense_lse_launch<__half>(p, scratch, (int32_t*)workspace, cs);
 }
 
-int dsa_sli_grad_workspace_bytes(const DsaSliGradParams* p, size_t* out_bytes) {
+int dsa_sli_grad_workspace_bytes_uncut(const DsaSliGradParams* p, size_t* out_bytes) {
   int st = sli_grad_validate(p);
   if (st != DSA_OK) return st;
   if (!out_bytes) return DSA_ERR_NULL;
   const size_t rows = (size_t)p->batch * p->s1;
   *out_bytes = kWorkspaceHeader + 2 * align256(rows * (size_t)sli_slots(p) * 4) + align256(rows * 4) +
-               align256(rows * 8) + align256((size_t)p->batch * p->s2 * p->d_idx * 4) + sli_grad_part_bytes(p);
+               align256(rows * 8) + align256((size_t)p->batch * p->s2 * p->d_idx * 4);
   return DSA_OK;
+}
+
+int dsa_sli_grad_workspace_bytes(const DsaSliGradParams* p, size_t* out_bytes) {
+  int st = dsa_sli_grad_workspace_bytes_uncut(p, out_bytes);
+  if (st == DSA_OK) *out_bytes += sli_grad_part_bytes(p);
+  return st;
 }
 
 int dsa_sli_grad(const DsaSliGradParams* p, void* workspace, size_t workspace_bytes, void* stream) {
   int st = sli_grad_validate(p);
   if (st != DSA_OK) return st;
   size_t need = 0;
-  dsa_sli_grad_workspace_bytes(p, &need);
+  dsa_sli_grad_workspace_bytes_uncut(p, &need);
   if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255u) != 0) return DSA_ERR_WORKSPACE;
   if ((int64_t)p->batch * p->s1 > 0x7FFFFFFF) return DSA_ERR_TOO_LARGE;
   cudaStream_t cs = (cudaStream_t)stream;
   if (cudaMemsetAsync(workspace, 0, kWorkspaceHeader, cs) != cudaSuccess) return DSA_ERR_CUDA;
   char* ws = (char*)workspace + kWorkspaceHeader;
-  if (p->dtype == DSA_DTYPE_BF16) return sli_grad_launch<__nv_bfloat16>(p, ws, (int32_t*)workspace, cs);
-  return sli_grad_launch<__half>(p, ws, (int32_t*)workspace, cs);
+  const bool cut = workspace_bytes - need >= sli_grad_part_bytes(p);    // there is room for the parts
+  if (p->dtype == DSA_DTYPE_BF16) return sli_grad_launch<__nv_bfloat16>(p, ws, cut, (int32_t*)workspace, cs);
+  return sli_grad_launch<__half>(p, ws, cut, (int32_t*)workspace, cs);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1104,7 +1104,8 @@ inline SliGradSplit sli_grad_split(int64_t items, int64_t slots) {
   if (parts < 2) return SliGradSplit{(int32_t)items, 1, (int32_t)items};
   return SliGradSplit{(int32_t)(items - rest), (int32_t)parts, (int32_t)(items - rest + rest * parts)};
 }
-// Bytes that the parts leave their sums in, after the dKI accumulators of the workspace.
+// Bytes that the parts leave their sums in, at the end of the workspace: without room for them the rows stay whole, so
+// that a workspace made for a larger call is enough for a smaller one with a thinner last round.
 inline size_t sli_grad_part_bytes(const DsaSliGradParams* p) {
   if (p->d_idx != 128) return 0;
   const SliGradSplit sp = sli_grad_split((int64_t)p->batch * p->s1 * ((p->g + 63) / 64), p->dense ? p->s2 : p->topk);
@@ -1244,7 +1245,9 @@ inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d,
   a.di_max = d.di_max;
   a.hchunks = (p->g + 63) / 64;
   if (rows * a.hchunks >= (1ll << 31)) return DSA_ERR_TOO_LARGE;
-  const SliGradSplit sp = sli_grad_split(rows * a.hchunks, p->dense ? p->s2 : p->topk);
+  const int64_t whole = rows * a.hchunks;
+  const SliGradSplit sp = part ? sli_grad_split(whole, p->dense ? p->s2 : p->topk)
+                               : SliGradSplit{(int32_t)whole, 1, (int32_t)whole};
   a.items = sp.items; a.full = sp.full; a.parts = sp.parts;
   a.part = part;
   a.key_rows = (int32_t)((int64_t)p->batch * p->s2);

@@ -12,8 +12,8 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, note_launch, packed, ptr, require_cuda,
-                    seq_tensor, workspace)
+from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, loss_workspace, note_launch, packed, ptr,
+                    require_cuda, seq_tensor, workspace)
 
 SUPPORTED_D = (128, 256, 512)
 
@@ -183,9 +183,7 @@ def dense_loss_backward_triton(query, key, query_index, key_index, weights, soft
     p.softmax_max_index, p.softmax_sum_index = ptr(softmax_max_index), ptr(softmax_sum_index)
 
     with device_guard(dev):
-        nbytes = ctypes.c_size_t(0)
-        _cabi.check(_cabi.lib.dsa_sli_grad_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)), "dense_loss_backward")
-        ws = workspace(nbytes.value, dev)
+        ws = loss_workspace(p, dev, "dense_loss_backward", workspace)
         _cabi.check(_cabi.lib.dsa_sli_grad(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
                     "dense_loss_backward")
         note_launch("dense_loss_backward", ws, dev)

@@ -13,8 +13,8 @@ import ctypes
 import torch
 
 from . import _cabi
-from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, note_launch, packed, ptr, require_cuda,
-                    seq_tensor, workspace)
+from ._host import (INT64_MAX, current_stream, device_guard, dtype_code, loss_workspace, note_launch, packed, ptr,
+                    require_cuda, seq_tensor, workspace)
 
 
 def sparse_lightning_indexer_grad_kl_loss_triton(
@@ -111,10 +111,7 @@ def sparse_lightning_indexer_grad_kl_loss_triton(
     p.scale = float(scale_value)
 
     with device_guard(dev):
-        nbytes = ctypes.c_size_t(0)
-        _cabi.check(_cabi.lib.dsa_sli_grad_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)),
-                    "sparse_lightning_indexer_grad_kl_loss")
-        ws = workspace(nbytes.value, dev)
+        ws = loss_workspace(p, dev, "sparse_lightning_indexer_grad_kl_loss", workspace)
         _cabi.check(_cabi.lib.dsa_sli_grad(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
                     "sparse_lightning_indexer_grad_kl_loss")
         note_launch("sparse_lightning_indexer_grad_kl_loss", ws, dev)

@@ -249,9 +249,15 @@ typedef struct DsaSliGradParams {
   const float* softmax_sum_index;
 } DsaSliGradParams;
 
-/* Workspace: status header + fp32 scratch (index scores / dI and attention probabilities, each
- * [rows, slots]; one loss term per row; the d_key_index accumulator [batch * s2, d_idx]). */
+/* Workspace: ..._uncut names the least, a status header + fp32 scratch (index scores / dI and attention
+ * probabilities, each [rows, slots]; three terms per row; the d_key_index accumulator [batch * s2, d_idx]); it grows
+ * with every size of the call.  The size named by dsa_sli_grad_workspace_bytes() may hold up to 148 fp32 blocks of 64 x
+ * 129 more (4.9 MB): with all of them, rows of a last round that would leave most SMs idle are cut into parts
+ * (dense, 512 rows x 4096 keys: 495 us against 508), whose d_query_index and d_weights sums are added up.  That can
+ * change their last place, by the number of rows and heads of the call; with less, a row's d_query_index and
+ * d_weights do not depend on the other rows. */
 int dsa_sli_grad_workspace_bytes(const DsaSliGradParams* p, size_t* out_bytes);
+int dsa_sli_grad_workspace_bytes_uncut(const DsaSliGradParams* p, size_t* out_bytes);
 int dsa_sli_grad(const DsaSliGradParams* p, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
