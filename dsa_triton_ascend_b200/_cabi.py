@@ -16,7 +16,6 @@ DTYPE_BF16, DTYPE_FP16, DTYPE_FP32 = 0, 1, 2
 RANK_IO_DTYPE, RANK_FP32 = 0, 1
 KERNEL_AUTO, KERNEL_PORTABLE, KERNEL_TENSOR = 0, 1, 2
 PHASE_SCORE, PHASE_TOPK, PHASE_ALL = 1, 2, 3
-OUT_ZEROS = 2   # return_value / return_lse: zeros in the place of the results
 
 ERR_VALUE = -3
 
@@ -110,8 +109,8 @@ class DsaDenseLseParams(_c.Structure):
 
 EXPORTS = (
     "dsa_abi_version", "dsa_status_string", "dsa_read_device_status",
-    "dsa_li_workspace_bytes", "dsa_li_forward", "dsa_li_uses_tensor_path",
-    "dsa_sfa_workspace_bytes", "dsa_sfa_forward", "dsa_sfa_uses_tensor_path",
+    "dsa_li_workspace_bytes", "dsa_li_forward", "dsa_li_forward_zeros", "dsa_li_uses_tensor_path",
+    "dsa_sfa_workspace_bytes", "dsa_sfa_forward", "dsa_sfa_forward_zeros", "dsa_sfa_uses_tensor_path",
     "dsa_li_forward_static", "dsa_li_static_scratch_bytes", "dsa_selftest_wait_timeout",
     "dsa_kernel_launch_count", "dsa_sfa_grad_workspace_bytes", "dsa_sfa_grad", "dsa_sfa_grad_uses_tensor_path",
     "dsa_sfa_grad_workspace_bytes_uncut", "dsa_sli_grad_workspace_bytes_uncut",
@@ -133,9 +132,9 @@ def _load():
         f = getattr(lib, f"dsa_{name}_workspace_bytes")
         f.argtypes = [_c.POINTER(ptype), _c.POINTER(_c.c_size_t)]
         f.restype = _c.c_int
-        f = getattr(lib, f"dsa_{name}_forward")
-        f.argtypes = [_c.POINTER(ptype), _c.c_void_p, _c.c_size_t, _c.c_void_p]
-        f.restype = _c.c_int
+        for f in (getattr(lib, f"dsa_{name}_forward"), getattr(lib, f"dsa_{name}_forward_zeros")):
+            f.argtypes = [_c.POINTER(ptype), _c.c_void_p, _c.c_size_t, _c.c_void_p]
+            f.restype = _c.c_int
         f = getattr(lib, f"dsa_{name}_uses_tensor_path")
         f.argtypes = [_c.POINTER(ptype)]
         f.restype = _c.c_int

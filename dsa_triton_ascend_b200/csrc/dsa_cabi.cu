@@ -61,7 +61,7 @@ static inline int64_t li_rows(const DsaLiParams* p) {
 }
 static inline int64_t li_score_ld(const DsaLiParams* p) { return round_up(p->s2 > 0 ? p->s2 : 1, 4); }
 
-static LiDev li_dev(const DsaLiParams* p) {
+static LiDev li_dev(const DsaLiParams* p, bool zeros) {
   LiDev d;
   d.seq.seq_q = p->seq_q; d.seq.seq_k = p->seq_k; d.seq.block_table = p->block_table;
   d.seq.layout_q = p->layout_q; d.seq.layout_k = p->layout_k;
@@ -75,8 +75,8 @@ static LiDev li_dev(const DsaLiParams* p) {
   d.dtype_w = p->dtype_w; d.n1 = p->n1; d.n2 = p->n2; d.d = p->d;
   d.rows = (int32_t)li_rows(p);
   d.sparse_count = p->sparse_count; d.rank_mode = p->rank_mode;
-  d.return_value = p->return_value == DSA_OUT_ZEROS ? 0 : p->return_value;
-  d.zero_values = p->return_value == DSA_OUT_ZEROS && p->out_values != nullptr;
+  d.return_value = p->return_value;
+  d.zero_values = zeros && !p->return_value;
   d.cta_status = nullptr; d.status = nullptr; d.n_cta_status = 0;
   return d;
 }
@@ -88,8 +88,8 @@ static bool li_takes_tensor_path(const DsaLiParams* p) {
 
 template <typename T>
 static int li_launch(const DsaLiParams* p, float* scores, cudaStream_t st, int32_t* status = nullptr,
-                     bool clear_status = false) {
-  LiDev d = li_dev(p);
+                     bool clear_status = false, bool zeros = false) {
+  LiDev d = li_dev(p, zeros);
   if (clear_status) { d.cta_status = (uint8_t*)status + 64; d.status = status; }
   const int64_t ld = li_score_ld(p);
   const int64_t rown = (int64_t)d.rows * p->n2;
@@ -172,7 +172,7 @@ static int sfa_validate(const DsaSfaParams* p) {
   return DSA_OK;
 }
 
-static SfaDev sfa_dev(const DsaSfaParams* p) {
+static SfaDev sfa_dev(const DsaSfaParams* p, bool zeros) {
   SfaDev d;
   d.seq.seq_q = p->seq_q; d.seq.seq_k = p->seq_k; d.seq.block_table = p->block_table;
   d.seq.layout_q = p->layout_q; d.seq.layout_k = p->layout_kv;
@@ -187,15 +187,15 @@ static SfaDev sfa_dev(const DsaSfaParams* p) {
   d.rows = p->layout_q == DSA_LAYOUT_TND ? p->s1 : p->batch * p->s1;
   d.n1 = p->n1; d.d = p->d; d.d_rope = p->d_rope;
   d.sparse_count = p->sparse_count; d.sparse_block_size = p->sparse_block_size;
-  d.return_lse = p->return_lse == DSA_OUT_ZEROS ? 0 : p->return_lse;
-  d.zero_lse = p->return_lse == DSA_OUT_ZEROS;
+  d.return_lse = p->return_lse;
+  d.zero_lse = zeros && !p->return_lse;
   d.scale = p->scale;
   return d;
 }
 
 template <typename T>
-static int sfa_launch_simt(const DsaSfaParams* p, cudaStream_t st) {
-  SfaDev d = sfa_dev(p);
+static int sfa_launch_simt(const DsaSfaParams* p, bool zeros, cudaStream_t st) {
+  SfaDev d = sfa_dev(p, zeros);
   if (d.rows == 0) return DSA_OK;
   const size_t stat_bytes = (size_t)d.rows * p->n1 * sizeof(float);
   if (d.zero_lse && (cudaMemsetAsync(p->softmax_max, 0, stat_bytes, st) != cudaSuccess ||
@@ -616,9 +616,10 @@ int dsa_li_workspace_bytes(const DsaLiParams* p, size_t* out_bytes) {
   return DSA_OK;
 }
 
-int dsa_li_forward(const DsaLiParams* p, void* workspace, size_t workspace_bytes, void* stream) {
+static int li_forward(const DsaLiParams* p, bool zeros, void* workspace, size_t workspace_bytes, void* stream) {
   int st = li_validate(p);
   if (st != DSA_OK) return st;
+  if (zeros && !p->out_values) return DSA_ERR_NULL;
   size_t need = 0;
   dsa_li_workspace_bytes(p, &need);
   if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255u) != 0) return DSA_ERR_WORKSPACE;
@@ -628,8 +629,16 @@ int dsa_li_forward(const DsaLiParams* p, void* workspace, size_t workspace_bytes
   const bool own = p->phases == DSA_PHASE_ALL && p->s2 > 0 && li_rows(p) > 0 && li_takes_tensor_path(p);
   if (!own && cudaMemsetAsync(workspace, 0, kWorkspaceHeader, cs) != cudaSuccess) return DSA_ERR_CUDA;
   float* scores = reinterpret_cast<float*>((char*)workspace + kWorkspaceHeader);
-  if (p->dtype_qk == DSA_DTYPE_BF16) return li_launch<__nv_bfloat16>(p, scores, cs, (int32_t*)workspace, own);
-  return li_launch<__half>(p, scores, cs, (int32_t*)workspace, own);
+  if (p->dtype_qk == DSA_DTYPE_BF16) return li_launch<__nv_bfloat16>(p, scores, cs, (int32_t*)workspace, own, zeros);
+  return li_launch<__half>(p, scores, cs, (int32_t*)workspace, own, zeros);
+}
+
+int dsa_li_forward(const DsaLiParams* p, void* workspace, size_t workspace_bytes, void* stream) {
+  return li_forward(p, false, workspace, workspace_bytes, stream);
+}
+
+int dsa_li_forward_zeros(const DsaLiParams* p, void* workspace, size_t workspace_bytes, void* stream) {
+  return li_forward(p, true, workspace, workspace_bytes, stream);
 }
 
 int dsa_sfa_workspace_bytes(const DsaSfaParams* p, size_t* out_bytes) {
@@ -640,23 +649,32 @@ int dsa_sfa_workspace_bytes(const DsaSfaParams* p, size_t* out_bytes) {
   return DSA_OK;
 }
 
-int dsa_sfa_forward(const DsaSfaParams* p, void* workspace, size_t workspace_bytes, void* stream) {
+static int sfa_forward(const DsaSfaParams* p, bool zeros, void* workspace, size_t workspace_bytes, void* stream) {
   int st = sfa_validate(p);
   if (st != DSA_OK) return st;
+  if (zeros && (!p->softmax_max || !p->softmax_sum)) return DSA_ERR_NULL;
   size_t need = 0;
   dsa_sfa_workspace_bytes(p, &need);
   if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255u) != 0) return DSA_ERR_WORKSPACE;
   if (p->kernel == DSA_KERNEL_TENSOR && !dsa_sfa_uses_tensor_path(p)) return DSA_ERR_UNSUPPORTED;
   cudaStream_t cs = (cudaStream_t)stream;
   if (dsa_sfa_uses_tensor_path(p)) {
-    SfaDev d = sfa_dev(p);
+    SfaDev d = sfa_dev(p, zeros);
     if (d.rows > 0)   // (the pre-pass kernel clears the header)
       return sfa_sm100_launch(p, d, (int32_t*)workspace, (char*)workspace + kWorkspaceHeader, cs);
   }
   if (cudaMemsetAsync(workspace, 0, kWorkspaceHeader, cs) != cudaSuccess) return DSA_ERR_CUDA;
   if (dsa_sfa_uses_tensor_path(p)) return DSA_OK;   // no rows
-  if (p->dtype == DSA_DTYPE_BF16) return sfa_launch_simt<__nv_bfloat16>(p, cs);
-  return sfa_launch_simt<__half>(p, cs);
+  if (p->dtype == DSA_DTYPE_BF16) return sfa_launch_simt<__nv_bfloat16>(p, zeros, cs);
+  return sfa_launch_simt<__half>(p, zeros, cs);
+}
+
+int dsa_sfa_forward(const DsaSfaParams* p, void* workspace, size_t workspace_bytes, void* stream) {
+  return sfa_forward(p, false, workspace, workspace_bytes, stream);
+}
+
+int dsa_sfa_forward_zeros(const DsaSfaParams* p, void* workspace, size_t workspace_bytes, void* stream) {
+  return sfa_forward(p, true, workspace, workspace_bytes, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

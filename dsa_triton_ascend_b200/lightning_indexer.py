@@ -132,7 +132,7 @@ def _build_params(query, key, weights, actual_seq_lengths_query, actual_seq_leng
     p.block_size, p.max_blocks = block_size, max_blocks
     p.sparse_count, p.sparse_mode = int(sparse_count), int(sparse_mode)
     p.rank_mode = _RANK_MODES[_rank_mode]
-    p.return_value = 1 if return_value else _cabi.OUT_ZEROS
+    p.return_value = 1 if return_value else 0
     p.phases = _cabi.PHASE_ALL
     p.key_rows = key.numel() // (N2 * D)
     keep = (query, key, weights, seq_q, seq_k, block_table, idx, val)
@@ -186,7 +186,7 @@ def lightning_indexer_triton(
         nbytes = ctypes.c_size_t(0)
         _cabi.check(_cabi.lib.dsa_li_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)), "lightning_indexer")
         ws = workspace(nbytes.value, dev)
-        _cabi.check(_cabi.lib.dsa_li_forward(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
+        _cabi.check(_cabi.lib.dsa_li_forward_zeros(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
                     "lightning_indexer")
         note_launch("lightning_indexer", ws, dev)
     del keep

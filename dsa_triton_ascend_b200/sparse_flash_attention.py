@@ -162,7 +162,7 @@ def sparse_flash_attention_triton(
     p.block_size, p.max_blocks = pa_block, max_blocks
     p.sparse_count, p.sparse_block_size = topk, sparse_block_size
     p.sparse_mode = sparse_mode
-    p.return_lse = 1 if return_softmax_lse else _cabi.OUT_ZEROS
+    p.return_lse = 1 if return_softmax_lse else 0
     p.scale = float(scale_value)
     p.key_rows = key.numel() // D
 
@@ -172,7 +172,7 @@ def sparse_flash_attention_triton(
             _cabi.check(_cabi.lib.dsa_sfa_workspace_bytes(ctypes.byref(p), ctypes.byref(nbytes)),
                         "sparse_flash_attention")
             ws = workspace(nbytes.value, dev)
-            _cabi.check(_cabi.lib.dsa_sfa_forward(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
+            _cabi.check(_cabi.lib.dsa_sfa_forward_zeros(ctypes.byref(p), ws.data_ptr(), ws.numel(), current_stream(dev)),
                         "sparse_flash_attention")
             note_launch("sparse_flash_attention", ws, dev)
     return out, sm_max, sm_sum

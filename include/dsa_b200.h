@@ -54,10 +54,6 @@ extern "C" {
 #define DSA_KERNEL_TENSOR 2   /* tensor-core path; forward calls: DSA_ERR_UNSUPPORTED when the shape is
                                  not eligible (the attention backward takes every legal shape) */
 
-/* return_value / return_lse: 0 the buffer is not written (it may be NULL), 1 the results, or zeros in their place
-   (what the reference's wrappers return for outputs that were not asked for) without a fill of the caller's */
-#define DSA_OUT_ZEROS 2
-
 #define DSA_PHASE_SCORE 1
 #define DSA_PHASE_TOPK 2
 #define DSA_PHASE_ALL 3
@@ -83,7 +79,7 @@ typedef struct DsaLiParams {
   const int32_t* seq_k; /* [batch] lengths, or cumulative ends when seq_k_cumulative; NULL = s2 */
   const int32_t* block_table; /* PA only: [batch, max_blocks], -1 = no block                  */
   int32_t* out_indices; /* [rows, n2, sparse_count]                                           */
-  void* out_values;     /* [rows, n2, sparse_count] in dtype_qk; may be NULL if !return_value (see DSA_OUT_ZEROS) */
+  void* out_values;     /* [rows, n2, sparse_count] in dtype_qk; may be NULL if !return_value */
   int32_t layout_q;     /* DSA_LAYOUT_BSND | DSA_LAYOUT_TND                                    */
   int32_t layout_k;     /* DSA_LAYOUT_*                                                        */
   int32_t dtype_qk;     /* DSA_DTYPE_BF16 | DSA_DTYPE_FP16                                     */
@@ -141,9 +137,14 @@ typedef struct DsaSfaParams {
 int dsa_li_workspace_bytes(const DsaLiParams* p, size_t* out_bytes);
 /* Enqueue the indexer on `stream` (a cudaStream_t passed as void*). */
 int dsa_li_forward(const DsaLiParams* p, void* workspace, size_t workspace_bytes, void* stream);
+/* The same, but values that are not asked for (return_value = 0) are zeros, which the top-k kernel stores: what the
+ * reference's wrappers return in their place, without a fill of the caller's.  out_values is required. */
+int dsa_li_forward_zeros(const DsaLiParams* p, void* workspace, size_t workspace_bytes, void* stream);
 
 int dsa_sfa_workspace_bytes(const DsaSfaParams* p, size_t* out_bytes);
 int dsa_sfa_forward(const DsaSfaParams* p, void* workspace, size_t workspace_bytes, void* stream);
+/* The same, but statistics that are not asked for (return_lse = 0) are zeros.  softmax_max and softmax_sum are required. */
+int dsa_sfa_forward_zeros(const DsaSfaParams* p, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * sparse_flash_attention backward - replaces `_sfa_grad_core`
