@@ -77,7 +77,7 @@ __device__ __forceinline__ void li_row_extras(const LiDev& p, int32_t rown) {
 
 // grid = rows * n2; block = 512 threads; dynamic smem = sort_cap * 8 + kTopkKeyCache * 4 bytes.
 template <typename T, bool kRank16>
-__global__ void __launch_bounds__(kTopkThreads) li_topk_kernel(LiDev p, const float* __restrict__ scores,
+__global__ void __launch_bounds__(kTopkThreads) li_topk_kernel(LiDev p, const float* scores,
                                                                int64_t ld, int32_t sort_cap) {
   extern __shared__ __align__(16) unsigned char topk_smem[];
   uint64_t* sbuf = reinterpret_cast<uint64_t*>(topk_smem);
@@ -285,7 +285,7 @@ __device__ __forceinline__ uint32_t block_count(uint32_t c, uint32_t* slot) {
 }
 
 template <typename T, bool kRank16, int E>
-__global__ void __launch_bounds__(kTopkThreads) li_topk_fast_kernel(LiDev p, const float* __restrict__ scores,
+__global__ void __launch_bounds__(kTopkThreads) li_topk_fast_kernel(LiDev p, const float* scores,
                                                                     int64_t ld) {
   typedef typename TopkComposite<kRank16>::type C;
   constexpr int P2 = kTopkThreads * E;
@@ -541,7 +541,7 @@ __device__ __forceinline__ uint32_t rank_key_of(T r) {
 }
 
 template <typename T, int E>
-__global__ void __launch_bounds__(kTopkThreads, 4) li_topk_bins_kernel(LiDev p, const float* __restrict__ scores,
+__global__ void __launch_bounds__(kTopkThreads, 4) li_topk_bins_kernel(LiDev p, const float* scores,
                                                                     int64_t ld) {
   constexpr int P2 = kTopkThreads * E;
   constexpr int NW = kTopkThreads / 32;
@@ -831,7 +831,7 @@ struct BinScale {
 };
 
 template <typename T, int E>
-__global__ void __launch_bounds__(kTopkThreads, 2) li_topk_bins_stream_kernel(LiDev p, const float* __restrict__ scores,
+__global__ void __launch_bounds__(kTopkThreads, 2) li_topk_bins_stream_kernel(LiDev p, const float* scores,
                                                                            int64_t ld) {
   constexpr int P2 = kTopkThreads * E;
   constexpr int NW = kTopkThreads / 32;

@@ -279,8 +279,8 @@ __global__ void __launch_bounds__(kSfaSimtThreads) sfa_fwd_mma_kernel(SfaDev p) 
 // tensor-core kernel's fixed reference maximum; normally none, and then every block leaves after
 // one load).  Any grid; blocks walk over (listed row, head chunk) pairs.
 template <typename T>
-__global__ void __launch_bounds__(kSfaSimtThreads) sfa_redo_kernel(SfaDev p, const int32_t* __restrict__ redo_list,
-                                                                   const int32_t* __restrict__ redo_count) {
+__global__ void __launch_bounds__(kSfaSimtThreads) sfa_redo_kernel(SfaDev p, const int32_t* redo_list,
+                                                                   const int32_t* redo_count) {
   grid_dep_wait();
   const int32_t chunks = (p.n1 + kSfaSimtHeads - 1) / kSfaSimtHeads;
   const int64_t work = (int64_t)min(*redo_count, p.rows) * chunks;

@@ -155,12 +155,12 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi, int is_bf16) {
 // loads as zeros - the slot takes part as a zero row, like the reference's un-paged cache
 // (sparse_flash_attention_triton.py:1012-1033).  Backward: -1, the slot is left out (it has no row to carry a
 // gradient to, and the list then names existing rows only).
-__global__ void __launch_bounds__(128) sfa_compact_kernel(SfaDev p, int2* __restrict__ nvalid,
-                                                          int32_t* __restrict__ key_list, int32_t split,
+__global__ void __launch_bounds__(128) sfa_compact_kernel(SfaDev p, int2* nvalid,
+                                                          int32_t* key_list, int32_t split,
                                                           int32_t part_keys, int32_t kv_rows, int32_t absent,
-                                                          int32_t* __restrict__ redo,
-                                                          int32_t* __restrict__ redo_count,
-                                                          int32_t* __restrict__ status) {
+                                                          int32_t* redo,
+                                                          int32_t* redo_count,
+                                                          int32_t* status) {
   const int lane = threadIdx.x & 31;
   const int32_t row = blockIdx.x * 4 + (threadIdx.x >> 5);
   grid_dep_launch();
@@ -266,12 +266,12 @@ inline bool sfa_compact_by_blocks(const SfaDev& p) {
   return p.rows <= rows && p.sparse_block_size == 1 && (p.sparse_count & 3) == 0 &&
          ((uintptr_t)p.sparse_indices & 15) == 0;
 }
-__global__ void __launch_bounds__(256) sfa_compact_block_kernel(SfaDev p, int2* __restrict__ nvalid,
-                                                                int32_t* __restrict__ key_list, int32_t split,
+__global__ void __launch_bounds__(256) sfa_compact_block_kernel(SfaDev p, int2* nvalid,
+                                                                int32_t* key_list, int32_t split,
                                                                 int32_t part_keys, int32_t kv_rows, int32_t absent,
-                                                                int32_t* __restrict__ redo,
-                                                                int32_t* __restrict__ redo_count,
-                                                                int32_t* __restrict__ status) {
+                                                                int32_t* redo,
+                                                                int32_t* redo_count,
+                                                                int32_t* status) {
   __shared__ int32_t counts[2][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t row = blockIdx.x;
@@ -1049,9 +1049,9 @@ inline bool sfa_sm100_eligible(const DsaSfaParams* p) {
 // unwritten).  All of a thread's loads are in flight together (8 rows x 8 parts x 128 heads: 11.2 -> 4.1 us against
 // the loop over parts that waited for each of them).
 constexpr int kSfaMaxSplit = 8;
-__global__ void __launch_bounds__(256) sfa_merge_kernel(SfaDev p, int32_t split, const float* __restrict__ part_o,
-                                                        const float* __restrict__ part_m,
-                                                        const float* __restrict__ part_l, int32_t is_bf16) {
+__global__ void __launch_bounds__(256) sfa_merge_kernel(SfaDev p, int32_t split, const float* part_o,
+                                                        const float* part_m,
+                                                        const float* part_l, int32_t is_bf16) {
   const int32_t row = blockIdx.x;
   grid_dep_wait();
   {
