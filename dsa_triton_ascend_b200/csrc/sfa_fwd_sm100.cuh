@@ -768,14 +768,14 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       // waits are warp-wide: the tcgen05 loads / stores that follow are warp-collective and must
       // never run with part of a warp gone
       auto wait_w = [&](uint64_t* bar, uint32_t parity) -> bool { return ptx::mbar_spin_warp(bar, parity, abort_flag); };
-      // One arrival per warp on a barrier of the even CTA.  From the odd CTA it is a relaxed remote
-      // arrival: a cluster-scope release costs ~1000 cycles here, and what the arrival announces has
-      // already been made visible by the fences before it (tcgen05.wait + tcgen05 fence for tensor
-      // memory, fence.proxy.async for the P rows, which lie in this CTA's own shared memory).
-      auto signal_lead = [&](uint64_t* local, uint32_t remote) {
+      // One arrival per warp on a barrier of the even CTA.  What it announces from the odd one: `publish`, rows of P that
+      // the warp stored (released to the issuer); else tensor memory that the warp has read (relaxed: the
+      // tcgen05 fence before it orders the reads).
+      auto signal_lead = [&](uint64_t* local, uint32_t remote, bool publish) {
         __syncwarp();
         if (lane == 0) {
           if (rank == 0) ptx::mbar_arrive(local);
+          else if (publish) ptx::mbar_arrive_remote_release(remote);
           else ptx::mbar_arrive_remote_relaxed(remote, 0u);
         }
       };
@@ -847,7 +847,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             for (int k = 0; k < kSfaHalfBK; ++k) sc[k] += s1[k];
           }
           ptx::tc_fence_before();
-          signal_lead(&s_empty[g], s_empty_lead);
+          signal_lead(&s_empty[g], s_empty_lead, false);
           SFA_PROF(1);
           // ---- softmax in the log2 domain; keys past `cnt` are padding
           if (cnt >= kSfaHalfBK) {
@@ -927,7 +927,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           }
           ptx::fence_proxy_async_smem();
           ptx::tc_fence_before();
-          signal_lead(&p_full[g], p_full_lead);
+          signal_lead(&p_full[g], p_full_lead, true);
           SFA_PROF(5);
         }
         if (!ok) break;
@@ -994,7 +994,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           }
         }
         ptx::tc_fence_before();
-        signal_lead(o_free, o_free_lead);
+        signal_lead(o_free, o_free_lead, false);
         SFA_PROF(6);
         if (g == 0 && half == 0) {
           // max of the scaled scores and sum of exp(score - max), back from the log2 domain

@@ -11,11 +11,15 @@ def _source(name):
 
 
 def test_copied_operands_are_released_to_the_other_cta():
-    """The odd CTA's relays announce blocks that other threads copied: a relaxed arrival orders nothing of theirs."""
+    """The odd CTA's relays announce blocks that other threads copied, its softmax warps rows of P that 32 lanes stored: a
+    relaxed arrival of one thread orders nothing of the others."""
     text = _source("sfa_fwd_sm100.cuh")
     arrivals = re.findall(r"mbar_arrive_remote_(\w+)\((\w+)", text)
     for target in ("k_ready_lead", "v_ready_lead"):
         assert [kind for kind, to in arrivals if to == target] == ["release"]
+    assert re.search(r"if \(publish\) ptx::mbar_arrive_remote_release\(remote\);", text)
+    assert re.findall(r"signal_lead\(&?(\w+)[^;]*?, (true|false)\);", text) == [
+        ("s_empty", "false"), ("p_full", "true"), ("o_free", "false")]
     helper = _source("ptx_sm100.cuh").split("void mbar_arrive_remote_release")[1].split("}")[0]
     assert helper.index("fence.release.sync_restrict::shared::cta.cluster") < helper.index("mbarrier.arrive")
 
