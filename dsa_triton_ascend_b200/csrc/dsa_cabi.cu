@@ -301,6 +301,7 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, bool tensor, char* ws, siz
   d.n1 = p->n1; d.d = p->d; d.d_rope = p->d_rope;
   d.sparse_count = p->sparse_count; d.sparse_block_size = p->sparse_block_size;
   d.scale = p->scale;
+  SfaBwdParts parts = {};
   if (d.rows > 0) {
     const unsigned gy = (unsigned)((p->n1 + kSfaGradHeads - 1) / kSfaGradHeads);
     dim3 grid((unsigned)d.rows, gy, 1);
@@ -308,7 +309,7 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, bool tensor, char* ws, siz
     // on request, or with a query or d_out off its 16-byte boundary, the CUDA-core kernel
     const bool mma = p->kernel != DSA_KERNEL_PORTABLE && !off16(p->query, p->query_rope) && !off16(p->d_out);
     if (tensor) {
-      const int rc = sfa_bwd_sm100_launch<T>(p, d, ws, ws_bytes, w, st);
+      const int rc = sfa_bwd_sm100_launch<T>(p, d, ws, ws_bytes, w, &parts, st);
       if (rc != DSA_OK) return rc;
     } else if (mma) {
       int rc;
@@ -329,8 +330,11 @@ static int sfa_grad_launch(const DsaSfaGradParams* p, bool tensor, char* ws, siz
   if (p->key_rows > 0) {
     const int64_t total = p->key_rows * (int64_t)(2 * p->d + p->d_rope);
     const unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16);
-    sfa_bwd_finalize_kernel<T><<<blocks, 256, 0, st>>>(d.dk_acc, d.dv_acc, (T*)p->d_key, (T*)p->d_key_rope,
-                                                      (T*)p->d_value, p->key_rows, p->d, p->d_rope);
+    const SfaBwdRounding<T> r = {d.dk_acc, d.dv_acc, (T*)p->d_key, (T*)p->d_key_rope, (T*)p->d_value, p->key_rows, p->d,
+                                 p->d_rope};
+    if (parts.items > 0)
+      sfa_bwd_finalize_parts_kernel<T><<<blocks + parts.items * 8, 256, 0, st>>>(r, parts, (int32_t)blocks);
+    else sfa_bwd_finalize_kernel<T><<<blocks, 256, 0, st>>>(r);
     if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
     count_launch();
   }

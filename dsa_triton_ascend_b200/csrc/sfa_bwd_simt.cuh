@@ -263,19 +263,30 @@ __global__ void __launch_bounds__(kSfaGradThreads) sfa_bwd_simt_kernel(SfaGradDe
 
 // fp32 accumulators -> d_key [key_rows, d], d_key_rope [key_rows, d_rope], d_value [key_rows, d]
 template <typename T>
-__global__ void __launch_bounds__(256) sfa_bwd_finalize_kernel(const float* __restrict__ dk_acc,
-                                                               const float* __restrict__ dv_acc, T* d_key,
-                                                               T* d_key_rope, T* d_value, int64_t key_rows, int32_t d,
-                                                               int32_t d_rope) {
-  const int32_t dq = d + d_rope, w = dq + d;
-  const int64_t total = key_rows * w;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+struct SfaBwdRounding {
+  const float *dk_acc, *dv_acc;
+  T *d_key, *d_key_rope, *d_value;
+  int64_t key_rows;
+  int32_t d, d_rope;
+};
+// The share of one of `blocks` blocks of 256 threads.
+template <typename T>
+__device__ __forceinline__ void sfa_bwd_finalize(const SfaBwdRounding<T>& a, int32_t block, int32_t blocks) {
+  const float *__restrict__ dk_acc = a.dk_acc, *__restrict__ dv_acc = a.dv_acc;
+  T *d_key = a.d_key, *d_key_rope = a.d_key_rope, *d_value = a.d_value;
+  const int32_t d = a.d, d_rope = a.d_rope, dq = d + d_rope, w = dq + d;
+  const int64_t total = a.key_rows * w;
+  for (int64_t i = (int64_t)block * 256 + threadIdx.x; i < total; i += (int64_t)blocks * 256) {
     const int64_t r = i / w;
     const int32_t c = (int32_t)(i - r * w);
     if (c < d) d_key[r * d + c] = from_f32<T>(dk_acc[r * dq + c]);
     else if (c < dq) d_key_rope[r * d_rope + (c - d)] = from_f32<T>(dk_acc[r * dq + c]);
     else d_value[r * d + (c - dq)] = from_f32<T>(dv_acc[r * d + (c - dq)]);
   }
+}
+template <typename T>
+__global__ void __launch_bounds__(256) sfa_bwd_finalize_kernel(SfaBwdRounding<T> a) {
+  sfa_bwd_finalize(a, blockIdx.x, gridDim.x);
 }
 
 }  // namespace dsa

@@ -91,8 +91,19 @@ struct SfaBwdArgs {
   float* dq_part;            // [items - full][64 heads][576]
   int32_t key_rows;
 };
+// Parts that a row with `tiles` tiles is cut into, at most `parts`, all of them with keys: of 3 tiles or more when rows
+// are cut in two, of 2 in three, of 1 in four.  A part loads Q and dO again (136 KB), which costs less the fewer blocks
+// do it.  Whole calls of 64 heads, rows whole / cut, us: 20 rows (four parts) of 100 keys 43 / 39, of 300 69 / 42; 222
+// rows (74 of them in two) of 300 keys (4 and 3 tiles) 126 / 115.  Cut by slots alone, as if every row had 2048 keys: 222
+// rows of 100 keys 83 for 73, of 40 keys 64 for 50 (with a kernel of its own for the sums).
+__device__ __forceinline__ int32_t bwd_row_parts(int32_t tiles, int32_t parts) {
+  if (parts == 1) return 1;
+  const int32_t n = max(1, min(parts, tiles / (5 - parts))), per = max(1, (tiles + n - 1) / n);
+  return max(1, (tiles + per - 1) / per);
+}
 struct BwdItem { int32_t base, row, h0, slot; int2 nv; };
-// Work item `i`: its (row, 64 heads), its share of the row's list, and its place in dq_part (-1: the whole row).
+// Work item `i`: its (row, 64 heads), its share of the row's list, and its place in dq_part (-1: the whole row, -2:
+// nothing to do, the row has fewer parts).
 __device__ __forceinline__ BwdItem bwd_item(const SfaBwdArgs& a, int32_t i) {
   BwdItem it;
   it.base = i;
@@ -109,9 +120,17 @@ __device__ __forceinline__ BwdItem bwd_item(const SfaBwdArgs& a, int32_t i) {
   it.h0 = (it.base - it.row * a.hblocks) * kBwdHeads;
   it.nv = a.nvalid[it.row];
   if (it.slot >= 0) {
-    const int32_t tiles = (it.nv.x + kBwdBK - 1) / kBwdBK, per = (tiles + a.parts - 1) / a.parts * kBwdBK;
-    it.nv.x = max(0, min(per, it.nv.x - part * per));
-    it.nv.y += part * per;
+    const int32_t tiles = (it.nv.x + kBwdBK - 1) / kBwdBK, n = bwd_row_parts(tiles, a.parts);
+    if (part >= n) {
+      it.slot = -2;
+      it.nv.x = 0;
+    } else if (n == 1) {
+      it.slot = -1;
+    } else {
+      const int32_t per = (tiles + n - 1) / n * kBwdBK;
+      it.nv.x = min(per, it.nv.x - part * per);
+      it.nv.y += part * per;
+    }
   }
   return it;
 }
@@ -273,6 +292,7 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       const BwdItem it = bwd_item(a, item);
+      if (it.slot == -2) continue;
       const int32_t row = it.row, h0 = it.h0, nvalid = it.nv.x, ntiles = tiles_of(nvalid);
       const bool head = h0 + hl < n1;
       const int64_t hi_ = (int64_t)row * n1 + h0 + hl;
@@ -678,35 +698,61 @@ sfa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, misaligned ? 2 : 1);
 }
 
-// d_query of the rows that were cut into parts: the parts' sums in their order, rounded once.
+// d_query of the rows that were cut into parts: the parts' sums in their order, rounded once.  A block per item and 8
+// heads, in front of the `blocks` blocks of the same kernel that round d_key and d_value (a kernel of its own costs a
+// call of short rows, in which there is nothing to add, 3 to 7 us).
+constexpr int kBwdMaxParts = 4;
+struct SfaBwdParts {
+  const int2* nvalid;
+  const float* dq_part;
+  void *d_query, *d_query_rope;
+  int32_t full, parts, items, hblocks, n1;    // items: of 64 heads, that may be cut
+};
 template <typename T>
-__global__ void __launch_bounds__(192) sfa_bwd_dq_kernel(const float* __restrict__ dq_part, T* __restrict__ d_query,
-                                                         T* __restrict__ d_query_rope, int32_t full, int32_t parts,
-                                                         int32_t hblocks, int32_t n1) {
-  const int32_t base = full + blockIdx.x, row = base / hblocks, hl = blockIdx.y;
-  const int32_t h = (base - row * hblocks) * kBwdHeads + hl;
-  if (h >= n1) return;
-  const float* src = dq_part + ((int64_t)blockIdx.x * parts * kBwdHeads + hl) * 576;
+__global__ void __launch_bounds__(256) sfa_bwd_finalize_parts_kernel(SfaBwdRounding<T> r, SfaBwdParts s, int32_t blocks) {
+  if ((int32_t)blockIdx.x >= s.items * 8) {
+    sfa_bwd_finalize(r, (int32_t)blockIdx.x - s.items * 8, blocks);
+    return;
+  }
+  const int32_t item = (int32_t)blockIdx.x >> 3, base = s.full + item, row = base / s.hblocks;
+  const int32_t hl0 = ((int32_t)blockIdx.x & 7) * 8, h0 = (base - row * s.hblocks) * kBwdHeads + hl0;
+  const int32_t n = bwd_row_parts((s.nvalid[row].x + kBwdBK - 1) / kBwdBK, s.parts), heads = min(8, s.n1 - h0);
+  if (n == 1) return;
+  const float* src = s.dq_part + ((int64_t)item * s.parts * kBwdHeads + hl0) * 576;
+#pragma unroll 5
+  for (int32_t i = threadIdx.x; i < heads * 144; i += 256) {
+    float4 x[kBwdMaxParts];
 #pragma unroll
-  for (int u = 0; u < 3; ++u) {
-    const int f = threadIdx.x + u * 192;
-    float v = src[f];
-    for (int32_t q = 1; q < parts; ++q) v += src[(int64_t)q * kBwdHeads * 576 + f];
-    const int64_t i = (int64_t)row * n1 + h;
-    if (f < 512) d_query[i * 512 + f] = from_f32<T>(v);
-    else d_query_rope[i * 64 + f - 512] = from_f32<T>(v);
+    for (int32_t q = 0; q < kBwdMaxParts; ++q)
+      x[q] = q < n ? reinterpret_cast<const float4*>(src + (int64_t)q * kBwdHeads * 576)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float v[4] = {x[0].x, x[0].y, x[0].z, x[0].w};
+#pragma unroll
+    for (int32_t q = 1; q < kBwdMaxParts; ++q) {
+      if (q < n) { v[0] += x[q].x; v[1] += x[q].y; v[2] += x[q].z; v[3] += x[q].w; }
+    }
+    const int32_t h = i / 144, f = (i - h * 144) * 4;
+    const int64_t o = (int64_t)row * s.n1 + h0 + h;
+    T* dst = f < 512 ? (T*)s.d_query + o * 512 + f : (T*)s.d_query_rope + o * 64 + f - 512;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dst[e] = from_f32<T>(v[e]);
   }
 }
 
 // ---- host side ---------------------------------------------------------------------------------
 // Items of the last round: a round lasts as long as its longest item, so where half of the SMs or more would idle in
-// it, its items are cut into 2 to 4 parts of 8 tiles or more, whose d_query is added up afterwards.  512 rows x 64
-// heads, 2048 of 4096 keys: 4 rounds -> 3.5, 1222 -> 1135 us.  148 SMs are assumed (the workspace is sized from it); any other
-// number is still correct.
+// it, its items are cut into 2 to 4 parts, whose d_query is added up afterwards.  This rule goes by the slots, all
+// that the host knows (8 tiles of them a part, or more); a row with fewer keys has fewer parts (bwd_row_parts).
+// Whole calls of 64 heads, 2048 of 4096 keys, rows of the last round whole / cut, us:
+//   first round   1 row 315 / 110,   20 rows 313 / 112,  37 (four parts) 316 / 118,  38 (three) 316 / 140,
+//                 49 316 / 144,      50 (two) 316 / 186, 74 316 / 190
+//   second        149 rows 609 / 400,  222 615 / 482     third 300 905 / 693     fourth 512 1206 / 1066
+//   fourteenth    1925 rows 4139 / 3957, 1998 4266 / 4111 (under the power cap)
+// and 222 rows of 768 slots, the fewest that two parts are made of, 261 / 218.  148 SMs are assumed (the workspace is
+// sized from it); any other number is still correct.
 struct SfaBwdSplit { int32_t full, parts, items; };
 inline SfaBwdSplit sfa_bwd_split(int64_t items, int64_t slots) {
   const int64_t sms = 148, rest = items % sms;
-  const int64_t parts = rest == 0 ? 1 : std::min<int64_t>(std::min<int64_t>(4, sms / rest), slots / (8 * kBwdBK));
+  const int64_t parts = rest == 0 ? 1 : std::min<int64_t>(std::min<int64_t>(kBwdMaxParts, sms / rest), slots / (8 * kBwdBK));
   if (parts < 2) return SfaBwdSplit{(int32_t)items, 1, (int32_t)items};
   return SfaBwdSplit{(int32_t)(items - rest), (int32_t)parts, (int32_t)(items - rest + rest * parts)};
 }
@@ -760,7 +806,7 @@ inline SfaBwdWs sfa_bwd_ws_layout(const DsaSfaGradParams* p, size_t header) {
 
 template <typename T>
 inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, char* ws, size_t ws_bytes,
-                                const SfaBwdWs& w, cudaStream_t st) {
+                                const SfaBwdWs& w, SfaBwdParts* parts, cudaStream_t st) {
   static std::atomic<int> sm_count[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DSA_ERR_CUDA;
@@ -834,12 +880,9 @@ inline int sfa_bwd_sm100_launch(const DsaSfaGradParams* p, const SfaGradDev& d, 
   sfa_bwd_sm100_kernel<T><<<grid, kBwdThreads, kBwdSmemBytes, st>>>(tq, tqr, tdo, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
-  if (sp.parts > 1) {
-    sfa_bwd_dq_kernel<T><<<dim3((unsigned)((sp.items - sp.full) / sp.parts), (unsigned)std::min(p->n1, kBwdHeads)), 192, 0, st>>>(
-        a.dq_part, (T*)p->d_query, (T*)p->d_query_rope, sp.full, sp.parts, hblocks, p->n1);
-    if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
-    count_launch();
-  }
+  if (sp.parts > 1)
+    *parts = SfaBwdParts{nvalid, a.dq_part, p->d_query, p->d_query_rope, sp.full, sp.parts, (sp.items - sp.full) / sp.parts,
+                         hblocks, p->n1};
   return DSA_OK;
 }
 

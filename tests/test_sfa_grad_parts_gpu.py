@@ -3,7 +3,7 @@ every row as a whole."""
 import pytest
 import torch
 
-from dsa_triton_ascend_b200 import check_status, sparse_flash_attention_grad_triton, sparse_flash_attention_triton
+from dsa_triton_ascend_b200 import _host, check_status, sparse_flash_attention_grad_triton, sparse_flash_attention_triton
 from dsa_triton_ascend_b200 import sparse_flash_attention_grad as grad
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +46,36 @@ def test_parts_add_up(q_lens, k_lens, heads, dtype):
     for g, w in zip(got, want):
         assert (g.double() - w.double()).norm() <= bound * w.double().norm()
     assert torch.equal(got[0], again[0]) and torch.equal(got[3], again[3])     # d_query, d_query_rope: no atomics
+
+
+@pytest.mark.parametrize("rows,keys,cut", [(222, 240, False), (222, 288, True), (20, 48, False), (20, 96, True)])
+def test_short_rows_stay_whole(rows, keys, cut, monkeypatch):
+    """Parts are made of the keys that a row has, whatever the width of its list: 1 to 6 tiles of 48 keys here, of 2048
+    slots.  The workspace shows whether any part left a sum."""
+    held = []
+
+    def marked(nbytes, device):
+        held.append(_host.workspace(nbytes, device).fill_(255))
+        return held[-1]
+
+    monkeypatch.setattr(grad, "workspace", marked)
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    normal = lambda *s: (torch.randn(s, generator=gen, device="cuda") * 0.3).bfloat16()   # noqa: E731
+    q, qr, k, kr, d_out = (normal(1, n, h, d) for n, h, d in ((rows, 64, 512), (rows, 64, 64), (keys, 1, 512), (keys, 1, 64),
+                                                               (rows, 64, 512)))
+    idx = torch.full((1, rows, 1, 2048), -1, dtype=torch.int32, device="cuda")
+    idx[..., :keys] = torch.arange(keys, device="cuda")
+    kw = dict(scale_value=576 ** -0.5, query_rope=qr, key_rope=kr, sparse_mode=0)
+    out, mx, sm = sparse_flash_attention_triton(q, k, k, idx, return_softmax_lse=True, **kw)
+    got = sparse_flash_attention_grad_triton(q, k, k, idx, d_out, out, mx, sm, **kw)
+    check_status()
+    left = rows % 148
+    size = left * min(4, 148 // left) * 64 * 576 * 4        # of the parts, at the end of the workspace
+    assert bool((held[0][-size:] != 255).any()) == cut
+    grad.set_kernel("portable")
+    try:
+        want = sparse_flash_attention_grad_triton(q, k, k, idx, d_out, out, mx, sm, **kw)
+    finally:
+        grad.set_kernel("auto")
+    for g, w in zip(got, want):
+        assert (g.double() - w.double()).norm() <= 2.0 ** -8 * w.double().norm()    # one rounding to bf16 each
