@@ -405,6 +405,7 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, bool cut, int32_
   d.g = p->g; d.d_idx = p->d_idx; d.topk = slots; d.dtype_w = p->dtype_w;
   d.scale = p->scale;
   if (cudaMemsetAsync(d.dki_acc, 0, (size_t)key_elems * 4, st) != cudaSuccess) return DSA_ERR_CUDA;
+  SliGradParts parts = {};
   if (rows > 0) {
     const int stride = std::max(p->d + p->d_rope, p->d_idx) + kSliPad;
     // teacher blocks of 32 heads when a side has more than 16 (half the key gathers per row)
@@ -498,7 +499,7 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, bool cut, int32_
     count_launch();
     if (tensor && p->d_idx == 128) {
       float* part = cut ? reinterpret_cast<float*>((char*)d.dki_acc + align256((size_t)key_elems * 4)) : nullptr;
-      const int rc = sli_grad_sm100_launch<T>(p, d, part, status, sms, st);
+      const int rc = sli_grad_sm100_launch<T>(p, d, part, &parts, status, sms, st);
       if (rc != DSA_OK) return rc;
     } else {
       if (cudaFuncSetAttribute(sli_grad_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b) !=
@@ -514,7 +515,9 @@ static int sli_grad_launch(const DsaSliGradParams* p, char* ws, bool cut, int32_
     }
   }
   const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((key_elems + 255) / 256, 148 * 16));
-  sli_finalize_kernel<T><<<blocks, 256, 0, st>>>(d, key_elems, (int32_t)rows);
+  if (parts.items > 0)
+    sli_finalize_parts_kernel<T><<<blocks + parts.items * 8, 256, 0, st>>>(d, key_elems, (int32_t)rows, parts, (int32_t)blocks);
+  else sli_finalize_kernel<T><<<blocks, 256, 0, st>>>(d, key_elems, (int32_t)rows);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
   return DSA_OK;

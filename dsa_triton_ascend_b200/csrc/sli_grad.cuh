@@ -646,12 +646,13 @@ __global__ void __launch_bounds__(kSliThreads) sli_lse_rows_kernel(SliGradDev p,
   if (tid == 0) { p.index_max[row] = m; p.index_sum[row] = se; }
 }
 
-// fp32 accumulator -> d_key_index; block 0 also adds up the rows' loss terms in a fixed order.
+// fp32 accumulator -> d_key_index; block 0 also adds up the rows' loss terms in a fixed order.  The share of one of
+// `blocks` blocks of 256 threads.
 template <typename T>
-__global__ void __launch_bounds__(256) sli_finalize_kernel(SliGradDev p, int64_t total, int32_t rows) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
+__device__ __forceinline__ void sli_finalize(const SliGradDev& p, int64_t total, int32_t rows, int32_t block, int32_t blocks) {
+  for (int64_t i = (int64_t)block * 256 + threadIdx.x; i < total; i += (int64_t)blocks * 256)
     ((T*)p.d_key_index)[i] = from_f32<T>(p.dki_acc[i]);
-  if (blockIdx.x == 0) {
+  if (block == 0) {
     __shared__ float red[256];
     float s = 0.f;
     for (int r = threadIdx.x; r < rows; r += 256) s += p.loss_parts[r];
@@ -663,6 +664,10 @@ __global__ void __launch_bounds__(256) sli_finalize_kernel(SliGradDev p, int64_t
     }
     if (threadIdx.x == 0) p.loss[0] = red[0];
   }
+}
+template <typename T>
+__global__ void __launch_bounds__(256) sli_finalize_kernel(SliGradDev p, int64_t total, int32_t rows) {
+  sli_finalize<T>(p, total, rows, blockIdx.x, gridDim.x);
 }
 
 }  // namespace dsa

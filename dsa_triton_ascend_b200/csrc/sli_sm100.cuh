@@ -556,6 +556,7 @@ static_assert(kSgSmemBytes <= kSlSmemMax, "shared memory");
 constexpr uint32_t kSgTmS = 0, kSgTmK = 128, kSgTmQ = 384;
 
 constexpr int kSgPart = 64 * 128 + 64;
+constexpr int kSgMaxParts = 4;
 
 struct SliGradArgs {
   SliGradDev p;
@@ -567,7 +568,13 @@ struct SliGradArgs {
   uint32_t idesc_s, idesc_k, idesc_q;
 };
 
-// Work item: (row, 64 heads) or, in the last round, a part of its slots (SliGradSplit): slots off .. off + n - 1.
+// Parts that a row with `tiles` tiles is cut into, at most `parts`: of 3 tiles or more, and all of them with slots
+// ((n - 1)^2 < tiles).  Whole calls, 2048 selected slots, rows whole / cut, us: 20 rows of 700 keys (6 tiles) 59 / 54, 222
+// rows of up to 700 101 / 97; cut by slots alone, as if every row had 2048 keys, 20 rows of 100 keys 60 for 46, 222 of
+// 300 85 for 78 (with a kernel of its own for the sums).
+__device__ __forceinline__ int32_t sli_row_parts(int32_t tiles, int32_t parts) { return max(1, min(parts, tiles / 3)); }
+// Work item: (row, 64 heads) or, in the last round, a part of its slots (SliGradSplit): slots off .. off + n - 1.  Its
+// place in `part`; -1: the whole row, -2: nothing to do, the row has fewer parts.
 struct SliGradItem { int32_t row, h0, b, n, off, slot; };
 __device__ __forceinline__ SliGradItem sli_grad_item(const SliGradArgs& a, int32_t i) {
   SliGradItem it;
@@ -585,9 +592,17 @@ __device__ __forceinline__ SliGradItem sli_grad_item(const SliGradArgs& a, int32
   it.n = sli_row_slots(a.p, it.row, &it.b);
   it.off = 0;
   if (it.slot >= 0) {
-    const int32_t tiles = (it.n + kSlKeys - 1) / kSlKeys, per = (tiles + a.parts - 1) / a.parts * kSlKeys;
-    it.off = part * per;
-    it.n = max(0, min(per, it.n - it.off));
+    const int32_t tiles = (it.n + kSlKeys - 1) / kSlKeys, n = sli_row_parts(tiles, a.parts);
+    if (part >= n) {
+      it.slot = -2;
+      it.n = 0;
+    } else if (n == 1) {
+      it.slot = -1;
+    } else {
+      const int32_t per = (tiles + n - 1) / n * kSlKeys;
+      it.off = part * per;
+      it.n = min(per, it.n - it.off);
+    }
   }
   return it;
 }
@@ -670,17 +685,14 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       const SliGradItem it = sli_grad_item(a, item);
+      if (it.slot == -2) continue;
       const int32_t row = it.row, h0 = it.h0, n = it.n, ntiles = tiles_of(n);
       const int32_t hn = min(32, g - h0 - half * 32);     // this warp's heads that exist
       float* part = it.slot >= 0 ? a.part + (int64_t)it.slot * kSgPart : nullptr;
       T* dq = (T*)a.p.d_query_index + ((int64_t)row * g + h0 + half * 32) * 128 + key;
       if (ntiles == 0) {
-        for (int h = 0; h < hn; ++h) {
-          if (part) part[(half * 32 + h) * 128 + key] = 0.f;
-          else dq[h * 128] = from_f32<T>(0.f);
-        }
-        if (part) { if (quarter == 0) part[64 * 128 + half * 32 + lane] = 0.f; }
-        else if (quarter == 0 && lane < hn)
+        for (int h = 0; h < hn; ++h) dq[h * 128] = from_f32<T>(0.f);
+        if (quarter == 0 && lane < hn)
           store_weight(a.p.d_weights, a.p.dtype_w, (int64_t)row * g + h0 + half * 32 + lane, 0.f);
         continue;
       }
@@ -1075,32 +1087,59 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, misaligned ? 2 : 1);
 }
 
-// dQI and dW of the items that were cut into parts: the parts' sums in their order.  A block per item, 128 features.
+// dQI and dW of the items that were cut into parts: the parts' sums in their order.  A block per item and 8 heads, before
+// the `blocks` blocks of the same kernel that round dKI (a kernel of its own costs a call of short rows, in which there
+// is nothing to add, 4 to 6 us).
+struct SliGradParts {
+  const float* part;
+  int32_t full, parts, items, hchunks;    // items: of 64 heads, that may be cut
+};
 template <typename T>
-__global__ void __launch_bounds__(128) sli_grad_parts_kernel(SliGradDev p, const float* __restrict__ part, int32_t full,
-                                                             int32_t parts, int32_t hchunks) {
-  const int32_t base = full + blockIdx.x, row = base / hchunks, h0 = (base - row * hchunks) * 64, hn = min(64, p.g - h0);
-  const float* src = part + (int64_t)blockIdx.x * parts * kSgPart;
-  const int64_t i0 = (int64_t)row * p.g + h0;
-  for (int32_t h = blockIdx.y; h < hn; h += gridDim.y) {
-    float v = src[h * 128 + threadIdx.x];
-    for (int32_t q = 1; q < parts; ++q) v += src[(int64_t)q * kSgPart + h * 128 + threadIdx.x];
-    ((T*)p.d_query_index)[(i0 + h) * 128 + threadIdx.x] = from_f32<T>(v * load_weight(p.weights, p.dtype_w, i0 + h));
-    if (threadIdx.x == 0) {
-      float w = src[64 * 128 + h];
-      for (int32_t q = 1; q < parts; ++q) w += src[(int64_t)q * kSgPart + 64 * 128 + h];
-      store_weight(p.d_weights, p.dtype_w, i0 + h, w);
-    }
+__global__ void __launch_bounds__(256) sli_finalize_parts_kernel(SliGradDev p, int64_t total, int32_t rows, SliGradParts s,
+                                                                 int32_t blocks) {
+  if ((int32_t)blockIdx.x >= s.items * 8) {
+    sli_finalize<T>(p, total, rows, (int32_t)blockIdx.x - s.items * 8, blocks);
+    return;
+  }
+  const int32_t item = (int32_t)blockIdx.x >> 3, base = s.full + item, row = base / s.hchunks;
+  const int32_t hl0 = ((int32_t)blockIdx.x & 7) * 8, h0 = (base - row * s.hchunks) * 64 + hl0;
+  int32_t b;
+  const int32_t n = sli_row_parts((sli_row_slots(p, row, &b) + kSlKeys - 1) / kSlKeys, s.parts), heads = min(8, p.g - h0);
+  if (n == 1) return;
+  const float* src = s.part + (int64_t)item * s.parts * kSgPart;
+  const int64_t o = (int64_t)row * p.g + h0;
+#pragma unroll 4
+  for (int32_t i = threadIdx.x; i < heads * 128; i += 256) {
+    float x[kSgMaxParts];
+#pragma unroll
+    for (int32_t q = 0; q < kSgMaxParts; ++q) x[q] = q < n ? src[(int64_t)q * kSgPart + hl0 * 128 + i] : 0.f;
+    float v = x[0];
+#pragma unroll
+    for (int32_t q = 1; q < kSgMaxParts; ++q)
+      if (q < n) v += x[q];
+    ((T*)p.d_query_index)[o * 128 + i] = from_f32<T>(v * load_weight(p.weights, p.dtype_w, o + (i >> 7)));
+  }
+  if ((int32_t)threadIdx.x < heads) {
+    const int32_t i = 64 * 128 + hl0 + threadIdx.x;
+    float v = src[i];
+    for (int32_t q = 1; q < n; ++q) v += src[(int64_t)q * kSgPart + i];
+    store_weight(p.d_weights, p.dtype_w, o + threadIdx.x, v);
   }
 }
 
 // ---- host side -----------------------------------------------------------------------------------
-// Gradient items of a last round that would leave half of the SMs idle or more: cut into 2 to 4 parts of 4 tiles or more (as
-// sfa_bwd_split).  Whole calls of 512 rows, 64 heads: dense over 4096 keys 508 -> 495 us, 2048 selected keys 381 -> 377.
+// Gradient items of a last round that would leave half of the SMs idle or more: cut into 2 to 4 parts, by the slots (4
+// tiles of them a part, or more; as sfa_bwd_split, a row with fewer keys has fewer: sli_row_parts).  Whole calls of
+// 64 index heads, rows of the last round whole / cut, us, 2048 selected of 4096 keys | dense over 4096:
+//   first round   1 row 77 / 54 | 115 / 69,  37 rows (four parts) 86 / 62 | 137 / 95,  38 (three) 88 / 68 | 138 / 100,
+//                 49 92 / 72 | 141 / 104,  50 (two) 92 / 75 | 140 / 112,  74 97 / 82 | 147 / 122
+//   second        149 156 / 133 | 231 / 187,  222 162 / 147 | 244 / 214      fourth  512 284 / 269 | 427 / 402
+//   fourteenth    1925 925 / 906 | 1137 / 1113,  1998 945 / 932 | 1161 / 1140
+// and 222 rows of 1024 slots, the fewest that two parts are made of, 110 / 101.
 struct SliGradSplit { int32_t full, parts, items; };
 inline SliGradSplit sli_grad_split(int64_t items, int64_t slots) {
   const int64_t sms = 148, rest = items % sms;
-  const int64_t parts = rest == 0 ? 1 : std::min<int64_t>(std::min<int64_t>(4, sms / rest), slots / (4 * kSlKeys));
+  const int64_t parts = rest == 0 ? 1 : std::min<int64_t>(std::min<int64_t>(kSgMaxParts, sms / rest), slots / (4 * kSlKeys));
   if (parts < 2) return SliGradSplit{(int32_t)items, 1, (int32_t)items};
   return SliGradSplit{(int32_t)(items - rest), (int32_t)parts, (int32_t)(items - rest + rest * parts)};
 }
@@ -1235,8 +1274,8 @@ inline int sli_mha_sm100_launch(const DsaSliGradParams* p, SliMhaArgs a, int32_t
 }
 
 template <typename T>
-inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d, float* part, int32_t* status, int sms,
-                                 cudaStream_t st) {
+inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d, float* part, SliGradParts* parts,
+                                 int32_t* status, int sms, cudaStream_t st) {
   const bool bf16 = p->dtype == DSA_DTYPE_BF16;
   const int64_t rows = (int64_t)p->batch * p->s1;
   SliGradArgs a;
@@ -1262,12 +1301,7 @@ inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d,
   sli_grad_sm100_kernel<T><<<std::min(a.items, sms), kSgThreads, kSgSmemBytes, st>>>(tk, tq, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
-  if (sp.parts > 1) {
-    sli_grad_parts_kernel<T><<<dim3((unsigned)((sp.items - sp.full) / sp.parts), 8), 128, 0, st>>>(d, part, sp.full, sp.parts,
-                                                                                                  a.hchunks);
-    if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
-    count_launch();
-  }
+  if (sp.parts > 1) *parts = SliGradParts{part, sp.full, sp.parts, (sp.items - sp.full) / sp.parts, a.hchunks};
   return DSA_OK;
 }
 
