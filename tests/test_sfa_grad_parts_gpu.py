@@ -1,22 +1,45 @@
 """Attention backward where the last round of work items is cut into parts: against the CUDA-core kernel, which takes
 every row as a whole."""
+import ctypes
+
 import pytest
 import torch
 
-from dsa_triton_ascend_b200 import _host, check_status, sparse_flash_attention_grad_triton, sparse_flash_attention_triton
+from dsa_triton_ascend_b200 import _cabi, _host, check_status, sparse_flash_attention_grad_triton, sparse_flash_attention_triton
 from dsa_triton_ascend_b200 import sparse_flash_attention_grad as grad
 
 pytestmark = pytest.mark.gpu
 
 
-# items of 64 heads left for the last round of 148: 2 (four parts), 52 (two parts), 2 of two head blocks
-# (the second of 16 heads), 49 (three parts, short rows: parts without keys), 75 (whole: more than half a round)
-@pytest.mark.parametrize("q_lens,k_lens,heads", [([150], [1200], 16), ([200], [1200], 64), ([75], [1300], 80),
-                                                 ([20, 177], [20, 1000], 16), ([223], [1200], 16)])
+def _parts(rows, keys, heads, count, left, dtype):
+    """Parts that the call's `left` last items are cut into, from the size of its workspace."""
+    p = _cabi.DsaSfaGradParams()
+    p.struct_size = ctypes.sizeof(p)
+    for name, kind in p._fields_:
+        if kind is ctypes.c_void_p and name not in ("seq_q", "seq_k"):
+            setattr(p, name, 256)
+    p.batch, p.s1, p.s2, p.n1, p.d, p.d_rope, p.key_rows = 1, rows, keys, heads, 512, 64, keys
+    p.sparse_count, p.sparse_block_size, p.sparse_mode = count, 1, 3
+    p.dtype = _cabi.DTYPE_BF16 if dtype == torch.bfloat16 else _cabi.DTYPE_FP16
+    total, uncut = ctypes.c_size_t(0), ctypes.c_size_t(0)
+    assert _cabi.lib.dsa_sfa_grad_workspace_bytes(ctypes.byref(p), ctypes.byref(total)) == 0
+    assert _cabi.lib.dsa_sfa_grad_workspace_bytes_uncut(ctypes.byref(p), ctypes.byref(uncut)) == 0
+    return max(1, (total.value - uncut.value) // (64 * 576 * 4) // left)
+
+
+# items of 64 heads left for the last round of 148 and the parts they are cut into: 2 in four; 52 in two; 2 of two head
+# blocks (the second of 16 heads), in three; 49 in three, of which 20 have 181 to 200 keys (4 or 5 tiles: two parts and
+# none in the place of the third) and the last 20 have 0 to 12 (whole); 75, more than half a round, as they are
+@pytest.mark.parametrize("q_lens,k_lens,heads,count,left,parts", [
+    ([150], [1700], 16, 1536, 2, 4), ([200], [1200], 64, 1152, 52, 2), ([75], [1300], 80, 1152, 2, 3),
+    ([157, 20, 20], [1000, 200, 12], 16, 1152, 49, 3), ([223], [1200], 16, 1152, 75, 1)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_parts_add_up(q_lens, k_lens, heads, dtype):
+def test_parts_add_up(q_lens, k_lens, heads, count, left, parts, dtype, monkeypatch):
+    assert _parts(sum(q_lens), sum(k_lens), heads, count, left, dtype) == parts
+    # (what is not written before it is read shows as a NaN)
+    monkeypatch.setattr(grad, "workspace", lambda nbytes, device: _host.workspace(nbytes, device).fill_(255))
     gen = torch.Generator(device="cuda").manual_seed(sum(q_lens) + heads)
-    rows, keys, count = sum(q_lens), sum(k_lens), 1152
+    rows, keys = sum(q_lens), sum(k_lens)
 
     def normal(*shape):
         return (torch.randn(shape, generator=gen, device="cuda") * 0.3).to(dtype)
