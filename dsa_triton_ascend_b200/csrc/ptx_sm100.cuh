@@ -71,9 +71,8 @@ __device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
 }
 // Arrive on an mbarrier of another CTA of the cluster, publishing shared memory of this CTA: what this thread wrote there,
 // and what it has seen other threads publish (release is cumulative), is ordered before the acquire over there.  The
-// fence is restricted to shared memory: mbarrier.arrive.release.cluster also waits for this SM's traffic to global
-// memory, of which a gather always has some in flight (attend 15360 tokens x 128 heads, each pair in turn: 7168 us
-// without a release, 7901 with that one; 7265 without, 7319 with this fence).
+// fence is restricted to shared memory; mbarrier.arrive.release.cluster orders global memory as well (attend 15360
+// tokens x 128 heads, each pair in turn: 7168 us without a release, 7901 with that one; 7265 without, 7319 with this).
 __device__ __forceinline__ void mbar_arrive_remote_release(uint32_t raddr_bar) {
   asm volatile(
       "fence.release.sync_restrict::shared::cta.cluster;\n\t"

@@ -21,12 +21,13 @@
 // Data movement.  Both blocks are gathered from L2 with 16-byte cp.async copies straight into the 128-byte-swizzled
 // MMA layout, K by six producer warps and V by four, from a front-packed list of physical KV rows that a pre-pass
 // kernel writes; a copy's completion is an arrival on the slot's barrier, so that no warp waits for its own copies.
-// An SM takes 72 B/clk this way (12 warps with 16 KB in flight each); TMA tile::gather4 takes one 512-byte load per
-// 16.5 cycles (31 B/clk), whatever else the SM does.  The 32 keys that both blocks share are loaded twice: building
-// V from the K block instead (loads, stores and st.async to the peer) holds the K slot until the copy is done
-// and costs the shared memory 512 cycles of traffic per tile against 256.  attend 15360 tokens x 128 heads, top-k
-// 2048, in turn with the version that gathered K with gather4 and copied V: 8130 -> 7167 us; 1471 ragged tokens x
-// 64 heads, indexer included: 629 -> 570 us.
+// A CTA loads 68 KB per tile of 2000 cycles, 35 B/clk; alone, with nothing but gathers on the SM, such copies were measured
+// at 58 (8 warps) to 72 B/clk (12 warps with 16 KB in flight each).  TMA tile::gather4 takes one 512-byte load per 16.5
+// cycles (31 B/clk), whatever else the SM does.  The 32 keys that both blocks share are loaded twice: building V from
+// the K block instead (loads, stores and st.async to the peer) holds the K slot until the copy is done and costs the
+// shared memory 512 cycles of traffic per tile against 256.  attend 15360 tokens x 128 heads, top-k 2048, in turn with the
+// version that gathered K with gather4 and copied V: 8130 -> 7167 us back to back under the power cap, 7437 -> 6524 as
+// single calls a second apart; 1471 ragged tokens x 64 heads, indexer included: 629 -> 570 us.
 //
 // Accumulator layout of a pair MMA with M = 128 (measured): lanes 0..63 hold a CTA's rows with the
 // first half of N, lanes 64..127 the same rows with the second half.  So TMEM lane L of CTA c
@@ -510,8 +511,9 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         load_rows(nxt, rn);
         const uint32_t s = n_tile & 1, use = n_tile >> 1;
         SFA_PROF(0);
-        // every lane polls (see ptx::mbar_wait_warp).  Like every wait of this kernel it spins without suspending: waking from a suspended try_wait costs hundreds of cycles at
-        // every hand-over (826 vs 640 TFLOP/s on a 4096-token, top-2048 case).
+        // every lane polls (see ptx::mbar_wait_warp).  Like every wait of this kernel it spins without suspending:
+        // waking from a suspended try_wait costs hundreds of cycles at every hand-over (826 vs 640 TFLOP/s on a
+        // 4096-token, top-2048 case).
         ok = ptx::mbar_spin_warp(&empty[s * 3], (use & 1) ^ 1, abort_flag);
         if (!ok) break;
         SFA_PROF(1);
@@ -657,7 +659,7 @@ sfa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
           const uint32_t b = n_tile & 1, use = n_tile >> 1;
           SFA_PROF(0);
-          ok = ptx::mbar_spin_cluster_warp(&v_full[b], use & 1, abort_flag);
+          ok = ptx::mbar_spin_warp(&v_full[b], use & 1, abort_flag);
           if (!ok) break;
           SFA_PROF(1);
           if (rank != 0) {

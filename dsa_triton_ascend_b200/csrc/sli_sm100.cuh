@@ -23,12 +23,13 @@ constexpr uint32_t kSlSmemMax = 232448;
 // ---- scores --------------------------------------------------------------------------------------
 // What bounds it: the hand-overs between gather, issuers and epilogue (512 rows x 2048 keys x 64 heads: 150 us; with a
 // quarter of the products and no global reads still 117).  A row's selected keys are its own, so each (row, key) pair
-// is a gather of 2 (D + Dr) bytes; cp.async copies bring 72 B/clk of them to an SM, TMA gather4 31 (one 512-byte
-// load per 16.5 cycles).  A block takes up to 128 heads of the row (every gathered byte serves all of them), Q stays
+// is a gather of 2 (D + Dr) bytes; cp.async copies of 8 warps bring 58 B/clk of them to an SM that does nothing else,
+// TMA gather4 31 (one 512-byte load per 16.5 cycles).  A block takes up to 128 heads of the row (every gathered byte serves all of them), Q stays
 // in shared memory and the keys stream through a ring of 64-feature blocks (16 KB each: a whole tile of 147 KB would
 // not fit beside 128 heads of Q).  Rows are cut into parts when there are few of them.
 // With gather4 and one issuer, and with the copies and two (attention / index side): 512 rows x 64 heads 191 / 67 us
-// -> 150 / 56, 2048 rows x 128 heads, fp16: 838 / 253 -> 680 / 202.
+// -> 150 / 56.  2048 rows x 128 heads, fp16, in calls back to back: 838 / 252 of a call of 1721 -> 705 / 209 of 1605;
+// the gradient kernel behind them, unchanged, takes 590 -> 629 there, at the lower clock that the power cap leaves.
 // Warps: 0..7 epilogue (two groups on alternate accumulators), 8..15 gather, 16, 17 MMA issuers, 18 Q and head
 // parameters.
 constexpr int kScThreads = 608, kScGatherWarp0 = 8, kScGatherWarps = 8, kScIssuer = 16, kScLoader = 18;
@@ -42,7 +43,7 @@ struct SliScoreArgs {
   int32_t heads;             // of this side
   int32_t nblk, nblk_a;      // 64-feature blocks in all / of the first tensor (the others: rope)
   int32_t hp;                // heads per item, padded to 16
-  int32_t hchunks, parts, items, stages, key_rows;
+  int32_t hchunks, parts, items, stages;
   uint32_t idesc, off_k, off_prm, off_bar;
 };
 
@@ -517,9 +518,9 @@ sli_mha_sm100_kernel(const __grid_constant__ CUtensorMap tmap_ka, const __grid_c
 // What it is built around: the scatter-adds of dKI (512 B per (row, key): 2300 cycles of the load / store unit
 // per 128 keys, 4.5 per line; all SMs together 6.2 TB/s), against 1300 cycles of tensor pipe and 1170 of
 // gather.  ncu, 512 rows x 2048 keys, 64 heads: 174 us, 3.1 TB/s of reductions, load / store data pipe 41 %, tensor
-// pipe 29 % (dense over 3840 keys a row: 286 us, 3.5 TB/s, 44 %, 33 %).  So a work item is (query row, 64 index heads), which makes every reduction carry all heads
-// of up to 64, and as in sfa_bwd_sm100.cuh the gradient products run with FEATURES on the lanes, so that a
-// reduction instruction is one full line.  Per tile of 128 gathered keys (M = the first named):
+// pipe 29 % (dense over 3840 keys a row: 286 us, 3.5 TB/s, 44 %, 33 %).  So a work item is (query row, 64 index heads),
+// which makes every reduction carry all heads of up to 64, and as in sfa_bwd_sm100.cuh the gradient products run with
+// FEATURES on the lanes, so that a reduction instruction is one full line.  Per tile of 128 gathered keys (M = the first named):
 //     S   [keys, heads]     = K . QI^T                              E = S > 0
 //     dKI^T [features, keys]  = (w QI)^T . E^T, times dI of the key   when it is drained
 //     dQI^T [features, heads] += K^T . (dI E), times w of the head      at the end of the row
@@ -1211,7 +1212,6 @@ inline int sli_score_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d
   a.parts = (int32_t)std::max<int64_t>(1, std::min<int64_t>(most, (6 * sms + rows * a.hchunks - 1) / (rows * a.hchunks)));
   if (rows * a.hchunks * a.parts >= (1ll << 31)) return DSA_ERR_TOO_LARGE;
   a.items = (int32_t)(rows * a.hchunks * a.parts);
-  a.key_rows = (int32_t)((int64_t)p->batch * p->s2);
   a.idesc = ptx::idesc_f16(bf16 ? 1u : 0u, 128, (uint32_t)a.hp, 0, 0);
   const uint32_t qbytes = (uint32_t)a.nblk * a.hp * 128, tail = 2 * 128 * 8 + 512;
   // (the ring starts on a 1024-byte boundary: hp * 128 is a multiple of 2048)
