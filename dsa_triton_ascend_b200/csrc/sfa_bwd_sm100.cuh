@@ -28,10 +28,10 @@
 //     (Cauchy-Schwarz over the item's heads and selected keys, taken by small kernels in front) below 2^13.
 //
 // Measured, whole operator call: B1 S1 512 S2 4096 N1 64 k 2048 in bf16 1.14 ms (sfa_bwd_mma_kernel: 4.63 ms); 4092
-// rows x 128 heads in bf16 7.3-7.4 ms back to back under the power cap (32.2 ms), 7.1 as single calls a second apart.  A tile of 48 keys takes 12 400 cycles: its
-// reductions alone would take 8400, its products 8000.  What is left is the chain of a tile (keys 1700, S 2200, P and
-// dS 5500, of which 1600 wait for dK of the tile before, dQ 2100) beside the chain of the dV / dK tiles (issue 6400,
-// ring slots 3100), and the reload of Q / dO between items.
+// rows x 128 heads in bf16 7.3-7.4 ms back to back under the power cap (32.2 ms), 7.1 as single calls a second apart.
+// A tile of 48 keys takes 12 400 cycles: its reductions alone would take 8400, its products 8000.  What is left is
+// the chain of a tile (keys 1700, S 2200, P and dS 5500, of which 1600 wait for dK of the tile before, dQ 2100) beside
+// the chain of the dV / dK tiles (issue 6400, ring slots 3100), and the reload of Q / dO between items.
 // ptxas spills 0 bytes (bf16) and 32 bytes (fp16) of a thread's 72 registers.
 //
 // Tensor memory: dQ^T 5 x 64 columns | S, dP 48 | rope part of S 48 | drain ring 2 x 48.
