@@ -444,7 +444,7 @@ def run_gpu(args):
             flush.fill_(i & 0xFF)
             a, b_ = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             a.record()
-            _cabi.check(_cabi.lib.dsa_li_forward(ctypes.byref(p), ws.data_ptr(), ws.numel(), stream), "li")
+            _cabi.check(_cabi.lib.dsa_li_forward_zeros(ctypes.byref(p), ws.data_ptr(), ws.numel(), stream), "li")
             b_.record()
             torch.cuda.synchronize()
             if i >= args.warmup:

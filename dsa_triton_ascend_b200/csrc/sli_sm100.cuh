@@ -29,7 +29,8 @@ constexpr uint32_t kSlSmemMax = 232448;
 // not fit beside 128 heads of Q).  Rows are cut into parts when there are few of them.
 // With gather4 and one issuer, and with the copies and two (attention / index side): 512 rows x 64 heads 191 / 67 us
 // -> 150 / 56.  2048 rows x 128 heads, fp16, in calls back to back: 838 / 252 of a call of 1721 -> 705 / 209 of 1605;
-// the gradient kernel behind them, unchanged, takes 590 -> 629 there, at the lower clock that the power cap leaves.
+// the gradient kernel behind them, the same code, takes 590 -> 629 there, at the lower clock that the power cap leaves
+// (602 and 603 in single calls).  Rows of one tile gain nothing: 1234 rows of 64 keys 58.4 / 19.3 -> 59.8 / 19.9.
 // Warps: 0..7 epilogue (two groups on alternate accumulators), 8..15 gather, 16, 17 MMA issuers, 18 Q and head
 // parameters.
 constexpr int kScThreads = 608, kScGatherWarp0 = 8, kScGatherWarps = 8, kScIssuer = 16, kScLoader = 18;
@@ -575,34 +576,35 @@ struct SliGradArgs {
 // 300 85 for 78 (with a kernel of its own for the sums).
 __device__ __forceinline__ int32_t sli_row_parts(int32_t tiles, int32_t parts) { return max(1, min(parts, tiles / 3)); }
 // Work item: (row, 64 heads) or, in the last round, a part of its slots (SliGradSplit): slots off .. off + n - 1.  Its
-// place in `part`; -1: the whole row, -2: nothing to do, the row has fewer parts.
-struct SliGradItem { int32_t row, h0, b, n, off, slot; };
+// place in `part`, -1: the whole row.  n = -1: nothing to do, the row has fewer parts.
+struct SliGradItem { int32_t row, h0, n, off, key0, slot; };      // key0: key row that dense slots and indices count from
+template <bool kCut>
 __device__ __forceinline__ SliGradItem sli_grad_item(const SliGradArgs& a, int32_t i) {
   SliGradItem it;
-  it.slot = i - a.full;
+  it.slot = -1;
+  it.off = 0;
   int32_t base = i, part = 0;
-  if (it.slot >= 0) {
+  if (kCut && i >= a.full) {
+    it.slot = i - a.full;
     const int32_t r = it.slot / a.parts;
     part = it.slot - r * a.parts;
     base = a.full + r;
-  } else {
-    it.slot = -1;
   }
   it.row = base / a.hchunks;
   it.h0 = (base - it.row * a.hchunks) * 64;
-  it.n = sli_row_slots(a.p, it.row, &it.b);
-  it.off = 0;
-  if (it.slot >= 0) {
+  int32_t b;
+  it.n = sli_row_slots(a.p, it.row, &b);
+  it.key0 = b * a.p.s2;
+  if (kCut && it.slot >= 0) {
     const int32_t tiles = (it.n + kSlKeys - 1) / kSlKeys, n = sli_row_parts(tiles, a.parts);
+    if (n == 1) it.slot = -1;
     if (part >= n) {
-      it.slot = -2;
-      it.n = 0;
-    } else if (n == 1) {
-      it.slot = -1;
-    } else {
+      it.n = -1;
+    } else if (n > 1) {
       const int32_t per = (tiles + n - 1) / n * kSlKeys;
       it.off = part * per;
       it.n = min(per, it.n - it.off);
+      if (a.p.sparse_indices == nullptr) it.key0 += it.off;
     }
   }
   return it;
@@ -610,7 +612,7 @@ __device__ __forceinline__ SliGradItem sli_grad_item(const SliGradArgs& a, int32
 // Key row of the item's j-th slot; past its n slots `none` (a row that does not exist: TMA fills zeros).
 __device__ __forceinline__ int32_t sli_key_row(const SliGradDev& p, const int32_t* idx_row, const SliGradItem& it, int32_t j,
                                                int32_t none) {
-  return j < it.n ? it.b * p.s2 + sli_slot_key(p, idx_row, it.off + j) : none;
+  return j < it.n ? it.key0 + sli_slot_key(p, idx_row, j) : none;
 }
 
 // Exponent of the power of two that brings magnitudes up to `m` below 2^14.
@@ -621,7 +623,10 @@ __device__ __forceinline__ int sli_exponent(float m) {
 template <typename T>
 __device__ __forceinline__ uint32_t sli_bits(T v) { return (uint32_t)*reinterpret_cast<const uint16_t*>(&v); }
 
-template <typename T>
+// kCut: items of the last round may be parts of rows.  Compiled apart because the other calls pay for it otherwise (this
+// kernel, 625 dense rows of 202 to 826 keys: 72.7 us apart, 74.3 together, 75.9 with the choice between part and row
+// inside the loop that stores dQI; 678 rows, fp16: 88.8, 89.2, 91.9).
+template <typename T, bool kCut>
 __global__ void __launch_bounds__(kSgThreads, 1)
 sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_q,
                       const SliGradArgs a) {
@@ -685,11 +690,11 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     uint32_t n_tile = 0, n_item = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const SliGradItem it = sli_grad_item(a, item);
-      if (it.slot == -2) continue;
+      const SliGradItem it = sli_grad_item<kCut>(a, item);
+      if (kCut && it.n < 0) continue;
       const int32_t row = it.row, h0 = it.h0, n = it.n, ntiles = tiles_of(n);
       const int32_t hn = min(32, g - h0 - half * 32);     // this warp's heads that exist
-      float* part = it.slot >= 0 ? a.part + (int64_t)it.slot * kSgPart : nullptr;
+      float* part = kCut && it.slot >= 0 ? a.part + (int64_t)it.slot * kSgPart : nullptr;
       T* dq = (T*)a.p.d_query_index + ((int64_t)row * g + h0 + half * 32) * 128 + key;
       if (ntiles == 0) {
         for (int h = 0; h < hn; ++h) dq[h * 128] = from_f32<T>(0.f);
@@ -697,7 +702,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
           store_weight(a.p.d_weights, a.p.dtype_w, (int64_t)row * g + h0 + half * 32 + lane, 0.f);
         continue;
       }
-      const int32_t* idx_row = a.p.sparse_indices ? a.p.sparse_indices + (int64_t)row * a.p.topk : nullptr;
+      const int32_t* idx_row = a.p.sparse_indices ? a.p.sparse_indices + (int64_t)row * a.p.topk + it.off : nullptr;
       const float* di_row = a.p.di + (int64_t)row * a.p.topk + it.off;
       float up = 1.f, down = 1.f, w_down = 1.f;
       if constexpr (kScaled) {
@@ -801,15 +806,18 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(dq_empty);
         }
+        if (part) {
 #pragma unroll
-        for (int h = 0; h < 16; ++h)
-          if (c + h < hn) {
-            const float x = kScaled ? v[h] * down : v[h];
-            if (part) part[(half * 32 + c + h) * 128 + key] = x;
-            else
-              dq[(c + h) * 128] =
-                  from_f32<T>(x * load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + half * 32 + c + h));
-          }
+          for (int h = 0; h < 16; ++h)
+            if (c + h < hn) part[(half * 32 + c + h) * 128 + key] = kScaled ? v[h] * down : v[h];
+        } else {
+#pragma unroll
+          for (int h = 0; h < 16; ++h)
+            if (c + h < hn) {
+              const float w = load_weight(a.p.weights, a.p.dtype_w, (int64_t)row * g + h0 + half * 32 + c + h);
+              dq[(c + h) * 128] = from_f32<T>((kScaled ? v[h] * down : v[h]) * w);
+            }
+        }
       }
       ++n_item;
     }
@@ -824,7 +832,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     uint32_t n_tile = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t n = sli_grad_item(a, item).n, ntiles = tiles_of(n);
+      const int32_t n = sli_grad_item<kCut>(a, item).n, ntiles = tiles_of(n);
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
         const int buf = n_tile & 1;
         const int4* rows4 = reinterpret_cast<const int4*>(rows_s + (n_tile & 3) * kSlKeys + k0);
@@ -884,9 +892,9 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     int stage = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const SliGradItem it = sli_grad_item(a, item);
+      const SliGradItem it = sli_grad_item<kCut>(a, item);
       const int32_t ntiles = tiles_of(it.n);
-      const int32_t* idx_row = a.p.sparse_indices ? a.p.sparse_indices + (int64_t)it.row * a.p.topk : nullptr;
+      const int32_t* idx_row = a.p.sparse_indices ? a.p.sparse_indices + (int64_t)it.row * a.p.topk + it.off : nullptr;
       int32_t rn[4];
       auto load = [&](int32_t t) {
 #pragma unroll
@@ -919,7 +927,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     int st_s = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const SliGradItem it = sli_grad_item(a, item);
+      const SliGradItem it = sli_grad_item<kCut>(a, item);
       const int32_t ntiles = tiles_of(it.n);
       if (ntiles == 0) continue;
       const int steps = (min(64, g - it.h0) + 15) / 16;
@@ -975,7 +983,7 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     int stage = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const int32_t ntiles = tiles_of(sli_grad_item(a, item).n);
+      const int32_t ntiles = tiles_of(sli_grad_item<kCut>(a, item).n);
       if (ntiles == 0) continue;
       ok = wait(dq_empty, (n_item & 1) ^ 1);
       for (int32_t t = 0; t < ntiles && ok; ++t, ++n_tile) {
@@ -1008,9 +1016,9 @@ sli_grad_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     uint32_t n_item = 0;
     bool ok = true;
     for (int32_t item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
-      const SliGradItem it = sli_grad_item(a, item);
+      const SliGradItem it = sli_grad_item<kCut>(a, item);
       const int32_t row = it.row, h0 = it.h0;
-      if (it.n == 0) continue;
+      if (it.n <= 0) continue;
       const int32_t hn = min(64, g - h0);
       if (warp == kSgStager0) {
         ok = wait(q_empty, (n_item & 1) ^ 1);
@@ -1173,16 +1181,19 @@ inline int sli_sm100_prepare(int* sms_out) {
         cudaFuncSetAttribute(sli_score_sm100_kernel<true, false>, attr, (int)kSlSmemMax) != cudaSuccess ||
         cudaFuncSetAttribute(sli_score_sm100_kernel<true, true>, attr, (int)kSlSmemMax) != cudaSuccess ||
         cudaFuncSetAttribute(sli_score_sm100_kernel<false, false>, attr, (int)kSlSmemMax) != cudaSuccess ||
-        cudaFuncSetAttribute(sli_mha_sm100_kernel, attr, (int)kMhSmemBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(sli_grad_sm100_kernel<__nv_bfloat16>, attr, (int)kSgSmemBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(sli_grad_sm100_kernel<__half>, attr, (int)kSgSmemBytes) != cudaSuccess)
+        cudaFuncSetAttribute(sli_mha_sm100_kernel, attr, (int)kMhSmemBytes) != cudaSuccess)
       return DSA_ERR_CUDA;
-    // (a build with another register count must not run: setmaxnreg.inc could block for good)
-    cudaFuncAttributes fa0, fa1;
-    if (cudaFuncGetAttributes(&fa0, sli_grad_sm100_kernel<__nv_bfloat16>) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa1, sli_grad_sm100_kernel<__half>) != cudaSuccess || fa0.numRegs != kSgLaunchRegs ||
-        fa1.numRegs != kSgLaunchRegs)
-      return DSA_ERR_CUDA;
+    const void* grads[] = {(const void*)sli_grad_sm100_kernel<__nv_bfloat16, false>,
+                           (const void*)sli_grad_sm100_kernel<__nv_bfloat16, true>,
+                           (const void*)sli_grad_sm100_kernel<__half, false>,
+                           (const void*)sli_grad_sm100_kernel<__half, true>};
+    for (const void* f : grads) {
+      // (a build with another register count must not run: setmaxnreg.inc could block for good)
+      cudaFuncAttributes fa;
+      if (cudaFuncSetAttribute(f, attr, (int)kSgSmemBytes) != cudaSuccess || cudaFuncGetAttributes(&fa, f) != cudaSuccess ||
+          fa.numRegs != kSgLaunchRegs)
+        return DSA_ERR_CUDA;
+    }
     sm_count[dev].store(sms, std::memory_order_release);
   }
   *sms_out = sms;
@@ -1298,7 +1309,9 @@ inline int sli_grad_sm100_launch(const DsaSliGradParams* p, const SliGradDev& d,
   if (!make_tmap_gather4_16bit(&tk, p->key_index, (uint64_t)a.key_rows, 128, 256, 64, bf16) ||
       !make_tmap_3d_16bit(&tq, p->query_index, (uint64_t)rows, (uint64_t)p->g, 128, 256, (uint64_t)p->g * 256, 64, 64, bf16))
     return DSA_ERR_CUDA;
-  sli_grad_sm100_kernel<T><<<std::min(a.items, sms), kSgThreads, kSgSmemBytes, st>>>(tk, tq, a);
+  const int grid = std::min(a.items, sms);
+  if (sp.parts > 1) sli_grad_sm100_kernel<T, true><<<grid, kSgThreads, kSgSmemBytes, st>>>(tk, tq, a);
+  else sli_grad_sm100_kernel<T, false><<<grid, kSgThreads, kSgSmemBytes, st>>>(tk, tq, a);
   if (cudaGetLastError() != cudaSuccess) return DSA_ERR_CUDA;
   count_launch();
   if (sp.parts > 1) *parts = SliGradParts{part, sp.full, sp.parts, (sp.items - sp.full) / sp.parts, a.hchunks};
