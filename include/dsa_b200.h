@@ -194,7 +194,7 @@ int dsa_sfa_grad_uses_tensor_path(const DsaSfaGradParams* p);
  * made for the largest call is enough for the others.  dsa_sfa_grad() with less than that runs on the mma.sync kernel:
  * the same results, 3.7 times the time at 512 rows x 64 heads.  The size named by dsa_sfa_grad_workspace_bytes() may
  * hold up to 148 fp32 blocks of 64 x (d + d_rope) more (21.8 MB): with all of them, rows of a last round that would
- * leave most SMs idle are cut into parts (1135 us against 1222 at 512 rows x 64 heads), whose d_query sums are
+ * leave most SMs idle are cut into parts (1066 us against 1206 at 512 rows x 64 heads), whose d_query sums are
  * added up.  That can change the last place of d_query and d_query_rope, by the number of rows and heads of the call;
  * with less, a row's d_query does not depend on the other rows. */
 int dsa_sfa_grad_workspace_bytes(const DsaSfaGradParams* p, size_t* out_bytes);
@@ -254,7 +254,7 @@ typedef struct DsaSliGradParams {
  * probabilities, each [rows, slots]; three terms per row; the d_key_index accumulator [batch * s2, d_idx]); it grows
  * with every size of the call.  The size named by dsa_sli_grad_workspace_bytes() may hold up to 148 fp32 blocks of 64 x
  * 129 more (4.9 MB): with all of them, rows of a last round that would leave most SMs idle are cut into parts
- * (dense, 512 rows x 4096 keys: 495 us against 508), whose d_query_index and d_weights sums are added up.  That can
+ * (dense, 512 rows x 4096 keys: 402 us against 427), whose d_query_index and d_weights sums are added up.  That can
  * change their last place, by the number of rows and heads of the call; with less, a row's d_query_index and
  * d_weights do not depend on the other rows. */
 int dsa_sli_grad_workspace_bytes(const DsaSliGradParams* p, size_t* out_bytes);
