@@ -91,14 +91,15 @@ struct SfaBwdArgs {
   float* dq_part;            // [items - full][64 heads][576]
   int32_t key_rows;
 };
-// Parts that a row with `tiles` tiles is cut into, at most `parts`, all of them with keys: of 3 tiles or more when rows
-// are cut in two, of 2 in three, of 1 in four.  A part loads Q and dO again (136 KB), which costs less the fewer blocks
-// do it.  Whole calls of 64 heads, rows whole / cut, us: 20 rows (four parts) of 100 keys 43 / 39, of 300 69 / 42; 222
-// rows (74 of them in two) of 300 keys (4 and 3 tiles) 126 / 115.  Cut by slots alone, as if every row had 2048 keys: 222
-// rows of 100 keys 83 for 73, of 40 keys 64 for 50 (with a kernel of its own for the sums).
+// Parts that a row with `tiles` tiles is cut into, at most `parts`, all of them with keys: of 2 tiles or more when rows
+// are cut in two, of a tile in three or four.  A part loads Q and dO again (136 KB), which costs less the fewer blocks do
+// it.  Whole calls, rows whole / parts of a tile / of two (a kernel of its own for the sums would add 3 to 7), us:
+//    45 rows, in three  16 heads: 90 keys 38 / 39 / 38,    140 43 / 38 / 45, 240 53 / 41 / 45;  64 heads: 140 45 / 39 / 47
+//   222, 74 of them in two  16 heads: 90 keys 58 / 55 / 58, 190 83 / 73 / 73; 64 heads: 90 62 / 64 / 64, 190 89 / 84 / 84
+//   500, 56 of them in two  64 heads: 90 keys 115 / 119 / 116, 190 168 / 165 / 164; with parts of three tiles 169
 __device__ __forceinline__ int32_t bwd_row_parts(int32_t tiles, int32_t parts) {
   if (parts == 1) return 1;
-  const int32_t n = max(1, min(parts, tiles / (5 - parts))), per = max(1, (tiles + n - 1) / n);
+  const int32_t n = max(1, min(parts, tiles / (parts == 2 ? 2 : 1))), per = max(1, (tiles + n - 1) / n);
   return max(1, (tiles + per - 1) / per);
 }
 struct BwdItem { int32_t base, row, h0, slot; int2 nv; };
